@@ -227,10 +227,14 @@ int tiles_dirty(silt_sheet* s) {
 }
 
 // Materialise the lazy dry cut before anything reads or writes the planes.
-int flush_cut(silt_sheet* s) {
+// `read_only`: the caller only reads them, so the tile flags still hold and
+// the next step keeps to its active tiles (a quiet tile has no depth, so after
+// the cut no velocity either); otherwise that step takes every tile.
+int flush_cut(silt_sheet* s, bool read_only = false) {
     if (!s->cut_pending) return SILT_OK;
     for (int l = 0; l < 2; ++l) CK(silt::launch_apply_cut(s->H(l), s->U(l), s->V(l), s->n, 1.0e-6f, s->st));
     s->cut_pending = false;
+    if (!read_only) s->tiles_all = true;
     return SILT_OK;
 }
 
@@ -432,7 +436,7 @@ void coarse_substep(silt_sheet* s, const CoarsePlan& cp, float dt, int k, silt::
     F.nxt = nxt;
     T.tf = s->tf;
     T.nxt = nxt;
-    all = (s->tiles_all || !(k > 0 || s->cut_pending)) ? 1 : 0;
+    all = s->tiles_all ? 1 : 0;
 }
 
 // After substep k: the other buffers are current and wait for the dry cut.
@@ -1636,7 +1640,7 @@ int silt_sample(silt_sheet* s, float x, float z, silt_ground_sample* out) {
     };
     const long i = axis(s->origin[0], x), j = axis(s->origin[1], z);
     if (i < 0 || j < 0) return SILT_OK_NOOP;  // outside the window: nothing parked per cell here
-    int rc = flush_cut(s);
+    int rc = flush_cut(s, true);
     if (rc) return rc;
     const size_t c = (size_t)j * s->res + (size_t)i;
     float vals[6];
@@ -1756,7 +1760,7 @@ int silt_get_ledger(silt_sheet* s, silt_ledger* out) {
 int silt_get_coarse_cell(silt_sheet* s, int32_t i, int32_t j, silt_coarse_cell* out) {
     if (!s || !out) return fail_arg("coarse_cell");
     if (i < 0 || j < 0 || i >= s->res || j >= s->res) return SILT_OK_NOOP;
-    int rc = flush_cut(s);
+    int rc = flush_cut(s, true);
     if (rc) return rc;
     size_t idx = (size_t)j * s->res + i;
     float vals[10];
@@ -1794,7 +1798,7 @@ int silt_export_maps(silt_sheet* s, float* height, float* vel_u, float* vel_v, f
     if (!s) return fail_arg("handle");
     int rc = silt::fine::restrict_all(s->fine, s);
     if (rc) return rc;
-    if ((rc = flush_cut(s))) return rc;
+    if ((rc = flush_cut(s, true))) return rc;
     // Four planes through the two staging buffers, two at a time.
     float* outs[4] = {height, vel_u, vel_v, moisture};
     for (int pass = 0; pass < 2; ++pass) {
@@ -1815,10 +1819,10 @@ int silt_export_maps(silt_sheet* s, float* height, float* vel_u, float* vel_v, f
 
 int silt_publish_film_flow_device(silt_sheet* s, float* d_film, float* d_flow) {
     if (!s || !d_film || !d_flow) return fail_arg("publish");
-    int rc = flush_cut(s);
-    if (rc) return rc;
+    // A pending dry cut is applied by the publish itself, which reads those planes anyway.
     CK(silt::op_publish(s->H(0), s->H(1), s->U(0), s->V(0), s->U(1), s->V(1), s->tr.susp[0], s->tr.turbid[0], d_film,
-                        d_flow, s->n, s->st));
+                        d_flow, s->n, s->cut_pending ? 1.0e-6f : 0.0f, s->st));
+    s->cut_pending = false;
     return SILT_OK;
 }
 
@@ -1887,7 +1891,7 @@ int silt_read_plane(silt_sheet* s, int32_t which, float* host) {
     if (!s || !host) return fail_arg("read_plane");
     float* p = plane_of(s, which);
     if (!p) return fail_arg("plane index");
-    int rc = flush_cut(s);
+    int rc = flush_cut(s, true);
     if (rc) return rc;
     CK(cudaMemcpyAsync(host, p, s->n * 4, cudaMemcpyDeviceToHost, s->st));
     CK(cudaStreamSynchronize(s->st));
@@ -1926,7 +1930,7 @@ int silt_plane_device(silt_sheet* s, int32_t which, void** out) {
 int silt_sheet_copy_state(silt_sheet* dst, silt_sheet* src) {
     if (!dst || !src || dst == src) return fail_arg("copy_state");
     if (dst->res != src->res || dst->cfg.device != src->cfg.device) return fail_arg("copy_state: different windows");
-    int rc = flush_cut(src);
+    int rc = flush_cut(src, true);
     if (rc) return rc;
     CK(cudaStreamSynchronize(src->st));
     rc = flush_cut(dst);

@@ -120,3 +120,36 @@ def test_fluid_sheet_publishes_film_and_flow():
     x0, z0, extent = dev.window_bounds()
     ox, oz = G.window_origin((0.0, 0.0))
     assert abs(x0 - ox) < 1e-4 and abs(z0 - oz) < 1e-4 and abs(extent - 40.0) < 1e-4
+
+
+@pytest.mark.parametrize("res", [96, 131, 640])
+def test_publish_between_steps_changes_no_bit(res):
+    """A grid sheet that publishes after every step (the publish applies the
+    pending dry cut itself and the next step keeps to its active tiles)
+    against one whose planes are handed out instead (the cut in passes of its
+    own, every tile stepped next): the same planes and maps bit for bit, with
+    fewer tiles stepped."""
+    import silt_scenes as S
+
+    scene = S.grid(res=res, puddles=2)
+    a, b = (G.Sheet(res=res, engine=G.ENGINE_GRID, fine_res=64, layout=G.FINE_PER_TIRE) for _ in range(2))
+    for sh in (a, b):
+        S.seed_core(sh, scene)
+        sh.set_inflow(2, -2.0, 2.0, 0.5)
+    p0 = a.step_parts(), b.step_parts()
+    for k in range(12):
+        for sh in (a, b):
+            for t in S.tires_at(k / 120.0, z0=-0.2 * res * 0.2):
+                sh.push_tire(**t)
+            sh.step(1.0 / 120.0, want_spray=False)
+        fa = a.publish()
+        b.plane_device("water")
+        fb = b.publish()
+        assert np.array_equal(fa[0].view(np.uint32), fb[0].view(np.uint32))
+        assert np.array_equal(fa[1].view(np.uint32), fb[1].view(np.uint32))
+    for name in ("water", "slurry", "uw", "vw", "us", "vs"):
+        assert np.array_equal(a.get(name).view(np.uint32), b.get(name).view(np.uint32)), name
+    cells = [sh.step_parts()["force_cells"] - p["force_cells"] for sh, p in zip((a, b), p0)]
+    assert cells[0] <= cells[1]
+    if res == 640:
+        assert cells[0] < cells[1]
