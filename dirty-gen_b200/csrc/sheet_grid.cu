@@ -24,6 +24,7 @@
 // depths and velocities on every cell that holds fluid.
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -36,10 +37,60 @@
 namespace silt {
 
 constexpr int FT = 32;       // force tile edge
-constexpr int FH = 9;        // force halo: p (2) + gravity (1) + vorticity (2) + projection (4)
-constexpr int FW = FT + 2 * FH;
-constexpr int FPLANE = FW * FW;
+// Shared-memory layout of a force tile: the halo its widest stage reads and
+// the eight planes' width and size.
+template <int HALO>
+struct TileGeom {
+    static constexpr int H = HALO;
+    static constexpr int W = FT + 2 * H;
+    static constexpr int PLANE = W * W;
+    static constexpr size_t BYTES = sizeof(float) * 8 * PLANE;
+};
 constexpr int FORCE_THREADS = 512;
+// The snapshot form carries every stage of a cell through one tile:
+// p (2) + gravity (1) + vorticity (2) + projection (4).
+using Snap = TileGeom<9>;
+// The sweep form's stages meet in global memory, so no stage reaches further
+// than the projection's 4 cells: 51 KB a tile instead of 80.
+using Sweep = TileGeom<4>;
+constexpr size_t SWEEP_SMEM = 2 * Sweep::BYTES;  // a CTA's two teams
+static_assert(2 * (SWEEP_SMEM + 2048) <= 228 * 1024, "two sweep CTAs share an SM");
+
+// The threads that step one tile: a whole CTA, or one half of it (a barrier
+// of its own). The sweep's time is block barriers between short stages (14.4
+// barrier stalls per issue with two 512-thread tiles on an SM), which more
+// and smaller teams fill for one another; with few tiles the latency of one
+// tile counts, and a whole CTA takes it. A 1501^2 flood (2300 tile-layers):
+// 376 us per launch by whole CTAs with a 9-cell halo, 348 by halves; 2048^2
+// with a vehicle (360): 94 by whole CTAs, 129 by halves.
+template <int N>
+struct Team {
+    static constexpr int NT = N;
+    int tid, bar;
+    __device__ Team() : tid((int)threadIdx.x % N), bar(N == FORCE_THREADS ? 0 : 1 + (int)threadIdx.x / N) {}
+    __device__ __forceinline__ void sync() const {
+        if constexpr (N == FORCE_THREADS)
+            __syncthreads();
+        else
+            asm volatile("barrier.cta.sync %0, %1;" ::"r"(bar), "n"(N) : "memory");
+    }
+    __device__ __forceinline__ bool any(bool x) const {
+        if constexpr (N == FORCE_THREADS) {
+            return __syncthreads_or(x) != 0;
+        } else {
+            int r;
+            asm volatile(
+                "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, %2, %3, q;\n\t"
+                "selp.s32 %0, 1, 0, p;\n\t}\n"
+                : "=r"(r)
+                : "r"((int)x), "r"(bar), "n"(N)
+                : "memory");
+            return r != 0;
+        }
+    }
+};
+using WholeCta = Team<FORCE_THREADS>;
+using HalfCta = Team<FORCE_THREADS / 2>;
 
 constexpr int TT = 32;       // transport tile edge
 constexpr int TW = TT + 3;   // rows [t0-2, t1+1)
@@ -53,7 +104,6 @@ static_assert((TPL * sizeof(float)) % 128 == 0, "each transport plane starts 128
 static_assert(TS * TW * sizeof(float) <= TPL * sizeof(float), "a TMA box fits its plane");
 constexpr int TRANSPORT_THREADS = 256;
 
-size_t force_smem_bytes() { return sizeof(float) * FPLANE * 8; }
 size_t transport_smem_bytes() { return sizeof(float) * TPL * 8; }
 
 // Five taps left to right. Away from the edge the reference starts from the
@@ -125,23 +175,22 @@ __device__ __forceinline__ float cell_decay(const LayerParams& P, size_t g, floa
 // the shared-memory index and g the global one. Edge tiles clip the region to
 // the grid and walk it one warp per row; interior tiles walk the rectangle as
 // one flat range (a compile-time width), which keeps every lane busy.
-template <bool EDGE, int RX, int RY, class F>
-__device__ __forceinline__ void region(int tx0, int ty0, int res, F f) {
-    const int ox = tx0 - FH, oy = ty0 - FH;
+template <class TM, class G, bool EDGE, int RX, int RY, class F>
+__device__ __forceinline__ void region(const TM& T, int tx0, int ty0, int res, F f) {
+    const int ox = tx0 - G::H, oy = ty0 - G::H;
     if (EDGE) {
-        const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-        constexpr int NW = FORCE_THREADS / 32;
+        const int lane = T.tid & 31, wy = T.tid >> 5, NW = TM::NT / 32;
         const int x0 = max(0, tx0 - RX), x1 = min(res, tx0 + FT + RX);
         const int y0 = max(0, ty0 - RY), y1 = min(res, ty0 + FT + RY);
         for (int gy = y0 + wy; gy < y1; gy += NW)
             for (int gx = x0 + lane; gx < x1; gx += 32)
-                f(gx, gy, (gy - oy) * FW + (gx - ox), (size_t)gy * res + gx);
+                f(gx, gy, (gy - oy) * G::W + (gx - ox), (size_t)gy * res + gx);
     } else {
-        constexpr int W = FT + 2 * RX, H = FT + 2 * RY;
-        for (int k = threadIdx.x; k < W * H; k += FORCE_THREADS) {
-            const int r = k / W;
-            const int gy = ty0 - RY + r, gx = tx0 - RX + (k - r * W);
-            f(gx, gy, (gy - oy) * FW + (gx - ox), (size_t)gy * res + gx);
+        constexpr int RW = FT + 2 * RX, RH = FT + 2 * RY;
+        for (int k = T.tid; k < RW * RH; k += TM::NT) {
+            const int r = k / RW;
+            const int gy = ty0 - RY + r, gx = tx0 - RX + (k - r * RW);
+            f(gx, gy, (gy - oy) * G::W + (gx - ox), (size_t)gy * res + gx);
         }
     }
 }
@@ -172,8 +221,9 @@ __device__ __forceinline__ void start_velocity(const LayerParams& P, int gx, int
     }
 }
 
-// Shared-memory planes of a force tile (FW x FW floats each, origin at the
-// tile corner minus FH).
+// Shared-memory planes of a force tile (G::W x G::W floats each, origin at the
+// tile corner minus G::H).
+template <class G>
 struct ForcePlanes {
     float* E;   // eta
     float* TG;  // x-pass scratch
@@ -184,34 +234,35 @@ struct ForcePlanes {
     float* HS;  // depth
     float* WQ;  // vorticity, then q
     __device__ explicit ForcePlanes(float* sm)
-        : E(sm), TG(sm + FPLANE), TS(sm + 2 * FPLANE), PB(sm + 3 * FPLANE), U(sm + 4 * FPLANE), V(sm + 5 * FPLANE),
-          HS(sm + 6 * FPLANE), WQ(sm + 7 * FPLANE) {}
+        : E(sm), TG(sm + G::PLANE), TS(sm + 2 * G::PLANE), PB(sm + 3 * G::PLANE), U(sm + 4 * G::PLANE), V(sm + 5 * G::PLANE),
+          HS(sm + 6 * G::PLANE), WQ(sm + 7 * G::PLANE) {}
 };
 
-#define NX(d) (EDGE ? (gy - oy) * FW + (clampi(gx + (d), 0, res - 1) - ox) : s + (d))
-#define NZ(d) (EDGE ? (clampi(gy + (d), 0, res - 1) - oy) * FW + (gx - ox) : s + (d) * FW)
+#define NX(d) (EDGE ? (gy - oy) * G::W + (clampi(gx + (d), 0, res - 1) - ox) : s + (d))
+#define NZ(d) (EDGE ? (clampi(gy + (d), 0, res - 1) - oy) * G::W + (gx - ox) : s + (d) * G::W)
 
 // Depth and eta on radius R + 2, then the pressure p = 0.45 (0.62 G + 0.38 S)
 // + 0.55 eta on radius R (src/fluid_core.rs:1950-1985): the two 5-tap blurs,
 // x pass then z pass. Ends with a barrier.
-template <bool EDGE, int R>
-__device__ __forceinline__ void pressure_field(const LayerParams& P, const ForcePlanes& F, int tx0, int ty0) {
+template <class TM, class G, bool EDGE, int R>
+__device__ __forceinline__ void pressure_field(const TM& T, const LayerParams& P, const ForcePlanes<G>& F, int tx0, int ty0) {
     const int res = P.res;
-    const int ox = tx0 - FH, oy = ty0 - FH;
-    region<EDGE, R + 2, R + 2>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-        float hv = P.h[g];
+    const int ox = tx0 - G::H, oy = ty0 - G::H;
+    const float *__restrict__ depth = P.h, *__restrict__ bed = P.bed;
+    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        float hv = depth[g];
         F.HS[s] = hv;
-        F.E[s] = P.bed[g] + hv;
+        F.E[s] = bed[g] + hv;
     });
-    __syncthreads();
-    region<EDGE, R, R + 2>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    T.sync();
+    region<TM, G, EDGE, R, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
         float e0 = F.E[NX(-2)], e1 = F.E[NX(-1)], e2 = F.E[s], e3 = F.E[NX(1)], e4 = F.E[NX(2)];
         F.TG[s] = tap5(e0, e1, e2, e3, e4, kG0, kG1, kG2, in);
         F.TS[s] = tap5(e0, e1, e2, e3, e4, kS0, kS1, kS2, in);
     });
-    __syncthreads();
-    region<EDGE, R, R>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    T.sync();
+    region<TM, G, EDGE, R, R>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         const bool in = EDGE ? (gy >= 2 && gy <= res - 3) : true;
         const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
         float gb = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
@@ -219,20 +270,20 @@ __device__ __forceinline__ void pressure_field(const LayerParams& P, const Force
         float filtered = 0.62f * gb + 0.38f * sc;
         F.PB[s] = 0.45f * filtered + 0.55f * F.E[s];
     });
-    __syncthreads();
+    T.sync();
 }
 
 // Projection, damping and the speed clamp from the confined velocity in U, V
 // (radius 4), depth and eta (radius 4) (src/fluid_core.rs:1992-2037). Writes
 // every cell of the tile to u_out, v_out.
-template <bool EDGE>
-__device__ __forceinline__ void finish_tile(const LayerParams& P, const ForcePlanes& F, int tx0, int ty0) {
+template <class TM, class G, bool EDGE>
+__device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, const ForcePlanes<G>& F, int tx0, int ty0) {
     const int res = P.res;
-    const int ox = tx0 - FH, oy = ty0 - FH;
+    const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float dt = P.dt, eps = P.eps;
     if (P.project) {
         // b = div * overload - 0.015 * overload * lap(eta), radius 3 (:1992-2003).
-        region<EDGE, 3, 3>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 3, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             const int sxp = NX(1), sxm = NX(-1), szp = NZ(1), szm = NZ(-1);
             float ux = fdiv(F.U[sxp] - F.U[sxm], P.div_two);
             float vz = fdiv(F.V[szp] - F.V[szm], P.div_two);
@@ -242,27 +293,27 @@ __device__ __forceinline__ void finish_tile(const LayerParams& P, const ForcePla
             float overload = 1.0f + rclamp(fdiv(cell_nu(P, g), P.div_231), 0.0f, 6.0f);
             F.PB[s] = div * overload - 0.015f * overload * lap_h;
         });
-        __syncthreads();
+        T.sync();
         // x pass of both blurs of b: rows radius 3, columns radius 1.
-        region<EDGE, 1, 3>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 1, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
             float b0 = F.PB[NX(-2)], b1 = F.PB[NX(-1)], b2 = F.PB[s], b3 = F.PB[NX(1)], b4 = F.PB[NX(2)];
             F.TG[s] = tap5(b0, b1, b2, b3, b4, kG0, kG1, kG2, in);
             F.TS[s] = tap5(b0, b1, b2, b3, b4, kS0, kS1, kS2, in);
         });
-        __syncthreads();
+        T.sync();
         // q = 0.62 G(b) + 0.38 S(b), radius 1 (:2004-2011).
-        region<EDGE, 1, 1>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 1, 1>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             const bool in = EDGE ? (gy >= 2 && gy <= res - 3) : true;
             const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
             float gq = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
             float sq = tap5(F.TS[s0], F.TS[s1], F.TS[s], F.TS[s3], F.TS[s4], kS0, kS1, kS2, in);
             F.WQ[s] = 0.62f * gq + 0.38f * sq;
         });
-        __syncthreads();
+        T.sync();
     }
     // Projection kick, damping and the speed clamp on wet cells (:2015-2037).
-    region<EDGE, 0, 0>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         float uu = F.U[s], vv = F.V[s];
         if (F.HS[s] > eps) {
             if (P.project) {
@@ -285,17 +336,17 @@ __device__ __forceinline__ void finish_tile(const LayerParams& P, const ForcePla
 // ever clamped there and every blur uses the interior form, so the stencils
 // are plain offsets. Threads walk the regions as rows (one warp per row,
 // lanes along x).
-template <bool EDGE>
-__device__ __forceinline__ void force_tile(const LayerParams& P, float* sm, int tx0, int ty0) {
+template <class TM, class G, bool EDGE>
+__device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0) {
     const int res = P.res;
-    const ForcePlanes F(sm);
-    const int ox = tx0 - FH, oy = ty0 - FH;
+    const ForcePlanes<G> F(sm);
+    const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float dt = P.dt, eps = P.eps;
     // 1-3. Depth, eta (radius 9) and the pressure (radius 7).
-    pressure_field<EDGE, 7>(P, F, tx0, ty0);
+    pressure_field<TM, G, EDGE, 7>(T, P, F, tx0, ty0);
     // Velocity on radius 6 and gravity down the pressure gradient on wet
     // cells (src/fluid_core.rs:2234-2253).
-    region<EDGE, 6, 6>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, 6, 6>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         float uu, vv;
         start_velocity(P, gx, gy, g, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
@@ -308,18 +359,18 @@ __device__ __forceinline__ void force_tile(const LayerParams& P, float* sm, int 
         F.U[s] = uu;
         F.V[s] = vv;
     });
-    __syncthreads();
+    T.sync();
     // Vorticity of the post-gravity snapshot, radius 5 (src/fluid_core.rs:3498-3506).
     if (P.vort > 0.0f) {
-        region<EDGE, 5, 5>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 5, 5>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             float dvdx = fdiv(F.V[NX(1)] - F.V[NX(-1)], P.div_two);
             float dudz = fdiv(F.U[NZ(1)] - F.U[NZ(-1)], P.div_two);
             F.WQ[s] = dvdx - dudz;
         });
-        __syncthreads();
+        T.sync();
         // Confinement kick from that snapshot, in place, radius 4
         // (src/fluid_core.rs:2348-2375, :2441-2470).
-        region<EDGE, 4, 4>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             if (F.HS[s] > eps) {
                 float w = F.WQ[s];
                 if (finite_f(w) && !(fabsf(w) < 1.0e-4f)) {
@@ -336,22 +387,22 @@ __device__ __forceinline__ void force_tile(const LayerParams& P, float* sm, int 
                 }
             }
         });
-        __syncthreads();
+        T.sync();
     }
-    finish_tile<EDGE>(P, F, tx0, ty0);
+    finish_tile<TM, G, EDGE>(T, P, F, tx0, ty0);
 }
 
 // Sweep form, part 1: the post-gravity velocity G of every cell of the tile
 // (gravity on wet cells only; a dry cell keeps its starting velocity), written
 // to u_out, v_out, and the sweep's first iterate F = G to fu, fv.
-template <bool EDGE>
-__device__ __forceinline__ void pre_tile(const LayerParams& P, float* sm, int tx0, int ty0) {
+template <class TM, class G, bool EDGE>
+__device__ __forceinline__ void pre_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0) {
     const int res = P.res;
-    const ForcePlanes F(sm);
-    const int ox = tx0 - FH, oy = ty0 - FH;
+    const ForcePlanes<G> F(sm);
+    const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float dt = P.dt, eps = P.eps;
-    pressure_field<EDGE, 1>(P, F, tx0, ty0);
-    region<EDGE, 0, 0>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    pressure_field<TM, G, EDGE, 1>(T, P, F, tx0, ty0);
+    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         float uu, vv;
         start_velocity(P, gx, gy, g, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
@@ -391,27 +442,27 @@ constexpr int SWEEP_LOCAL_PASSES = SILT_SWEEP_LOCAL_PASSES;
 // pass of the launch (the CTA solves no other tile), so only the ring of
 // other tiles' wet cells around it is read again; the starting and
 // post-gravity velocities and the tile's own iterate are current.
-template <bool EDGE>
-__device__ bool sweep_tile(const LayerParams& P, float* sm, int tx0, int ty0, bool reuse, int& passes) {
+template <class TM, class G, bool EDGE>
+__device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0, bool reuse, int& passes) {
     const int res = P.res;
     float* PU = sm;              // starting velocity (the values of cells after a cell)
-    float* PV = sm + FPLANE;
-    float* FU = sm + 2 * FPLANE;  // current iterate (the values of cells before it)
-    float* FV = sm + 3 * FPLANE;
-    float* GU = sm + 4 * FPLANE;  // post-gravity velocity of the tile's own cells
-    float* GV = sm + 5 * FPLANE;
-    float* WT = sm + 6 * FPLANE;  // 1: wet
-    const int ox = tx0 - FH, oy = ty0 - FH;
+    float* PV = sm + G::PLANE;
+    float* FU = sm + 2 * G::PLANE;  // current iterate (the values of cells before it)
+    float* FV = sm + 3 * G::PLANE;
+    float* GU = sm + 4 * G::PLANE;  // post-gravity velocity of the tile's own cells
+    float* GV = sm + 5 * G::PLANE;
+    float* WT = sm + 6 * G::PLANE;  // 1: wet
+    const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float eps = P.eps;
     if (reuse) {
-        region<EDGE, 2, 2>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             if (gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT) return;
             if (WT[s] != 0.0f) {
                 FU[s] = P.fu[g];
                 FV[s] = P.fv[g];
             }
         });
-    } else region<EDGE, 2, 2>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    } else region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         const float hv = P.h[g];
         float uu, vv;
         start_velocity(P, gx, gy, g, hv, uu, vv);
@@ -428,7 +479,7 @@ __device__ bool sweep_tile(const LayerParams& P, float* sm, int tx0, int ty0, bo
             GV[s] = P.v_out[g];
         }
     });
-    __syncthreads();
+    T.sync();
     bool tile_changed = false;
     passes = 0;
     // Interior tiles recompute, after the first local pass, only the cells
@@ -437,24 +488,24 @@ __device__ bool sweep_tile(const LayerParams& P, float* sm, int tx0, int ty0, bo
     // marks the cells that read c's iterate: c + (1,0), (2,0), (0,1),
     // (-1,1), (1,1), (0,2). Marks for pass it + 1 go to one byte plane while
     // pass it reads the other (plane 7 of the force layout, unused here).
-    uint8_t* const marks = reinterpret_cast<uint8_t*>(sm + 7 * FPLANE);
+    uint8_t* const marks = reinterpret_cast<uint8_t*>(sm + 7 * G::PLANE);
     for (int it = 0; it < SWEEP_LOCAL_PASSES; ++it) {
         ++passes;
         int changed = 0;
-        const uint8_t* dirty = marks + (it & 1) * FPLANE;
-        uint8_t* dirty_next = marks + ((it + 1) & 1) * FPLANE;
+        const uint8_t* dirty = marks + (it & 1) * G::PLANE;
+        uint8_t* dirty_next = marks + ((it + 1) & 1) * G::PLANE;
         if (!EDGE) {
-            region<false, 0, 0>(tx0, ty0, res, [&](int, int, int s, size_t) { dirty_next[s] = 0; });
-            __syncthreads();
+            region<TM, G, false, 0, 0>(T, tx0, ty0, res, [&](int, int, int s, size_t) { dirty_next[s] = 0; });
+            T.sync();
         }
-        region<EDGE, 0, 0>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             if (WT[s] == 0.0f) return;
             if (!EDGE) {
                 // Interior tile: no stencil index is clamped.
                 if (it > 0 && !dirty[s]) return;
                 float du, dv, nu_ = GU[s], nv_ = GV[s];
-                if (conf_kick_inner(P.div_two, P.dt, P.vort, SweepRead{FU, PU, GU, s, FW},
-                                    SweepRead{FV, PV, GV, s, FW}, du, dv)) {
+                if (conf_kick_inner(P.div_two, P.dt, P.vort, SweepRead{FU, PU, GU, s, G::W},
+                                    SweepRead{FV, PV, GV, s, G::W}, du, dv)) {
                     nu_ = GU[s] + du;
                     nv_ = GV[s] + dv;
                 }
@@ -464,14 +515,14 @@ __device__ bool sweep_tile(const LayerParams& P, float* sm, int tx0, int ty0, bo
                     changed = 1;
                     dirty_next[s + 1] = 1;
                     dirty_next[s + 2] = 1;
-                    dirty_next[s + FW - 1] = 1;
-                    dirty_next[s + FW] = 1;
-                    dirty_next[s + FW + 1] = 1;
-                    dirty_next[s + 2 * FW] = 1;
+                    dirty_next[s + G::W - 1] = 1;
+                    dirty_next[s + G::W] = 1;
+                    dirty_next[s + G::W + 1] = 1;
+                    dirty_next[s + 2 * G::W] = 1;
                 }
                 return;
             }
-            auto at = [&](int a, int b) { return (b - oy) * FW + (a - ox); };
+            auto at = [&](int a, int b) { return (b - oy) * G::W + (a - ox); };
             auto before = [&](int a, int b) { return b < gy || (b == gy && a < gx); };
             auto uu = [&](int a, int b) {
                 if (a == gx && b == gy) return GU[s];
@@ -492,28 +543,28 @@ __device__ bool sweep_tile(const LayerParams& P, float* sm, int tx0, int ty0, bo
                 changed = 1;
             }
         });
-        if (!__syncthreads_or(changed)) break;
+        if (!T.any(changed != 0)) break;
         tile_changed = true;
     }
     if (tile_changed) {
-        region<EDGE, 0, 0>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             if (WT[s] != 0.0f) {
                 P.fu[g] = FU[s];
                 P.fv[g] = FV[s];
             }
         });
     }
-    __syncthreads();  // shared memory is read again by the next tile or pass
+    T.sync();  // shared memory is read again by the next tile or pass
     return tile_changed;
 }
 
 // Sweep form, part 3: projection, damping and clamp from the solved sweep.
-template <bool EDGE>
-__device__ __forceinline__ void post_tile(const LayerParams& P, float* sm, int tx0, int ty0) {
+template <class TM, class G, bool EDGE>
+__device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0) {
     const int res = P.res;
-    const ForcePlanes F(sm);
+    const ForcePlanes<G> F(sm);
     const float eps = P.eps;
-    region<EDGE, 4, 4>(tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         const float hv = P.h[g];
         F.HS[s] = hv;
         F.E[s] = P.bed[g] + hv;
@@ -527,8 +578,8 @@ __device__ __forceinline__ void post_tile(const LayerParams& P, float* sm, int t
         F.U[s] = uu;
         F.V[s] = vv;
     });
-    __syncthreads();
-    finish_tile<EDGE>(P, F, tx0, ty0);
+    T.sync();
+    finish_tile<TM, G, EDGE>(T, P, F, tx0, ty0);
 }
 
 #undef NX
@@ -548,54 +599,56 @@ __device__ __forceinline__ LayerParams force_params(const LayerParams& P0, const
     return P;
 }
 
-// A tile whose whole radius-9 region lies at least 2 cells inside the grid:
-// no stencil index is clamped there and every blur uses the interior form.
+// A tile whose whole region lies at least 2 cells inside the grid: no stencil
+// index is clamped there and every blur uses the interior form.
+template <class G>
 __device__ __forceinline__ bool tile_interior(int res, int tx0, int ty0) {
-    return tx0 - FH >= 2 && ty0 - FH >= 2 && tx0 + FT + FH <= res - 2 && ty0 + FT + FH <= res - 2;
+    return tx0 - G::H >= 2 && ty0 - G::H >= 2 && tx0 + FT + G::H <= res - 2 && ty0 + FT + G::H <= res - 2;
 }
 
 // One list entry of the force pass (the sweep form's first part for a
 // sweeping layer). Returns true when it used shared memory.
-__device__ __forceinline__ bool force_entry(const LayerParams& P, const TileFlags& tf, int nxt, int e, float* sm) {
+template <class G, class TM>
+__device__ __forceinline__ bool force_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int nxt, int e, float* sm) {
     const int l = e >> 30, zero_fill = (e & ENTRY_ZERO) != 0, copy = (e & ENTRY_COPY) != 0, t = e & ENTRY_TILE;
     const int res = P.res;
     const int tx0 = (t % tf.tiles_x) * FT, ty0 = (t / tf.tiles_x) * FT;
     if (copy) {
         // Identity substep of a layer that has taken all its substeps.
         const int w = min(FT, res - tx0), h = min(FT, res - ty0);
-        for (int q = threadIdx.x; q < w * h; q += blockDim.x) {
+        for (int q = T.tid; q < w * h; q += TM::NT) {
             const size_t g = (size_t)(ty0 + q / w) * res + tx0 + q % w;
             P.u_out[g] = P.u[g];
             P.v_out[g] = P.v[g];
         }
-        if (threadIdx.x == 0) pick(tf.zero_uv, l, nxt)[t] = pick(tf.zero_uv, l, nxt ^ 1)[t];
+        if (T.tid == 0) pick(tf.zero_uv, l, nxt)[t] = pick(tf.zero_uv, l, nxt ^ 1)[t];
         return false;
     }
     if (zero_fill) {
         // A quiet tile: dry in its whole neighbourhood, so after the dry cut
         // its velocity is zero.
         const int w = min(FT, res - tx0), h = min(FT, res - ty0);
-        for (int q = threadIdx.x; q < w * h; q += blockDim.x) {
+        for (int q = T.tid; q < w * h; q += TM::NT) {
             const size_t g = (size_t)(ty0 + q / w) * res + tx0 + q % w;
             P.u_out[g] = 0.0f;
             P.v_out[g] = 0.0f;
         }
-        if (threadIdx.x == 0) pick(tf.zero_uv, l, nxt)[t] = 1;
+        if (T.tid == 0) pick(tf.zero_uv, l, nxt)[t] = 1;
         return false;
     }
-    const bool interior = tile_interior(res, tx0, ty0);
-    if (P.sweep) {
+    const bool interior = tile_interior<G>(res, tx0, ty0);
+    if constexpr (std::is_same_v<G, Sweep>) {
         // Sweep form: this launch's first part; the sweep and the projection follow.
         if (interior)
-            pre_tile<false>(P, sm, tx0, ty0);
+            pre_tile<TM, G, false>(T, P, sm, tx0, ty0);
         else
-            pre_tile<true>(P, sm, tx0, ty0);
+            pre_tile<TM, G, true>(T, P, sm, tx0, ty0);
     } else if (interior) {
-        force_tile<false>(P, sm, tx0, ty0);
+        force_tile<TM, G, false>(T, P, sm, tx0, ty0);
     } else {
-        force_tile<true>(P, sm, tx0, ty0);
+        force_tile<TM, G, true>(T, P, sm, tx0, ty0);
     }
-    if (threadIdx.x == 0) pick(tf.zero_uv, l, nxt)[t] = 0;
+    if (T.tid == 0) pick(tf.zero_uv, l, nxt)[t] = 0;
     return true;
 }
 
@@ -610,7 +663,8 @@ __device__ __forceinline__ bool entry_steps(int e) { return (e & (ENTRY_ZERO | E
 // whether the tile changed (block-uniform) and stamps it when it did.
 // `reuse`: the CTA solves only this entry in the launch, so its shared
 // memory keeps the tile between passes.
-__device__ __forceinline__ bool sweep_entry(const LayerParams& P, const TileFlags& tf, int e, float* sm, int pass,
+template <class TM>
+__device__ __forceinline__ bool sweep_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int e, float* sm, int pass,
                                             unsigned int epoch, bool reuse) {
     if (!entry_steps(e) || !P.sweep || !(P.vort > 0.0f)) return false;
     const int l = e >> 30, t = e & ENTRY_TILE;
@@ -620,20 +674,21 @@ __device__ __forceinline__ bool sweep_entry(const LayerParams& P, const TileFlag
     if (pass > 0 && stamp) {
         // Nine threads read the nine stamps at once.
         bool hit = false;
-        if (threadIdx.x < 9) {
-            const int x = ti + (int)(threadIdx.x % 3) - 1, y = tj + (int)(threadIdx.x / 3) - 1;
+        if (T.tid < 9) {
+            const int x = ti + T.tid % 3 - 1, y = tj + T.tid / 3 - 1;
             const unsigned int since = epoch * 256u + (unsigned int)pass;
             hit = x >= 0 && y >= 0 && x < tf.tiles_x && y < tf.tiles_x &&
                   *(volatile unsigned int*)&stamp[y * tf.tiles_x + x] >= since;
         }
-        if (!__syncthreads_or(hit)) return false;
+        if (!T.any(hit)) return false;
     }
     const int tx0 = ti * FT, ty0 = tj * FT;
     int passes = 0;
     const bool keep = reuse && pass > 0;
-    const bool changed = tile_interior(P.res, tx0, ty0) ? sweep_tile<false>(P, sm, tx0, ty0, keep, passes)
-                                                        : sweep_tile<true>(P, sm, tx0, ty0, keep, passes);
-    if (threadIdx.x == 0) {
+    const bool changed = tile_interior<Sweep>(P.res, tx0, ty0)
+                             ? sweep_tile<TM, Sweep, false>(T, P, sm, tx0, ty0, keep, passes)
+                             : sweep_tile<TM, Sweep, true>(T, P, sm, tx0, ty0, keep, passes);
+    if (T.tid == 0) {
         if (changed && stamp) {
             __threadfence();
             stamp[t] = epoch * 256u + (unsigned int)pass + 1u;
@@ -647,14 +702,15 @@ __device__ __forceinline__ bool sweep_entry(const LayerParams& P, const TileFlag
 }
 
 // Sweep-form projection of one list entry. Returns true when it used shared memory.
-__device__ __forceinline__ bool post_entry(const LayerParams& P, const TileFlags& tf, int e, float* sm) {
+template <class TM>
+__device__ __forceinline__ bool post_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int e, float* sm) {
     if (!entry_steps(e) || !P.sweep) return false;
     const int t = e & ENTRY_TILE;
     const int tx0 = (t % tf.tiles_x) * FT, ty0 = (t / tf.tiles_x) * FT;
-    if (tile_interior(P.res, tx0, ty0))
-        post_tile<false>(P, sm, tx0, ty0);
+    if (tile_interior<Sweep>(P.res, tx0, ty0))
+        post_tile<TM, Sweep, false>(T, P, sm, tx0, ty0);
     else
-        post_tile<true>(P, sm, tx0, ty0);
+        post_tile<TM, Sweep, true>(T, P, sm, tx0, ty0);
     return true;
 }
 
@@ -701,21 +757,35 @@ __device__ bool grid_barrier(SweepState* S, unsigned int& target) {
     return ok != 0;
 }
 
+// A team's share of a launch over its list: the first entry it takes, the
+// step to its next, its shared memory and its half of the CTA.
+template <class TM>
+struct SweepTeam {
+    TM T;
+    int half, first, stride;
+    float* sm;
+    __device__ explicit SweepTeam(float* shared) {
+        constexpr int TEAMS = FORCE_THREADS / TM::NT;
+        half = (int)threadIdx.x / TM::NT;
+        first = (int)blockIdx.x + half * (int)gridDim.x;
+        stride = TEAMS * (int)gridDim.x;
+        sm = shared + half * (Sweep::BYTES / sizeof(float));
+    }
+};
+
 // Passes of the fixed point until one changes nothing anywhere. `visit(k)`
 // runs list entry k's pass and returns whether it changed a value. Returns
 // the number of passes, 0 at the pass limit, -1 after a failed barrier.
-template <class Visit>
-__device__ int sweep_fixed_point(SweepState* S, unsigned int& target, int n, Visit visit) {
+template <class TM, class Visit>
+__device__ int sweep_fixed_point(const SweepTeam<TM>& W, SweepState* S, unsigned int& target, int n, Visit visit) {
     __shared__ unsigned int verdict;
     for (int pass = 0; pass < SWEEP_MAX_PASSES; ++pass) {
         bool changed = false;
-        for (int k = blockIdx.x; k < n; k += gridDim.x) changed |= visit(k, pass);
-        if (threadIdx.x == 0) {
-            if (changed) atomicOr(&S->flag[pass % 3], 1u);
-            // The next pass's verdict starts clear; the one cleared here was
-            // last read before the previous barrier.
-            if (blockIdx.x == 0) S->flag[(pass + 1) % 3] = 0u;
-        }
+        for (int k = W.first; k < n; k += W.stride) changed |= visit(k, pass);
+        if (W.T.tid == 0 && changed) atomicOr(&S->flag[pass % 3], 1u);
+        // The next pass's verdict starts clear; the one cleared here was
+        // last read before the previous barrier.
+        if (threadIdx.x == 0 && blockIdx.x == 0) S->flag[(pass + 1) % 3] = 0u;
         if (!grid_barrier(S, target)) return -1;
         if (threadIdx.x == 0) verdict = ld_acquire_u32(&S->flag[pass % 3]);
         __syncthreads();
@@ -768,27 +838,23 @@ __device__ __forceinline__ void sweep_stats(SweepState* S, int passes) {
     }
 }
 
-// One sheet's force pass in the sweep form (cooperative launch): pre-sweep
-// tiles (and the list's zero and copy entries), the fixed point, projection.
-__global__ void __launch_bounds__(FORCE_THREADS) k_force_sweep(ForceLaunch L) {
-    ::silt::dep_wait();
-    extern __shared__ float sm[];
-    __shared__ LayerParams Ps[2];
-    if (threadIdx.x < 2) Ps[threadIdx.x] = force_params(L.lay[threadIdx.x], L.sc, threadIdx.x, blockIdx.x == 0);
-    __syncthreads();
+// One sheet's force pass in the sweep form: pre-sweep tiles (and the list's
+// zero and copy entries), the fixed point, projection.
+template <class TM>
+__device__ __forceinline__ void force_sweep(const ForceLaunch& L, const LayerParams* Ps, int n, float* sm) {
     SweepState* S = L.tf.sweep;
     const unsigned int epoch = ld_acquire_u32(&S->epoch);
-    const int n = *L.tf.count;
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+    const SweepTeam<TM> W(sm);
+    for (int k = W.first; k < n; k += W.stride) {
         const int e = L.tf.list[k];
-        if (force_entry(Ps[e >> 30], L.tf, L.nxt, e, sm)) __syncthreads();
+        if (force_entry<Sweep>(W.T, Ps[e >> 30], L.tf, L.nxt, e, W.sm)) W.T.sync();
     }
     unsigned int target = 0;
     if (!grid_barrier(S, target)) return;
-    const bool reuse = n <= (int)gridDim.x;  // one entry per CTA: its tile stays in shared memory
-    const int passes = sweep_fixed_point(S, target, n, [&](int k, int pass) {
+    const bool reuse = n <= W.stride;  // one entry per team: its tile stays in shared memory
+    const int passes = sweep_fixed_point(W, S, target, n, [&](int k, int pass) {
         const int e = L.tf.list[k];
-        return sweep_entry(Ps[e >> 30], L.tf, e, sm, pass, epoch, reuse);
+        return sweep_entry(W.T, Ps[e >> 30], L.tf, e, W.sm, pass, epoch, reuse);
     });
     if (passes < 0) return;
     if (passes == 0) {
@@ -799,10 +865,25 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force_sweep(ForceLaunch L) {
         if (!grid_barrier(S, target)) return;
     }
     sweep_stats(S, passes);
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+    for (int k = W.first; k < n; k += W.stride) {
         const int e = L.tf.list[k];
-        if (post_entry(Ps[e >> 30], L.tf, e, sm)) __syncthreads();
+        if (post_entry(W.T, Ps[e >> 30], L.tf, e, W.sm)) W.T.sync();
     }
+}
+
+// force_sweep as a cooperative launch; its teams are whole CTAs while every
+// entry of the list has one.
+__global__ void __launch_bounds__(FORCE_THREADS, 2) k_force_sweep(ForceLaunch L) {
+    ::silt::dep_wait();
+    extern __shared__ float sm[];
+    __shared__ LayerParams Ps[2];
+    if (threadIdx.x < 2) Ps[threadIdx.x] = force_params(L.lay[threadIdx.x], L.sc, threadIdx.x, blockIdx.x == 0);
+    __syncthreads();
+    const int n = *L.tf.count;
+    if (n <= (int)gridDim.x)
+        force_sweep<WholeCta>(L, Ps, n, sm);
+    else
+        force_sweep<HalfCta>(L, Ps, n, sm);
 }
 
 // Persistent over the substep's tile list.
@@ -813,9 +894,10 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_force(ForceLaunch L) {
     if (threadIdx.x < 2) Ps[threadIdx.x] = force_params(L.lay[threadIdx.x], L.sc, threadIdx.x, blockIdx.x == 0);
     __syncthreads();
     const int n = *L.tf.count;
+    const WholeCta T;
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const int e = L.tf.list[k];
-        if (force_entry(Ps[e >> 30], L.tf, L.nxt, e, sm)) __syncthreads();  // shared memory is reused by the next tile
+        if (force_entry<Snap>(T, Ps[e >> 30], L.tf, L.nxt, e, sm)) T.sync();  // shared memory is reused by the next tile
     }
 }
 
@@ -1360,6 +1442,7 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_batch_force(const WindowSubst
     __shared__ TileFlags Tf;
     __shared__ int nxt_s;
     const int n = *count;
+    const WholeCta T;
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const int e = list[k];
         if (threadIdx.x == 0) {
@@ -1369,47 +1452,50 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_batch_force(const WindowSubst
             nxt_s = D.F.nxt;
         }
         __syncthreads();
-        force_entry(Ps, Tf, nxt_s, e, sm);
+        if (!Ps.sweep) force_entry<Snap>(T, Ps, Tf, nxt_s, e, sm);  // the others are k_batch_force_sweep's
         __syncthreads();  // the parameters and shared memory are reused by the next entry
     }
 }
 
-// Every window's force pass in the sweep form (cooperative launch), as
-// k_force_sweep does for one sheet; windows without the sweep take the
-// snapshot form in the first part and sit out the rest.
-__global__ void __launch_bounds__(FORCE_THREADS) k_batch_force_sweep(const WindowSubstep* ws, int nwin, const int* list,
-                                                                     const int* entry_win, const int* count,
-                                                                     SweepState* S) {
-    ::silt::dep_wait();
-    extern __shared__ float sm[];
-    __shared__ LayerParams Ps;
-    __shared__ TileFlags Tf;
-    __shared__ int nxt_s;
-    const int n = *count;
+// Every window's force pass in the sweep form, as force_sweep does for one
+// sheet; a window in the snapshot form is k_batch_force's. Each team keeps
+// its entry's parameters in its own slot.
+struct BatchEntry {
+    LayerParams P;
+    TileFlags tf;
+    int nxt;
+};
+
+template <class TM>
+__device__ __forceinline__ void batch_force_sweep(const WindowSubstep* ws, int nwin, const int* list,
+                                                  const int* entry_win, int n, SweepState* S, BatchEntry* slots,
+                                                  float* sm) {
+    const SweepTeam<TM> W(sm);
+    BatchEntry& B = slots[W.half];
     auto fetch = [&](int k, bool report) {
         const int e = list[k];
-        if (threadIdx.x == 0) {
+        if (W.T.tid == 0) {
             const WindowSubstep& D = ws[entry_win[k]];
-            Ps = force_params(D.F.lay[e >> 30], D.F.sc, e >> 30, report);
-            Tf = D.F.tf;
-            nxt_s = D.F.nxt;
+            B.P = force_params(D.F.lay[e >> 30], D.F.sc, e >> 30, report);
+            B.tf = D.F.tf;
+            B.nxt = D.F.nxt;
         }
-        __syncthreads();
+        W.T.sync();
         return e;
     };
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+    for (int k = W.first; k < n; k += W.stride) {
         const int e = fetch(k, true);
-        force_entry(Ps, Tf, nxt_s, e, sm);
-        __syncthreads();  // the parameters and shared memory are reused by the next entry
+        if (B.P.sweep) force_entry<Sweep>(W.T, B.P, B.tf, B.nxt, e, W.sm);
+        W.T.sync();  // the parameters and shared memory are reused by the next entry
     }
     unsigned int target = 0;
     const unsigned int epoch = ld_acquire_u32(&S->epoch);
     if (!grid_barrier(S, target)) return;
-    const bool reuse = n <= (int)gridDim.x;  // one entry per CTA: its tile stays in shared memory
-    const int passes = sweep_fixed_point(S, target, n, [&](int k, int pass) {
+    const bool reuse = n <= W.stride;  // one entry per team: its tile stays in shared memory
+    const int passes = sweep_fixed_point(W, S, target, n, [&](int k, int pass) {
         const int e = fetch(k, false);
-        const bool r = sweep_entry(Ps, Tf, e, sm, pass, epoch, reuse);
-        __syncthreads();
+        const bool r = sweep_entry(W.T, B.P, B.tf, e, W.sm, pass, epoch, reuse);
+        W.T.sync();
         return r;
     });
     if (passes < 0) return;
@@ -1425,11 +1511,24 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_batch_force_sweep(const Windo
         if (!grid_barrier(S, target)) return;
     }
     sweep_stats(S, passes);
-    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+    for (int k = W.first; k < n; k += W.stride) {
         const int e = fetch(k, false);
-        post_entry(Ps, Tf, e, sm);
-        __syncthreads();
+        post_entry(W.T, B.P, B.tf, e, W.sm);
+        W.T.sync();
     }
+}
+
+__global__ void __launch_bounds__(FORCE_THREADS, 2) k_batch_force_sweep(const WindowSubstep* ws, int nwin,
+                                                                        const int* list, const int* entry_win,
+                                                                        const int* count, SweepState* S) {
+    ::silt::dep_wait();
+    extern __shared__ float sm[];
+    __shared__ BatchEntry slots[2];
+    const int n = *count;
+    if (n <= (int)gridDim.x)
+        batch_force_sweep<WholeCta>(ws, nwin, list, entry_win, n, S, slots, sm);
+    else
+        batch_force_sweep<HalfCta>(ws, nwin, list, entry_win, n, S, slots, sm);
 }
 
 __global__ void __launch_bounds__(TRANSPORT_THREADS) k_batch_transport(const WindowSubstep* ws, const int* list,
@@ -1476,11 +1575,12 @@ cudaError_t launch_batch_speed2(const WindowSubstep* d_ws, const int* list, cons
 
 // Grid of a cooperative force launch: every CTA the device holds at once.
 template <class K>
-int coop_grid(K kernel, size_t smem) {
+int coop_grid(K kernel) {
     int dev = 0, nsm = 0, per = 0;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SWEEP_SMEM);
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, FORCE_THREADS, smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, FORCE_THREADS, SWEEP_SMEM) != cudaSuccess) return 0;
     return nsm * per;
 }
 
@@ -1490,7 +1590,7 @@ cudaError_t launch_coop(K kernel, int grid, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(FORCE_THREADS);
-    cfg.dynamicSmemBytes = force_smem_bytes();
+    cfg.dynamicSmemBytes = SWEEP_SMEM;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1503,13 +1603,12 @@ cudaError_t launch_coop(K kernel, int grid, cudaStream_t st, Args... args) {
 }
 
 cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* list, const int* entry_win,
-                               const int* count, SweepState* sweep, cudaStream_t st, int ctas_per_sm) {
+                               const int* count, SweepState* sweep, bool snapshot, cudaStream_t st, int ctas_per_sm) {
     if (sweep) {
         static std::once_flag sattr;
         static int grid = 0, nsm = 148;
         std::call_once(sattr, [] {
-            cudaFuncSetAttribute(k_batch_force_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem_bytes());
-            grid = coop_grid(k_batch_force_sweep, force_smem_bytes());
+            grid = coop_grid(k_batch_force_sweep);
             int dev = 0;
             if (cudaGetDevice(&dev) != cudaSuccess ||
                 cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0)
@@ -1519,11 +1618,11 @@ cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* l
         // Fewer CTAs than the device holds stay co-resident: the launch is still cooperative.
         const int g = ctas_per_sm > 0 ? std::min(grid, ctas_per_sm * nsm) : grid;
         const cudaError_t e = launch_coop(k_batch_force_sweep, g, st, d_ws, nwin, list, entry_win, count, sweep);
-        return e != cudaSuccess ? e : cudaGetLastError();
+        if (e != cudaSuccess || !snapshot) return e != cudaSuccess ? e : cudaGetLastError();
     }
     static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_batch_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem_bytes()); });
-    ::silt::launch_dep(k_batch_force, dim3(148 * 2), dim3(FORCE_THREADS), force_smem_bytes(), st, d_ws, list, entry_win, count);
+    std::call_once(attr, [] { cudaFuncSetAttribute(k_batch_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Snap::BYTES); });
+    ::silt::launch_dep(k_batch_force, dim3(148 * 2), dim3(FORCE_THREADS), Snap::BYTES, st, d_ws, list, entry_win, count);
     ::silt::count_launch();
     return cudaGetLastError();
 }
@@ -1544,17 +1643,16 @@ cudaError_t launch_force(const ForceLaunch& L, int res, int layers, cudaStream_t
         static std::once_flag sattr;
         static int grid = 0;
         std::call_once(sattr, [] {
-            cudaFuncSetAttribute(k_force_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem_bytes());
-            grid = coop_grid(k_force_sweep, force_smem_bytes());
+            grid = coop_grid(k_force_sweep);
         });
         const cudaError_t e = launch_coop(k_force_sweep, grid, st, L);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
     static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)force_smem_bytes()); });
+    std::call_once(attr, [] { cudaFuncSetAttribute(k_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Snap::BYTES); });
     (void)res;
     (void)layers;
-    ::silt::launch_dep(k_force, dim3(148 * 2), dim3(FORCE_THREADS), force_smem_bytes(), st, L);
+    ::silt::launch_dep(k_force, dim3(148 * 2), dim3(FORCE_THREADS), Snap::BYTES, st, L);
     ::silt::count_launch();
     return cudaGetLastError();
 }

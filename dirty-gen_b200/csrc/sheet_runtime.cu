@@ -2366,7 +2366,7 @@ int batch_coarse(silt_batch* b, float dt) {
     // The batch's sweep launches keep their state in the first window's
     // slot, so their errors come back through that window's flags.
     silt::SweepState* sweep = b->sheets[0]->sweep_state();
-    bool sweeping = false;
+    bool sweeping = false, snapshot = false;
     if (b->ev[slot]) CK(cudaEventSynchronize(b->ev[slot]));  // this slot's last copy has left its pinned half
     if (need > b->ws_cap[slot]) {
         cudaFree(b->d_ws[slot]);
@@ -2391,6 +2391,7 @@ int batch_coarse(silt_batch* b, float dt) {
             int all = 0;
             coarse_substep(s, plans[w], dt, k, D.F, D.T, all);
             sweeping = sweeping || D.F.lay[0].sweep || D.F.lay[1].sweep;
+            snapshot = snapshot || !D.F.lay[0].sweep || !D.F.lay[1].sweep;
             D.cur = s->cur;
             D.all = all;
             D.apply_cut = s->cut_pending ? 1 : 0;
@@ -2418,7 +2419,7 @@ int batch_coarse(silt_batch* b, float dt) {
             if (!e0 || !e1 || !e2) return fail_cuda(cudaErrorMemoryAllocation, "batch timing events");
             CK(cudaEventRecord(e0, b->st));
         }
-        CK(silt::launch_batch_force(d, n, b->list, b->entry_win, count, sweeping ? sweep : nullptr, b->st,
+        CK(silt::launch_batch_force(d, n, b->list, b->entry_win, count, sweeping ? sweep : nullptr, snapshot, b->st,
                                     b->tune.sweep_ctas_per_sm));
         if (b->timing) CK(cudaEventRecord(e1, b->st));
         CK(silt::launch_batch_transport(d, b->list, b->entry_win, count, b->st, b->tune.transport_blocks));
