@@ -172,26 +172,18 @@ __device__ __forceinline__ float cell_decay(const LayerParams& P, size_t g, floa
 }
 
 // Every cell of the tile's region of radius (RX, RY): f(gx, gy, s, g) with s
-// the shared-memory index and g the global one. Edge tiles clip the region to
-// the grid and walk it one warp per row; interior tiles walk the rectangle as
-// one flat range (a compile-time width), which keeps every lane busy.
+// the shared-memory index and g the global one. The rectangle is walked as one
+// flat range (a compile-time width), which keeps every lane busy; on edge
+// tiles cells outside the grid are left out.
 template <class TM, class G, bool EDGE, int RX, int RY, class F>
 __device__ __forceinline__ void region(const TM& T, int tx0, int ty0, int res, F f) {
     const int ox = tx0 - G::H, oy = ty0 - G::H;
-    if (EDGE) {
-        const int lane = T.tid & 31, wy = T.tid >> 5, NW = TM::NT / 32;
-        const int x0 = max(0, tx0 - RX), x1 = min(res, tx0 + FT + RX);
-        const int y0 = max(0, ty0 - RY), y1 = min(res, ty0 + FT + RY);
-        for (int gy = y0 + wy; gy < y1; gy += NW)
-            for (int gx = x0 + lane; gx < x1; gx += 32)
-                f(gx, gy, (gy - oy) * G::W + (gx - ox), (size_t)gy * res + gx);
-    } else {
-        constexpr int RW = FT + 2 * RX, RH = FT + 2 * RY;
-        for (int k = T.tid; k < RW * RH; k += TM::NT) {
-            const int r = k / RW;
-            const int gy = ty0 - RY + r, gx = tx0 - RX + (k - r * RW);
-            f(gx, gy, (gy - oy) * G::W + (gx - ox), (size_t)gy * res + gx);
-        }
+    constexpr int RW = FT + 2 * RX, RH = FT + 2 * RY;
+    for (int k = T.tid; k < RW * RH; k += TM::NT) {
+        const int r = k / RW;
+        const int gy = ty0 - RY + r, gx = tx0 - RX + (k - r * RW);
+        if (EDGE && ((unsigned)gx >= (unsigned)res || (unsigned)gy >= (unsigned)res)) continue;
+        f(gx, gy, (gy - oy) * G::W + (gx - ox), (size_t)gy * res + gx);
     }
 }
 
@@ -419,13 +411,6 @@ __device__ __forceinline__ void pre_tile(const TM& T, const LayerParams& P, floa
     });
 }
 
-// Local passes of the sweep's fixed point on one tile before its values go
-// back to global memory.
-#ifndef SILT_SWEEP_LOCAL_PASSES
-#define SILT_SWEEP_LOCAL_PASSES 16
-#endif
-constexpr int SWEEP_LOCAL_PASSES = SILT_SWEEP_LOCAL_PASSES;
-
 // Sweep form, part 2: one pass of the raster-order Gauss-Seidel confinement
 // (force_gravity_open, src/fluid_core.rs:2234-2260) solved as a fixed point.
 // In the reference's sweep a wet cell's final velocity is its post-gravity
@@ -433,17 +418,29 @@ constexpr int SWEEP_LOCAL_PASSES = SILT_SWEEP_LOCAL_PASSES;
 // in raster order, its own G, and the starting values of the cells after it;
 // dry cells never change. The tile iterates that equation for its own wet
 // cells in shared memory, reading the current iterate of other tiles' cells
-// from fu, fv, until a local pass changes no bit, and writes back what
-// changed. Returns true (block-uniform) when any value of the tile changed.
-// When a whole pass over every tile changes nothing, every cell satisfies its
-// equation with the values it read, and since each cell depends only on
-// earlier cells that solution is the sequential sweep's, bit for bit.
-// `reuse`: this CTA's shared memory still holds this tile from an earlier
-// pass of the launch (the CTA solves no other tile), so only the ring of
+// from fu, fv, until a local pass changes no bit (each pass settles at least
+// the first unsettled cell in raster order, so it ends), and writes back what
+// changed. Returns true (block-uniform) when a value another tile reads
+// changed. When a whole pass over every tile changes none, every cell
+// satisfies its equation with the values it read, and since each cell depends
+// only on earlier cells that solution is the sequential sweep's, bit for bit.
+//
+// A change at c reaches the cells that read c's iterate: c + (1,0), (2,0),
+// (0,1), (-1,1), (1,1), (0,2) (index clamping at the grid's edge reads no
+// other cells). So a local pass after the first recomputes only the marked
+// ones; the first pass of a tile solved before (`again`) only those that read
+// the ring of other tiles' cells, the 154 of rows 0-1 and columns 0, 1 and
+// 31, since the tile's own values satisfy their equations; and only a change
+// in column 0, 30 or 31 or in row 30 or 31 is another tile's business.
+// Recomputing whole tiles in every pass a flood's launch of 2300 tile-layers
+// (2.5 solves each) took 348 us; TIMED.
+// `reuse`: this team's shared memory still holds this tile from an earlier
+// pass of the launch (the team solves no other tile), so only the ring of
 // other tiles' wet cells around it is read again; the starting and
 // post-gravity velocities and the tile's own iterate are current.
 template <class TM, class G, bool EDGE>
-__device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0, bool reuse, int& passes) {
+__device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0, bool again, bool reuse,
+                           int& passes) {
     const int res = P.res;
     float* PU = sm;              // starting velocity (the values of cells after a cell)
     float* PV = sm + G::PLANE;
@@ -452,76 +449,55 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     float* GU = sm + 4 * G::PLANE;  // post-gravity velocity of the tile's own cells
     float* GV = sm + 5 * G::PLANE;
     float* WT = sm + 6 * G::PLANE;  // 1: wet
+    // Marks of the cells to recompute: pass it reads one byte plane, clearing
+    // it, and marks in the other; both are clear when a solve ends.
+    uint8_t* const marks = reinterpret_cast<uint8_t*>(sm + 7 * G::PLANE);
     const int ox = tx0 - G::H, oy = ty0 - G::H;
-    const float eps = P.eps;
+    const float eps = P.eps, dt = P.dt, vort = P.vort;
+    const FixedDiv two = P.div_two;
+    float *__restrict__ fu = P.fu, *__restrict__ fv = P.fv;
+    auto own = [&](int gx, int gy) { return gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT; };
     if (reuse) {
         region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-            if (gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT) return;
-            if (WT[s] != 0.0f) {
-                FU[s] = P.fu[g];
-                FV[s] = P.fv[g];
+            if (!own(gx, gy) && WT[s] != 0.0f) {
+                FU[s] = fu[g];
+                FV[s] = fv[g];
             }
         });
-    } else region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-        const float hv = P.h[g];
-        float uu, vv;
-        start_velocity(P, gx, gy, g, hv, uu, vv);
-        const bool wet = hv > eps;
-        PU[s] = uu;
-        PV[s] = vv;
-        WT[s] = wet ? 1.0f : 0.0f;
-        // A wet cell's tile is always stepped this substep, so its iterate
-        // is current; a dry cell keeps its starting velocity.
-        FU[s] = wet ? P.fu[g] : uu;
-        FV[s] = wet ? P.fv[g] : vv;
-        if (wet && gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT) {
-            GU[s] = P.u_out[g];
-            GV[s] = P.v_out[g];
-        }
-    });
-    T.sync();
-    bool tile_changed = false;
-    passes = 0;
-    // Interior tiles recompute, after the first local pass, only the cells
-    // one of whose earlier-cell reads changed since they were last computed:
-    // a cell whose inputs did not change keeps its value. A change at c
-    // marks the cells that read c's iterate: c + (1,0), (2,0), (0,1),
-    // (-1,1), (1,1), (0,2). Marks for pass it + 1 go to one byte plane while
-    // pass it reads the other (plane 7 of the force layout, unused here).
-    uint8_t* const marks = reinterpret_cast<uint8_t*>(sm + 7 * G::PLANE);
-    for (int it = 0; it < SWEEP_LOCAL_PASSES; ++it) {
-        ++passes;
-        int changed = 0;
-        const uint8_t* dirty = marks + (it & 1) * G::PLANE;
-        uint8_t* dirty_next = marks + ((it + 1) & 1) * G::PLANE;
-        if (!EDGE) {
-            region<TM, G, false, 0, 0>(T, tx0, ty0, res, [&](int, int, int s, size_t) { dirty_next[s] = 0; });
-            T.sync();
-        }
-        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-            if (WT[s] == 0.0f) return;
-            if (!EDGE) {
-                // Interior tile: no stencil index is clamped.
-                if (it > 0 && !dirty[s]) return;
-                float du, dv, nu_ = GU[s], nv_ = GV[s];
-                if (conf_kick_inner(P.div_two, P.dt, P.vort, SweepRead{FU, PU, GU, s, G::W},
-                                    SweepRead{FV, PV, GV, s, G::W}, du, dv)) {
-                    nu_ = GU[s] + du;
-                    nv_ = GV[s] + dv;
+    } else {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+            const float hv = P.h[g];
+            float uu, vv;
+            start_velocity(P, gx, gy, g, hv, uu, vv);
+            const bool wet = hv > eps;
+            PU[s] = uu;
+            PV[s] = vv;
+            WT[s] = wet ? 1.0f : 0.0f;
+            // A wet cell's tile is always stepped this substep, so its iterate
+            // is current; a dry cell keeps its starting velocity.
+            FU[s] = wet ? fu[g] : uu;
+            FV[s] = wet ? fv[g] : vv;
+            if (own(gx, gy)) {
+                marks[s] = marks[G::PLANE + s] = 0;
+                if (wet) {
+                    GU[s] = P.u_out[g];
+                    GV[s] = P.v_out[g];
                 }
-                if (__float_as_uint(nu_) != __float_as_uint(FU[s]) || __float_as_uint(nv_) != __float_as_uint(FV[s])) {
-                    FU[s] = nu_;
-                    FV[s] = nv_;
-                    changed = 1;
-                    dirty_next[s + 1] = 1;
-                    dirty_next[s + 2] = 1;
-                    dirty_next[s + G::W - 1] = 1;
-                    dirty_next[s + G::W] = 1;
-                    dirty_next[s + G::W + 1] = 1;
-                    dirty_next[s + 2 * G::W] = 1;
-                }
-                return;
             }
+        });
+    }
+    T.sync();
+    bool exported = false;
+    int changed = 0;
+    uint8_t* mark_next = nullptr;
+    auto solve = [&](int gx, int gy, int s) {
+        float du, dv, nu_ = GU[s], nv_ = GV[s];
+        bool kick;
+        if (!EDGE || (gx >= 2 && gy >= 2 && gx < res - 2 && gy < res - 2)) {
+            // No stencil index is clamped.
+            kick = conf_kick_inner(two, dt, vort, SweepRead{FU, PU, GU, s, G::W}, SweepRead{FV, PV, GV, s, G::W}, du,
+                                   dv);
+        } else {
             auto at = [&](int a, int b) { return (b - oy) * G::W + (a - ox); };
             auto before = [&](int a, int b) { return b < gy || (b == gy && a < gx); };
             auto uu = [&](int a, int b) {
@@ -532,30 +508,62 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
                 if (a == gx && b == gy) return GV[s];
                 return before(a, b) ? FV[at(a, b)] : PV[at(a, b)];
             };
-            float du, dv, nu_ = GU[s], nv_ = GV[s];
-            if (conf_kick(gx, gy, res, P.div_two, P.dt, P.vort, uu, vv, du, dv)) {
-                nu_ = GU[s] + du;
-                nv_ = GV[s] + dv;
+            kick = conf_kick(gx, gy, res, two, dt, vort, uu, vv, du, dv);
+        }
+        if (kick) {
+            nu_ = GU[s] + du;
+            nv_ = GV[s] + dv;
+        }
+        if (__float_as_uint(nu_) != __float_as_uint(FU[s]) || __float_as_uint(nv_) != __float_as_uint(FV[s])) {
+            FU[s] = nu_;
+            FV[s] = nv_;
+            changed |= (gx == tx0 || gx >= tx0 + FT - 2 || gy >= ty0 + FT - 2) ? 3 : 1;
+            mark_next[s + 1] = 1;
+            mark_next[s + 2] = 1;
+            mark_next[s + G::W - 1] = 1;
+            mark_next[s + G::W] = 1;
+            mark_next[s + G::W + 1] = 1;
+            mark_next[s + 2 * G::W] = 1;
+        }
+    };
+    bool tile_changed = false;
+    passes = 0;
+    for (int it = 0; it <= FT * FT; ++it) {
+        ++passes;
+        changed = 0;
+        uint8_t* const mark = marks + (it & 1) * G::PLANE;
+        mark_next = marks + ((it + 1) & 1) * G::PLANE;
+        if (it == 0 && again) {
+            constexpr int N = 2 * FT + 3 * (FT - 2);
+            for (int k = T.tid; k < N; k += TM::NT) {
+                const int q = k - 2 * FT, c = q % 3;
+                const int gx = tx0 + (q < 0 ? k % FT : (c == 2 ? FT - 1 : c)), gy = ty0 + (q < 0 ? k / FT : 2 + q / 3);
+                if (EDGE && (gx >= res || gy >= res)) continue;
+                const int s = (gy - oy) * G::W + (gx - ox);
+                if (WT[s] != 0.0f) solve(gx, gy, s);
             }
-            if (__float_as_uint(nu_) != __float_as_uint(FU[s]) || __float_as_uint(nv_) != __float_as_uint(FV[s])) {
-                FU[s] = nu_;
-                FV[s] = nv_;
-                changed = 1;
-            }
-        });
+        } else {
+            region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
+                if (it > 0) {
+                    if (!mark[s]) return;
+                    mark[s] = 0;
+                }
+                if (WT[s] != 0.0f) solve(gx, gy, s);
+            });
+        }
+        exported |= (changed & 2) != 0;
         if (!T.any(changed != 0)) break;
         tile_changed = true;
     }
     if (tile_changed) {
         region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
             if (WT[s] != 0.0f) {
-                P.fu[g] = FU[s];
-                P.fv[g] = FV[s];
+                fu[g] = FU[s];
+                fv[g] = FV[s];
             }
         });
     }
-    T.sync();  // shared memory is read again by the next tile or pass
-    return tile_changed;
+    return T.any(exported);  // and shared memory is read again by the next tile or pass
 }
 
 // Sweep form, part 3: projection, damping and clamp from the solved sweep.
@@ -657,39 +665,39 @@ __device__ __forceinline__ bool entry_steps(int e) { return (e & (ENTRY_ZERO | E
 
 // Sweep-form pass `pass` over one list entry: the fixed-point pass of a
 // stepped tile of a sweeping layer with confinement on. After the first
-// pass a tile is solved again only when some tile of its 3 x 3
-// neighbourhood (itself included) changed since the previous pass began: it
-// is otherwise still at the fixed point of the values around it. Returns
-// whether the tile changed (block-uniform) and stamps it when it did.
-// `reuse`: the CTA solves only this entry in the launch, so its shared
-// memory keeps the tile between passes.
+// pass a tile is solved again only when a tile whose cells it reads as
+// earlier ones (left, right and the three above) changed since the previous
+// pass began: it is otherwise still at the fixed point of the values around
+// it. Returns whether a value another tile reads changed (block-uniform) and
+// stamps the tile when one did. `reuse`: the team solves only this entry in
+// the launch, so its shared memory keeps the tile between passes.
 template <class TM>
-__device__ __forceinline__ bool sweep_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int e, float* sm, int pass,
-                                            unsigned int epoch, bool reuse) {
+__device__ __forceinline__ bool sweep_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int e, float* sm,
+                                            int pass, unsigned int epoch, bool reuse) {
     if (!entry_steps(e) || !P.sweep || !(P.vort > 0.0f)) return false;
     const int l = e >> 30, t = e & ENTRY_TILE;
     const int nt = tf.tiles_x * tf.tiles_x;
     const int ti = t % tf.tiles_x, tj = t / tf.tiles_x;
-    unsigned int* stamp = tf.stamp ? tf.stamp + (size_t)l * nt : nullptr;
-    if (pass > 0 && stamp) {
-        // Nine threads read the nine stamps at once.
+    unsigned int* stamp = tf.stamp + (size_t)l * nt;
+    if (pass > 0) {
+        // Five threads read the five stamps at once.
         bool hit = false;
-        if (T.tid < 9) {
-            const int x = ti + T.tid % 3 - 1, y = tj + T.tid / 3 - 1;
+        if (T.tid < 5) {
+            const int x = ti + (T.tid < 3 ? T.tid - 1 : 2 * T.tid - 7), y = tj - (T.tid < 3 ? 1 : 0);
             const unsigned int since = epoch * 256u + (unsigned int)pass;
-            hit = x >= 0 && y >= 0 && x < tf.tiles_x && y < tf.tiles_x &&
+            hit = x >= 0 && y >= 0 && x < tf.tiles_x &&
                   *(volatile unsigned int*)&stamp[y * tf.tiles_x + x] >= since;
         }
         if (!T.any(hit)) return false;
     }
     const int tx0 = ti * FT, ty0 = tj * FT;
     int passes = 0;
-    const bool keep = reuse && pass > 0;
+    const bool again = pass > 0, keep = reuse && again;
     const bool changed = tile_interior<Sweep>(P.res, tx0, ty0)
-                             ? sweep_tile<TM, Sweep, false>(T, P, sm, tx0, ty0, keep, passes)
-                             : sweep_tile<TM, Sweep, true>(T, P, sm, tx0, ty0, keep, passes);
+                             ? sweep_tile<TM, Sweep, false>(T, P, sm, tx0, ty0, again, keep, passes)
+                             : sweep_tile<TM, Sweep, true>(T, P, sm, tx0, ty0, again, keep, passes);
     if (T.tid == 0) {
-        if (changed && stamp) {
+        if (changed) {
             __threadfence();
             stamp[t] = epoch * 256u + (unsigned int)pass + 1u;
         }
