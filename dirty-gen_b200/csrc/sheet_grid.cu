@@ -187,13 +187,11 @@ __device__ __forceinline__ void region(const TM& T, int tx0, int ty0, int res, F
     }
 }
 
-// The velocity a substep starts from at (gx, gy): the lazy dry cut of the
-// previous substep, then the soft window border (src/fluid_core.rs:9594-9622;
-// a river reach's band keeps its current through the window ends).
-__device__ __forceinline__ void start_velocity(const LayerParams& P, int gx, int gy, size_t g, float hv, float& uu,
-                                               float& vv) {
-    uu = P.u[g];
-    vv = P.v[g];
+// The velocity a substep starts from at (gx, gy), from the plane's (uu, vv):
+// the lazy dry cut of the previous substep, then the soft window border
+// (src/fluid_core.rs:9594-9622; a river reach's band keeps its current through
+// the window ends).
+__device__ __forceinline__ void start_velocity(const LayerParams& P, int gx, int gy, float hv, float& uu, float& vv) {
     if (P.apply_cut && hv < P.eps) {
         uu = 0.0f;
         vv = 0.0f;
@@ -233,19 +231,37 @@ struct ForcePlanes {
 #define NX(d) (EDGE ? (gy - oy) * G::W + (clampi(gx + (d), 0, res - 1) - ox) : s + (d))
 #define NZ(d) (EDGE ? (clampi(gy + (d), 0, res - 1) - oy) * G::W + (gx - ox) : s + (d) * G::W)
 
-// Depth and eta on radius R + 2, then the pressure p = 0.45 (0.62 G + 0.38 S)
-// + 0.55 eta on radius R (src/fluid_core.rs:1950-1985): the two 5-tap blurs,
+// Tiles are staged by cp.async, one copy per value and plane, all of a stage
+// in flight at once: a loop of loads and shared stores waits for each round
+// trip in turn, since the compiler cannot move a load past a store through
+// another pointer. (4-byte copies: rows start at any column.) A 1501^2 flood's
+// sweep launch 305 -> 269 us, k_force on a flooded 1000^2 grid 100 -> 90.
+__device__ __forceinline__ void stage(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+// Every thread's own copies have landed; a barrier publishes them to the team.
+__device__ __forceinline__ void staged() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// Depth and eta on radius R + 2, the velocity as stored on radius RV, then the
+// pressure p = 0.45 (0.62 G + 0.38 S) + 0.55 eta on radius R (src/fluid_core.rs:1950-1985): the two 5-tap blurs,
 // x pass then z pass. Ends with a barrier.
-template <class TM, class G, bool EDGE, int R>
-__device__ __forceinline__ void pressure_field(const TM& T, const LayerParams& P, const ForcePlanes<G>& F, int tx0, int ty0) {
+template <class TM, class G, bool EDGE, int R, int RV>
+__device__ __forceinline__ void pressure_field(const TM& T, const LayerParams& P, const ForcePlanes<G>& F, int tx0,
+                                               int ty0) {
     const int res = P.res;
     const int ox = tx0 - G::H, oy = ty0 - G::H;
-    const float *__restrict__ depth = P.h, *__restrict__ bed = P.bed;
+    const float *depth = P.h, *bed = P.bed, *u = P.u, *v = P.v;
     region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-        float hv = depth[g];
-        F.HS[s] = hv;
-        F.E[s] = bed[g] + hv;
+        stage(&F.HS[s], depth + g);
+        stage(&F.E[s], bed + g);
     });
+    region<TM, G, EDGE, RV, RV>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        stage(&F.U[s], u + g);
+        stage(&F.V[s], v + g);
+    });
+    staged();
+    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int, int, int s, size_t) { F.E[s] += F.HS[s]; });
     T.sync();
     region<TM, G, EDGE, R, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
         const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
@@ -335,12 +351,12 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
     const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float dt = P.dt, eps = P.eps;
     // 1-3. Depth, eta (radius 9) and the pressure (radius 7).
-    pressure_field<TM, G, EDGE, 7>(T, P, F, tx0, ty0);
+    pressure_field<TM, G, EDGE, 7, 6>(T, P, F, tx0, ty0);
     // Velocity on radius 6 and gravity down the pressure gradient on wet
     // cells (src/fluid_core.rs:2234-2253).
     region<TM, G, EDGE, 6, 6>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-        float uu, vv;
-        start_velocity(P, gx, gy, g, F.HS[s], uu, vv);
+        float uu = F.U[s], vv = F.V[s];
+        start_velocity(P, gx, gy, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
             float px = fdiv(F.PB[NX(1)] - F.PB[NX(-1)], P.div_two);
             float pz = fdiv(F.PB[NZ(1)] - F.PB[NZ(-1)], P.div_two);
@@ -393,10 +409,10 @@ __device__ __forceinline__ void pre_tile(const TM& T, const LayerParams& P, floa
     const ForcePlanes<G> F(sm);
     const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float dt = P.dt, eps = P.eps;
-    pressure_field<TM, G, EDGE, 1>(T, P, F, tx0, ty0);
+    pressure_field<TM, G, EDGE, 1, 0>(T, P, F, tx0, ty0);
     region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-        float uu, vv;
-        start_velocity(P, gx, gy, g, F.HS[s], uu, vv);
+        float uu = F.U[s], vv = F.V[s];
+        start_velocity(P, gx, gy, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
             float px = fdiv(F.PB[NX(1)] - F.PB[NX(-1)], P.div_two);
             float pz = fdiv(F.PB[NZ(1)] - F.PB[NZ(-1)], P.div_two);
@@ -432,8 +448,8 @@ __device__ __forceinline__ void pre_tile(const TM& T, const LayerParams& P, floa
 // the ring of other tiles' cells, the 154 of rows 0-1 and columns 0, 1 and
 // 31, since the tile's own values satisfy their equations; and only a change
 // in column 0, 30 or 31 or in row 30 or 31 is another tile's business.
-// Recomputing whole tiles in every pass a flood's launch of 2300 tile-layers
-// (2.5 solves each) took 348 us; TIMED.
+// Recomputing whole tiles in every pass, a flood's launch of 2300 tile-layers
+// (2.5 solves each) took 348 us instead of 305.
 // `reuse`: this team's shared memory still holds this tile from an earlier
 // pass of the launch (the team solves no other tile), so only the ring of
 // other tiles' wet cells around it is read again; the starting and
@@ -448,7 +464,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     float* FV = sm + 3 * G::PLANE;
     float* GU = sm + 4 * G::PLANE;  // post-gravity velocity of the tile's own cells
     float* GV = sm + 5 * G::PLANE;
-    float* WT = sm + 6 * G::PLANE;  // 1: wet
+    float* HS = sm + 6 * G::PLANE;  // depth
     // Marks of the cells to recompute: pass it reads one byte plane, clearing
     // it, and marks in the other; both are clear when a solve ends.
     uint8_t* const marks = reinterpret_cast<uint8_t*>(sm + 7 * G::PLANE);
@@ -459,30 +475,39 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     auto own = [&](int gx, int gy) { return gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT; };
     if (reuse) {
         region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-            if (!own(gx, gy) && WT[s] != 0.0f) {
-                FU[s] = fu[g];
-                FV[s] = fv[g];
+            if (!own(gx, gy) && HS[s] > eps) {
+                stage(&FU[s], fu + g);
+                stage(&FV[s], fv + g);
             }
         });
+        staged();
     } else {
+        const float *depth = P.h, *u = P.u, *v = P.v, *gu = P.u_out, *gv = P.v_out;
         region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-            const float hv = P.h[g];
-            float uu, vv;
-            start_velocity(P, gx, gy, g, hv, uu, vv);
-            const bool wet = hv > eps;
+            stage(&HS[s], depth + g);
+            stage(&PU[s], u + g);
+            stage(&PV[s], v + g);
+            stage(&FU[s], fu + g);
+            stage(&FV[s], fv + g);
+            if (own(gx, gy)) {
+                stage(&GU[s], gu + g);
+                stage(&GV[s], gv + g);
+                marks[s] = marks[G::PLANE + s] = 0;
+            }
+        });
+        staged();
+        // The same thread's cells again.
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
+            const float hv = HS[s];
+            float uu = PU[s], vv = PV[s];
+            start_velocity(P, gx, gy, hv, uu, vv);
             PU[s] = uu;
             PV[s] = vv;
-            WT[s] = wet ? 1.0f : 0.0f;
             // A wet cell's tile is always stepped this substep, so its iterate
             // is current; a dry cell keeps its starting velocity.
-            FU[s] = wet ? fu[g] : uu;
-            FV[s] = wet ? fv[g] : vv;
-            if (own(gx, gy)) {
-                marks[s] = marks[G::PLANE + s] = 0;
-                if (wet) {
-                    GU[s] = P.u_out[g];
-                    GV[s] = P.v_out[g];
-                }
+            if (!(hv > eps)) {
+                FU[s] = uu;
+                FV[s] = vv;
             }
         });
     }
@@ -540,7 +565,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
                 const int gx = tx0 + (q < 0 ? k % FT : (c == 2 ? FT - 1 : c)), gy = ty0 + (q < 0 ? k / FT : 2 + q / 3);
                 if (EDGE && (gx >= res || gy >= res)) continue;
                 const int s = (gy - oy) * G::W + (gx - ox);
-                if (WT[s] != 0.0f) solve(gx, gy, s);
+                if (HS[s] > eps) solve(gx, gy, s);
             }
         } else {
             region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
@@ -548,7 +573,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
                     if (!mark[s]) return;
                     mark[s] = 0;
                 }
-                if (WT[s] != 0.0f) solve(gx, gy, s);
+                if (HS[s] > eps) solve(gx, gy, s);
             });
         }
         exported |= (changed & 2) != 0;
@@ -557,7 +582,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     }
     if (tile_changed) {
         region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-            if (WT[s] != 0.0f) {
+            if (HS[s] > eps) {
                 fu[g] = FU[s];
                 fv[g] = FV[s];
             }
@@ -572,16 +597,25 @@ __device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, flo
     const int res = P.res;
     const ForcePlanes<G> F(sm);
     const float eps = P.eps;
-    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
-        const float hv = P.h[g];
-        F.HS[s] = hv;
-        F.E[s] = P.bed[g] + hv;
-        float uu, vv;
+    const float *depth = P.h, *bed = P.bed, *u = P.u, *v = P.v, *fu = P.fu, *fv = P.fv;
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int, int, int s, size_t g) {
+        stage(&F.HS[s], depth + g);
+        stage(&F.E[s], bed + g);
+        stage(&F.U[s], u + g);
+        stage(&F.V[s], v + g);
+        stage(&F.TG[s], fu + g);
+        stage(&F.TS[s], fv + g);
+    });
+    staged();
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
+        const float hv = F.HS[s];
+        F.E[s] += hv;
+        float uu = F.U[s], vv = F.V[s];
         if (hv > eps) {
-            uu = P.fu[g];
-            vv = P.fv[g];
+            uu = F.TG[s];
+            vv = F.TS[s];
         } else {
-            start_velocity(P, gx, gy, g, hv, uu, vv);
+            start_velocity(P, gx, gy, hv, uu, vv);
         }
         F.U[s] = uu;
         F.V[s] = vv;
@@ -816,8 +850,8 @@ __device__ void sweep_serial(const LayerParams& P) {
                 if (a == i && b == j) return is_u ? P.u_out[q] : P.v_out[q];
                 const float hq = P.h[q];
                 if (hq > eps && (b < j || (b == j && a < i))) return is_u ? P.fu[q] : P.fv[q];
-                float uu, vv;
-                start_velocity(P, a, b, q, hq, uu, vv);
+                float uu = P.u[q], vv = P.v[q];
+                start_velocity(P, a, b, hq, uu, vv);
                 return is_u ? uu : vv;
             };
             auto uu = [&](int a, int b) { return val(true, a, b); };
