@@ -183,32 +183,41 @@ __device__ __forceinline__ void region(const TM& T, int tx0, int ty0, int res, F
         const int r = k / RW;
         const int gy = ty0 - RY + r, gx = tx0 - RX + (k - r * RW);
         if (EDGE && ((unsigned)gx >= (unsigned)res || (unsigned)gy >= (unsigned)res)) continue;
-        f(gx, gy, (gy - oy) * G::W + (gx - ox), (size_t)gy * res + gx);
+        f(gx, gy, (gy - oy) * G::W + (gx - ox), gy * res + gx);
     }
 }
 
 // The velocity a substep starts from at (gx, gy), from the plane's (uu, vv):
 // the lazy dry cut of the previous substep, then the soft window border
 // (src/fluid_core.rs:9594-9622; a river reach's band keeps its current through
-// the window ends).
-__device__ __forceinline__ void start_velocity(const LayerParams& P, int gx, int gy, float hv, float& uu, float& vv) {
+// the window ends). `band`: the border's width, 0 where no cell of the
+// caller's tile lies in it (tile_band), which spares most tiles the distances.
+__device__ __forceinline__ void start_velocity(const LayerParams& P, int band, int gx, int gy, float hv, float& uu,
+                                               float& vv) {
     if (P.apply_cut && hv < P.eps) {
         uu = 0.0f;
         vv = 0.0f;
     }
-    if (P.soften_edge > 0) {
+    if (band > 0) {
         const int res = P.res;
         const int dx = min(gx, res - 1 - gx), dz = min(gy, res - 1 - gy);
         int d = min(dx, dz);
         if (P.open_axis == 1 && gy >= P.open_c0 && gy < P.open_c1) d = dz;
         else if (P.open_axis == 2 && gx >= P.open_c0 && gx < P.open_c1) d = dx;
-        if (d < P.soften_edge) {
-            float t = (float)d / (float)P.soften_edge;
+        if (d < band) {
+            float t = (float)d / (float)band;
             float w = t * t * (3.0f - 2.0f * t);
             uu *= w;
             vv *= w;
         }
     }
+}
+
+// P.soften_edge for a tile whose cells and halo reach the soft border, else 0.
+template <class G>
+__device__ __forceinline__ int tile_band(const LayerParams& P, int tx0, int ty0) {
+    const int e = P.soften_edge + G::H;
+    return min(tx0, ty0) < e || max(tx0, ty0) + FT + e > P.res ? P.soften_edge : 0;
 }
 
 // Shared-memory planes of a force tile (G::W x G::W floats each, origin at the
@@ -252,25 +261,25 @@ __device__ __forceinline__ void pressure_field(const TM& T, const LayerParams& P
     const int res = P.res;
     const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float *depth = P.h, *bed = P.bed, *u = P.u, *v = P.v;
-    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         stage(&F.HS[s], depth + g);
         stage(&F.E[s], bed + g);
     });
-    region<TM, G, EDGE, RV, RV>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, RV, RV>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         stage(&F.U[s], u + g);
         stage(&F.V[s], v + g);
     });
     staged();
-    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int, int, int s, size_t) { F.E[s] += F.HS[s]; });
+    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int, int, int s, int) { F.E[s] += F.HS[s]; });
     T.sync();
-    region<TM, G, EDGE, R, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, R, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
         float e0 = F.E[NX(-2)], e1 = F.E[NX(-1)], e2 = F.E[s], e3 = F.E[NX(1)], e4 = F.E[NX(2)];
         F.TG[s] = tap5(e0, e1, e2, e3, e4, kG0, kG1, kG2, in);
         F.TS[s] = tap5(e0, e1, e2, e3, e4, kS0, kS1, kS2, in);
     });
     T.sync();
-    region<TM, G, EDGE, R, R>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, R, R>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         const bool in = EDGE ? (gy >= 2 && gy <= res - 3) : true;
         const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
         float gb = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
@@ -291,7 +300,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
     const float dt = P.dt, eps = P.eps;
     if (P.project) {
         // b = div * overload - 0.015 * overload * lap(eta), radius 3 (:1992-2003).
-        region<TM, G, EDGE, 3, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 3, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             const int sxp = NX(1), sxm = NX(-1), szp = NZ(1), szm = NZ(-1);
             float ux = fdiv(F.U[sxp] - F.U[sxm], P.div_two);
             float vz = fdiv(F.V[szp] - F.V[szm], P.div_two);
@@ -303,7 +312,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         });
         T.sync();
         // x pass of both blurs of b: rows radius 3, columns radius 1.
-        region<TM, G, EDGE, 1, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 1, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
             float b0 = F.PB[NX(-2)], b1 = F.PB[NX(-1)], b2 = F.PB[s], b3 = F.PB[NX(1)], b4 = F.PB[NX(2)];
             F.TG[s] = tap5(b0, b1, b2, b3, b4, kG0, kG1, kG2, in);
@@ -311,7 +320,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         });
         T.sync();
         // q = 0.62 G(b) + 0.38 S(b), radius 1 (:2004-2011).
-        region<TM, G, EDGE, 1, 1>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 1, 1>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             const bool in = EDGE ? (gy >= 2 && gy <= res - 3) : true;
             const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
             float gq = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
@@ -321,7 +330,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         T.sync();
     }
     // Projection kick, damping and the speed clamp on wet cells (:2015-2037).
-    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         float uu = F.U[s], vv = F.V[s];
         if (F.HS[s] > eps) {
             if (P.project) {
@@ -349,14 +358,15 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
     const int res = P.res;
     const ForcePlanes<G> F(sm);
     const int ox = tx0 - G::H, oy = ty0 - G::H;
+    const int band = tile_band<G>(P, tx0, ty0);
     const float dt = P.dt, eps = P.eps;
     // 1-3. Depth, eta (radius 9) and the pressure (radius 7).
     pressure_field<TM, G, EDGE, 7, 6>(T, P, F, tx0, ty0);
     // Velocity on radius 6 and gravity down the pressure gradient on wet
     // cells (src/fluid_core.rs:2234-2253).
-    region<TM, G, EDGE, 6, 6>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, 6, 6>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         float uu = F.U[s], vv = F.V[s];
-        start_velocity(P, gx, gy, F.HS[s], uu, vv);
+        start_velocity(P, band, gx, gy, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
             float px = fdiv(F.PB[NX(1)] - F.PB[NX(-1)], P.div_two);
             float pz = fdiv(F.PB[NZ(1)] - F.PB[NZ(-1)], P.div_two);
@@ -370,7 +380,7 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
     T.sync();
     // Vorticity of the post-gravity snapshot, radius 5 (src/fluid_core.rs:3498-3506).
     if (P.vort > 0.0f) {
-        region<TM, G, EDGE, 5, 5>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 5, 5>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             float dvdx = fdiv(F.V[NX(1)] - F.V[NX(-1)], P.div_two);
             float dudz = fdiv(F.U[NZ(1)] - F.U[NZ(-1)], P.div_two);
             F.WQ[s] = dvdx - dudz;
@@ -378,7 +388,7 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
         T.sync();
         // Confinement kick from that snapshot, in place, radius 4
         // (src/fluid_core.rs:2348-2375, :2441-2470).
-        region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             if (F.HS[s] > eps) {
                 float w = F.WQ[s];
                 if (finite_f(w) && !(fabsf(w) < 1.0e-4f)) {
@@ -408,11 +418,12 @@ __device__ __forceinline__ void pre_tile(const TM& T, const LayerParams& P, floa
     const int res = P.res;
     const ForcePlanes<G> F(sm);
     const int ox = tx0 - G::H, oy = ty0 - G::H;
+    const int band = tile_band<G>(P, tx0, ty0);
     const float dt = P.dt, eps = P.eps;
     pressure_field<TM, G, EDGE, 1, 0>(T, P, F, tx0, ty0);
-    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
         float uu = F.U[s], vv = F.V[s];
-        start_velocity(P, gx, gy, F.HS[s], uu, vv);
+        start_velocity(P, band, gx, gy, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
             float px = fdiv(F.PB[NX(1)] - F.PB[NX(-1)], P.div_two);
             float pz = fdiv(F.PB[NZ(1)] - F.PB[NZ(-1)], P.div_two);
@@ -469,12 +480,13 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     // it, and marks in the other; both are clear when a solve ends.
     uint8_t* const marks = reinterpret_cast<uint8_t*>(sm + 7 * G::PLANE);
     const int ox = tx0 - G::H, oy = ty0 - G::H;
+    const int band = tile_band<G>(P, tx0, ty0);
     const float eps = P.eps, dt = P.dt, vort = P.vort;
     const FixedDiv two = P.div_two;
     float *__restrict__ fu = P.fu, *__restrict__ fv = P.fv;
     auto own = [&](int gx, int gy) { return gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT; };
     if (reuse) {
-        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             if (!own(gx, gy) && HS[s] > eps) {
                 stage(&FU[s], fu + g);
                 stage(&FV[s], fv + g);
@@ -483,7 +495,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
         staged();
     } else {
         const float *depth = P.h, *u = P.u, *v = P.v, *gu = P.u_out, *gv = P.v_out;
-        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             stage(&HS[s], depth + g);
             stage(&PU[s], u + g);
             stage(&PV[s], v + g);
@@ -497,10 +509,10 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
         });
         staged();
         // The same thread's cells again.
-        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int) {
             const float hv = HS[s];
             float uu = PU[s], vv = PV[s];
-            start_velocity(P, gx, gy, hv, uu, vv);
+            start_velocity(P, band, gx, gy, hv, uu, vv);
             PU[s] = uu;
             PV[s] = vv;
             // A wet cell's tile is always stepped this substep, so its iterate
@@ -517,12 +529,11 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     uint8_t* mark_next = nullptr;
     auto solve = [&](int gx, int gy, int s) {
         float du, dv, nu_ = GU[s], nv_ = GV[s];
-        bool kick;
-        if (!EDGE || (gx >= 2 && gy >= 2 && gx < res - 2 && gy < res - 2)) {
-            // No stencil index is clamped.
-            kick = conf_kick_inner(two, dt, vort, SweepRead{FU, PU, GU, s, G::W}, SweepRead{FV, PV, GV, s, G::W}, du,
+        int kick = -1;
+        if (!EDGE || (gx >= 2 && gy >= 2 && gx < res - 2 && gy < res - 2))
+            kick = conf_kick_inner<false>(two, dt, vort, SweepRead{FU, PU, GU, s, G::W}, SweepRead{FV, PV, GV, s, G::W}, du,
                                    dv);
-        } else {
+        if (kick < 0) {
             auto at = [&](int a, int b) { return (b - oy) * G::W + (a - ox); };
             auto before = [&](int a, int b) { return b < gy || (b == gy && a < gx); };
             auto uu = [&](int a, int b) {
@@ -568,7 +579,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
                 if (HS[s] > eps) solve(gx, gy, s);
             }
         } else {
-            region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
+            region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int) {
                 if (it > 0) {
                     if (!mark[s]) return;
                     mark[s] = 0;
@@ -581,7 +592,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
         tile_changed = true;
     }
     if (tile_changed) {
-        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t g) {
+        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             if (HS[s] > eps) {
                 fu[g] = FU[s];
                 fv[g] = FV[s];
@@ -596,9 +607,10 @@ template <class TM, class G, bool EDGE>
 __device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0) {
     const int res = P.res;
     const ForcePlanes<G> F(sm);
+    const int band = tile_band<G>(P, tx0, ty0);
     const float eps = P.eps;
     const float *depth = P.h, *bed = P.bed, *u = P.u, *v = P.v, *fu = P.fu, *fv = P.fv;
-    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int, int, int s, size_t g) {
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int, int, int s, int g) {
         stage(&F.HS[s], depth + g);
         stage(&F.E[s], bed + g);
         stage(&F.U[s], u + g);
@@ -607,7 +619,7 @@ __device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, flo
         stage(&F.TS[s], fv + g);
     });
     staged();
-    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, size_t) {
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, int) {
         const float hv = F.HS[s];
         F.E[s] += hv;
         float uu = F.U[s], vv = F.V[s];
@@ -615,7 +627,7 @@ __device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, flo
             uu = F.TG[s];
             vv = F.TS[s];
         } else {
-            start_velocity(P, gx, gy, hv, uu, vv);
+            start_velocity(P, band, gx, gy, hv, uu, vv);
         }
         F.U[s] = uu;
         F.V[s] = vv;
@@ -851,7 +863,7 @@ __device__ void sweep_serial(const LayerParams& P) {
                 const float hq = P.h[q];
                 if (hq > eps && (b < j || (b == j && a < i))) return is_u ? P.fu[q] : P.fv[q];
                 float uu = P.u[q], vv = P.v[q];
-                start_velocity(P, a, b, hq, uu, vv);
+                start_velocity(P, P.soften_edge, a, b, hq, uu, vv);
                 return is_u ? uu : vv;
             };
             auto uu = [&](int a, int b) { return val(true, a, b); };

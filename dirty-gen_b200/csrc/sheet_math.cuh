@@ -149,22 +149,49 @@ struct SweepRead {
 
 // conf_kick at a cell at least two cells inside the grid, where no stencil
 // index is clamped: the same arithmetic in the same order, reading the nine
-// neighbours through SweepRead's fixed offsets.
-__device__ __forceinline__ bool conf_kick_inner(const FixedDiv& two, float dt, float vort, const SweepRead& uu,
-                                                const SweepRead& vv, float& du, float& dv) {
+// neighbours through SweepRead's fixed offsets. Returns 1 for a kick, 0 for
+// none and -1 when the caller has to ask conf_kick.
+// The twelve divisions take fdiv's product form and are tested together: -1
+// when some operand lies outside the range where that form is known to be
+// exact ([2^-90, 2^90] and zeros). (A test per division: 261 us a launch on a
+// 1501^2 flood, 258 together; 1569 and 1535 on 256 windows.) A zero's sign,
+// which fdiv keeps, is lost: it reaches only the sign of a zero vorticity,
+// which kicks nothing or whose magnitude is taken (the differences of
+// magnitudes that nx and nz divide have positive zeros). Under 0.9e-4 the
+// vorticity kicks nothing whatever its operands: the product form's error
+// outside the range is below 2^-88, and an overflow ends in no kick either way.
+// IEEE: a divisor without the product form divides by IEEE division here; the
+// code for that, unused, costs a full register file (the grid's sweep 258 ->
+// 292 us), which leaves it out and takes -1.
+template <bool IEEE>
+__device__ __forceinline__ int conf_kick_inner(const FixedDiv& two, float dt, float vort, const SweepRead& uu,
+                                               const SweepRead& vv, float& du, float& dv) {
+    constexpr unsigned int LO = 0x12800000u;  // 2^-90
+    unsigned int lo = 0xffffffffu;
+    float hi = 0.0f;
+    auto by_two = [&](float x) {
+        if (IEEE && !two.exact) return x / two.d;
+        lo = min(lo, 2u * __float_as_uint(x) - 1u);  // the sign shifted out; a zero wraps to the top
+        hi = fmaxf(hi, fabsf(x));
+        const float q = x * two.r;
+        return __fmaf_rn(__fmaf_rn(-q, two.d, x), two.r, q);
+    };
     auto vort_of = [&](float vp, float vm, float up, float um) {
-        float dvdx = fdiv(vp - vm, two);
-        float dudz = fdiv(up - um, two);
+        float dvdx = by_two(vp - vm);
+        float dudz = by_two(up - um);
         return dvdx - dudz;
     };
+    if (!IEEE && !two.exact) return -1;
     float w = vort_of(vv.at<1, 0>(), vv.at<-1, 0>(), uu.at<0, 1>(), uu.at<0, -1>());
-    if (!finite_f(w) || fabsf(w) < 1.0e-4f) return false;
+    if (!(fabsf(w) >= 0.9e-4f)) return 0;
     float wxp = fabsf(vort_of(vv.at<2, 0>(), vv.at<0, 0>(), uu.at<1, 1>(), uu.at<1, -1>()));
     float wxm = fabsf(vort_of(vv.at<0, 0>(), vv.at<-2, 0>(), uu.at<-1, 1>(), uu.at<-1, -1>()));
     float wzp = fabsf(vort_of(vv.at<1, 1>(), vv.at<-1, 1>(), uu.at<0, 2>(), uu.at<0, 0>()));
     float wzm = fabsf(vort_of(vv.at<1, -1>(), vv.at<-1, -1>(), uu.at<0, 0>(), uu.at<0, -2>()));
-    float nx = fdiv(wxp - wxm, two);
-    float nz = fdiv(wzp - wzm, two);
+    float nx = by_two(wxp - wxm);
+    float nz = by_two(wzp - wzm);
+    if (lo < 2u * LO - 1u || !(hi <= 0x1p90f)) return -1;
+    if (fabsf(w) < 1.0e-4f) return 0;
     du = vort * dt * (-nz * w);
     dv = vort * dt * (nx * w);
     return finite_f(du) && finite_f(dv) && du * du + dv * dv <= 0.0625f;

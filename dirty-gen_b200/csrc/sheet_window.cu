@@ -736,9 +736,11 @@ __device__ int cta_gravity_gs(Shared& S, const Job& J, const Box& b, const float
                 float nu_ = UG[g], nv_ = VG[g];
                 // Two cells inside the window no stencil index is clamped.
                 const bool inner = i >= 2 && j >= 2 && i + 2 < res && j + 2 < res;
-                if (inner ? conf_kick_inner(two, dt, J.vort, SweepRead{J.u, U0, UG, g, res},
-                                            SweepRead{J.v, V0, VG, g, res}, du, dv)
-                          : conf_kick(i, j, res, two, dt, J.vort, uu, vv, du, dv)) {
+                int kick = inner ? conf_kick_inner<true>(two, dt, J.vort, SweepRead{J.u, U0, UG, g, res},
+                                                         SweepRead{J.v, V0, VG, g, res}, du, dv)
+                                 : -1;
+                if (kick < 0) kick = conf_kick(i, j, res, two, dt, J.vort, uu, vv, du, dv);
+                if (kick) {
                     nu_ = UG[g] + du;
                     nv_ = VG[g] + dv;
                 }
