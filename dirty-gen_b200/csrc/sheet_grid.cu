@@ -244,7 +244,8 @@ struct ForcePlanes {
 // in flight at once: a loop of loads and shared stores waits for each round
 // trip in turn, since the compiler cannot move a load past a store through
 // another pointer. (4-byte copies: rows start at any column.) A 1501^2 flood's
-// sweep launch 305 -> 269 us, k_force on a flooded 1000^2 grid 100 -> 90.
+// sweep launch 305 -> 269 us, k_force on a flooded 1000^2 grid 100 -> 90, the
+// transport there 39 -> 34.
 __device__ __forceinline__ void stage(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -1086,21 +1087,14 @@ __device__ bool tma_stage_transport(const CUtensorMap* maps, float* HSm, float* 
     return true;
 }
 
-// Cells [x0, x0 + W) x [y0, y0 + H) of a transport tile: edge tiles walk
-// clipped rows one warp per row; interior tiles (W, H exact) one flat range
-// of compile-time width, so every lane is busy on the 33-35 wide passes.
+// Cells [x0, x1) x [y0, y1) of a transport tile, at most W x H of them, walked
+// as one flat range of compile-time width so that every lane is busy on the
+// 33-35 wide passes; interior tiles have exactly W x H, edge tiles fewer.
 template <bool EDGE, int W, int H, class F>
 __device__ __forceinline__ void trows(int x0, int x1, int y0, int y1, F f) {
-    if (EDGE) {
-        const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
-        constexpr int NW = TRANSPORT_THREADS / 32;
-        for (int gy = y0 + wy; gy < y1; gy += NW)
-            for (int gx = x0 + lane; gx < x1; gx += 32) f(gx, gy);
-    } else {
-        for (int k = threadIdx.x; k < W * H; k += TRANSPORT_THREADS) {
-            const int r = k / W;
-            f(x0 + (k - r * W), y0 + r);
-        }
+    for (int k = threadIdx.x; k < W * H; k += TRANSPORT_THREADS) {
+        const int r = k / W, gx = x0 + (k - r * W), gy = y0 + r;
+        if (!EDGE || (gx < x1 && gy < y1)) f(gx, gy);
     }
 }
 
@@ -1134,15 +1128,17 @@ __device__ __forceinline__ void transport_tile(const TransportParams& P, float* 
     const bool with_bed = P.bank_bed != nullptr;
     const uint8_t* gate = P.gate;
     // An interior tile of a layer with tensor maps arrives by TMA.
-    const bool staged = !EDGE && maps && ts && !ts->off &&
+    const bool by_tma = !EDGE && maps && ts && !ts->off &&
                         tma_stage_transport(maps, HSm, US, VS, tx0, ty0, *ts, tf.sweep ? &tf.sweep->err : nullptr);
-    if (!staged) {
+    if (!by_tma) {
+        const float *h = P.h, *u = P.u, *v = P.v;
         trows<EDGE, TT + 3, TT + 3>(cx0, cx1, ry0, ry1, [&](int gx, int gy) {
-            size_t g = (size_t)gy * res + gx;
-            HSm[TIDX(gx, gy)] = P.h[g];
-            US[TIDX(gx, gy)] = P.u[g];
-            if (gx >= tx0 && gx < tx1) VS[TIDX(gx, gy)] = P.v[g];
+            const int g = gy * res + gx, s = TIDX(gx, gy);
+            stage(&HSm[s], h + g);
+            stage(&US[s], u + g);
+            if (gx >= tx0 && gx < tx1) stage(&VS[s], v + g);
         });
+        staged();
         __syncthreads();
     }
     // x pass. Edge e joins cells e and e+1 and exists for 0 <= e < res-1.
