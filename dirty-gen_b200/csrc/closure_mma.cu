@@ -3,23 +3,38 @@
 // accumulators in tensor memory), their weight gradient, the loss gradient,
 // Adam and weight packing.
 //
-// Forward / input gradient (k_conv3x3): one CTA of 128 threads per 8 x 16
-// pixel tile (M = 128 rows = pixels). K runs over (tap, input channel): for
-// each of the 9 taps the tile's shifted pixels are copied into shared memory
-// in the K-major no-swizzle core-matrix layout (8 rows x 16 bytes per core
-// matrix), and one elected thread issues 9 x cin/16 MMAs of 128 x cout x 16
-// into one TMEM accumulator; a commit to an mbarrier tells the CTA when the
-// accumulator is complete, and each warp reads its 32 rows back with
-// tcgen05.ld for the epilogue (bias, ReLU or the ReLU-derivative gate,
-// BF16/FP32 store).
+// Both contractions read the input from one shared-memory form: per 8-channel
+// chunk a plane of pixels, 16 bytes each. Eight neighbouring pixels are then
+// one 8 x 16-byte core matrix wherever they start, so a tap's shifted pixels
+// are the same plane at another address and nothing is copied per tap. Tiles
+// are 16 x 8 pixels (M = 128 rows of the forward, K = 128 of the weight
+// gradient): a tile row is one core matrix, and the rows lie a pitch apart.
 //
-// Weight gradient (k_conv3x3_wgrad): M = (tap, input channel) rows (padded to
-// a multiple of 128), N = output channels, K = pixels. Each CTA accumulates
-// its tiles' 128-pixel K slices in TMEM and adds its partial sums to the
-// global gradient once at the end.
+// Forward / input gradient (k_conv3x3): M = pixels, K = (tap, input channel),
+// both operands K-major. One elected thread issues 9 x cin/16 MMAs of
+// 128 x cout x 16 into one TMEM accumulator, each on the plane at its tap's
+// offset; a commit to an mbarrier tells the CTA when the accumulator is
+// complete, and each warp reads its 32 rows back with tcgen05.ld for the
+// epilogue (bias, ReLU or the ReLU-derivative gate, BF16/FP32 store).
+//
+// Weight gradient (k_conv3x3_wgrad): M = (dx, input channel), N = output
+// channels, K = pixels, both operands MN-major (the channels of a pixel are
+// contiguous), so no transposition is staged. The planes are staged once per
+// dx; a dy is a row offset and an accumulator of its own. A plane of ones
+// beside them makes its row of the product the bias gradient.
+//
+// Both are persistent and stage the next tile with cp.async while the tensor
+// core works on the current one. What bounds them is the latency of a tile's
+// loads and stores, covered by several CTAs an SM: the MMAs of 256 crops of
+// 32 x 32 take about 16 us of the tensor cores for a whole training step. With
+// the taps' slices copied (and, for the weights, transposed) tile by tile, one
+// tile at a time, those crops took 55, 34 and 43 us (32 -> 32, 16 -> 32,
+// 32 -> 16 forward) and 164, 122 and 131 us (weights); now 31, 24, 27 and 39,
+// 31, 30, launches included.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 
@@ -41,7 +56,7 @@ int fail(int rc, const char* what) {
 
 namespace {
 
-constexpr int TILE_H = 8, TILE_W = 16, TILE_M = 128;
+constexpr int TILE_H = 16, TILE_W = 8, TILE_M = 128;
 constexpr int THREADS = 128;
 constexpr int WAIT_LIMIT = 1 << 22;  // mbarrier polls before a kernel gives up and flags an error
 
@@ -51,16 +66,25 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 // Shared-memory matrix descriptor, no swizzle: start address, leading byte
 // offset (between the two 8-element K chunks of one MMA), stride byte offset
-// (between 8-row groups), all in 16-byte units; bit 46 = descriptor version 1.
+// (between 8-row groups of M or N), all in 16-byte units; bit 46 = descriptor
+// version 1.
 __device__ __forceinline__ uint64_t mat_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
 
-// kind::f16 instruction descriptor: D FP32, A and B BF16, both K-major, M = 128.
-__host__ __device__ constexpr uint32_t idesc_bf16(int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
+// kind::f16 instruction descriptor: D FP32, A and B BF16, both K-major or both
+// MN-major, M = 128.
+__host__ __device__ constexpr uint32_t idesc_bf16(int n, bool mn_major) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn_major ? 3u << 15 : 0u) | ((uint32_t)(n >> 3) << 17) |
+           ((uint32_t)(TILE_M >> 4) << 24);
 }
+
+// 16 bytes global -> shared without a register; zeros when !in.
+__device__ __forceinline__ void stage16(uint32_t dst, const void* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void staged_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
@@ -135,17 +159,32 @@ struct ConvArgs {
     const uint16_t* gate;
     uint16_t* y;
     float* y32;
-    int n_img, H, W, relu;
+    int n_img, H, W, relu, gate_vec;  // gate_vec: the gate is 16-byte aligned
     int* err;
+};
+
+// The tile's place in the image batch.
+struct Tile {
+    int img, y0, x0;
+    __device__ __forceinline__ Tile(int t, int H, int W) {
+        const int tiles_x = (W + TILE_W - 1) / TILE_W, per_img = tiles_x * ((H + TILE_H - 1) / TILE_H);
+        img = t / per_img;
+        const int r = t - img * per_img, ty = r / tiles_x;
+        y0 = ty * TILE_H;
+        x0 = (r - ty * tiles_x) * TILE_W;
+    }
 };
 
 template <int CIN, int COUT>
 struct ConvShape {
-    static constexpr int TAP_BYTES = TILE_M * CIN * 2;  // one tap's 128 x cin slice of A
-    static constexpr int A_BYTES = 9 * TAP_BYTES;
-    static constexpr int KC = 9 * CIN / 8;              // 8-element K chunks of a weight row
+    static constexpr int CH = CIN / 8;                    // 8-channel chunks
+    static constexpr int PW = TILE_W + 2, PH = TILE_H + 2;  // the tile with its halo
+    static constexpr int PLANE = PW * PH * 16 + 16;       // a chunk's pixels; the pad spreads the chunks over the banks
+    static constexpr int A_BYTES = CH * PLANE;
+    static constexpr int KC = 9 * CH;                     // 8-element K chunks of a weight row
     static constexpr int B_BYTES = COUT * 9 * CIN * 2;
-    static constexpr int SMEM = A_BYTES + B_BYTES;
+    static constexpr int SMEM = B_BYTES + 2 * A_BYTES;
+    static constexpr int CTAS = 4;                        // CTAs per SM
 };
 
 template <int CIN, int COUT>
@@ -154,12 +193,24 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(ConvArgs a) {
     static_assert(CIN % 16 == 0 && COUT % 16 == 0 && COUT <= 32, "shape");
     using S = ConvShape<CIN, COUT>;
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* As = smem;
-    uint8_t* Bs = smem + S::A_BYTES;
+    uint8_t* Bs = smem;
+    const uint32_t As = smem_u32(smem) + S::B_BYTES;
     __shared__ uint64_t bar;
     __shared__ uint32_t tslot;
     __shared__ float bias_s[COUT];
     const int tid = threadIdx.x, warp = tid >> 5;
+    const int ntiles = a.n_img * ((a.W + TILE_W - 1) / TILE_W) * ((a.H + TILE_H - 1) / TILE_H);
+    auto stage_tile = [&](int t, uint32_t buf) {
+        const Tile T(t, a.H, a.W);
+        for (int q = tid; q < S::CH * S::PW * S::PH; q += THREADS) {
+            const int cc = q % S::CH, p = q / S::CH;
+            const int yy = T.y0 + p / S::PW - 1, xx = T.x0 + p % S::PW - 1;
+            const bool in = yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
+            const size_t pix = in ? ((size_t)T.img * a.H + yy) * a.W + xx : 0;
+            stage16(buf + cc * S::PLANE + p * 16, a.x + pix * CIN + cc * 8, in);
+        }
+    };
+    if ((int)blockIdx.x < ntiles) stage_tile(blockIdx.x, As);
     // Weights, row n = output channel, K = tap * CIN + c, in 8-element chunks.
     for (int q = tid; q < COUT * S::KC; q += THREADS) {
         const int n = q / S::KC, kc = q - n * S::KC;
@@ -173,55 +224,60 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(ConvArgs a) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tslot;
-    const int tiles_x = (a.W + TILE_W - 1) / TILE_W, tiles_y = (a.H + TILE_H - 1) / TILE_H;
-    const int per_img = tiles_x * tiles_y, ntiles = a.n_img * per_img;
-    constexpr uint32_t IDESC = idesc_bf16(COUT);
-    uint32_t parity = 0;
+    constexpr uint32_t IDESC = idesc_bf16(COUT, false);
     bool ok = true;
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        const int img = t / per_img, r = t - img * per_img, ty = r / tiles_x, tx = r - ty * tiles_x;
-        const int py = ty * TILE_H + (tid >> 4), px = tx * TILE_W + (tid & 15);  // row m = tid of A and D
-        for (int tap = 0; tap < 9; ++tap) {
-            const int yy = py + tap / 3 - 1, xx = px + tap % 3 - 1;
-            const bool in = yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-            const uint4* src = reinterpret_cast<const uint4*>(a.x + (((size_t)img * a.H + yy) * a.W + xx) * CIN);
-            uint8_t* dst = As + tap * S::TAP_BYTES + (tid >> 3) * (CIN * 16) + (tid & 7) * 16;
-#pragma unroll
-            for (int c = 0; c < CIN / 8; ++c)
-                *reinterpret_cast<uint4*>(dst + c * 128) = in ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-        }
+    int it = 0;
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++it) {
+        const uint32_t buf = As + (it & 1) * S::A_BYTES;
+        // This tile has landed, and every warp has read the last accumulator.
+        staged_wait();
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t a0 = smem_u32(As), b0 = smem_u32(Bs);
+            const uint32_t b0 = smem_u32(Bs);
             uint32_t acc = 0;
             for (int tap = 0; tap < 9; ++tap)
 #pragma unroll
                 for (int s = 0; s < CIN / 16; ++s) {
-                    const uint64_t ad = mat_desc(a0 + tap * S::TAP_BYTES + s * 256, 128, CIN * 16);
-                    const uint64_t bd = mat_desc(b0 + (tap * (CIN / 8) + 2 * s) * 128, 128, S::KC * 128);
+                    const uint32_t at = buf + 2 * s * S::PLANE + ((tap / 3) * S::PW + tap % 3) * 16;
+                    const uint64_t ad = mat_desc(at, S::PLANE, S::PW * 16);
+                    const uint64_t bd = mat_desc(b0 + (tap * S::CH + 2 * s) * 128, 128, S::KC * 128);
                     mma_bf16(tmem, ad, bd, IDESC, acc);
                     acc = 1;
                 }
             mma_commit(&bar);
         }
-        ok = __syncthreads_and(bar_wait(&bar, parity) ? 1 : 0) != 0;  // uniform across the CTA
-        parity ^= 1u;
+        // The other buffer's last reader is the tile before, waited for below.
+        if (t + (int)gridDim.x < ntiles) stage_tile(t + gridDim.x, As + ((it + 1) & 1) * S::A_BYTES);
+        const Tile T(t, a.H, a.W);
+        const int py = T.y0 + (tid >> 3), px = T.x0 + (tid & 7);  // row m = tid of A and D
+        ok = __syncthreads_and(bar_wait(&bar, it & 1) ? 1 : 0) != 0;  // uniform across the CTA
         tc_fence_after();
         float v[COUT];
 #pragma unroll
         for (int c0 = 0; c0 < COUT; c0 += 8) tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v + c0);
         tmem_wait_ld();
         if (ok && py < a.H && px < a.W) {
-            const size_t pix = ((size_t)img * a.H + py) * a.W + px;
-            const uint16_t* g = a.gate ? a.gate + pix * COUT : nullptr;
+            const size_t pix = ((size_t)T.img * a.H + py) * a.W + px;
 #pragma unroll
             for (int c = 0; c < COUT; ++c) {
-                float o = v[c] + bias_s[c];
-                if (a.relu) o = fmaxf(o, 0.0f);
-                if (g && !(from_bf16(g[c]) > 0.0f)) o = 0.0f;
-                v[c] = o;
+                v[c] += bias_s[c];
+                if (a.relu) v[c] = fmaxf(v[c], 0.0f);
+            }
+            if (a.gate) {
+                const uint16_t* g = a.gate + pix * COUT;
+#pragma unroll
+                for (int c = 0; c < COUT; c += 8) {
+                    uint16_t gv[8];
+                    if (a.gate_vec)
+                        *reinterpret_cast<uint4*>(gv) = *reinterpret_cast<const uint4*>(g + c);
+                    else
+                        for (int k = 0; k < 8; ++k) gv[k] = g[c + k];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if (!(from_bf16(gv[k]) > 0.0f)) v[c + k] = 0.0f;
+                }
             }
             if (a.y32) {
                 float4* d = reinterpret_cast<float4*>(a.y32 + pix * COUT);
@@ -242,9 +298,9 @@ __global__ void __launch_bounds__(THREADS) k_conv3x3(ConvArgs a) {
             }
         }
         tc_fence_before();
-        __syncthreads();
     }
     if (!ok && tid == 0 && a.err) atomicExch(a.err, 1);
+    staged_wait();
     __syncthreads();
     tc_fence_after();
     if (warp == 0) tmem_free(tmem, 32);
@@ -255,150 +311,140 @@ struct WgradArgs {
     const uint16_t* dy;
     float* dw;
     float* db;
-    int n_img, H, W;
+    int n_img, H, W, dw_vec;  // dw_vec: dw is 16-byte aligned
     int* err;
 };
 
 template <int CIN, int COUT>
 struct WgradShape {
-    static constexpr int ROWS = 9 * CIN;                    // (tap, cin)
-    static constexpr int MT = (ROWS + TILE_M - 1) / TILE_M;  // 128-row M tiles
-    static constexpr int SBO = (TILE_M / 8) * 128;           // 16 pixel chunks per row group
-    static constexpr int A_BYTES = MT * TILE_M * TILE_M * 2;
-    static constexpr int B_BYTES = COUT * TILE_M * 2;
-    static constexpr int SMEM = A_BYTES + B_BYTES;
-    static constexpr int COLS = MT * COUT <= 32 ? 32 : (MT * COUT <= 64 ? 64 : 128);
+    static constexpr int CH = CIN / 8, OH = COUT / 8;       // 8-channel chunks of x and of dy
+    static constexpr int PH = TILE_H + 2;
+    static constexpr int A_PLANE = PH * TILE_W * 16 + 32;   // (dx, chunk): the tile's columns shifted by dx, with the
+    static constexpr int B_PLANE = TILE_M * 16 + 32;        // rows' halo; the pads spread the chunks over the banks
+    static constexpr int ONES = 3 * CH;                     // the plane of ones
+    static constexpr int B_AT = (ONES + 1) * A_PLANE;
+    // M = 128 reads 16 planes; those past the ones give rows nobody uses.
+    static constexpr int BUF0 = B_AT + OH * B_PLANE, BUF1 = 16 * A_PLANE;
+    static constexpr int BUF = BUF0 > BUF1 ? BUF0 : BUF1;
+    static constexpr int SMEM = 2 * BUF;
+    static constexpr int COLS = 3 * COUT <= 64 ? 64 : 128;  // one accumulator per dy
 };
+constexpr int WG_THREADS = 256;
 
-// Eight pixels' 8-channel vectors (v[j] = pixel j) -> eight channels'
-// 8-pixel vectors (out[r] = channel r), BF16 lanes.
-__device__ __forceinline__ void transpose8(const uint4 (&v)[8], uint4 (&out)[8]) {
-    uint16_t e[8][8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            e[j][2 * q] = (uint16_t)(w[q] & 0xFFFFu);
-            e[j][2 * q + 1] = (uint16_t)(w[q] >> 16);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        out[r].x = (uint32_t)e[0][r] | ((uint32_t)e[1][r] << 16);
-        out[r].y = (uint32_t)e[2][r] | ((uint32_t)e[3][r] << 16);
-        out[r].z = (uint32_t)e[4][r] | ((uint32_t)e[5][r] << 16);
-        out[r].w = (uint32_t)e[6][r] | ((uint32_t)e[7][r] << 16);
-    }
+__device__ __forceinline__ void red_add4(float* d, float x, float y, float z, float w) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(THREADS) k_conv3x3_wgrad(WgradArgs a) {
+__global__ void __launch_bounds__(WG_THREADS) k_conv3x3_wgrad(WgradArgs a) {
     ::silt::dep_wait();
     using S = WgradShape<CIN, COUT>;
+    static_assert(S::ONES < 16 && S::BUF % 16 == 0, "planes of one M = 128 operand");
     extern __shared__ __align__(128) uint8_t smem[];
-    uint8_t* As = smem;
-    uint8_t* Bs = smem + S::A_BYTES;
-    __shared__ uint64_t bar;
+    const uint32_t base = smem_u32(smem);
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t tslot;
     const int tid = threadIdx.x, warp = tid >> 5;
-    // Rows past 9 * CIN are zero for the whole kernel.
-    for (int q = S::ROWS * 16 + tid; q < S::MT * TILE_M * 16; q += THREADS)
-        *reinterpret_cast<uint4*>(As + (q / 16 >> 3) * S::SBO + (q % 16) * 128 + (q / 16 & 7) * 16) =
-            make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) bar_init(&bar, 1);
+    const int ntiles = a.n_img * ((a.W + TILE_W - 1) / TILE_W) * ((a.H + TILE_H - 1) / TILE_H);
+    auto stage_tile = [&](int t, uint32_t buf) {
+        const Tile T(t, a.H, a.W);
+        // x, per dx the tile's columns shifted by dx - 1, rows from one above.
+        for (int q = tid; q < 3 * S::PH * TILE_W * S::CH; q += WG_THREADS) {
+            const int cc = q % S::CH, p = q / S::CH, px = p % TILE_W, r = p / TILE_W;
+            const int dx = r / S::PH, py = r - dx * S::PH;
+            const int yy = T.y0 + py - 1, xx = T.x0 + px + dx - 1;
+            const bool in = yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
+            const size_t pix = in ? ((size_t)T.img * a.H + yy) * a.W + xx : 0;
+            stage16(buf + (dx * S::CH + cc) * S::A_PLANE + (py * TILE_W + px) * 16, a.x + pix * CIN + cc * 8, in);
+        }
+        // dy; pixels outside the image give 0.
+        for (int q = tid; q < TILE_M * S::OH; q += WG_THREADS) {
+            const int oc = q % S::OH, p = q / S::OH;
+            const int yy = T.y0 + p / TILE_W, xx = T.x0 + p % TILE_W;
+            const bool in = yy < a.H && xx < a.W;
+            const size_t pix = in ? ((size_t)T.img * a.H + yy) * a.W + xx : 0;
+            stage16(buf + S::B_AT + oc * S::B_PLANE + p * 16, a.dy + pix * COUT + oc * 8, in);
+        }
+    };
+    if ((int)blockIdx.x < ntiles) stage_tile(blockIdx.x, base);
+    for (int q = tid; q < 2 * (S::A_PLANE / 4); q += WG_THREADS) {
+        const int b = q / (S::A_PLANE / 4), k = q - b * (S::A_PLANE / 4);
+        *reinterpret_cast<uint32_t*>(smem + b * S::BUF + S::ONES * S::A_PLANE + k * 4) = 0x3F803F80u;  // BF16 1, 1
+    }
+    if (tid == 0) {
+        bar_init(&bar[0], 1);
+        bar_init(&bar[1], 1);
+    }
     if (warp == 0) tmem_alloc(&tslot, S::COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tslot;
-    const int tiles_x = (a.W + TILE_W - 1) / TILE_W, tiles_y = (a.H + TILE_H - 1) / TILE_H;
-    const int per_img = tiles_x * tiles_y, ntiles = a.n_img * per_img;
-    constexpr uint32_t IDESC = idesc_bf16(COUT);
-    constexpr int B_ITEMS = (COUT / 8) * 16;  // (channel chunk, pixel chunk)
-    float bsum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint32_t parity = 0;
-    bool ok = true, any = false;
-    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        const int img = t / per_img, r = t - img * per_img, ty = r / tiles_x, tx = r - ty * tiles_x;
-        // A: row (tap, cin), K = the tile's 128 pixels (pixel m at (m / 16, m % 16)).
-        for (int q = tid; q < 9 * (CIN / 8) * 16; q += THREADS) {
-            const int pc = q & 15, cc = (q >> 4) % (CIN / 8), tap = (q >> 4) / (CIN / 8);
-            uint4 v[8], o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int m = pc * 8 + j;
-                const int yy = ty * TILE_H + (m >> 4) + tap / 3 - 1, xx = tx * TILE_W + (m & 15) + tap % 3 - 1;
-                const bool in = yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-                v[j] = in ? *reinterpret_cast<const uint4*>(a.x + (((size_t)img * a.H + yy) * a.W + xx) * CIN + cc * 8)
-                          : make_uint4(0u, 0u, 0u, 0u);
-            }
-            transpose8(v, o);
-            uint8_t* dst = As + (tap * (CIN / 8) + cc) * S::SBO + pc * 128;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4*>(dst + k * 16) = o[k];
-        }
-        // B: row = output channel, K = pixels; pixels outside the image give 0.
-        if (tid < B_ITEMS) {
-            const int pc = tid & 15, cc = tid >> 4;
-            uint4 v[8], o[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int m = pc * 8 + j;
-                const int yy = ty * TILE_H + (m >> 4), xx = tx * TILE_W + (m & 15);
-                const bool in = yy < a.H && xx < a.W;
-                v[j] = in ? *reinterpret_cast<const uint4*>(a.dy + (((size_t)img * a.H + yy) * a.W + xx) * COUT + cc * 8)
-                          : make_uint4(0u, 0u, 0u, 0u);
-            }
-            transpose8(v, o);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                *reinterpret_cast<uint4*>(Bs + cc * S::SBO + pc * 128 + k * 16) = o[k];
-                const uint32_t w[4] = {o[k].x, o[k].y, o[k].z, o[k].w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    bsum[k] += from_bf16((uint16_t)(w[q] & 0xFFFFu)) + from_bf16((uint16_t)(w[q] >> 16));
-            }
-        }
+    constexpr uint32_t IDESC = idesc_bf16(COUT, true);
+    bool ok = true;
+    int it = 0;
+    // Tile `k` of this CTA is done: its MMAs have read their buffer.
+    auto done = [&](int k) { return __syncthreads_and(bar_wait(&bar[k & 1], (uint32_t)(k >> 1) & 1u) ? 1 : 0) != 0; };
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++it) {
+        const uint32_t buf = base + (it & 1) * S::BUF;
+        staged_wait();
         fence_async_smem();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t a0 = smem_u32(As), b0 = smem_u32(Bs);
 #pragma unroll
-            for (int mt = 0; mt < S::MT; ++mt)
+            for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
                 for (int s = 0; s < TILE_M / 16; ++s) {
-                    const uint64_t ad = mat_desc(a0 + mt * (TILE_M / 8) * S::SBO + s * 256, 128, S::SBO);
-                    const uint64_t bd = mat_desc(b0 + s * 256, 128, S::SBO);
-                    mma_bf16(tmem + (uint32_t)(mt * COUT), ad, bd, IDESC, (any || s > 0) ? 1u : 0u);
+                    const uint64_t ad = mat_desc(buf + (dy + 2 * s) * (TILE_W * 16), TILE_W * 16, S::A_PLANE);
+                    const uint64_t bd = mat_desc(buf + S::B_AT + s * 256, TILE_W * 16, S::B_PLANE);
+                    mma_bf16(tmem + (uint32_t)(dy * COUT), ad, bd, IDESC, (it > 0 || s > 0) ? 1u : 0u);
                 }
-            mma_commit(&bar);
+            mma_commit(&bar[it & 1]);
         }
-        any = true;
-        // Uniform across the CTA; the shared operands are rewritten by the next tile.
-        ok = __syncthreads_and(bar_wait(&bar, parity) ? 1 : 0) != 0;
-        parity ^= 1u;
-        tc_fence_after();
+        if (t + (int)gridDim.x < ntiles) {
+            if (it > 0 && !(ok = done(it - 1))) {
+                ++it;
+                break;
+            }
+            stage_tile(t + gridDim.x, base + ((it + 1) & 1) * S::BUF);
+        }
     }
-    if (ok && any) {
+    if (it > 0) ok = done(it - 1) && ok;
+    tc_fence_after();
+    if (ok && it > 0 && warp < 4) {
+        // Row m = (dx, input channel), or the ones' row.
+        const int j = tid >> 3, dx = j / S::CH, c = (j - dx * S::CH) * 8 + (tid & 7);
 #pragma unroll
-        for (int mt = 0; mt < S::MT; ++mt) {
+        for (int dy = 0; dy < 3; ++dy) {
             float v[COUT];
 #pragma unroll
             for (int c0 = 0; c0 < COUT; c0 += 8)
-                tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mt * COUT + c0), v + c0);
+                tmem_ld8(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dy * COUT + c0), v + c0);
             tmem_wait_ld();
-            const int row = mt * TILE_M + tid;
-            if (row < S::ROWS)
+            float* row = nullptr;
+            bool vec = false;
+            if (j < S::ONES) {
+                row = a.dw + ((size_t)(dy * 3 + dx) * CIN + c) * COUT;
+                vec = a.dw_vec;
+            } else if (dy == 0 && tid == 8 * S::ONES) {
+                row = a.db;
+            }
+            if (row) {
 #pragma unroll
-                for (int c = 0; c < COUT; ++c) atomicAdd(a.dw + (size_t)row * COUT + c, v[c]);
+                for (int k = 0; k < COUT; k += 4) {
+                    if (vec) {
+                        red_add4(row + k, v[k], v[k + 1], v[k + 2], v[k + 3]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) atomicAdd(row + k + q, v[k + q]);
+                    }
+                }
+            }
         }
-        if (tid < B_ITEMS && a.db)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) atomicAdd(a.db + (tid >> 4) * 8 + k, bsum[k]);
     }
     if (!ok && tid == 0 && a.err) atomicExch(a.err, 1);
+    staged_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -433,6 +479,9 @@ __global__ void k_loss_grad(const float* y, const float* t, const float* wgt, ui
 }
 
 // One crop per block, one cell per thread (the crop edge has no outgoing face).
+// VEC: y, t and dy are 16-byte aligned, and a cell's values move as float4s
+// (33 MB for 256 crops: 39 us by scalars, 13 so, launch included).
+template <bool VEC>
 __global__ void __launch_bounds__(SILT_CLOSURE_CROP * SILT_CLOSURE_CROP)
     k_step_loss(const float* y, const float* t, const float* scale, const float* inv_var, float lam, uint16_t* dy,
                 double* loss, float norm) {
@@ -445,12 +494,22 @@ __global__ void __launch_bounds__(SILT_CLOSURE_CROP * SILT_CLOSURE_CROP)
     const size_t pix = (size_t)blockIdx.x * NC + p;
     const float* yo = y + pix * CO;
     const float* to = t + pix * NT;
-    float yv[8], sc[8];
+    float yv[8], tv[8], sc[8];
+    if constexpr (VEC) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        yv[c] = yo[c];
-        sc[c] = scale[c];
+        for (int c = 0; c < 8; c += 4) {
+            *reinterpret_cast<float4*>(yv + c) = *reinterpret_cast<const float4*>(yo + c);
+            *reinterpret_cast<float4*>(tv + c) = *reinterpret_cast<const float4*>(to + c);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            yv[c] = yo[c];
+            tv[c] = to[c];
+        }
     }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) sc[c] = scale[c];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const bool edge = (c % 2 == 0) ? cx == N - 1 : cy == N - 1;
@@ -462,22 +521,22 @@ __global__ void __launch_bounds__(SILT_CLOSURE_CROP * SILT_CLOSURE_CROP)
     for (int l = 0; l < 2; ++l) {
         const float in = (cx > 0 ? g[2 * l][p - 1] : 0.0f) + (cy > 0 ? g[2 * l + 1][p - N] : 0.0f);
         const float div = in - g[2 * l][p] - g[2 * l + 1][p];
-        const float r = div - to[l];
+        const float r = div - tv[l];
         e[l][p] = r;
         part += (double)(inv_var[l] * r * r);
     }
     float gv[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float w = to[6 + k / 2];
-        const float r = yv[4 + k] * sc[4 + k] - to[2 + k];
+        const float w = tv[6 + k / 2];
+        const float r = yv[4 + k] * sc[4 + k] - tv[2 + k];
         part += (double)(inv_var[2 + k] * w * r * r);
         gv[k] = 2.0f * inv_var[2 + k] * w * r * sc[4 + k];
     }
 #pragma unroll
     for (int c = 0; c < 8; ++c) part += (double)(lam * yv[c] * yv[c]);
     __syncthreads();
-    uint16_t* out = dy + pix * CO;
+    __align__(16) uint16_t out[CO];
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
         const float gx = cx < N - 1 ? 2.0f * inv_var[l] * (e[l][p + 1] - e[l][p]) : 0.0f;
@@ -489,6 +548,14 @@ __global__ void __launch_bounds__(SILT_CLOSURE_CROP * SILT_CLOSURE_CROP)
     for (int k = 0; k < 4; ++k) out[4 + k] = to_bf16((gv[k] + 2.0f * lam * yv[4 + k]) * norm);
 #pragma unroll
     for (int c = 8; c < CO; ++c) out[c] = 0;
+    uint16_t* const d = dy + pix * CO;
+    if constexpr (VEC) {
+#pragma unroll
+        for (int c = 0; c < CO; c += 8) *reinterpret_cast<uint4*>(d + c) = *reinterpret_cast<const uint4*>(out + c);
+    } else {
+#pragma unroll
+        for (int c = 0; c < CO; ++c) d[c] = out[c];
+    }
     for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
     if ((p & 31) == 0) red[p >> 5] = part;
     __syncthreads();
@@ -557,7 +624,7 @@ cudaError_t conv_launch(const ConvArgs& a, cudaStream_t st) {
     static cudaError_t attr = set_smem(k_conv3x3<CIN, COUT>, S::SMEM);
     if (attr != cudaSuccess) return attr;
     const int tiles = a.n_img * ((a.H + TILE_H - 1) / TILE_H) * ((a.W + TILE_W - 1) / TILE_W);
-    const int grid = tiles < 2 * sm_count() ? tiles : 2 * sm_count();
+    const int grid = std::min(tiles, S::CTAS * sm_count());
     ::silt::launch_dep(k_conv3x3<CIN, COUT>, dim3(grid), dim3(THREADS), S::SMEM, st, a);
     ::silt::count_launch();
     return cudaGetLastError();
@@ -569,8 +636,8 @@ cudaError_t wgrad_launch(const WgradArgs& a, cudaStream_t st) {
     static cudaError_t attr = set_smem(k_conv3x3_wgrad<CIN, COUT>, S::SMEM);
     if (attr != cudaSuccess) return attr;
     const int tiles = a.n_img * ((a.H + TILE_H - 1) / TILE_H) * ((a.W + TILE_W - 1) / TILE_W);
-    const int grid = tiles < sm_count() ? tiles : sm_count();
-    ::silt::launch_dep(k_conv3x3_wgrad<CIN, COUT>, dim3(grid), dim3(THREADS), S::SMEM, st, a);
+    const int grid = std::min(tiles, 2 * sm_count());  // two CTAs an SM by shared memory
+    ::silt::launch_dep(k_conv3x3_wgrad<CIN, COUT>, dim3(grid), dim3(WG_THREADS), S::SMEM, st, a);
     ::silt::count_launch();
     return cudaGetLastError();
 }
@@ -585,7 +652,7 @@ int* err_slot() {
 
 cudaError_t conv3x3(const uint16_t* x, const uint16_t* w, const float* bias, const uint16_t* gate, uint16_t* y,
                     float* y32, int n_img, int h, int wd, int cin, int cout, int relu, cudaStream_t st) {
-    ConvArgs a{x, w, bias, gate, y, y32, n_img, h, wd, relu, err_slot()};
+    ConvArgs a{x, w, bias, gate, y, y32, n_img, h, wd, relu, ((uintptr_t)gate & 15u) == 0, err_slot()};
     if (n_img <= 0 || h <= 0 || wd <= 0) return cudaSuccess;
     if (cin == 16 && cout == 32) return conv_launch<16, 32>(a, st);
     if (cin == 32 && cout == 32) return conv_launch<32, 32>(a, st);
@@ -596,7 +663,7 @@ cudaError_t conv3x3(const uint16_t* x, const uint16_t* w, const float* bias, con
 
 cudaError_t conv3x3_wgrad(const uint16_t* x, const uint16_t* dy, float* dw, float* db, int n_img, int h, int wd,
                           int cin, int cout, cudaStream_t st) {
-    WgradArgs a{x, dy, dw, db, n_img, h, wd, err_slot()};
+    WgradArgs a{x, dy, dw, db, n_img, h, wd, ((uintptr_t)dw & 15u) == 0, err_slot()};
     if (n_img <= 0 || h <= 0 || wd <= 0) return cudaSuccess;
     if (cin == 16 && cout == 32) return wgrad_launch<16, 32>(a, st);
     if (cin == 32 && cout == 32) return wgrad_launch<32, 32>(a, st);
@@ -675,7 +742,8 @@ int silt_closure_step_loss_grad(const float* y, const float* t, const float* sca
     if (!y || !t || !scale || !inv_var || !dy || n_img < 0)
         return fail(SILT_EINVAL, "invalid argument: closure_step_loss_grad");
     if (n_img == 0) return SILT_OK;
-    ::silt::launch_dep(k_step_loss, dim3(n_img), dim3(SILT_CLOSURE_CROP * SILT_CLOSURE_CROP), 0, (cudaStream_t)stream, 
+    const bool vec = aligned16(y) && aligned16(t) && aligned16(dy);
+    ::silt::launch_dep(vec ? k_step_loss<true> : k_step_loss<false>, dim3(n_img), dim3(SILT_CLOSURE_CROP * SILT_CLOSURE_CROP), 0, (cudaStream_t)stream, 
         y, t, scale, inv_var, lambda, (uint16_t*)dy, loss, norm);
     ::silt::count_launch();
     return cuda_rc(cudaGetLastError(), "closure_step_loss_grad");

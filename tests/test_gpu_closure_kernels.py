@@ -164,3 +164,40 @@ def test_bounded_wait_gives_up_and_reports_without_a_fault():
     ok, err = close(y32, ref_conv(x.float(), w32), 1e-4)
     assert ok, err
     assert C.wait_status() == 0
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 32), (32, 32), (32, 16)])
+@pytest.mark.parametrize("n,h,w", [(1, 1, 1), (1, 16, 8), (1, 17, 9), (2, 15, 7), (1, 3, 40), (5, 33, 31), (23, 32, 32)])
+def test_convolutions_at_tile_edges(cin, cout, n, h, w):
+    """Images of one pixel, of whole 16 x 8 tiles, of one more and one less,
+    flat ones, and more tiles than CTAs hold at once are all of one kind: the
+    forward, the gated form (gate at an odd 2-byte offset as well), and both
+    gradients against FP32 references of the same BF16 operands. The sums have
+    at most 9 * 32 (forward) and n * h * w (weights) BF16 products in FP32:
+    1e-4 of the output scale, BF16 stores 2^-7."""
+    x, dy = rand_bf16((n, h, w, cin), seed=21), rand_bf16((n, h, w, cout), seed=22)
+    w32 = rand_bf16((9, cin, cout), 0.2, seed=23).float().contiguous()
+    b = torch.randn(cout, device="cuda") * 0.1
+    fwd = torch.empty((cout, 9, cin), dtype=torch.bfloat16, device="cuda")
+    C.pack(w32, cin, cout, fwd=fwd)
+    flat = rand_bf16((n * h * w * cout + 1,), seed=24)
+    for gate in (flat[:-1].clone(), flat[1:]):
+        y, y32 = C.conv3x3(x, fwd, b, gate=gate.view(n, h, w, cout), want_f32=True)
+        ref = ref_conv(x.float(), w32, b) * (gate.view(n, h, w, cout).float() > 0)
+        ok, err = close(y32, ref, 1e-4)
+        assert ok, err
+        ok, err = close(y.float(), ref, 2.0 ** -7)
+        assert ok, err
+    room = torch.zeros(9 * cin * cout + 1, device="cuda")
+    for dw in (room[:-1].clone(), room[1:]):  # 16-byte aligned, and not
+        dw.zero_()
+        db = torch.zeros(cout, device="cuda")
+        C.wgrad(x, dy, dw.view(9, cin, cout), db)
+        wr = torch.zeros((9, cin, cout), device="cuda", requires_grad=True)
+        br = torch.zeros(cout, device="cuda", requires_grad=True)
+        ref_conv(x.float(), wr, br).backward(dy.float())
+        ok, err = close(dw.view(9, cin, cout), wr.grad, 1e-4)
+        assert ok, err
+        ok, err = close(db, br.grad, 1e-4)
+        assert ok, err
+    assert C.wait_status() == 0
