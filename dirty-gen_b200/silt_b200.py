@@ -208,6 +208,10 @@ TIRE_DTYPE = np.dtype([("x", np.float32), ("z", np.float32), ("forward_x", np.fl
                        ("radius", np.float32), ("width", np.float32), ("speed", np.float32), ("slip", np.float32)])
 
 
+# A spray event as a numpy record (the layout of silt_spray_event).
+SPRAY_DTYPE = np.dtype([(k, np.float32) for k in ("x", "y", "z", "vx", "vy", "vz", "volume")] + [("kind", np.int32)])
+
+
 def make_push(t):
     return TirePush(t["x"], t["z"], t.get("forward_x", 0.0), t.get("forward_z", 1.0), t["radius"], t["width"],
                     t["speed"], t.get("slip", 0.0))
@@ -299,7 +303,10 @@ class Sheet:
         n = _i(0)
         buf = self._spray_buf
         check(lib().silt_step(self.h, dt, buf, cap, ctypes.byref(n)), "step")
-        return [(e.x, e.y, e.z, e.vx, e.vy, e.vz, e.volume, e.kind) for e in buf[:min(n.value, cap)]]
+        # numpy makes the list of tuples: a vehicle's spray is hundreds of events a
+        # step, and eight attribute reads each took longer than the step.
+        k = min(n.value, cap)
+        return np.frombuffer(buf, SPRAY_DTYPE, k).tolist() if k > 0 else []
 
     def ledger(self):
         led = Ledger()
