@@ -36,6 +36,9 @@ constexpr int SLEEP_TILE = 8;      // src/fluid_core.rs:1528
 constexpr int MAX_TILES = (MAX_RES / SLEEP_TILE) * (MAX_RES / SLEEP_TILE);
 constexpr int MAX_BOXES = 512;
 constexpr int GS_MAX_PASSES = 256;
+constexpr int MAX_CREW = 16;       // CTAs of a crew: the non-portable cluster size B200 allows
+constexpr int MAX_RUNS = MAX_TILES;  // wet runs rank 0 labels in its shared memory (S.lab)
+static_assert(MAX_RES <= NT, "one thread takes a row");
 
 struct Box {
     int i0, i1, j0, j1;
@@ -55,11 +58,17 @@ struct Shared {
     int lchg[3];     // wet-body label rounds' verdicts, rotating the same way
     float red_f[NT / 32];
     double red_d[NT / 32];
-    double crew_d;   // this CTA's share of a crew-wide sum or maximum, read by the crew
-    int crew_ext[5]; // this CTA's share of the wet extent: count, i0, -i1, j0, j1
-    float crew_f;
-    int red_i[4][NT / 32];
+    double crew_d[MAX_CREW];  // on rank 0: every CTA's share of the ledger's sum
+    float crew_f;    // this CTA's share of the crew's largest speed
+    int ext[5];      // on rank 0: the wet extent (wet cells, i0, -i1, j0, j1)
+    int by_cells;    // on rank 0: more runs than the tables hold, label by cells
+    int scan[NT / 32];
 };
+
+// The wet cells of the window, one bit each, rows of wet_words(res) words: on
+// rank 0, written by the whole crew.
+extern __shared__ unsigned int wet_bits[];
+__host__ __device__ constexpr int wet_words(int res) { return (res + 31) / 32; }
 
 // Every cell of the inclusive rectangle, one warp per row and the lanes along
 // x (no division per cell). Bodies may `continue` to the next cell.
@@ -159,82 +168,34 @@ __device__ __forceinline__ T crew_fold(const T* mine, T init, F combine) {
     return acc;
 }
 
-// A crew-wide sum of per-thread partials: each CTA reduces its own, then every
-// CTA adds the CTAs' results in rank order (the same value in every CTA).
-__device__ double crew_sum_d(Shared& S, double v) {
-    const double part = block_sum_d(S, v);
-    if (threadIdx.x == 0) S.crew_d = part;
-    crew_sync();
-    const double tot = crew_fold(&S.crew_d, 0.0, [](double a, double b) { return a + b; });
-    crew_sync();  // every CTA has read the shares before they are reused
-    return tot;
-}
-
-// A crew-wide maximum of non-negative per-thread values.
+// A crew-wide maximum of non-negative per-thread values, once per step (its
+// slot is not written again, so no barrier follows the read).
 __device__ float crew_max_f(Shared& S, float v) {
     const float part = block_max_f(S, v);
     if (threadIdx.x == 0) S.crew_f = part;
     crew_sync();
-    const float m = crew_fold(&S.crew_f, 0.0f, [](float a, float b) { return fmaxf(a, b); });
-    crew_sync();
-    return m;
+    return crew_fold(&S.crew_f, 0.0f, [](float a, float b) { return fmaxf(a, b); });
 }
 
-// Four ints reduced together: op 0 = sum, 1 = min, 2 = max.
-__device__ void block_reduce4(Shared& S, int v[4], const int op[4]) {
-    for (int q = 0; q < 4; ++q)
-        for (int o = 16; o > 0; o >>= 1) {
-            int w = __shfl_down_sync(0xffffffffu, v[q], o);
-            v[q] = op[q] == 0 ? v[q] + w : (op[q] == 1 ? min(v[q], w) : max(v[q], w));
-        }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0)
-        for (int q = 0; q < 4; ++q) S.red_i[q][threadIdx.x >> 5] = v[q];
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        for (int q = 0; q < 4; ++q) {
-            const int ident = op[q] == 0 ? 0 : (op[q] == 1 ? 0x7fffffff : (int)0x80000000);
-            int t = threadIdx.x < NT / 32 ? S.red_i[q][threadIdx.x] : ident;
-            for (int o = 16; o > 0; o >>= 1) {
-                int w = __shfl_down_sync(0xffffffffu, t, o);
-                t = op[q] == 0 ? t + w : (op[q] == 1 ? min(t, w) : max(t, w));
-            }
-            if (threadIdx.x == 0) S.red_i[q][0] = t;
-        }
+// Exclusive prefix sum of one int per thread over the CTA; *total gets the sum.
+__device__ int block_scan(Shared& S, int v, int* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
     __syncthreads();
-    for (int q = 0; q < 4; ++q) v[q] = S.red_i[q][0];
+    if (lane == 31) S.scan[warp] = x;
     __syncthreads();
-}
-
-// The crew-wide wet sum and wet extent of one pass: ws summed as crew_sum_d
-// does; ext = {wet cells, min i, -max i, min j, max j} over the crew, in the
-// same barriers.
-__device__ double crew_sum_extent(Shared& S, double v, int ext[5]) {
-    const double part = block_sum_d(S, v);
-    int a[4] = {ext[0], ext[1], ext[2], ext[3]};
-    const int op[4] = {0, 1, 1, 1};
-    block_reduce4(S, a, op);
-    int b[4] = {ext[4], 0, 0, 0};
-    const int op2[4] = {2, 2, 2, 2};
-    block_reduce4(S, b, op2);
-    if (threadIdx.x == 0) {
-        S.crew_d = part;
-        for (int q = 0; q < 4; ++q) S.crew_ext[q] = a[q];
-        S.crew_ext[4] = b[0];
+    int base = 0, all = 0;
+    for (int w = 0; w < NT / 32; ++w) {
+        if (w < warp) base += S.scan[w];
+        all += S.scan[w];
     }
-    crew_sync();
-    const double tot = crew_fold(&S.crew_d, 0.0, [](double a, double b) { return a + b; });
-    auto mn = [](int a, int b) { return min(a, b); };
-    ext[0] = crew_fold(&S.crew_ext[0], 0, [](int a, int b) { return a + b; });
-    ext[1] = crew_fold(&S.crew_ext[1], 0x7fffffff, mn);
-    ext[2] = crew_fold(&S.crew_ext[2], 0x7fffffff, mn);
-    ext[3] = crew_fold(&S.crew_ext[3], 0x7fffffff, mn);
-    ext[4] = crew_fold(&S.crew_ext[4], -1, [](int a, int b) { return max(a, b); });
-    crew_sync();  // every CTA has read the shares before they are reused
-    return tot;
+    *total = all;
+    return base + x - v;
 }
-
 
 // Five taps along one axis, clamped at the grid edge. Cells at least 2 from
 // the edge start from the first product (accum5), others from 0.0
@@ -998,19 +959,23 @@ __device__ void cta_awake_boxes(Shared& S, const Job& J) {
         if (!S.changed) break;
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        int nb = 0;
-        for (int t = 0; t < ntile; ++t)
-            if (S.grown[t] && S.lab[t] == t && nb < MAX_BOXES) {
-                S.bbox[0][nb] = t % tiles;
-                S.bbox[1][nb] = t % tiles;
-                S.bbox[2][nb] = t / tiles;
-                S.bbox[3][nb] = t / tiles;
-                S.lab[t] = -(nb + 1);
-                ++nb;
-            }
-        S.nbox = nb;
+    // Roots numbered in raster order: a block scan over NT tiles at a time.
+    int nroots = 0;
+    for (int t0 = 0; t0 < ntile; t0 += NT) {
+        const int t = t0 + (int)threadIdx.x;
+        const bool root = t < ntile && S.grown[t] && S.lab[t] == t;
+        int found = 0;
+        const int nb = nroots + block_scan(S, root ? 1 : 0, &found);
+        if (root && nb < MAX_BOXES) {
+            S.bbox[0][nb] = t % tiles;
+            S.bbox[1][nb] = t % tiles;
+            S.bbox[2][nb] = t / tiles;
+            S.bbox[3][nb] = t / tiles;
+            S.lab[t] = -(nb + 1);
+        }
+        nroots += found;
     }
+    if (threadIdx.x == 0) S.nbox = min(nroots, MAX_BOXES);
     __syncthreads();
     for (int t = threadIdx.x; t < ntile; t += NT) {
         if (!S.grown[t]) continue;
@@ -1051,10 +1016,232 @@ __device__ void set_whole(Shared& S, int x0, int x1, int y0, int y1) {
     __syncthreads();
 }
 
-// sheet_work_boxes (src/fluid_core.rs:1325-1447). Wet bodies are labelled in
-// the f2 plane (as ints) by hooking and pointer jumping; a body's root is its
-// first wet cell in raster order, the order the reference's run merge keeps.
-// The wet-body labels of sheet_work_boxes (src/fluid_core.rs:1378-1457) over
+// The bodies' boxes (S.bbox, in body order) grown by 6 and merged
+// (src/fluid_core.rs:1459-1487, swap_remove order); one box, or more than 8,
+// become the whole wet box [x0, x1] x [y0, y1]. The first warp: the lanes test
+// 32 boxes at a time against box a, the first that touches is merged, and the
+// search goes on from its place with the grown box, as a loop over c does.
+__device__ void merge_bodies(Shared& S, int nbodies, int x0, int x1, int y0, int y1, int res) {
+    for (int k = threadIdx.x; k < nbodies; k += NT) {
+        S.bbox[0][k] = max(S.bbox[0][k] - 6, 0);
+        S.bbox[1][k] = min(S.bbox[1][k] + 6, res - 1);
+        S.bbox[2][k] = max(S.bbox[2][k] - 6, 0);
+        S.bbox[3][k] = min(S.bbox[3][k] + 6, res - 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int nb = nbodies;
+        for (bool did = true; did;) {
+            did = false;
+            for (int a = 0; a < nb; ++a) {
+                int b0 = S.bbox[0][a], b1 = S.bbox[1][a], b2 = S.bbox[2][a], b3 = S.bbox[3][a];
+                bool grew = false;
+                for (int c = a + 1; c < nb;) {
+                    const int k = c + lane;
+                    const bool in = k < nb;
+                    const int k0 = in ? S.bbox[0][k] : 0, k1 = in ? S.bbox[1][k] : 0, k2 = in ? S.bbox[2][k] : 0,
+                              k3 = in ? S.bbox[3][k] : 0;
+                    const unsigned hit =
+                        __ballot_sync(0xffffffffu, in && boxes_touch(b0, b1, b2, b3, k0, k1, k2, k3));
+                    if (!hit) {
+                        c += 32;
+                        continue;
+                    }
+                    const int l = __ffs(hit) - 1;
+                    c += l;
+                    b0 = min(b0, __shfl_sync(0xffffffffu, k0, l));
+                    b1 = max(b1, __shfl_sync(0xffffffffu, k1, l));
+                    b2 = min(b2, __shfl_sync(0xffffffffu, k2, l));
+                    b3 = max(b3, __shfl_sync(0xffffffffu, k3, l));
+                    --nb;
+                    if (lane < 4) S.bbox[lane][c] = S.bbox[lane][nb];
+                    __syncwarp();
+                    grew = did = true;
+                }
+                if (grew && lane == 0) {
+                    S.bbox[0][a] = b0;
+                    S.bbox[1][a] = b1;
+                    S.bbox[2][a] = b2;
+                    S.bbox[3][a] = b3;
+                }
+                __syncwarp();
+            }
+        }
+        if (lane == 0) {
+            if (nb == 1 || nb > 8) {
+                nb = 1;
+                S.bbox[0][0] = x0;
+                S.bbox[1][0] = x1;
+                S.bbox[2][0] = y0;
+                S.bbox[3][0] = y1;
+            }
+            S.nbox = nb;
+        }
+    }
+    __syncthreads();
+}
+
+// The next run of set bits at or after `pos` in a row of W words: [s, e].
+__device__ __forceinline__ bool next_run(const unsigned int* row, int W, int pos, int& s, int& e) {
+    int w = pos >> 5;
+    if (w >= W) return false;
+    unsigned m = row[w] & (0xffffffffu << (pos & 31));
+    while (m == 0u) {
+        if (++w >= W) return false;
+        m = row[w];
+    }
+    const int b = __ffs(m) - 1;
+    s = 32 * w + b;
+    m = ~row[w] & (0xffffffffu << b);
+    while (m == 0u) {
+        if (++w >= W) {
+            e = 32 * W - 1;
+            return true;
+        }
+        m = ~row[w];
+    }
+    e = 32 * w + __ffs(m) - 2;
+    return true;
+}
+
+// sheet_work_boxes (src/fluid_core.rs:1325-1447) on rank 0 from the window's
+// wet bits: the wet extent, the bodies (4-connected, in the order of their
+// first raster cells), their boxes. Everything is in shared memory: one thread
+// takes a row's runs, joins them to the row above's by union-find over run
+// indices (raster order, so a body's root is its first run), and the bodies'
+// boxes are the runs'. By cells in global memory (crew_label_bodies, still
+// taken past MAX_RUNS) the labels took 28 us and the boxes 17 of the 104 of a
+// 200 x 200 window with a puddle; TIMED.
+__device__ void rank0_wet_boxes(Shared& S, const Job& J) {
+    const int res = J.res, W = wet_words(res), j = threadIdx.x;
+    const unsigned int* const row = wet_bits + (size_t)min(j, res - 1) * W;
+    int runs = 0, wet = 0, lo = MAX_RES, hi = -1;
+    if (j < res) {
+        unsigned carry = 0u;
+        for (int w = 0; w < W; ++w) {
+            const unsigned m = row[w];
+            runs += __popc(m & ~((m << 1) | carry));
+            carry = m >> 31;
+            wet += __popc(m);
+            if (m) {
+                if (lo == MAX_RES) lo = 32 * w + __ffs(m) - 1;
+                hi = 32 * w + 31 - __clz(m);
+            }
+        }
+    }
+    if (j == 0) {
+        S.ext[0] = 0;
+        S.ext[1] = MAX_RES;
+        S.ext[2] = MAX_RES;
+        S.ext[3] = MAX_RES;
+        S.ext[4] = -1;
+    }
+    int nruns = 0;
+    const int first = block_scan(S, runs, &nruns);
+    if (wet > 0) {
+        atomicAdd(&S.ext[0], wet);
+        atomicMin(&S.ext[1], lo);
+        atomicMin(&S.ext[2], -hi);
+        atomicMin(&S.ext[3], j);
+        atomicMax(&S.ext[4], j);
+    }
+    __syncthreads();
+    const int i0 = S.ext[1], i1 = -S.ext[2], j0 = S.ext[3], j1 = S.ext[4];
+    if (j == 0) {
+        S.by_cells = 0;
+        S.nbox = 0;
+    }
+    __syncthreads();
+    if (S.ext[0] == 0) return;
+    const int x0 = max(i0 - 3, 0), x1 = min(i1 + 3, res - 1), y0 = max(j0 - 3, 0), y1 = min(j1 + 3, res - 1);
+    if (S.ext[0] == (i1 - i0 + 1) * (j1 - j0 + 1)) {
+        set_whole(S, x0, x1, y0, y1);
+        return;
+    }
+    if (nruns > MAX_RUNS) {
+        if (j == 0) S.by_cells = 1;
+        __syncthreads();
+        return;
+    }
+    volatile int* const lab = S.lab;
+    S.row_count[min(j, MAX_RES - 1)] = first;
+    for (int k = 0; k < runs; ++k) lab[first + k] = first + k;
+    __syncthreads();
+    auto root = [&](int x) {
+        for (int y = lab[x]; y != x; y = lab[x]) x = y;  // labels fall along the way, so it ends
+        return x;
+    };
+    if (j > 0 && runs > 0) {
+        // This row's runs against the row above's, both from the left.
+        const unsigned int* const above = row - W;
+        int a = S.row_count[j - 1], b = first, as, ae, bs, be;
+        bool ha = next_run(above, W, 0, as, ae), hb = next_run(row, W, 0, bs, be);
+        while (ha && hb) {
+            if (as <= be && bs <= ae) {
+                for (int x = a, y = b;;) {
+                    x = root(x);
+                    y = root(y);
+                    if (x == y) break;
+                    const int up = max(x, y), down = min(x, y);
+                    if (atomicCAS(&S.lab[up], up, down) == up) break;
+                }
+            }
+            if (ae < be) {
+                ++a;
+                ha = next_run(above, W, ae + 1, as, ae);
+            } else {
+                ++b;
+                hb = next_run(row, W, be + 1, bs, be);
+            }
+        }
+    }
+    __syncthreads();
+    int roots = 0;
+    for (int k = 0; k < runs; ++k) {
+        const int r = root(first + k);
+        if (r == first + k)
+            ++roots;
+        else
+            lab[first + k] = r;
+    }
+    int nbodies = 0;
+    int slot = block_scan(S, roots, &nbodies);
+    // More than MAX_BOXES bodies: step the whole box. The reference merges the
+    // grown bodies first and only then falls back at more than 8 boxes, so
+    // this differs from it only when over 512 separate bodies would merge
+    // into 8 or fewer boxes.
+    if (nbodies > MAX_BOXES) {
+        set_whole(S, x0, x1, y0, y1);
+        return;
+    }
+    for (int k = threadIdx.x; k < nbodies; k += NT) {
+        S.bbox[0][k] = S.bbox[2][k] = MAX_RES;
+        S.bbox[1][k] = S.bbox[3][k] = -1;
+    }
+    __syncthreads();
+    for (int k = 0; k < runs; ++k)
+        if (lab[first + k] == first + k) lab[first + k] = -(slot++) - 1;
+    __syncthreads();
+    int s = 0, e = -1;
+    for (int k = 0; k < runs; ++k) {
+        next_run(row, W, e + 1, s, e);
+        int v = lab[first + k];
+        if (v >= 0) v = lab[v];
+        const int body = -v - 1;
+        atomicMin(&S.bbox[0][body], s);
+        atomicMax(&S.bbox[1][body], e);
+        atomicMin(&S.bbox[2][body], j);
+        atomicMax(&S.bbox[3][body], j);
+    }
+    __syncthreads();
+    merge_bodies(S, nbodies, x0, x1, y0, y1, res);
+}
+
+// The same by cells, for a window of more wet runs than rank 0's tables hold:
+// wet bodies are labelled in the f2 plane (as ints) by hooking and pointer
+// jumping; a body's root is its first wet cell in raster order, the order the
+// reference's run merge keeps. The wet-body labels of sheet_work_boxes (src/fluid_core.rs:1378-1457) over
 // the wet extent, by the whole crew, into the plane f2: every wet cell ends
 // holding its body's smallest index (its first raster cell). Hook and jump:
 // each round lowers the label of the larger of two neighbours' labels to the
@@ -1149,7 +1336,7 @@ __device__ void crew_label_bodies(Shared& S, const Job& J, const int ext[5]) {
     }
 }
 
-// `ext`: the crew's wet extent of the layer (crew_sum_extent).
+// `ext`: the layer's wet extent (rank0_wet_boxes).
 __device__ void cta_wet_boxes(Shared& S, const Job& J, const int ext[5]) {
     const int res = J.res;
     const int wet = ext[0], i0 = ext[1], i1 = -ext[2], j0 = ext[3], j1 = ext[4];
@@ -1224,51 +1411,11 @@ __device__ void cta_wet_boxes(Shared& S, const Job& J, const int ext[5]) {
         }
     })
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int nb = nbodies;
-        for (int k = 0; k < nb; ++k) {
-            S.bbox[0][k] = max(S.bbox[0][k] - 6, 0);
-            S.bbox[1][k] = min(S.bbox[1][k] + 6, res - 1);
-            S.bbox[2][k] = max(S.bbox[2][k] - 6, 0);
-            S.bbox[3][k] = min(S.bbox[3][k] + 6, res - 1);
-        }
-        // merge_boxes (src/fluid_core.rs:1459-1487), swap_remove order.
-        for (;;) {
-            bool did = false;
-            int a = 0;
-            while (a < nb) {
-                int c = a + 1;
-                while (c < nb) {
-                    if (boxes_touch(S.bbox[0][a], S.bbox[1][a], S.bbox[2][a], S.bbox[3][a], S.bbox[0][c],
-                                    S.bbox[1][c], S.bbox[2][c], S.bbox[3][c])) {
-                        S.bbox[0][a] = min(S.bbox[0][a], S.bbox[0][c]);
-                        S.bbox[1][a] = max(S.bbox[1][a], S.bbox[1][c]);
-                        S.bbox[2][a] = min(S.bbox[2][a], S.bbox[2][c]);
-                        S.bbox[3][a] = max(S.bbox[3][a], S.bbox[3][c]);
-                        for (int q = 0; q < 4; ++q) S.bbox[q][c] = S.bbox[q][nb - 1];
-                        --nb;
-                        did = true;
-                    } else {
-                        ++c;
-                    }
-                }
-                ++a;
-            }
-            if (!did) break;
-        }
-        if (nb == 1 || nb > 8) {
-            nb = 1;
-            S.bbox[0][0] = x0;
-            S.bbox[1][0] = x1;
-            S.bbox[2][0] = y0;
-            S.bbox[3][0] = y1;
-        }
-        S.nbox = nb;
-    }
-    __syncthreads();
+    merge_bodies(S, nbodies, x0, x1, y0, y1, res);
 }
 
-// soften_border (src/fluid_core.rs:9594-9622) on the whole layer.
+// soften_border (src/fluid_core.rs:9594-9622) on the whole layer; the caller's
+// next barrier publishes it.
 __device__ void cta_soften(const Job& J) {
     const int res = J.res, edge = J.soften_edge;
     // The band's rows and columns: [0, lo] and [hi, res).
@@ -1295,16 +1442,23 @@ __device__ void cta_soften(const Job& J) {
     CLU_RECT(0, lo, lo + 1, hi - 1, SOFTEN_CELL)
     CLU_RECT(hi, res - 1, lo + 1, hi - 1, SOFTEN_CELL)
 #undef SOFTEN_CELL
-    crew_sync();
 }
 
-// The layer's FP64 depth sum over the crew; rank 0 writes it.
+// The layer's FP64 depth sum over the crew, the CTAs' shares added in rank
+// order by rank 0. The barrier here is the step's last: after it no CTA reads
+// another's shared memory, so each may leave.
 __device__ void cta_ledger(Shared& S, const Job& J) {
     const int res = J.res;
     double part = 0.0;
     CLU_RECT(0, res - 1, 0, res - 1, { part += (double)fmaxf(J.h[g], 0.0f); })
-    part = crew_sum_d(S, part);
-    if (threadIdx.x == 0 && J.ledger && crew_rank() == 0) *J.ledger = part;
+    part = block_sum_d(S, part);
+    if (threadIdx.x == 0) *cg::this_cluster().map_shared_rank(&S.crew_d[crew_rank()], 0) = part;
+    crew_sync();
+    if (threadIdx.x == 0 && J.ledger && crew_rank() == 0) {
+        double sum = 0.0;
+        for (int r = 0; r < crew_size(); ++r) sum += S.crew_d[r];
+        *J.ledger = sum;
+    }
 }
 
 // step_sheet_eps_in + step_sheet_scratch (src/fluid_core.rs:821-852, :1659-1831).
@@ -1314,40 +1468,45 @@ __device__ __forceinline__ int window_body(Shared& S, const Job& J) {
     const int res = J.res;
     const float eps = J.eps;
     if (J.soften_edge > 0) cta_soften(J);
-    if (J.solid) cta_displace(J);
-    // wet_sum early out (src/fluid_core.rs:1306-1319, :840-844), over the crew.
-    double ws = 0.0;
-    int ext[5] = {0, res, 1, res, -1};  // wet cells, min i, -max i, min j, max j
-    CLU_RECT(0, res - 1, 0, res - 1, {
-        float hv = J.h[g];
-        if (hv > eps) {
-            ws += (double)hv;
-            ext[0] += 1;
-            ext[1] = min(ext[1], i);
-            ext[2] = min(ext[2], -i);
-            ext[3] = min(ext[3], j);
-            ext[4] = max(ext[4], j);
-        }
-    })
-    ws = crew_sum_extent(S, ws, ext);
-    if (!(ws > (double)eps)) {
-        cta_ledger(S, J);
-        return 0;
+    if (J.solid) {
+        crew_sync();
+        cta_displace(J);
     }
     const bool open_fine = !J.solid && J.cell <= kFineCell + 1.0e-6f;
     const bool fine_open = open_fine && J.pace == 0;
     const bool whole_wet = open_fine && (J.pace == 2 || J.pace == 3);
     const bool awake = open_fine && !whole_wet && !fine_open;
-    // Work boxes on rank 0 (the wet-body labels use a global plane; the awake
-    // scan is shared by the crew), then every other CTA copies them from its
-    // shared memory.
+    // Work boxes on rank 0, then every other CTA copies them from its shared
+    // memory. None when nothing is wet: the reference's wet_sum early out
+    // (src/fluid_core.rs:1306-1319, :840-844) sums the cells deeper than eps
+    // and asks for more than eps, which is to ask for one such cell.
     if (fine_open || awake) {
         cta_awake_boxes(S, J);
     } else {
-        crew_label_bodies(S, J, ext);
-        if (crew_rank() == 0) cta_wet_boxes(S, J, ext);
+        {
+            // The wet cells' bits to rank 0: a warp takes 32 cells of a row.
+            unsigned int* const bits = cg::this_cluster().map_shared_rank(wet_bits, 0);
+            const int W = wet_words(res), lane = (int)(threadIdx.x & 31);
+            for (int it = crew_rank() * (NT / 32) + (int)(threadIdx.x >> 5); it < res * W;
+                 it += crew_size() * (NT / 32)) {
+                const int j = it / W, i = 32 * (it - j * W) + lane;
+                const unsigned m = __ballot_sync(0xffffffffu, i < res && J.h[j * res + i] > eps);
+                if (lane == 0) bits[it] = m;
+            }
+        }
+        crew_sync();
+        if (crew_rank() == 0) rank0_wet_boxes(S, J);
+        crew_sync();
+        const Shared* S0 = cg::this_cluster().map_shared_rank(&S, 0);
+        if (S0->by_cells) {
+            int ext[5];
+            for (int q = 0; q < 5; ++q) ext[q] = S0->ext[q];
+            crew_label_bodies(S, J, ext);
+            if (crew_rank() == 0) cta_wet_boxes(S, J, ext);
+            crew_sync();
+        }
     }
-    crew_sync();
+    if (fine_open || awake) crew_sync();
     if (crew_rank() != 0) {
         const Shared* S0 = cg::this_cluster().map_shared_rank(&S, 0);
         const int n0 = S0->nbox;
@@ -1406,6 +1565,12 @@ __device__ __forceinline__ int window_body(Shared& S, const Job& J) {
     return gs_passes;
 }
 
+// Every CTA of the crew has started, which a write to another's shared memory
+// needs: the arrival comes first thing in the kernel, before its dependency,
+// so the wait here finds it done.
+__device__ __forceinline__ void crew_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void crew_started() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ void window_job(Job* jp) {
     __shared__ Shared S;
     __shared__ Job Js;
@@ -1414,26 +1579,25 @@ __device__ __forceinline__ void window_job(Job* jp) {
     // memory after each store through a plane pointer.
     if (threadIdx.x == 0) Js = *jp;
     __syncthreads();
+    crew_started();
     if (!Js.active) return;  // the same for the whole crew
     const int gs_passes = window_body(S, Js);
     if (threadIdx.x == 0 && crew_rank() == 0) jp->gs_iters = gs_passes;
-    crew_sync();  // no CTA leaves while another may still read its shared memory
 }
 
 // Job k of an array.
 __global__ void __launch_bounds__(NT, 1) k_window_step(Job* jobs) {
+    crew_arrive();
     ::silt::dep_wait();
     window_job(jobs + blockIdx.x / (unsigned)crew_size());
 }
 
 // Job k of a list of jobs that live in different tables (batched windows).
 __global__ void __launch_bounds__(NT, 1) k_window_step_list(Job* const* jobs) {
+    crew_arrive();
     ::silt::dep_wait();
     window_job(jobs[blockIdx.x / (unsigned)crew_size()]);
 }
-
-// Largest crew: 16 CTAs, the non-portable cluster size B200 allows.
-constexpr int MAX_CREW = 16;
 
 // CTAs per job: enough warps for one (row, 32-cell chunk) item each on a
 // 64-cell patch, up to the largest crew.
@@ -1445,8 +1609,13 @@ static int crew_for(int max_res) {
     return c;
 }
 
+// Dynamic shared memory of a launch: the wet bits of its largest window.
+static size_t wet_bytes(int max_res) { return (size_t)max_res * wet_words(max_res) * 4; }
+
 // The largest crew the device can hold at once (a cluster of full-SM CTAs).
 static int crew_limit_query(cudaStream_t st) {
+    cudaFuncSetAttribute(k_window_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wet_bytes(MAX_RES));
+    cudaFuncSetAttribute(k_window_step_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wet_bytes(MAX_RES));
     if (cudaFuncSetAttribute(k_window_step, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaFuncSetAttribute(k_window_step_list, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
@@ -1456,6 +1625,7 @@ static int crew_limit_query(cudaStream_t st) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)c, 1, 1);
         cfg.blockDim = dim3(NT, 1, 1);
+        cfg.dynamicSmemBytes = wet_bytes(MAX_RES);
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1490,6 +1660,7 @@ cudaError_t launch_window_step_list(Job* const* d_job_list, int njobs, int max_r
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(njobs * crew), 1, 1);
     cfg.blockDim = dim3(NT, 1, 1);
+    cfg.dynamicSmemBytes = wet_bytes(max_res);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1512,7 +1683,7 @@ cudaError_t launch_window_step(const Job* d_jobs, int njobs, int max_res, cudaSt
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(njobs * crew), 1, 1);
     cfg.blockDim = dim3(NT, 1, 1);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = wet_bytes(max_res);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
