@@ -66,7 +66,8 @@ struct Shared {
 };
 
 // The wet cells of the window, one bit each, rows of wet_words(res) words: on
-// rank 0, written by the whole crew.
+// rank 0, written by the whole crew. After them its runs of wet cells, row by
+// row from the left (first cell, last cell and row, 10 bits each).
 extern __shared__ unsigned int wet_bits[];
 __host__ __device__ constexpr int wet_words(int res) { return (res + 31) / 32; }
 
@@ -1107,12 +1108,15 @@ __device__ __forceinline__ bool next_run(const unsigned int* row, int W, int pos
 
 // sheet_work_boxes (src/fluid_core.rs:1325-1447) on rank 0 from the window's
 // wet bits: the wet extent, the bodies (4-connected, in the order of their
-// first raster cells), their boxes. Everything is in shared memory: one thread
-// takes a row's runs, joins them to the row above's by union-find over run
-// indices (raster order, so a body's root is its first run), and the bodies'
-// boxes are the runs'. By cells in global memory (crew_label_bodies, still
-// taken past MAX_RUNS) the labels took 28 us and the boxes 17 of the 104 of a
-// 200 x 200 window with a puddle; TIMED.
+// first raster cells), their boxes. Everything is in shared memory. One thread
+// lists a row's runs; runs that touch the row above's then hook the larger of
+// the two bodies' labels to the smaller and every run jumps to its root, until
+// a round finds nothing to hook (run indices are in raster order, so a body's
+// root is its first run; jumping halves the chains that hooking makes, where
+// walking them took 17 to 33 us). By cells in global memory
+// (crew_label_bodies, still taken past MAX_RUNS) the labels took 28 us and the
+// boxes 17 of the 104 of a 200 x 200 window with a puddle; this takes 3 (148
+// runs of a half-flooded 64 x 64: 11).
 __device__ void rank0_wet_boxes(Shared& S, const Job& J) {
     const int res = J.res, W = wet_words(res), j = threadIdx.x;
     const unsigned int* const row = wet_bits + (size_t)min(j, res - 1) * W;
@@ -1165,74 +1169,84 @@ __device__ void rank0_wet_boxes(Shared& S, const Job& J) {
         return;
     }
     volatile int* const lab = S.lab;
-    S.row_count[min(j, MAX_RES - 1)] = first;
-    for (int k = 0; k < runs; ++k) lab[first + k] = first + k;
-    __syncthreads();
-    auto root = [&](int x) {
-        for (int y = lab[x]; y != x; y = lab[x]) x = y;  // labels fall along the way, so it ends
-        return x;
-    };
-    if (j > 0 && runs > 0) {
-        // This row's runs against the row above's, both from the left.
-        const unsigned int* const above = row - W;
-        int a = S.row_count[j - 1], b = first, as, ae, bs, be;
-        bool ha = next_run(above, W, 0, as, ae), hb = next_run(row, W, 0, bs, be);
-        while (ha && hb) {
-            if (as <= be && bs <= ae) {
-                for (int x = a, y = b;;) {
-                    x = root(x);
-                    y = root(y);
-                    if (x == y) break;
-                    const int up = max(x, y), down = min(x, y);
-                    if (atomicCAS(&S.lab[up], up, down) == up) break;
-                }
-            }
-            if (ae < be) {
-                ++a;
-                ha = next_run(above, W, ae + 1, as, ae);
-            } else {
-                ++b;
-                hb = next_run(row, W, be + 1, bs, be);
-            }
+    unsigned int* const list = wet_bits + (size_t)res * W;
+    S.row_count[j] = first;
+    {
+        int s = 0, e = -1;
+        for (int k = 0; k < runs; ++k) {
+            next_run(row, W, e + 1, s, e);
+            list[first + k] = (unsigned)s | (unsigned)e << 10 | (unsigned)j << 20;
+            lab[first + k] = first + k;
         }
     }
     __syncthreads();
-    int roots = 0;
-    for (int k = 0; k < runs; ++k) {
-        const int r = root(first + k);
-        if (r == first + k)
-            ++roots;
-        else
-            lab[first + k] = r;
+    for (int round = 0; round <= nruns; ++round) {
+        // Labels are roots here. Two that touch: the larger goes to the smaller.
+        int hooked = 0;
+        if (j > 0 && runs > 0) {
+            int a = S.row_count[j - 1], b = first;
+            const int a_end = first, b_end = first + runs;
+            while (a < a_end && b < b_end) {
+                const unsigned ra = list[a], rb = list[b];
+                const int as = ra & 1023u, ae = ra >> 10 & 1023u, bs = rb & 1023u, be = rb >> 10 & 1023u;
+                if (as <= be && bs <= ae) {
+                    const int x = lab[a], y = lab[b];
+                    if (x != y) {
+                        atomicMin(&S.lab[max(x, y)], min(x, y));
+                        hooked = 1;
+                    }
+                }
+                if (ae < be)
+                    ++a;
+                else
+                    ++b;
+            }
+        }
+        if (!__syncthreads_or(hooked)) break;
+        for (;;) {
+            int jumped = 0;
+            for (int r = threadIdx.x; r < nruns; r += NT) {
+                const int x = lab[r], y = lab[x];
+                if (x != y) {
+                    lab[r] = y;
+                    jumped = 1;
+                }
+            }
+            if (!__syncthreads_or(jumped)) break;
+        }
     }
+    // The bodies numbered by their roots' order. More than MAX_BOXES: step the
+    // whole box. The reference merges the grown bodies first and only then
+    // falls back at more than 8 boxes, so this differs from it only when over
+    // 512 separate bodies would merge into 8 or fewer boxes.
     int nbodies = 0;
-    int slot = block_scan(S, roots, &nbodies);
-    // More than MAX_BOXES bodies: step the whole box. The reference merges the
-    // grown bodies first and only then falls back at more than 8 boxes, so
-    // this differs from it only when over 512 separate bodies would merge
-    // into 8 or fewer boxes.
+    for (int r0 = 0; r0 < nruns; r0 += NT) {
+        const int r = r0 + (int)threadIdx.x;
+        const bool is_root = r < nruns && lab[r] == r;
+        int found = 0;
+        const int body = nbodies + block_scan(S, is_root ? 1 : 0, &found);
+        if (is_root && body < MAX_BOXES) {
+            S.bbox[0][body] = S.bbox[2][body] = MAX_RES;
+            S.bbox[1][body] = S.bbox[3][body] = -1;
+            lab[r] = -body - 1;
+        }
+        nbodies += found;
+    }
+    __syncthreads();
     if (nbodies > MAX_BOXES) {
         set_whole(S, x0, x1, y0, y1);
         return;
     }
-    for (int k = threadIdx.x; k < nbodies; k += NT) {
-        S.bbox[0][k] = S.bbox[2][k] = MAX_RES;
-        S.bbox[1][k] = S.bbox[3][k] = -1;
-    }
-    __syncthreads();
-    for (int k = 0; k < runs; ++k)
-        if (lab[first + k] == first + k) lab[first + k] = -(slot++) - 1;
-    __syncthreads();
-    int s = 0, e = -1;
-    for (int k = 0; k < runs; ++k) {
-        next_run(row, W, e + 1, s, e);
-        int v = lab[first + k];
+    for (int r = threadIdx.x; r < nruns; r += NT) {
+        int v = lab[r];
         if (v >= 0) v = lab[v];
         const int body = -v - 1;
+        const unsigned run = list[r];
+        const int s = run & 1023u, e = run >> 10 & 1023u, row_j = run >> 20;
         atomicMin(&S.bbox[0][body], s);
         atomicMax(&S.bbox[1][body], e);
-        atomicMin(&S.bbox[2][body], j);
-        atomicMax(&S.bbox[3][body], j);
+        atomicMin(&S.bbox[2][body], row_j);
+        atomicMax(&S.bbox[3][body], row_j);
     }
     __syncthreads();
     merge_bodies(S, nbodies, x0, x1, y0, y1, res);
@@ -1609,8 +1623,8 @@ static int crew_for(int max_res) {
     return c;
 }
 
-// Dynamic shared memory of a launch: the wet bits of its largest window.
-static size_t wet_bytes(int max_res) { return (size_t)max_res * wet_words(max_res) * 4; }
+// Dynamic shared memory of a launch: the wet bits of its largest window and the runs.
+static size_t wet_bytes(int max_res) { return ((size_t)max_res * wet_words(max_res) + MAX_RUNS) * 4; }
 
 // The largest crew the device can hold at once (a cluster of full-SM CTAs).
 static int crew_limit_query(cudaStream_t st) {
