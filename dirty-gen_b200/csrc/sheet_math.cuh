@@ -149,7 +149,7 @@ struct SweepRead {
 
 // conf_kick at a cell at least two cells inside the grid, where no stencil
 // index is clamped: the same arithmetic in the same order, reading the nine
-// neighbours through SweepRead's fixed offsets. Returns 1 for a kick, 0 for
+// neighbours at fixed offsets by SweepRead's rule. Returns 1 for a kick, 0 for
 // none and -1 when the caller has to ask conf_kick.
 // The twelve divisions take fdiv's product form and are tested together: -1
 // when some operand lies outside the range where that form is known to be
@@ -163,9 +163,9 @@ struct SweepRead {
 // IEEE: a divisor without the product form divides by IEEE division here; the
 // code for that, unused, costs a full register file (the grid's sweep 258 ->
 // 292 us), which leaves it out and takes -1.
-template <bool IEEE>
-__device__ __forceinline__ int conf_kick_inner(const FixedDiv& two, float dt, float vort, const SweepRead& uu,
-                                               const SweepRead& vv, float& du, float& dv) {
+template <bool IEEE, class Read>
+__device__ __forceinline__ int conf_kick_inner(const FixedDiv& two, float dt, float vort, const Read& uu,
+                                               const Read& vv, float& du, float& dv) {
     constexpr unsigned int LO = 0x12800000u;  // 2^-90
     unsigned int lo = 0xffffffffu;
     float hi = 0.0f;
@@ -182,12 +182,12 @@ __device__ __forceinline__ int conf_kick_inner(const FixedDiv& two, float dt, fl
         return dvdx - dudz;
     };
     if (!IEEE && !two.exact) return -1;
-    float w = vort_of(vv.at<1, 0>(), vv.at<-1, 0>(), uu.at<0, 1>(), uu.at<0, -1>());
+    float w = vort_of(vv.template at<1, 0>(), vv.template at<-1, 0>(), uu.template at<0, 1>(), uu.template at<0, -1>());
     if (!(fabsf(w) >= 0.9e-4f)) return 0;
-    float wxp = fabsf(vort_of(vv.at<2, 0>(), vv.at<0, 0>(), uu.at<1, 1>(), uu.at<1, -1>()));
-    float wxm = fabsf(vort_of(vv.at<0, 0>(), vv.at<-2, 0>(), uu.at<-1, 1>(), uu.at<-1, -1>()));
-    float wzp = fabsf(vort_of(vv.at<1, 1>(), vv.at<-1, 1>(), uu.at<0, 2>(), uu.at<0, 0>()));
-    float wzm = fabsf(vort_of(vv.at<1, -1>(), vv.at<-1, -1>(), uu.at<0, 0>(), uu.at<0, -2>()));
+    float wxp = fabsf(vort_of(vv.template at<2, 0>(), vv.template at<0, 0>(), uu.template at<1, 1>(), uu.template at<1, -1>()));
+    float wxm = fabsf(vort_of(vv.template at<0, 0>(), vv.template at<-2, 0>(), uu.template at<-1, 1>(), uu.template at<-1, -1>()));
+    float wzp = fabsf(vort_of(vv.template at<1, 1>(), vv.template at<-1, 1>(), uu.template at<0, 2>(), uu.template at<0, 0>()));
+    float wzm = fabsf(vort_of(vv.template at<1, -1>(), vv.template at<-1, -1>(), uu.template at<0, 0>(), uu.template at<0, -2>()));
     float nx = by_two(wxp - wxm);
     float nz = by_two(wzp - wzm);
     if (lo < 2u * LO - 1u || !(hi <= 0x1p90f)) return -1;

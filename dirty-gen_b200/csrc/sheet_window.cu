@@ -63,6 +63,7 @@ struct Shared {
     int ext[5];      // on rank 0: the wet extent (wet cells, i0, -i1, j0, j1)
     int by_cells;    // on rank 0: more runs than the tables hold, label by cells
     int scan[NT / 32];
+    unsigned char wall_row[MAX_RES];  // the row holds a wall
 };
 
 // The wet cells of the window, one bit each, rows of wet_words(res) words: on
@@ -119,6 +120,36 @@ __device__ __forceinline__ void crew_sync() { cg::this_cluster().sync(); }
             }                                                                            \
         }                                                                                \
     }
+
+// The same cells with each item's loads split off: use(i, j, v) gets what
+// load(i, j) read, and the next item's loads are issued before this item's
+// use. A phase finds its planes in L2 (the barrier before it emptied L1), and
+// written as one body an item waits for one round trip after another, as the
+// branches and stores of the body allow; so it waits for one at most (a 160-cell
+// patch and its window: 77 us a launch, 68 so; a flooded window with walls:
+// 241, 216). `load` is called for cells of the rectangle only and must not
+// depend on what `use` writes for other cells.
+template <class Load, class Use>
+__device__ __forceinline__ void clu_items(int i0, int i1, int j0, int j1, Load load, Use use) {
+    if (i1 < i0 || j1 < j0) return;
+    const int ch = (i1 - i0 + 32) >> 5, items = (j1 - j0 + 1) * ch, gs = crew_size() * (NT / 32);
+    const int lane = (int)(threadIdx.x & 31);
+    int it = crew_rank() * (NT / 32) + (int)(threadIdx.x >> 5);
+    if (it >= items) return;
+    int j = j0 + it / ch, i = i0 + (it % ch) * 32 + lane;
+    auto v = load(min(i, i1), j);
+    for (;;) {
+        it += gs;
+        if (it >= items) break;
+        const int nj = j0 + it / ch, ni = i0 + (it % ch) * 32 + lane;
+        auto next = load(min(ni, i1), nj);
+        if (i <= i1) use(i, j, v);
+        v = next;
+        i = ni;
+        j = nj;
+    }
+    if (i <= i1) use(i, j, v);
+}
 
 __device__ __forceinline__ double block_sum_d(Shared& S, double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -198,38 +229,25 @@ __device__ int block_scan(Shared& S, int v, int* total) {
     return base + x - v;
 }
 
-// Five taps along one axis, clamped at the grid edge. Cells at least 2 from
+// Five taps along one axis at position p of [0, res): cells at least 2 from
 // the edge start from the first product (accum5), others from 0.0
 // (accum5_clamped), src/fluid_core.rs:3680-3697.
-__device__ __forceinline__ float tap5c(const float* line, int res, int i, float k0, float k1, float k2, int stride) {
-    const bool in = i >= 2 && i <= res - 3;
-    const int i0 = i < 2 ? 0 : i - 2, i1 = i < 1 ? 0 : i - 1;
-    const int i3 = i + 1 > res - 1 ? res - 1 : i + 1, i4 = i + 2 > res - 1 ? res - 1 : i + 2;
-    float a0 = line[i0 * stride], a1 = line[i1 * stride], a2 = line[i * stride], a3 = line[i3 * stride],
-          a4 = line[i4 * stride];
-    float a = in ? a0 * k0 : 0.0f + a0 * k0;
-    a += a1 * k1;
-    a += a2 * k2;
-    a += a3 * k1;
-    a += a4 * k0;
+struct Taps {
+    float a[5];
+};
+__device__ __forceinline__ float tap5c(const Taps& t, int p, int res, float k0, float k1, float k2) {
+    const bool in = p >= 2 && p <= res - 3;
+    float a = in ? t.a[0] * k0 : 0.0f + t.a[0] * k0;
+    a += t.a[1] * k1;
+    a += t.a[2] * k2;
+    a += t.a[3] * k1;
+    a += t.a[4] * k0;
     return a;
 }
-
-// tap5c down column i where rows [lo, hi] come from `in_box` and the other
-// rows from `outside`.
-__device__ __forceinline__ float tap5c_pick(const float* in_box, const float* outside, int lo, int hi, int res, int i,
-                                            int j, float k0, float k1, float k2) {
-    const bool in = j >= 2 && j <= res - 3;
-    const int r0 = j < 2 ? 0 : j - 2, r1 = j < 1 ? 0 : j - 1;
-    const int r3 = j + 1 > res - 1 ? res - 1 : j + 1, r4 = j + 2 > res - 1 ? res - 1 : j + 2;
-    auto at = [&](int r) { return (r >= lo && r <= hi ? in_box : outside)[r * res + i]; };
-    float a0 = at(r0), a1 = at(r1), a2 = at(j), a3 = at(r3), a4 = at(r4);
-    float a = in ? a0 * k0 : 0.0f + a0 * k0;
-    a += a1 * k1;
-    a += a2 * k2;
-    a += a3 * k1;
-    a += a4 * k0;
-    return a;
+// The taps' values: at(q) at the positions around p, clamped to the grid.
+template <class At>
+__device__ __forceinline__ Taps taps_at(int p, int res, At at) {
+    return Taps{{at(max(p - 2, 0)), at(max(p - 1, 0)), at(p), at(min(p + 1, res - 1)), at(min(p + 2, res - 1))}};
 }
 
 // The reference's two blurs of one source in a row, blur_box with GAUSS into
@@ -239,25 +257,42 @@ __device__ __forceinline__ float tap5c_pick(const float* in_box, const float* ou
 // (STEEP, where the reference's second blur leaves it). Each z pass reads box
 // rows from its own x pass and the rows outside the box from tmp as they are:
 // the reference's x passes write only the box, so both of its z passes see
-// the same stale rows there. `combine(g, gauss, steep)` runs on each box cell
-// in the z phase.
+// the same stale rows there. `combine(g, gauss, steep, own)` runs on each box
+// cell in the z phase, `own` the cell's value in the plane `also`.
 template <class Comb>
 __device__ void cta_blur_pair(const float* __restrict__ src, float* __restrict__ dst_g, float* __restrict__ dst_s,
-                              float* __restrict__ tmp, float* __restrict__ tmp_g, int res, const Box& b,
-                              Comb combine) {
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        const float* line = src + j * res;
-        tmp_g[g] = tap5c(line, res, i, kG0, kG1, kG2, 1);
-        tmp[g] = tap5c(line, res, i, kS0, kS1, kS2, 1);
-    })
+                              float* __restrict__ tmp, float* __restrict__ tmp_g, const float* also, int res,
+                              const Box& b, Comb combine) {
+    clu_items(b.i0, b.i1, b.j0, b.j1,
+              [&](int i, int j) {
+                  const float* line = src + j * res;
+                  return taps_at(i, res, [&](int q) { return line[q]; });
+              },
+              [&](int i, int j, const Taps& t) {
+                  const int g = j * res + i;
+                  tmp_g[g] = tap5c(t, i, res, kG0, kG1, kG2);
+                  tmp[g] = tap5c(t, i, res, kS0, kS1, kS2);
+              });
     crew_sync();
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        const float gv = tap5c_pick(tmp_g, tmp, b.j0, b.j1, res, i, j, kG0, kG1, kG2);
-        const float sv = tap5c(tmp + i, res, j, kS0, kS1, kS2, res);
-        dst_g[g] = gv;
-        dst_s[g] = sv;
-        combine(g, gv, sv);
-    })
+    struct Pair {
+        Taps g, s;
+        float own;
+    };
+    clu_items(b.i0, b.i1, b.j0, b.j1,
+              [&](int i, int j) {
+                  Pair p;
+                  p.g = taps_at(j, res, [&](int r) { return (r >= b.j0 && r <= b.j1 ? tmp_g : tmp)[r * res + i]; });
+                  p.s = taps_at(j, res, [&](int r) { return tmp[r * res + i]; });
+                  p.own = also[j * res + i];
+                  return p;
+              },
+              [&](int i, int j, const Pair& p) {
+                  const int g = j * res + i;
+                  const float gv = tap5c(p.g, j, res, kG0, kG1, kG2), sv = tap5c(p.s, j, res, kS0, kS1, kS2);
+                  dst_g[g] = gv;
+                  dst_s[g] = sv;
+                  combine(g, gv, sv, p.own);
+              });
     crew_sync();
 }
 
@@ -274,10 +309,14 @@ __device__ __forceinline__ float job_mob(const Job& J, int g) {
     return sheet_mobility_for(job_nu(J, g));
 }
 
-// The cell's damping factor over dt: exp(-sheet_damp(nu) dt).
-__device__ __forceinline__ float job_decay(const Job& J, int g, float dt, float decay_c) {
+// What the cell's damping factor is made of, and the factor over dt:
+// exp(-sheet_damp(nu) dt).
+__device__ __forceinline__ float job_damp_source(const Job& J, int g) {
+    return J.nu_mode == NU_CONST ? 0.0f : (J.nu_mode == NU_TABLE ? J.damp_plane[g] : job_nu(J, g));
+}
+__device__ __forceinline__ float job_decay(const Job& J, float source, float dt, float decay_c) {
     if (J.nu_mode == NU_CONST) return decay_c;
-    const float rate = J.nu_mode == NU_TABLE ? J.damp_plane[g] : sheet_damp(job_nu(J, g));
+    const float rate = J.nu_mode == NU_TABLE ? source : sheet_damp(source);
     return exp_rn(-rate * dt);
 }
 
@@ -306,62 +345,61 @@ __device__ void cta_transport(const Job& J, const Box& b, float dt) {
     // (FP64) sum of the fluxes across its faces.
     const bool book_round = J.round != nullptr;
     double rnd = 0.0;
-    // dh of the edge from donor d to receiver r on depths hp, 0 across a wall.
-    auto edge = [&](const float* hp, int d, int r, float remd, float speed) {
-        const float dh = open_edge_dh(walled, hp[d], hp[r], remd, gate ? gate[r] : 1, walled ? bed[d] : 0.0f,
-                                      walled ? bed[r] : 0.0f, speed, dt, cell, 0.45f);
-        return walled && (W[d] | W[r]) ? 0.0f : dh;
+    // The four cells around a cell's two edges along one axis, q = p - 2 .. p + 1
+    // (clamped to the box, whose ends have no edge beyond): depth, velocity
+    // along the axis, and bed, wall and gate where there are any.
+    struct Line {
+        float h[4], s[4], bed[4];
+        unsigned char wall[4], gate[4];
     };
-    // x pass. Edge e joins cells e and e+1 of the row, e in [i0, i1 - 1]: its
-    // left-going flux (donor e+1) when the face speed is not positive, else
-    // its right-going flux (donor e, after what e gave across edge e-1).
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        const int row = j * res;
-        auto speed = [&](int e) { return 0.5f * (U[row + e] + U[row + e + 1]); };
-        auto left = [&](int e) {
-            const float sp = speed(e);
-            const float dh = edge(h, row + e + 1, row + e, 0.0f, sp);
+    auto line = [&](const float* hp, const float* sp, int p, int lo, int hi, int first, int step) {
+        Line L;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int g = first + min(max(p - 2 + k, lo), hi) * step;
+            L.h[k] = hp[g];
+            L.s[k] = sp[g];
+            L.bed[k] = walled ? bed[g] : 0.0f;
+            L.wall[k] = walled ? W[g] : 0;
+            L.gate[k] = gate ? gate[g] : 1;
+        }
+        return L;
+    };
+    // Depth after the pass along the axis. Edge e joins cells e and e + 1 of
+    // the line: its flux toward e when the face speed is not positive (donor
+    // e + 1), else toward e + 1 (donor e, after what it gave the other way).
+    auto pass = [&](const Line& L, int p, int lo, int hi) {
+        auto edge = [&](int d, int r, float remd, float speed) {
+            const float dh = open_edge_dh(walled, L.h[d], L.h[r], remd, L.gate[r], L.bed[d], L.bed[r], speed, dt, cell,
+                                          0.45f);
+            return (L.wall[d] | L.wall[r]) ? 0.0f : dh;
+        };
+        auto back = [&](int k) {
+            const float sp = 0.5f * (L.s[k] + L.s[k + 1]);
+            const float dh = edge(k + 1, k, 0.0f, sp);
             return sp > 0.0f ? 0.0f : dh;
         };
-        auto right = [&](int e) {
-            const float sp = speed(e);
-            const float prev = e > b.i0 ? left(e - 1) : 0.0f;
-            const float dh = edge(h, row + e, row + e + 1, 0.0f + prev, sp);
+        auto ahead = [&](int k, float gave) {
+            const float sp = 0.5f * (L.s[k] + L.s[k + 1]);
+            const float dh = edge(k, k + 1, 0.0f + gave, sp);
             return sp > 0.0f ? dh : 0.0f;
         };
-        const float flm = i > b.i0 ? left(i - 1) : 0.0f, frm = i > b.i0 ? right(i - 1) : 0.0f;
-        const float flc = i < b.i1 ? left(i) : 0.0f, frc = i < b.i1 ? right(i) : 0.0f;
-        const float rem = (0.0f + flm) + frc, add = (0.0f + frm) + flc;
-        const float hv = h[g];
-        const float moved = fmaxf(hv - rem + add, 0.0f);
-        const float hx = (rem > 0.0f || add > 0.0f) ? moved : hv;
-        HX[g] = hx;
-        if (book_round) rnd += ((double)hx - (double)hv) - (((double)frm + (double)flc) - ((double)flm + (double)frc));
-    })
-    crew_sync();
-    // z pass on the x pass's depths: row pair r joins rows r and r+1, r in [j0, j1 - 1].
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        auto speed = [&](int r) { return 0.5f * (V[r * res + i] + V[(r + 1) * res + i]); };
-        auto up = [&](int r) {
-            const float sp = speed(r);
-            const float dh = edge(HX, (r + 1) * res + i, r * res + i, 0.0f, sp);
-            return sp > 0.0f ? 0.0f : dh;
-        };
-        auto down = [&](int r) {
-            const float sp = speed(r);
-            const float ra = r > b.j0 ? 0.0f + up(r - 1) : 0.0f;
-            const float dh = edge(HX, r * res + i, (r + 1) * res + i, ra, sp);
-            return sp > 0.0f ? dh : 0.0f;
-        };
-        const float upm = j > b.j0 ? up(j - 1) : 0.0f, dnm = j > b.j0 ? down(j - 1) : 0.0f;
-        const float upc = j < b.j1 ? up(j) : 0.0f, dnc = j < b.j1 ? down(j) : 0.0f;
-        const float rem = (0.0f + upm) + dnc, add = (0.0f + dnm) + upc;
-        const float hv = HX[g];
+        const bool has_m = p > lo, has_c = p < hi;
+        const float give2 = p - 1 > lo ? back(0) : 0.0f;
+        const float bm = has_m ? back(1) : 0.0f, am = has_m ? ahead(1, give2) : 0.0f;
+        const float bc = has_c ? back(2) : 0.0f, ac = has_c ? ahead(2, bm) : 0.0f;
+        const float rem = (0.0f + bm) + ac, add = (0.0f + am) + bc;
+        const float hv = L.h[2];
         const float moved = fmaxf(hv - rem + add, 0.0f);
         const float hn = (rem > 0.0f || add > 0.0f) ? moved : hv;
-        h[g] = hn;
-        if (book_round) rnd += ((double)hn - (double)hv) - (((double)dnm + (double)upc) - ((double)upm + (double)dnc));
-    })
+        if (book_round) rnd += ((double)hn - (double)hv) - (((double)am + (double)bc) - ((double)bm + (double)ac));
+        return hn;
+    };
+    clu_items(b.i0, b.i1, b.j0, b.j1, [&](int i, int j) { return line(h, U, i, b.i0, b.i1, j * res, 1); },
+              [&](int i, int j, const Line& L) { HX[j * res + i] = pass(L, i, b.i0, b.i1); });
+    crew_sync();
+    clu_items(b.i0, b.i1, b.j0, b.j1, [&](int i, int j) { return line(HX, V, j, b.j0, b.j1, i, res); },
+              [&](int i, int j, const Line& L) { h[j * res + i] = pass(L, j, b.j0, b.j1); });
     if (book_round) {
         for (int o = 16; o > 0; o >>= 1) rnd += __shfl_down_sync(0xffffffffu, rnd, o);
         if ((threadIdx.x & 31) == 0 && rnd != 0.0) atomicAdd(J.round, rnd * J.cut_area);
@@ -415,12 +453,72 @@ __device__ __forceinline__ bool wall_near(const uint8_t* W, int res, int i, int 
     return false;
 }
 
+// The rows that hold a wall, each CTA for itself (the mask is a byte a cell).
+__device__ void find_wall_rows(Shared& S, const Job& J) {
+    const int res = J.res, n = res * res;
+    for (int j = threadIdx.x; j < res; j += NT) S.wall_row[j] = 0;
+    __syncthreads();
+    const int n16 = ((uintptr_t)J.solid & 15u) == 0 ? n / 16 : 0;
+    for (int k = threadIdx.x; k < n16; k += NT) {
+        const uint4 q = reinterpret_cast<const uint4*>(J.solid)[k];
+        if (q.x | q.y | q.z | q.w)
+            for (int e = 0; e < 16; ++e)
+                if (J.solid[16 * k + e]) S.wall_row[(16 * k + e) / res] = 1;
+    }
+    for (int k = 16 * n16 + (int)threadIdx.x; k < n; k += NT)
+        if (J.solid[k]) S.wall_row[k / res] = 1;
+    __syncthreads();
+}
+
+// Whether a wall lies within R cells of any of the 32 cells (i0 + lane, j) of a
+// work item: asked by the whole warp, so that items clear of the walls (nearly
+// all of a window with one vehicle) skip the passes that only act beside one.
+template <int R>
+__device__ __forceinline__ bool item_near_wall(const Shared& S, const uint8_t* W, int res, int i0, int j) {
+    bool row = false;
+    for (int r = max(j - R, 0); r <= min(j + R, res - 1); ++r) row |= S.wall_row[r] != 0;
+    if (!row) return false;
+    const int lane = (int)(threadIdx.x & 31), i = i0 + lane;
+    // Each lane its own column, the first and last R also those beyond.
+    const int far = lane < R ? i - R : (lane >= 32 - R ? i + R : i);
+    bool hit = false;
+#pragma unroll
+    for (int d = -R; d <= R; ++d) {
+        const int r = j + d;
+        if (r < 0 || r >= res) continue;
+        if (i < res) hit |= W[r * res + i] != 0;
+        if (far >= 0 && far < res) hit |= W[r * res + far] != 0;
+    }
+    return __any_sync(0xffffffffu, hit);
+}
+
+// CLU_RECT whose items' bodies see `beside`: a wall lies within R cells of the item.
+#define CLU_WALLS(R, I0, I1, J0, J1, ...)                                                  \
+    {                                                                                    \
+        const int ri0_ = (I0), ri1_ = (I1), rj0_ = (J0), rj1_ = (J1);                    \
+        const int ch_ = (ri1_ - ri0_ + 32) >> 5;                                         \
+        const int items_ = rj1_ >= rj0_ ? (rj1_ - rj0_ + 1) * ch_ : 0;                   \
+        for (int it_ = crew_rank() * (NT / 32) + (int)(threadIdx.x >> 5); it_ < items_;  \
+             it_ += crew_size() * (NT / 32)) {                                           \
+            const int r_ = it_ / ch_;                                                    \
+            const int j = rj0_ + r_;                                                     \
+            const int i_ = ri0_ + (it_ - r_ * ch_) * 32;                                 \
+            const bool beside = item_near_wall<R>(S, J.solid, res, i_, j);                   \
+            const int i = i_ + (int)(threadIdx.x & 31);                                  \
+            if (i <= ri1_) {                                                             \
+                const int g = j * res + i;                                               \
+                (void)g;                                                                 \
+                __VA_ARGS__                                                              \
+            }                                                                            \
+        }                                                                                \
+    }
+
 // displace_occupied (:4382-4444) on the whole window: a covered column goes,
 // in equal shares, to its open four-neighbours (to the open cells of its 5 x 5
 // block when none is open) and the cell empties; with nowhere to go it stays.
 // Each open cell gathers its shares in the reference's order (sources in
 // raster order) into f1, then every cell applies its change.
-__device__ void cta_displace(const Job& J) {
+__device__ void cta_displace(Shared& S, const Job& J) {
     const int res = J.res;
     const uint8_t* __restrict__ W = J.solid;
     float* __restrict__ H = J.h;
@@ -436,8 +534,8 @@ __device__ void cta_displace(const Job& J) {
             for (int di = -2; di <= 2; ++di) n += open_at(W, res, si + di, sj + dj) ? 1 : 0;
         return n;
     };
-    CLU_RECT(0, res - 1, 0, res - 1, {
-        if (W[g] == 0) {
+    CLU_WALLS(2, 0, res - 1, 0, res - 1, {
+        if (beside && W[g] == 0) {
             float acc = 0.0f;
             for (int sj = j - 2; sj <= j + 2; ++sj)
                 for (int si = i - 2; si <= i + 2; ++si) {
@@ -453,7 +551,8 @@ __device__ void cta_displace(const Job& J) {
         }
     })
     crew_sync();
-    CLU_RECT(0, res - 1, 0, res - 1, {
+    CLU_WALLS(2, 0, res - 1, 0, res - 1, {
+        if (!beside) continue;
         if (W[g] != 0) {
             const float vol = H[g];
             bool four;
@@ -517,12 +616,12 @@ __device__ void cta_ghost(const Job& J, const Box& b) {
 
 // block_into_solid (:4328-4380): a wet open cell drops the part of its
 // velocity that points into a wall neighbour, direction by direction.
-__device__ void cta_block(const Job& J, const Box& b) {
+__device__ void cta_block(Shared& S, const Job& J, const Box& b) {
     const int res = J.res;
     const uint8_t* __restrict__ W = J.solid;
     const float eps = J.eps;
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        if (W[g] == 0 && J.h[g] > eps) {
+    CLU_WALLS(1, b.i0, b.i1, b.j0, b.j1, {
+        if (beside && W[g] == 0 && J.h[g] > eps) {
             float ux = J.u[g], vx = J.v[g];
             bool hit = false;
             for (int k = 0; k < 4; ++k) {
@@ -551,7 +650,7 @@ __device__ void cta_block(const Job& J, const Box& b) {
 // books live in the transient planes (the Gauss-Seidel snapshots and f2): the
 // scratch sets keep what the reference's blurs left there, which the next
 // step's blurs read beyond its box.
-__device__ void cta_redirect(const Job& J, const Box& b, float dt) {
+__device__ void cta_redirect(Shared& S, const Job& J, const Box& b, float dt) {
     const int res = J.res;
     const uint8_t* __restrict__ W = J.solid;
     float* __restrict__ H = J.h;
@@ -563,10 +662,13 @@ __device__ void cta_redirect(const Job& J, const Box& b, float dt) {
     auto accepts = [&](int q, int s) {
         return W[q] == 0 && !(H[q] <= 1.0e-6f && bed[q] > bed[s] + H[s] + 1.0e-3f);
     };
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
+    // A source has a wall beside it and its flanks lie one cell off, so only
+    // items within one cell of a wall give and only items within two receive;
+    // the books are written everywhere, for the cells that read them.
+    CLU_WALLS(1, b.i0, b.i1, b.j0, b.j1, {
         float rem = 0.0f;
         float share[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        if (W[g] == 0 && !(H[g] < 0.02f)) {
+        if (beside && W[g] == 0 && !(H[g] < 0.02f)) {
             for (int k = 0; k < 4; ++k) {
                 const int di = nb_di(k), dj = nb_dj(k);
                 if (!wall_at(W, res, i + di, j + dj)) continue;
@@ -608,7 +710,8 @@ __device__ void cta_redirect(const Job& J, const Box& b, float dt) {
     const int ri0 = max(b.i0 - 1, 0), ri1 = min(b.i1 + 1, res - 1);
     const int rj0 = max(b.j0 - 1, 0), rj1 = min(b.j1 + 1, res - 1);
     auto in_box = [&](int i, int j) { return i >= b.i0 && i <= b.i1 && j >= b.j0 && j <= b.j1; };
-    CLU_RECT(ri0, ri1, rj0, rj1, {
+    CLU_WALLS(2, ri0, ri1, rj0, rj1, {
+        if (!beside) continue;
         // Sources whose flank this cell is: the cell above (horizontal
         // directions), left and right (vertical directions), below
         // (horizontal directions), in raster order.
@@ -629,9 +732,33 @@ __device__ void cta_redirect(const Job& J, const Box& b, float dt) {
         J.f1[g] = (rem > 0.0f || add > 0.0f) ? fmaxf(hv - rem + add, 0.0f) : hv;
     })
     crew_sync();
-    CLU_RECT(ri0, ri1, rj0, rj1, { H[g] = J.f1[g]; })
+    CLU_WALLS(2, ri0, ri1, rj0, rj1, { if (beside) H[g] = J.f1[g]; })
     crew_sync();
 }
+
+// The values conf_kick_inner reads of one component around a cell (SweepRead's
+// rule), read together.
+struct KickReads {
+    float before[6], self, after[6];
+    // dx, dy: 1 and the row stride, or 0 and 0 where the neighbours are not to
+    // be read (the cell's own values stand in).
+    __device__ __forceinline__ KickReads(const float* cur, const float* start, const float* own, int g, int dx, int dy)
+        : before{cur[g - dx], cur[g - 2 * dx], cur[g - dy], cur[g - dy - dx], cur[g - dy + dx], cur[g - 2 * dy]},
+          self(own[g]),
+          after{start[g + dx], start[g + 2 * dx], start[g + dy], start[g + dy + dx], start[g + dy - dx],
+                start[g + 2 * dy]} {}
+    template <int DX, int DY>
+    __device__ __forceinline__ float at() const {
+        if constexpr (DX == 0 && DY == 0) {
+            return self;
+        } else {
+            constexpr bool later = DY > 0 || (DY == 0 && DX > 0);
+            constexpr int X = later ? DX : -DX, Y = later ? DY : -DY;  // the mirrored place among the later ones
+            constexpr int k = Y == 0 ? X - 1 : (Y == 2 ? 5 : (X == 0 ? 2 : (X == 1 ? 3 : 4)));
+            return later ? after[k] : before[k];
+        }
+    }
+};
 
 // Gravity then the raster-order Gauss-Seidel confinement on one box
 // (force_gravity_open's serial sweep, src/fluid_core.rs:2234-2260).
@@ -650,25 +777,45 @@ __device__ int cta_gravity_gs(Shared& S, const Job& J, const Box& b, const float
         const int x0 = max(b.i0 - 2, 0), x1 = min(b.i1 + 2, res - 1), y0 = max(b.j0 - 2, 0),
                   y1 = min(b.j1 + 2, res - 1);
         if (threadIdx.x == 0) S.chg[0] = S.chg[1] = S.chg[2] = 0;
-        CLU_RECT(x0, x1, y0, y1, {
-            const float u0 = J.u[g], v0 = J.v[g];
-            U0[g] = u0;
-            V0[g] = v0;
-            if (i >= b.i0 && i <= b.i1 && j >= b.j0 && j <= b.j1 && J.h[g] > eps) {
-                const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
-                float px = fdiv(p[j * res + ip] - p[j * res + im], two);
-                float pz = fdiv(p[jp * res + i] - p[jm * res + i], two);
-                float mob = job_mob(J, g);
+        {
+            int* const clear = reinterpret_cast<int*>(J.f2);
+            const int n = (b.j1 - b.j0 + 1) * ((b.i1 - b.i0 + 32) >> 5);
+            for (int k = crew_rank() * NT + (int)threadIdx.x; k < n; k += crew_size() * NT) clear[k] = 0;
+        }
+        struct Cell {
+            float u, v, h, p[4], mob;
+        };
+        auto load = [&](int i, int j) {
+            const int g = j * res + i;
+            const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
+            return Cell{J.u[g], J.v[g], J.h[g], {p[j * res + ip], p[j * res + im], p[jp * res + i], p[jm * res + i]},
+                        job_mob(J, g)};
+        };
+        auto start = [&](int i, int j, const Cell& c, bool beside) {
+            const int g = j * res + i;
+            U0[g] = c.u;
+            V0[g] = c.v;
+            if (i >= b.i0 && i <= b.i1 && j >= b.j0 && j <= b.j1 && c.h > eps) {
+                float px = fdiv(c.p[0] - c.p[1], two);
+                float pz = fdiv(c.p[2] - c.p[3], two);
+                float mob = c.mob;
                 // force_gravity_solid (:2084-2129): at least 1 beside a wall.
-                if (J.solid && J.h[g] > 0.08f && wall_near(J.solid, res, i, j)) mob = fmaxf(mob, 1.0f);
-                float ug = u0 + -kGravity * px * mob * dt;
-                float vg = v0 + -kGravity * pz * mob * dt;
+                if (beside && c.h > 0.08f && wall_near(J.solid, res, i, j)) mob = fmaxf(mob, 1.0f);
+                float ug = c.u + -kGravity * px * mob * dt;
+                float vg = c.v + -kGravity * pz * mob * dt;
                 UG[g] = ug;
                 VG[g] = vg;
                 J.u[g] = ug;
                 J.v[g] = vg;
             }
-        })
+        };
+        if (J.solid)
+            CLU_WALLS(1, x0, x1, y0, y1, {
+                (void)g;
+                start(i, j, load(i, j), beside);
+            })
+        else
+            clu_items(x0, x1, y0, y1, load, [&](int i, int j, const Cell& c) { start(i, j, c, false); });
     }
     crew_sync();
     if (!(J.vort > 0.0f)) return 0;
@@ -680,39 +827,78 @@ __device__ int cta_gravity_gs(Shared& S, const Job& J, const Box& b, const float
     // three slots, so a pass needs one barrier: pass k sets chg[k % 3] and
     // clears chg[(k + 1) % 3], which the crew last read before the barrier
     // that ended pass k - 1.
-    cg::cluster_group crew = cg::this_cluster();
+    // An item's stamp is one past the last pass that changed it. A later pass
+    // solves an item again only when it or an item whose cells it reads as
+    // earlier ones (left, the three above, the one two above) was changed in
+    // the pass before or since: otherwise its cells still satisfy their
+    // equations. A late pass over a whole 200 x 200 window takes 3 to 5 us
+    // instead of the first ones' 12.
+    volatile int* const stamp = reinterpret_cast<int*>(J.f2);
+    const int lane = (int)(threadIdx.x & 31), warp = (int)(threadIdx.x >> 5);
+    const int ch = (b.i1 - b.i0 + 32) >> 5, items = (b.j1 - b.j0 + 1) * ch, gs = crew_size() * (NT / 32);
+    const int near = lane % 6;  // itself, left, above left, above, above right, two above
+    const int near_r = near < 2 ? 0 : (near < 5 ? -1 : -2);
+    const int near_c = near == 0 || near == 3 || near == 5 ? 0 : (near == 4 ? 1 : -1);
     int passes = 0;
     for (; passes < GS_MAX_PASSES; ++passes) {
         const int slot = passes % 3;
         if (threadIdx.x == 0) S.chg[(slot + 1) % 3] = 0;
-        CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-            if (J.h[g] > eps) {
-                auto pick = [&](const float* X, const float* G0, const float* SG, int a, int c) {
-                    if (a == i && c == j) return SG[g];
-                    const bool before = c < j || (c == j && a < i);
-                    return before ? X[c * res + a] : G0[c * res + a];
-                };
-                auto uu = [&](int a, int c) { return pick(J.u, U0, UG, a, c); };
-                auto vv = [&](int a, int c) { return pick(J.v, V0, VG, a, c); };
-                float du, dv;
-                float nu_ = UG[g], nv_ = VG[g];
+        // Items (row, 32 cells of the box), dealt round-robin to the crew's
+        // warps; after the first pass five at a time are asked whether an item
+        // whose cells they read as earlier ones changed since.
+        for (int it0 = crew_rank() * (NT / 32) + warp; it0 < items; it0 += 5 * gs) {
+            unsigned due = 0x1fu;
+            if (passes > 0) {
+                const int q = lane / 6, it = it0 + q * gs;
+                bool hit = false;
+                if (lane < 30 && it < items) {
+                    const int r = it / ch + near_r, c = it % ch + near_c;
+                    hit = r >= 0 && c >= 0 && c < ch && stamp[r * ch + c] >= passes;
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                due = 0u;
+                for (int k = 0; k < 5; ++k) due |= (m >> (6 * k) & 0x3fu) ? 1u << k : 0u;
+            }
+            for (int k = 0; k < 5; ++k) {
+                const int it = it0 + k * gs;
+                if (it >= items) break;
+                if (!(due >> k & 1u)) continue;
+                const int r = it / ch, j = b.j0 + r, i = b.i0 + 32 * (it - r * ch) + lane, g = j * res + i;
+                bool changed = false;
                 // Two cells inside the window no stencil index is clamped.
                 const bool inner = i >= 2 && j >= 2 && i + 2 < res && j + 2 < res;
-                int kick = inner ? conf_kick_inner<true>(two, dt, J.vort, SweepRead{J.u, U0, UG, g, res},
-                                                         SweepRead{J.v, V0, VG, g, res}, du, dv)
-                                 : -1;
-                if (kick < 0) kick = conf_kick(i, j, res, two, dt, J.vort, uu, vv, du, dv);
-                if (kick) {
-                    nu_ = UG[g] + du;
-                    nv_ = VG[g] + dv;
+                // Every read at once, before the first branch on one of them.
+                const int own = j * res + min(i, b.i1), at = inner ? g : own, dx = inner ? 1 : 0, dy = inner ? res : 0;
+                const KickReads uu(J.u, U0, UG, at, dx, dy), vv(J.v, V0, VG, at, dx, dy);
+                const float hc = J.h[own], uc = J.u[own], vc = J.v[own], ug = UG[own], vg = VG[own];
+                if (i <= b.i1 && hc > eps) {
+                    float du, dv, nu_ = ug, nv_ = vg;
+                    int kick = inner ? conf_kick_inner<true>(two, dt, J.vort, uu, vv, du, dv) : -1;
+                    if (kick < 0) {
+                        auto pick = [&](const float* X, const float* G0, const float* SG, int a, int c) {
+                            if (a == i && c == j) return SG[g];
+                            const bool before = c < j || (c == j && a < i);
+                            return before ? X[c * res + a] : G0[c * res + a];
+                        };
+                        kick = conf_kick(i, j, res, two, dt, J.vort, [&](int a, int c) { return pick(J.u, U0, UG, a, c); },
+                                         [&](int a, int c) { return pick(J.v, V0, VG, a, c); }, du, dv);
+                    }
+                    if (kick) {
+                        nu_ = ug + du;
+                        nv_ = vg + dv;
+                    }
+                    if (__float_as_uint(nu_) != __float_as_uint(uc) || __float_as_uint(nv_) != __float_as_uint(vc)) {
+                        J.u[g] = nu_;
+                        J.v[g] = nv_;
+                        changed = true;
+                    }
                 }
-                if (__float_as_uint(nu_) != __float_as_uint(J.u[g]) || __float_as_uint(nv_) != __float_as_uint(J.v[g])) {
-                    J.u[g] = nu_;
-                    J.v[g] = nv_;
+                if (__ballot_sync(0xffffffffu, changed) && lane == 0) {
+                    stamp[it] = passes + 1;
                     S.chg[slot] = 1;
                 }
             }
-        })
+        }
         crew_sync();
         const int any = crew_fold(&S.chg[slot], 0, [](int a, int b) { return a | b; });
         if (!any) break;
@@ -755,49 +941,63 @@ __device__ void cta_gravity_jacobi(const Job& J, const Box& b, const float* __re
     const float* __restrict__ H = J.h;
     float* __restrict__ U = J.u;
     float* __restrict__ V = J.v;
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        if (H[g] > eps) {
-            const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
-            float px = fdiv(p[j * res + ip] - p[j * res + im], two);
-            float pz = fdiv(p[jp * res + i] - p[jm * res + i], two);
-            float mob = job_mob(J, g);
-            U[g] += -kGravity * px * mob * dt;
-            V[g] += -kGravity * pz * mob * dt;
-        }
-    })
+    struct Cell {
+        float u, v, h, p[4], mob;
+    };
+    clu_items(b.i0, b.i1, b.j0, b.j1,
+              [&](int i, int j) {
+                  const int g = j * res + i;
+                  const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
+                  return Cell{U[g], V[g], H[g],
+                              {p[j * res + ip], p[j * res + im], p[jp * res + i], p[jm * res + i]}, job_mob(J, g)};
+              },
+              [&](int i, int j, const Cell& c) {
+                  const int g = j * res + i;
+                  if (!(c.h > eps)) return;
+                  float px = fdiv(c.p[0] - c.p[1], two);
+                  float pz = fdiv(c.p[2] - c.p[3], two);
+                  U[g] = c.u + -kGravity * px * c.mob * dt;
+                  V[g] = c.v + -kGravity * pz * c.mob * dt;
+              });
     crew_sync();
     if (!(J.vort > 0.0f)) return;
     float* __restrict__ W = J.f1;
-    {
-        const int wi0 = max(b.i0 - 1, 0), wi1 = min(b.i1 + 1, res - 1);
-        const int wj0 = max(b.j0 - 1, 0), wj1 = min(b.j1 + 1, res - 1);
-        CLU_RECT(wi0, wi1, wj0, wj1, {
-            const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
-            float dvdx = fdiv(V[j * res + ip] - V[j * res + im], two);
-            float dudz = fdiv(U[jp * res + i] - U[jm * res + i], two);
-            W[g] = dvdx - dudz;
-        })
-    }
+    struct Four {
+        float a[4];
+    };
+    clu_items(max(b.i0 - 1, 0), min(b.i1 + 1, res - 1), max(b.j0 - 1, 0), min(b.j1 + 1, res - 1),
+              [&](int i, int j) {
+                  const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
+                  return Four{{V[j * res + ip], V[j * res + im], U[jp * res + i], U[jm * res + i]}};
+              },
+              [&](int i, int j, const Four& f) {
+                  float dvdx = fdiv(f.a[0] - f.a[1], two);
+                  float dudz = fdiv(f.a[2] - f.a[3], two);
+                  W[j * res + i] = dvdx - dudz;
+              });
     crew_sync();
     const float vort = J.vort;
-    CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-        if (H[g] > eps) {
-            float w = W[g];
-            if (finite_f(w) && !(fabsf(w) < 1.0e-4f)) {
-                const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
-                float wxp = fabsf(W[j * res + ip]), wxm = fabsf(W[j * res + im]);
-                float wzp = fabsf(W[jp * res + i]), wzm = fabsf(W[jm * res + i]);
-                float nx = fdiv(wxp - wxm, two);
-                float nz = fdiv(wzp - wzm, two);
-                float du = vort * dt * (-nz * w);
-                float dv = vort * dt * (nx * w);
-                if (finite_f(du) && finite_f(dv) && du * du + dv * dv <= 0.0625f) {
-                    U[g] += du;
-                    V[g] += dv;
-                }
-            }
-        }
-    })
+    struct Kick {
+        float h, w, u, v, n[4];
+    };
+    clu_items(b.i0, b.i1, b.j0, b.j1,
+              [&](int i, int j) {
+                  const int g = j * res + i;
+                  const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
+                  return Kick{H[g], W[g], U[g], V[g], {W[j * res + ip], W[j * res + im], W[jp * res + i], W[jm * res + i]}};
+              },
+              [&](int i, int j, const Kick& k) {
+                  if (!(k.h > eps) || !finite_f(k.w) || fabsf(k.w) < 1.0e-4f) return;
+                  const int g = j * res + i;
+                  float nx = fdiv(fabsf(k.n[0]) - fabsf(k.n[1]), two);
+                  float nz = fdiv(fabsf(k.n[2]) - fabsf(k.n[3]), two);
+                  float du = vort * dt * (-nz * k.w);
+                  float dv = vort * dt * (nx * k.w);
+                  if (finite_f(du) && finite_f(dv) && du * du + dv * dv <= 0.0625f) {
+                      U[g] = k.u + du;
+                      V[g] = k.v + dv;
+                  }
+              });
     crew_sync();
 }
 
@@ -818,16 +1018,20 @@ __device__ __forceinline__ int cta_substep(Shared& S, const Job& J, const Box& b
         const float* __restrict__ H = J.h;
         const int hi0 = max(b.i0 - 2, 0), hi1 = min(b.i1 + 2, res - 1);
         const int hj0 = max(b.j0 - 2, 0), hj1 = min(b.j1 + 2, res - 1);
-        CLU_RECT(hi0, hi1, hj0, hj1, { sa[g] = bed[g] + H[g]; })
+        struct Two {
+            float a, b;
+        };
+        clu_items(hi0, hi1, hj0, hj1, [&](int i, int j) { return Two{bed[j * res + i], H[j * res + i]}; },
+                  [&](int i, int j, const Two& t) { sa[j * res + i] = t.a + t.b; });
     }
     crew_sync();
     if (walled) {
         cta_lift(J, b, sa);
         crew_sync();
     }
-    cta_blur_pair(sa, sb, scc, se, J.f1, res, b, [&](int g, float gauss, float steep) {
+    cta_blur_pair(sa, sb, scc, se, J.f1, sa, res, b, [&](int g, float gauss, float steep, float eta) {
         float filtered = 0.62f * gauss + 0.38f * steep;
-        sd[g] = 0.45f * filtered + 0.55f * sa[g];
+        sd[g] = 0.45f * filtered + 0.55f * eta;
     });
     const bool par = (b.j1 - b.j0 >= 47) && (b.i1 - b.i0 >= 31) && inner_par;
     int passes = 0;
@@ -844,45 +1048,65 @@ __device__ __forceinline__ int cta_substep(Shared& S, const Job& J, const Box& b
     }
     const bool project = !fine || walled;
     if (project) {
-        CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-            const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1), jm = max(j - 1, 0);
-            float ux = fdiv(J.u[j * res + ip] - J.u[j * res + im], J.div.two);
-            float vz = fdiv(J.v[jp * res + i] - J.v[jm * res + i], J.div.two);
-            float div = ux + vz;
-            float s = sa[j * res + ip] + sa[j * res + im] + sa[jp * res + i] + sa[jm * res + i] - 4.0f * sa[g];
-            float lap_h = fdiv(s, J.div.cell2);
-            float overload = 1.0f + rclamp(fdiv(job_nu(J, g), J.div.d231), 0.0f, 6.0f);
-            sb[g] = div * overload - 0.015f * overload * lap_h;
-        })
+        struct Cell {
+            float u[2], v[2], e[5], nu;
+        };
+        const float *__restrict__ U = J.u, *__restrict__ V = J.v;
+        clu_items(b.i0, b.i1, b.j0, b.j1,
+                  [&](int i, int j) {
+                      const int g = j * res + i;
+                      const int l = j * res + max(i - 1, 0), r = j * res + min(i + 1, res - 1);
+                      const int d = max(j - 1, 0) * res + i, u = min(j + 1, res - 1) * res + i;
+                      return Cell{{U[r], U[l]}, {V[u], V[d]}, {sa[r], sa[l], sa[u], sa[d], sa[g]}, job_nu(J, g)};
+                  },
+                  [&](int i, int j, const Cell& c) {
+                      float ux = fdiv(c.u[0] - c.u[1], J.div.two);
+                      float vz = fdiv(c.v[0] - c.v[1], J.div.two);
+                      float div = ux + vz;
+                      float s = c.e[0] + c.e[1] + c.e[2] + c.e[3] - 4.0f * c.e[4];
+                      float lap_h = fdiv(s, J.div.cell2);
+                      float overload = 1.0f + rclamp(fdiv(c.nu, J.div.d231), 0.0f, 6.0f);
+                      sb[j * res + i] = div * overload - 0.015f * overload * lap_h;
+                  });
         crew_sync();
-        cta_blur_pair(sb, scc, sa, se, J.f1, res, b,
-                      [&](int g, float gauss, float steep) { sd[g] = 0.62f * gauss + 0.38f * steep; });
+        // No own value is needed here: `also` is any plane of the window.
+        cta_blur_pair(sb, scc, sa, se, J.f1, J.h, res, b, [&](int g, float gauss, float steep, float) {
+            sd[g] = 0.62f * gauss + 0.38f * steep;
+        });
     }
     {
         const float* __restrict__ H = J.h;
         float* __restrict__ U = J.u;
         float* __restrict__ V = J.v;
-        CLU_RECT(b.i0, b.i1, b.j0, b.j1, {
-            if (H[g] > eps) {
-                float uu = U[g], vv = V[g];
-                if (project) {
-                    const int ip = min(i + 1, res - 1), im = max(i - 1, 0), jp = min(j + 1, res - 1),
-                              jm = max(j - 1, 0);
-                    float qx = fdiv(sd[j * res + ip] - sd[j * res + im], J.div.two);
-                    float qz = fdiv(sd[jp * res + i] - sd[jm * res + i], J.div.two);
-                    uu += 0.012f * dt * qx;
-                    vv += 0.012f * dt * qz;
-                }
-                float decay = job_decay(J, g, dt, decay_c);
-                U[g] = finite_speed(uu * decay, kSpeedCap);
-                V[g] = finite_speed(vv * decay, kSpeedCap);
-            }
-        })
+        struct Cell {
+            float h, u, v, q[4], damp;
+        };
+        clu_items(b.i0, b.i1, b.j0, b.j1,
+                  [&](int i, int j) {
+                      const int g = j * res + i;
+                      const int l = j * res + max(i - 1, 0), r = j * res + min(i + 1, res - 1);
+                      const int d = max(j - 1, 0) * res + i, u = min(j + 1, res - 1) * res + i;
+                      return Cell{H[g], U[g], V[g], {sd[r], sd[l], sd[u], sd[d]}, job_damp_source(J, g)};
+                  },
+                  [&](int i, int j, const Cell& c) {
+                      if (!(c.h > eps)) return;
+                      const int g = j * res + i;
+                      float uu = c.u, vv = c.v;
+                      if (project) {
+                          float qx = fdiv(c.q[0] - c.q[1], J.div.two);
+                          float qz = fdiv(c.q[2] - c.q[3], J.div.two);
+                          uu += 0.012f * dt * qx;
+                          vv += 0.012f * dt * qz;
+                      }
+                      float decay = job_decay(J, c.damp, dt, decay_c);
+                      U[g] = finite_speed(uu * decay, kSpeedCap);
+                      V[g] = finite_speed(vv * decay, kSpeedCap);
+                  });
     }
     crew_sync();
     if (walled) {
-        cta_redirect(J, b, dt);
-        cta_block(J, b);
+        cta_redirect(S, J, b, dt);
+        cta_block(S, J, b);
         crew_sync();
         cta_ghost(J, b);
         crew_sync();
@@ -1109,11 +1333,11 @@ __device__ __forceinline__ bool next_run(const unsigned int* row, int W, int pos
 // sheet_work_boxes (src/fluid_core.rs:1325-1447) on rank 0 from the window's
 // wet bits: the wet extent, the bodies (4-connected, in the order of their
 // first raster cells), their boxes. Everything is in shared memory. One thread
-// lists a row's runs; runs that touch the row above's then hook the larger of
-// the two bodies' labels to the smaller and every run jumps to its root, until
-// a round finds nothing to hook (run indices are in raster order, so a body's
-// root is its first run; jumping halves the chains that hooking makes, where
-// walking them took 17 to 33 us). By cells in global memory
+// lists a row's runs; each run goes under the first it touches in the row
+// above, every run jumps to its root, and the parts this leaves are joined by
+// union-find (run indices are in raster order and the smaller label wins, so a
+// body's root is its first run; the jumps halve the chains, where walking them
+// took 17 to 33 us). By cells in global memory
 // (crew_label_bodies, still taken past MAX_RUNS) the labels took 28 us and the
 // boxes 17 of the 104 of a 200 x 200 window with a puddle; this takes 3 (148
 // runs of a half-flooded 64 x 64: 11).
@@ -1180,41 +1404,64 @@ __device__ void rank0_wet_boxes(Shared& S, const Job& J) {
         }
     }
     __syncthreads();
-    for (int round = 0; round <= nruns; ++round) {
-        // Labels are roots here. Two that touch: the larger goes to the smaller.
-        int hooked = 0;
-        if (j > 0 && runs > 0) {
-            int a = S.row_count[j - 1], b = first;
-            const int a_end = first, b_end = first + runs;
-            while (a < a_end && b < b_end) {
-                const unsigned ra = list[a], rb = list[b];
-                const int as = ra & 1023u, ae = ra >> 10 & 1023u, bs = rb & 1023u, be = rb >> 10 & 1023u;
-                if (as <= be && bs <= ae) {
-                    const int x = lab[a], y = lab[b];
-                    if (x != y) {
-                        atomicMin(&S.lab[max(x, y)], min(x, y));
-                        hooked = 1;
-                    }
-                }
-                if (ae < be)
-                    ++a;
-                else
-                    ++b;
-            }
+    // Every pair of runs that touch, this row's against the row above's.
+    auto pairs = [&](auto join) {
+        if (j == 0 || runs == 0) return;
+        int a = S.row_count[j - 1], b = first;
+        const int a_end = first, b_end = first + runs;
+        while (a < a_end && b < b_end) {
+            const unsigned ra = list[a], rb = list[b];
+            const int as = ra & 1023u, ae = ra >> 10 & 1023u, bs = rb & 1023u, be = rb >> 10 & 1023u;
+            if (as <= be && bs <= ae) join(a, b);
+            if (ae < be)
+                ++a;
+            else
+                ++b;
         }
-        if (!__syncthreads_or(hooked)) break;
+    };
+    // The root of x, halving the way there (only roots are hooked, so a label
+    // written along the way is an ancestor still).
+    auto root = [&](int x) {
         for (;;) {
-            int jumped = 0;
-            for (int r = threadIdx.x; r < nruns; r += NT) {
-                const int x = lab[r], y = lab[x];
-                if (x != y) {
-                    lab[r] = y;
-                    jumped = 1;
-                }
-            }
-            if (!__syncthreads_or(jumped)) break;
+            const int y = lab[x];
+            if (y == x) return x;
+            const int z = lab[y];
+            if (z != y) lab[x] = z;
+            x = z;
         }
+    };
+    // First each run under the smallest it touches above, which may leave a
+    // body in a few parts; then the parts by union-find, whose walks are short.
+    pairs([&](int a, int b) { atomicMin(&S.lab[b], a); });
+    __syncthreads();
+    // These chains are as long as the window is high: all runs jump until none
+    // moves.
+    for (;;) {
+        int jumped = 0;
+        for (int r = threadIdx.x; r < nruns; r += NT) {
+            const int x = lab[r], y = lab[x];
+            if (x != y) {
+                lab[r] = y;
+                jumped = 1;
+            }
+        }
+        if (!__syncthreads_or(jumped)) break;
     }
+    pairs([&](int a, int b) {
+        for (int x = a, y = b;;) {
+            x = root(x);
+            y = root(y);
+            if (x == y) break;
+            const int up = max(x, y), down = min(x, y);
+            if (atomicCAS(&S.lab[up], up, down) == up) break;
+        }
+    });
+    __syncthreads();
+    for (int r = threadIdx.x; r < nruns; r += NT) {
+        const int x = root(r);
+        if (x != r) lab[r] = x;
+    }
+    __syncthreads();
     // The bodies numbered by their roots' order. More than MAX_BOXES: step the
     // whole box. The reference merges the grown bodies first and only then
     // falls back at more than 8 boxes, so this differs from it only when over
@@ -1484,7 +1731,8 @@ __device__ __forceinline__ int window_body(Shared& S, const Job& J) {
     if (J.soften_edge > 0) cta_soften(J);
     if (J.solid) {
         crew_sync();
-        cta_displace(J);
+        find_wall_rows(S, J);
+        cta_displace(S, J);
     }
     const bool open_fine = !J.solid && J.cell <= kFineCell + 1.0e-6f;
     const bool fine_open = open_fine && J.pace == 0;
