@@ -22,6 +22,7 @@
 // reads is a value the full-grid pass computes the same way; dry cells carry
 // no flux and no force. The full-grid pass therefore gives the reference's
 // depths and velocities on every cell that holds fluid.
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <type_traits>
@@ -31,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include "sheet_grid.cuh"
+#include "block_sum.cuh"
 #include "sheet_math.cuh"
 #include "launch_count.cuh"
 
@@ -1354,22 +1356,40 @@ __global__ void k_apply_cut(const float* h, float* u, float* v, size_t n, float 
         if (h[i] < eps) { u[i] = 0.0f; v[i] = 0.0f; }
 }
 
-// Largest squared speed, for the CFL substep count (src/fluid_core.rs:1723-1744).
-__global__ void k_max_speed2(const float* h, const float* u, const float* v, size_t n, float eps, int apply_cut,
-                             unsigned int* out_bits) {
+// Largest squared speed, for the CFL substep count (src/fluid_core.rs:1723-1744),
+// and the depth sum of the wet test (:840-844), in one reading of the planes:
+// as two passes they took 26 us of a flooded 1000^2 operator step's 214.
+__global__ void __launch_bounds__(256) k_speed_sum(const float* h, const float* u, const float* v, size_t n,
+                                                   unsigned int* bits, double* sum) {
     ::silt::dep_wait();
     float m = 0.0f;
+    double s = 0.0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        float uu = u[i], vv = v[i];
-        if (apply_cut && h[i] < eps) continue;
-        float s2 = uu * uu + vv * vv;
+        const float uu = u[i], vv = v[i], hv = h[i];
+        const float s2 = uu * uu + vv * vv;
         if (s2 > m) m = s2;
+        s += (double)fmaxf(hv, 0.0f);
     }
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out_bits, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax(bits, __float_as_uint(m));
+    block_add(s, sum);
 }
 
-// k_max_speed2 over the stepped tiles of substep 0's list (every tile that
+// One pass for what were three plane copies and the dry cut.
+__global__ void __launch_bounds__(256) k_finish(const float* h1, const float* u1, const float* v1, float* h, float* u,
+                                                float* v, size_t n, float eps, const double* sum, double wet) {
+    ::silt::dep_wait();
+    if (!(*sum > wet)) return;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const float hv = h1[i], uu = u1[i], vv = v1[i];
+        const bool dry = hv < eps;
+        h[i] = hv;
+        u[i] = dry ? 0.0f : uu;
+        v[i] = dry ? 0.0f : vv;
+    }
+}
+
+// The largest squared speed over the stepped tiles of substep 0's list (every tile that
 // may hold water is one of them; a tile without water has no cell at or above
 // eps and, after the dry cut, no velocity). Each thread loads its four cells
 // before comparing, so a tile costs one memory round trip.
@@ -1804,11 +1824,18 @@ cudaError_t launch_apply_cut(const float* h, float* u, float* v, size_t n, float
     return cudaGetLastError();
 }
 
-cudaError_t launch_max_speed2(const float* h, const float* u, const float* v, size_t n, float eps, int apply_cut,
-                              unsigned int* out_bits, cudaStream_t st) {
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    ::silt::launch_dep(k_max_speed2, dim3(blocks), dim3(256), 0, st, h, u, v, n, eps, apply_cut, out_bits);
+cudaError_t launch_speed_sum(const float* h, const float* u, const float* v, size_t n, unsigned int* bits, double* sum,
+                             cudaStream_t st) {
+    const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 8);
+    ::silt::launch_dep(k_speed_sum, dim3(blocks), dim3(256), 0, st, h, u, v, n, bits, sum);
+    ::silt::count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_finish(const float* h1, const float* u1, const float* v1, float* h, float* u, float* v, size_t n,
+                          float eps, const double* sum, double wet, cudaStream_t st) {
+    const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+    ::silt::launch_dep(k_finish, dim3(blocks), dim3(256), 0, st, h1, u1, v1, h, u, v, n, eps, sum, wet);
     ::silt::count_launch();
     return cudaGetLastError();
 }

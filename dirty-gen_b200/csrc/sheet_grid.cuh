@@ -202,7 +202,13 @@ cudaError_t launch_transport(const TransportLaunch& L, int res, int layers, cuda
 cudaError_t launch_material(const uint8_t* grain, const float* moisture, float* nu, float* mob, float* damp, size_t n,
                             cudaStream_t st);
 cudaError_t launch_apply_cut(const float* h, float* u, float* v, size_t n, float eps, cudaStream_t st);
-cudaError_t launch_max_speed2(const float* h, const float* u, const float* v, size_t n, float eps, int apply_cut,
-                              unsigned int* out_bits, cudaStream_t st);
+// The largest squared speed of every cell (atomicMax of its bits into *bits)
+// and the FP64 sum of max(h, 0) (into *sum); both start at zero.
+cudaError_t launch_speed_sum(const float* h, const float* u, const float* v, size_t n, unsigned int* bits, double* sum,
+                             cudaStream_t st);
+// A free-operator substep's results into the caller's planes, dry cut applied;
+// nothing when *sum is not above `wet` (the sheet was dry).
+cudaError_t launch_finish(const float* h1, const float* u1, const float* v1, float* h, float* u, float* v, size_t n,
+                          float eps, const double* sum, double wet, cudaStream_t st);
 
 }  // namespace silt

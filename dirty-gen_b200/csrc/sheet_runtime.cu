@@ -2880,6 +2880,28 @@ static int step_sheet_window(float* h, float* u, float* v, const float* bed, con
     return SILT_OK;
 }
 
+// Where silt_step_sheet reads the speed bits and the depth sum back: 48 pinned
+// bytes and an event per calling thread and device, given back when the
+// thread ends. (A pageable read-back holds the host until the copy is done
+// and with it the launches behind it.)
+struct SpeedSum {
+    unsigned int* host = nullptr;
+    cudaEvent_t ev = nullptr;
+    ~SpeedSum() {
+        if (host) cudaFreeHost(host);
+        if (ev) cudaEventDestroy(ev);
+    }
+};
+static SpeedSum* speed_sum_slot() {
+    static thread_local std::map<int, SpeedSum> slots;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    SpeedSum& s = slots[dev];
+    if (!s.host && cudaMallocHost(&s.host, 48) != cudaSuccess) s.host = nullptr;
+    if (!s.ev && cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming) != cudaSuccess) s.ev = nullptr;
+    return s.host && s.ev ? &s : nullptr;
+}
+
 int silt_step_sheet(float* h, float* u, float* v, const float* bed, const float* nu, const uint8_t* gate, int32_t res,
                     float cell, float dt, float vorticity, void* scratch, void* stream) {
     if (!h || !u || !v || !bed || !nu || !scratch || res <= 0) return fail_arg("step_sheet");
@@ -2917,21 +2939,17 @@ int silt_step_sheet(float* h, float* u, float* v, const float* bed, const float*
         tf.count = tf.list + 2 * nt;
         tf.tiles_x = tx;
     }
-    CK(cudaMemsetAsync(d_bits, 0, 32, st));
-    CK(silt::launch_max_speed2(h, u, v, n, 1.0e-6f, 0, d_bits, st));
-    CK(silt::op_sum2(h, h, n, d_sum, st));
-    unsigned int bits = 0;
-    double sums[2];
-    CK(cudaMemcpyAsync(&bits, d_bits, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(sums, d_sum, 16, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (!(sums[0] > 1.0e-6)) return SILT_OK_NOOP;  // nothing wet (src/fluid_core.rs:873-879)
-    float m2;
-    memcpy(&m2, &bits, 4);
-    float max_s = std::max(0.15f, sqrtf(m2));
-    int nsub = (int)silt::host::rclamp(ceilf((dt * max_s) / (0.42f * std::max(cell, 1.0e-3f))), 1.0f, 8.0f);
-    float dts = dt / (float)nsub;
-    for (int k = 0; k < nsub; ++k) {
+    CK(cudaMemsetAsync(d_bits, 0, 48, st));
+    CK(silt::launch_speed_sum(h, u, v, n, d_bits, d_sum, st));
+    SpeedSum* const back = speed_sum_slot();
+    if (!back) return fail_cuda(cudaErrorMemoryAllocation, "step_sheet read-back");
+    CK(cudaMemcpyAsync(back->host, scratch, 48, cudaMemcpyDeviceToHost, st));
+    CK(cudaEventRecord(back->ev, st));
+    // Substep k: the first one's dt is the device's own (dt over the count of
+    // the speed it just measured), so it is queued before the host has read
+    // the speed and the sum and runs while it does; a sheet with nothing wet
+    // takes it into the scratch planes and no further (launch_finish).
+    auto substep = [&](float dts, const silt::SubstepCount& count) -> int {
         silt::ForceLaunch F;
         silt::TransportLaunch T;
         memset(&F, 0, sizeof F);
@@ -2973,16 +2991,38 @@ int silt_step_sheet(float* h, float* u, float* v, const float* bed, const float*
         T.tf = tf;
         F.nxt = 1;
         T.nxt = 1;
+        F.sc = count;
+        T.sc = count;
         silt::SubstepCount host_count;
         memset(&host_count, 0, sizeof host_count);
         CK(silt::launch_tile_list(tf, 0, 1, 1, 0, 1, host_count, nullptr, nullptr, nullptr, st));
         CK(silt::launch_force(F, res, 1, st));
         CK(silt::launch_transport(T, res, 1, st));
-        CK(cudaMemcpyAsync(h, h_next, n * 4, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(u, u_mid, n * 4, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(v, v_mid, n * 4, cudaMemcpyDeviceToDevice, st));
-        CK(silt::launch_apply_cut(h, u, v, n, 1.0e-6f, st));
-    }
+        CK(silt::launch_finish(h_next, u_mid, v_mid, h, u, v, n, 1.0e-6f, d_sum, 1.0e-6, st));
+        return SILT_OK;
+    };
+    silt::SubstepCount count;
+    memset(&count, 0, sizeof count);
+    count.speed2 = d_bits;
+    count.overflow = d_bits + 2;  // never set: the host launches every substep the device counts
+    count.dt = dt;
+    count.cell = cell;
+    count.cap = 8.0f;
+    count.launched = 8;
+    int rc = substep(dt, count);
+    if (rc) return rc;
+    CK(cudaEventSynchronize(back->ev));
+    const unsigned int bits = back->host[0];
+    double sum;
+    memcpy(&sum, back->host + 8, sizeof sum);
+    if (!(sum > 1.0e-6)) return SILT_OK_NOOP;  // nothing wet (src/fluid_core.rs:873-879)
+    float m2;
+    memcpy(&m2, &bits, 4);
+    float max_s = std::max(0.15f, sqrtf(m2));
+    int nsub = (int)silt::host::rclamp(ceilf((dt * max_s) / (0.42f * std::max(cell, 1.0e-3f))), 1.0f, 8.0f);
+    memset(&count, 0, sizeof count);
+    for (int k = 1; k < nsub; ++k)
+        if ((rc = substep(dt / (float)nsub, count))) return rc;
     return SILT_OK;
 }
 

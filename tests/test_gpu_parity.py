@@ -167,6 +167,85 @@ def test_free_step_sheet_matches_oracle(res, cell, dt, vort):
     assert dh <= TOL_H, dh
 
 
+def free_operator(res, speed, depth):
+    """A disc of water on a wavy slope for the operator on tiles: step(dt) on
+    the device, its planes, and the host's copies."""
+    import torch
+    n = res * res
+    jj, ii = np.mgrid[0:res, 0:res]
+    bed = (-0.01 * jj + 0.02 * np.sin(ii * 0.3)).astype(np.float32).ravel()
+    wet = (((ii - res / 2) ** 2 + (jj - res / 3) ** 2) < (res / 5) ** 2).ravel()
+    h = np.where(wet, depth, 0.0).astype(np.float32)
+    u = np.where(wet, speed, 0.0).astype(np.float32)
+    v = np.where(wet, -0.25 * speed, 0.0).astype(np.float32)
+    nu = np.full(n, 0.05, np.float32)
+    dev = [torch.tensor(x, device="cuda") for x in (h, u, v, bed, nu)]
+    gate = torch.ones(n, dtype=torch.uint8, device="cuda")
+    scratch = torch.zeros(G.lib().silt_step_sheet_scratch_bytes(res) // 4 + 16, dtype=torch.float32, device="cuda")
+
+    def step(dt):
+        rc = G.step_sheet_device(*[x.data_ptr() for x in dev], gate.data_ptr(), res, 0.1, dt, 0.02, scratch.data_ptr())
+        torch.cuda.synchronize()
+        return rc
+
+    return step, dev, (h, u, v, bed, nu)
+
+
+@pytest.mark.parametrize("res,speed,depth", [(513, 0.0, 0.05), (520, 0.4, 3.0e-6)])
+def test_free_step_sheet_above_512_matches_oracle(res, speed, depth):
+    """Still water, and a film whose cells cross the dry cut."""
+    step, dev, (h, u, v, bed, nu) = free_operator(res, speed, depth)
+    gate, sc = np.ones(res * res, np.uint8), O.Scratch()
+    for _ in range(3):
+        O.step_sheet(h, u, v, bed, nu, gate, res, 0.1, 0.05, 0.02, scratch=sc)
+        assert step(0.05) == 0
+    dh = np.abs(dev[0].cpu().numpy() - h).max()
+    assert dh <= TOL_H, dh
+
+
+@pytest.mark.parametrize("res,speed,count", [(513, 0.5, 1), (600, 2.6, 4), (515, 5.0, 7)])
+def test_free_step_sheet_above_512_counts_its_substeps(res, speed, count):
+    """The first substep's dt is the device's own count of the speed, the
+    others' is the host's: one call gives the same bits as `count` calls with
+    a `count`-th of its dt, each of which takes one substep."""
+    import torch
+    dt = np.float32(0.05)
+    assert int(np.ceil(dt * np.float32(np.hypot(speed, 0.25 * speed)) / np.float32(0.042))) == count
+    whole, a, _ = free_operator(res, speed, 0.05)
+    parts, b, _ = free_operator(res, speed, 0.05)
+    assert whole(float(dt)) == 0
+    for _ in range(count):
+        assert parts(float(dt / np.float32(count))) == 0
+    assert all(torch.equal(x, y) for x, y in zip(a[:3], b[:3]))
+
+
+def test_free_step_sheet_above_512_leaves_a_dry_sheet_alone():
+    """At or below 1e-6 of summed depth the operator is a no-op: its return
+    value says so and no plane changes, on a fresh sheet and after a wet one."""
+    import torch
+    res = 520
+    scratch = torch.zeros(G.lib().silt_step_sheet_scratch_bytes(res) // 4 + 16, dtype=torch.float32, device="cuda")
+    z = torch.zeros(res * res, device="cuda")
+    gate = torch.ones(res * res, dtype=torch.uint8, device="cuda")
+    nu = torch.full_like(z, 0.05)
+
+    def step(h, u, v):
+        return G.lib().silt_step_sheet(h.data_ptr(), u.data_ptr(), v.data_ptr(), z.data_ptr(), nu.data_ptr(),
+                                       gate.data_ptr(), res, 0.1, 0.05, 0.0, scratch.data_ptr(), None)
+
+    for k in range(3):
+        dry = [z.clone(), torch.full_like(z, 0.3), torch.full_like(z, -0.2)]
+        dry[0][:5] = 1.0e-7
+        was = [x.clone() for x in dry]
+        torch.cuda.synchronize()
+        assert step(*dry) == 1  # SILT_OK_NOOP
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(dry, was)), k
+        wet = [torch.full_like(z, 0.05), z.clone(), z.clone()]
+        torch.cuda.synchronize()
+        assert step(*wet) == 0
+
+
 @pytest.mark.parametrize("engine", [G.ENGINE_WINDOW, G.ENGINE_GRID])
 def test_open_water_and_surface_diffusion_match_oracle(engine):
     """Open-water mode (mobility 1, Manning 0.035, eddy 0.06 m^2/s, the ford
