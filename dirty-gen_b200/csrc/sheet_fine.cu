@@ -625,7 +625,13 @@ __device__ void near_capture_col(int q, const PatchRef* refs, int fres, int sub,
 
 __device__ void restrict_column(const PatchRef* refs, int fres, const SheetView& W, const RestrictEntry& E,
                                 const Segment* segs, float fine_area, float coarse_area, int lane) {
-    float aw = 0.0f, as = 0.0f, auw = 0.0f, avw = 0.0f, aus = 0.0f, avs = 0.0f;
+    // Lane q < 6 keeps sum q. The products of 32 cells go through shared
+    // memory; a cell that is not taken holds +0, which changes no sum (a sum
+    // that starts at +0 is never -0), and 32 cells of which none is taken are
+    // passed over.
+    __shared__ __align__(16) float prod[4][6][32];
+    float(*const mine)[32] = prod[(threadIdx.x >> 5) & 3];
+    float sum = 0.0f;
     for (int sgi = 0; sgi < E.seg_n; ++sgi) {
         const Segment S = segs[E.seg_off + sgi];
         const PatchRef& R = refs[S.patch];
@@ -633,7 +639,7 @@ __device__ void restrict_column(const PatchRef* refs, int fres, const SheetView&
         constexpr int G = 4;  // chunks loaded together before they are summed
         for (int g0 = 0; g0 < nc; g0 += 32 * G) {
             float pw[G], ps[G], puw[G], pvw[G], pus[G], pvs[G];
-            unsigned takes[G];
+            bool takes[G];
 #pragma unroll
             for (int q = 0; q < G; ++q) {
                 const int c = g0 + 32 * q + lane;
@@ -652,27 +658,34 @@ __device__ void restrict_column(const PatchRef* refs, int fres, const SheetView&
                         pvs[q] = R.vs[f] * fs * fine_area;
                     }
                 }
-                takes[q] = __ballot_sync(0xffffffffu, take);
+                takes[q] = __any_sync(0xffffffffu, take);
             }
 #pragma unroll
             for (int q = 0; q < G; ++q) {
-                const int m = min(32, nc - (g0 + 32 * q));
-                for (int b = 0; b < m; ++b) {
-                    const float xw = __shfl_sync(0xffffffffu, pw[q], b), xs = __shfl_sync(0xffffffffu, ps[q], b);
-                    const float xuw = __shfl_sync(0xffffffffu, puw[q], b), xvw = __shfl_sync(0xffffffffu, pvw[q], b);
-                    const float xus = __shfl_sync(0xffffffffu, pus[q], b), xvs = __shfl_sync(0xffffffffu, pvs[q], b);
-                    if ((takes[q] >> b) & 1u) {
-                        aw += xw;
-                        as += xs;
-                        auw += xuw;
-                        avw += xvw;
-                        aus += xus;
-                        avs += xvs;
-                    }
+                if (!takes[q]) continue;
+                mine[0][lane] = pw[q];
+                mine[1][lane] = ps[q];
+                mine[2][lane] = puw[q];
+                mine[3][lane] = pvw[q];
+                mine[4][lane] = pus[q];
+                mine[5][lane] = pvs[q];
+                __syncwarp();
+                const float4* row = reinterpret_cast<const float4*>(mine[lane < 6 ? lane : 5]);
+#pragma unroll
+                for (int b = 0; b < 8; ++b) {
+                    const float4 x = row[b];
+                    sum += x.x;
+                    sum += x.y;
+                    sum += x.z;
+                    sum += x.w;
                 }
+                __syncwarp();
             }
         }
     }
+    const float aw = __shfl_sync(0xffffffffu, sum, 0), as = __shfl_sync(0xffffffffu, sum, 1);
+    const float auw = __shfl_sync(0xffffffffu, sum, 2), avw = __shfl_sync(0xffffffffu, sum, 3);
+    const float aus = __shfl_sync(0xffffffffu, sum, 4), avs = __shfl_sync(0xffffffffu, sum, 5);
     if (lane != 0) return;
     const size_t idx = E.cidx;
     const float w = aw / coarse_area, s = as / coarse_area;
@@ -716,8 +729,8 @@ __device__ void restrict_column(const PatchRef* refs, int fres, const SheetView&
 
 // restrict_fine (src/fluid_core.rs:8462-8555): one warp per touched coarse
 // column. The lanes load 32 fine cells at a time and form their products in
-// parallel; the six sums then take the products one by one in the
-// reference's raster order (every lane adds the same sequence).
+// parallel; six lanes then add one sum each, product by product in the
+// reference's raster order.
 // Blocks [0, ncap) capture the near-field residual of one held column each
 // (with `ncap` = 0 when the near field is off); the rest restrict, a warp per
 // touched coarse column. Both read the fine cells after the peel and write

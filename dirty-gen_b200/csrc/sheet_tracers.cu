@@ -44,6 +44,7 @@ enum : uint8_t { WET = 1, SHORE = 2, LIVE = 4 };
 struct Ctl {
     int active;     // the tracer step runs at all (wake, live silt or live foam)
     int cbox[4];    // the step's collection box
+    int tspan1[4];  // silt span at the step's start
     int tspan2[4];  // silt span after the transport
     int tspan3[4];  // silt span after the sources
     int mbox[4];    // where wet and shore marks may be set (the last collection box)
@@ -220,50 +221,45 @@ __device__ __forceinline__ void grown(const int* b, int res, int& i0, int& i1, i
     j1 = min(b[3] + 1, res - 1);
 }
 
-// Every cell of the job's window (blockIdx.y is the job, blockIdx.x strides
-// its cells). Indices are 32-bit: a window holds fewer than 2^32 cells.
+// Every cell of the job's window (block at_ of the of_ that work on it). Indices are 32-bit: a window holds fewer than 2^32 cells.
 #define CELLS(S)                                                                                                  \
-    for (unsigned g = blockIdx.x * blockDim.x + threadIdx.x, n_ = (unsigned)(S).res * (unsigned)(S).res; g < n_; \
-         g += gridDim.x * blockDim.x)
+    for (unsigned g = at_ * blockDim.x + threadIdx.x, n_ = (unsigned)(S).res * (unsigned)(S).res; g < n_; \
+         g += of_ * blockDim.x)
 
 // The cells (i, j, g) of the box [i0, i1] x [j0, j1] (inclusive) of a window
 // `res` cells wide; `continue` moves to the next cell.
 #define BOX_CELLS(res, i0, i1, j0, j1)                                                                  \
-    for (unsigned q_ = blockIdx.x * blockDim.x + threadIdx.x, w_ = (unsigned)max((i1) - (i0) + 1, 0),    \
+    for (unsigned q_ = at_ * blockDim.x + threadIdx.x, w_ = (unsigned)max((i1) - (i0) + 1, 0),    \
                   n_ = w_ * (unsigned)max((j1) - (j0) + 1, 0);                                          \
-         q_ < n_; q_ += gridDim.x * blockDim.x)                                                        \
+         q_ < n_; q_ += of_ * blockDim.x)                                                        \
         for (int once_ = 1, i = (i0) + (int)(q_ % w_), j = (j0) + (int)(q_ / w_); once_; once_ = 0)        \
             for (unsigned g = (unsigned)j * (unsigned)(res) + (unsigned)i; once_; once_ = 0)
 
-// The 128-cell segments of a row of a `res`-wide window (cells 128 s .. 128 s + 127).
-__host__ __device__ __forceinline__ int segments(int res) { return (res + 127) / 128; }
+// The passes over whole windows give a warp 128 cells of a row of the box at a
+// time (a run; each load coalesced, a thread's four independent): lane l has
+// the cells ib, ib + 32, ib + 64 and ib + 96 with ib = the run's first + l.
+struct Runs {
+    int i0, j0;
+    unsigned nx, n;
+    __device__ __forceinline__ Runs(int i0_, int i1, int j0_, int j1)
+        : i0(i0_), j0(j0_), nx((unsigned)max(i1 - i0_ + 128, 0) / 128u), n(nx * (unsigned)max(j1 - j0_ + 1, 0)) {}
+    __device__ __forceinline__ void at(unsigned r, int& ib, int& j) const {
+        j = j0 + (int)(r / nx);
+        ib = i0 + (int)(r % nx) * 128 + (int)(threadIdx.x & 31);
+    }
+};
 
-// QUAD_ROWS over whole segments: every segment that meets the columns
-// [i0, i1], in the rows [j0, j1], one per warp iteration. Declares j, s and
-// ib = 128 s + lane; the cells outside [i0, i1] are the caller's to skip.
-#define QUAD_SEGS(res, i0, i1, j0, j1)                                                                          \
-    for (unsigned it_ = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, s0_ = (unsigned)max((i0), 0) >> 7,        \
-                  nx_ = (i1) >= (i0) ? ((unsigned)(i1) >> 7) - s0_ + 1u : 0u,                                 \
-                  n_ = nx_ * (unsigned)max((j1) - (j0) + 1, 0);                                               \
-         it_ < n_; it_ += (gridDim.x * blockDim.x) >> 5)                                                        \
-        for (int once_ = 1, j = (j0) + (int)(it_ / nx_), s = (int)(s0_ + it_ % nx_), ib = s * 128 + (int)(threadIdx.x & 31); \
-             once_; once_ = 0)
-
-// Four cells per thread for the passes over whole windows: a warp takes 128
-// consecutive cells of a row of the box, lane l the cells ib, ib + 32,
-// ib + 64, ib + 96 with ib = start + l (each load coalesced; a thread's four
-// loads independent). Declares j and ib.
-#define QUAD_ROWS(res, i0, i1, j0, j1)                                                                          \
-    for (unsigned it_ = (blockIdx.x * blockDim.x + threadIdx.x) >> 5,                                           \
-                  nx_ = (unsigned)max((i1) - (i0) + 128, 0) / 128u, n_ = nx_ * (unsigned)max((j1) - (j0) + 1, 0); \
-         it_ < n_; it_ += (gridDim.x * blockDim.x) >> 5)                                                        \
-        for (int once_ = 1, j = (j0) + (int)(it_ / nx_), ib = (i0) + (int)(it_ % nx_) * 128 + (int)(threadIdx.x & 31); \
-             once_; once_ = 0)
-
+// This block's job, and which of the of_ blocks on that job it is (at_). A
+// launch over several windows lists its blocks (`slices`, see split_blocks);
+// one over a single window, or with one block per job, has no list.
 // The job is copied into registers: the planes' stores would otherwise make
 // the compiler reload its fields from memory after every write.
-#define JOB                              \
-    const Job J = jobs[blockIdx.y];      \
+#define JOB                                                                                                      \
+    const Slice slice_ = slices ? slices[blockIdx.x] : Slice{(int)blockIdx.y, blockIdx.x, gridDim.x};             \
+    const unsigned at_ = slice_.at, of_ = slice_.of;                                                              \
+    (void)at_;                                                                                                    \
+    (void)of_;                                                                                                    \
+    const Job J = jobs[slice_.job];                                                                               \
     const Sheet& S = J.S;                \
     const Planes& T = J.T;               \
     (void)S;                             \
@@ -286,25 +282,13 @@ __device__ __forceinline__ Box box_union(Box a, Box b) {
     return Box{min(a.i0, b.i0), max(a.i1, b.i1), min(a.j0, b.j0), max(a.j1, b.j1)};
 }
 
-// True when the warp's 128 cells of row j from column ib0 on hold no wet or
-// foam-live mark (the flags of the one or two segments they meet, as this
-// step's wet-set pass left them) and meet no cell of box b: a pass that acts
-// only on such marks and on the cells of b has nothing to do there. Flags of
-// segments the wet-set pass did not visit may be stale, but such segments
-// lie outside its box, where no cell carries a mark.
-__device__ __forceinline__ bool quiet_run(const uint8_t* occ, int res, int j, int ib0, const Box& b) {
-    const int ns = segments(res);
-    const int s0 = ib0 >> 7, s1 = min((ib0 + 127) >> 7, ns - 1);
-    if (occ[j * ns + s0] | occ[j * ns + s1]) return false;
-    return b.empty() || j < b.j0 || j > b.j1 || ib0 + 127 < b.i0 || ib0 > b.i1;
-}
 __device__ __forceinline__ bool in_box(const Box& b, int i, int j) {
     return i >= b.i0 && i <= b.i1 && j >= b.j0 && j <= b.j1;
 }
 
 // ------------------------------------------------------------ entrain_wake
 
-__global__ void k_entrain(const Job* jobs) {
+__global__ void k_entrain(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     float* susp = T.susp[0];
@@ -312,7 +296,7 @@ __global__ void k_entrain(const Job* jobs) {
     const int res = S.res;
     const float cell = S.cell, area = cell * cell;
     double b = 0.0;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && J.ebox[0] <= J.ebox[1]) {
+    if (at_ == 0 && threadIdx.x == 0 && J.ebox[0] <= J.ebox[1]) {
         int* sup = ctl_of(T.st)->ssup_next;  // the wake's cells may now hold a load
         atomicMin(&sup[0], J.ebox[0]);
         atomicMax(&sup[1], J.ebox[1]);
@@ -365,11 +349,12 @@ __global__ void k_entrain(const Job* jobs) {
 // whole window runs only after the planes were rewritten wholesale (attach,
 // window moves). Launches: [scan], begin (control words and the collection
 // box), collect (with the foam advection into scratch), the silt advection
-// into scratch, commit, settle (with the sync's start), spawn, clear and sync.
+// into scratch (with the sync's start), apply (everything that a cell does
+// alone), clear.
 
 // The start span of the jobs whose planes were rewritten (`rescan`); the
 // reset that rewrote them left the span empty.
-__global__ void k_scan(const Job* jobs) {
+__global__ void k_scan(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     if (!J.rescan) return;
@@ -386,17 +371,21 @@ __global__ void k_scan(const Job* jobs) {
 // tracer_visit_box (:6296-6337). `wake`: a tire with speed or slip, or a
 // surface drive (host-known); `pbox`: the tires' reach boxes (host-computed;
 // empty when none).
-__global__ void k_begin(const Job* jobs) {
+__global__ void k_begin(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (threadIdx.x != 0 || at_ != 0) return;
     State* st = T.st;
     const int res = S.res, wake = J.wake;
     Ctl* c = ctl_of(st);
     box_clear(c->tspan2, res);
     box_clear(c->tspan3, res);
     box_clear(c->cbox, res);
-    st->live_silt = box_empty(st->tspan) ? 0u : 1u;
+    // The start span moves to the step's own words, and k_clear rebuilds it.
+    // (A step that goes no further than the wet set has an empty one.)
+    for (int k = 0; k < 4; ++k) c->tspan1[k] = st->tspan[k];
+    box_clear(st->tspan, res);
+    st->live_silt = box_empty(c->tspan1) ? 0u : 1u;
     st->wet_any = 0;
     c->live_foam_prev = st->live_foam;
     c->active = (wake || st->live_silt || c->live_foam_prev) ? 1 : 0;
@@ -418,9 +407,9 @@ __global__ void k_begin(const Job* jobs) {
         any = true;
     };
     if (c->live_foam_prev) take(st->live_box[0], st->live_box[1], st->live_box[2], st->live_box[3]);
-    if (!box_empty(st->tspan)) {
+    if (st->live_silt) {
         int i0, i1, j0, j1;
-        grown(st->tspan, res, i0, i1, j0, j1);
+        grown(c->tspan1, res, i0, i1, j0, j1);
         take(i0, i1, j0, j1);
     }
     if (J.pbox[0] <= J.pbox[1]) take(J.pbox[0], J.pbox[1], J.pbox[2], J.pbox[3]);
@@ -512,8 +501,8 @@ __device__ __forceinline__ float turbid_after(const Sheet& S, const float* T, in
 // The wet set (marks) and, into scratch, advect_foam (:6352-6397) of every
 // wet or foam-live cell; k_turbid_advect puts advect_turbid of the grown span
 // beside it. Both read only fields no step kernel has changed yet; whether
-// they take effect is decided once the wet set is known (k_go, k_commit).
-__global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs) {
+// they take effect is decided once the wet set is known (k_apply).
+__global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     uint8_t* mark = T.mark;
@@ -530,54 +519,58 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs) {
     const Box b = box_of(c->cbox);
     const Box u = box_union(b, box_of(c->mbox));
     bool any = false;
-    const int ns = segments(res);
-    QUAD_SEGS(res, u.i0, u.i1, u.j0, u.j1) {
-        // The four cells' loads in two rounds: marks and depths, then, for the
-        // wet cells only, the four neighbours' water of the shore test
-        // (shore_wet_cell, :9752-9764: a cell on the window's border is never
-        // shore) and the velocity the foam advection reads.
-        uint8_t mk[4];
-        float hw[4], hs[4], nb[4][4], uw4[4], vw4[4];
-        bool here[4], wet[4], inner[4];
+    // A run's marks and depths are loaded while the run before is worked on
+    // (a cell outside the box holds no water here); for its wet cells only,
+    // the four neighbours' water of the shore test (shore_wet_cell,
+    // :9752-9764: a cell on the window's border is never shore) and the
+    // velocity that the foam advection reads are then the wait of a round.
+    const Runs runs(u.i0, u.i1, u.j0, u.j1);
+    const unsigned warps = (of_ * blockDim.x) >> 5;
+    unsigned run = (at_ * blockDim.x + threadIdx.x) >> 5;
+    unsigned m_next[4];
+    float w_next[4], s_next[4];
+    int ib_next = 0, j_next = 0;
+    auto load_head = [&](unsigned r) {
+        runs.at(r, ib_next, j_next);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            here[k] = i >= u.i0 && i <= u.i1;
-            wet[k] = false;
-            if (here[k]) mk[k] = mark[g];
-            if (here[k] && in_box(b, i, j)) {
-                hw[k] = S.water[g];
-                hs[k] = S.slurry[g];
-                wet[k] = true;
-            }
+            const int i = ib_next + 32 * k;
+            const unsigned g = (unsigned)j_next * (unsigned)res + (unsigned)i;
+            const bool inside = in_box(b, i, j_next);
+            m_next[k] = i <= u.i1 ? mark[g] : 0u;
+            w_next[k] = inside ? S.water[g] : 0.0f;
+            s_next[k] = inside ? S.slurry[g] : 0.0f;
         }
-        // A segment with no wet cell and no foam-live mark: its cells' marks
-        // become 0 and nothing else happens there.
+    };
+    if (run < runs.n) load_head(run);
+    for (; run < runs.n; run += warps) {
+        const int ib = ib_next, j = j_next;
+        const unsigned g0 = (unsigned)j * (unsigned)res + (unsigned)ib;
+        unsigned mk[4];
+        bool wet[4];
+        // A run with no wet cell and no foam-live mark: its cells' marks become
+        // 0 and nothing else happens there.
         bool busy = false;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (here[k] && (mk[k] & LIVE)) busy = true;
-            if (wet[k]) {
-                const float h = hw[k] + hs[k];
-                if (finite_f(h) && !(h < 0.004f)) busy = true;
-            }
+            mk[k] = m_next[k];
+            const float h = w_next[k] + s_next[k];
+            wet[k] = finite_f(h) && !(h < 0.004f);
+            busy = busy || wet[k] || (mk[k] & LIVE);
         }
+        if (run + warps < runs.n) load_head(run + warps);
         if (!__any_sync(0xffffffffu, busy)) {
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-                if (here[k] && mk[k] != 0) mark[(unsigned)j * (unsigned)res + (unsigned)(ib + 32 * k)] = 0;
-            if ((threadIdx.x & 31) == 0) T.occ[j * ns + s] = 0;
+                if (mk[k] != 0) mark[g0 + 32u * k] = 0;
             continue;
         }
+        float nb[4][4], uw4[4], vw4[4];
+        bool inner[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            if (wet[k]) {
-                const float h = hw[k] + hs[k];
-                wet[k] = finite_f(h) && !(h < 0.004f);
-            }
+            const unsigned g = g0 + 32u * k;
             inner[k] = i > 0 && j > 0 && i + 1 < res && j + 1 < res;
             if (!wet[k]) continue;
             if (inner[k]) {
@@ -591,13 +584,11 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs) {
                 vw4[k] = S.vw[g];
             }
         }
-        bool marked = false;  // a wet or foam-live mark among this thread's cells
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (!here[k]) continue;
             const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            uint8_t m = mk[k] & LIVE;
+            const unsigned g = g0 + 32u * k;
+            unsigned m = mk[k] & LIVE;
             if (wet[k]) {
                 m |= WET;
                 any = true;
@@ -606,8 +597,7 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs) {
                     for (int q = 0; q < 4; ++q) shore = shore || (finite_f(nb[k][q]) && nb[k][q] < 0.004f);
                 if (shore) m |= SHORE;
             }
-            mark[g] = m;
-            marked = marked || m != 0;
+            if (m != mk[k]) mark[g] = (uint8_t)m;
             if (foam_on) {
                 if (m & WET) {
                     const float uu = uw4[k], vv = vw4[k];  // wet cells are far above the dry cut
@@ -624,133 +614,47 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs) {
                 }
             }
         }
-        // The warp holds the whole segment (the cells outside the box carry no mark).
-        const unsigned seg = __ballot_sync(0xffffffffu, marked);
-        if ((threadIdx.x & 31) == 0) T.occ[j * ns + s] = seg != 0u ? 1 : 0;
     }
     block_flag(any, &st->wet_any);
 }
 
 // advect_turbid of the grown span into scratch, spread over every block of
 // the launch (a cell's donor sequences are long; in the wet-set pass the
-// few warps holding the span's rows would carry all of them).
-__global__ void k_turbid_advect(const Job* jobs) {
+// few warps holding the span's rows would carry all of them). The cells it
+// leaves above 1e-8 are the span after the transport (outside the grown span
+// no cell holds more). Its first block also makes the sync's start (:6339):
+// the marks' box for the next step's wet set, and the live set, which k_apply
+// rebuilds.
+__global__ void k_turbid_advect(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     State* st = T.st;
-    if (!ctl_of(st)->active || box_empty(st->tspan)) return;
+    Ctl* c = ctl_of(st);
+    if (!c->active) return;
     const int res = S.res;
-    const Box tb = grown_box(st->tspan, res);
+    if (at_ == 0 && threadIdx.x == 0) {
+        for (int k = 0; k < 4; ++k) c->mbox[k] = c->cbox[k];
+        if (step_goes(st)) {
+            st->live_foam = 0;
+            box_clear(st->live_box, res);
+        }
+    }
+    if (box_empty(c->tspan1)) return;
+    const Box tb = grown_box(c->tspan1, res);
     const float* silt = T.turbid[0];
     float* ttmp = T.turbid[1];
+    LocalBox lb;
     BOX_CELLS(res, tb.i0, tb.i1, tb.j0, tb.j1) {
         // A cell without silt beside neighbours without silt (those inside the
         // span) keeps its value: every edge of those columns gives 0.
         const bool still = silt[g] == 0.0f && (i - 1 < tb.i0 || silt[g - 1] == 0.0f) &&
                            (i + 1 > tb.i1 || silt[g + 1] == 0.0f) && (j - 1 < tb.j0 || silt[g - res] == 0.0f) &&
                            (j + 1 > tb.j1 || silt[g + res] == 0.0f);
-        ttmp[g] = still ? silt[g] : turbid_after(S, silt, i, j, tb.i0, tb.i1, tb.j0, tb.j1, J.dt);
-    }
-}
-
-// The advections take effect: foam on every wet or foam-live cell, silt on
-// the grown span, whose cells above 1e-8 are the span after the transport
-// (outside it no cell holds more than 1e-8).
-__global__ void k_commit(const Job* jobs) {
-    ::silt::dep_wait();
-    JOB;
-    State* st = T.st;
-    Ctl* c = ctl_of(st);
-    if (!step_goes(st)) return;
-    const int res = S.res;
-    const bool foam_on = c->live_foam_prev != 0, silt_on = !box_empty(st->tspan);
-    if (!foam_on && !silt_on) return;
-    const Box fb = foam_on ? box_of(c->cbox) : Box{0, -1, 0, -1};
-    const Box tb = silt_on ? grown_box(st->tspan, res) : Box{0, -1, 0, -1};
-    const Box u = box_union(fb, tb);
-    float* foam = T.foam[0];
-    const float* ftmp = T.foam[1];
-    float* silt = T.turbid[0];
-    const float* ttmp = T.turbid[1];
-    const uint8_t* mark = T.mark;
-    LocalBox lb;
-    QUAD_ROWS(res, u.i0, u.i1, u.j0, u.j1) {
-        if (quiet_run(T.occ, res, j, ib - (int)(threadIdx.x & 31), tb)) continue;
-        bool fo[4];
-        float fv[4], tv[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            fo[k] = i <= u.i1 && in_box(fb, i, j) && (mark[(unsigned)j * (unsigned)res + (unsigned)i] & (WET | LIVE));
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            if (fo[k]) fv[k] = ftmp[g];
-            if (i <= u.i1 && in_box(tb, i, j)) tv[k] = ttmp[g];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            if (fo[k]) foam[g] = fv[k];
-            if (i <= u.i1 && in_box(tb, i, j)) {
-                silt[g] = tv[k];
-                if (tv[k] > 1.0e-8f) lb.add(i, j);
-            }
-        }
+        const float t = still ? silt[g] : turbid_after(S, silt, i, j, tb.i0, tb.i1, tb.j0, tb.j1, J.dt);
+        ttmp[g] = t;
+        if (t > 1.0e-8f) lb.add(i, j);
     }
     lb.commit(c->tspan2);
-}
-
-// settle_turbid (:6473-6509) on the span after the transport; the cells it
-// leaves above 1e-8 go into the span after the sources.
-__global__ void k_settle(const Job* jobs) {
-    ::silt::dep_wait();
-    const Job J = jobs[blockIdx.y];
-    const Sheet& S = J.S;
-    float* T = J.T.turbid[0];
-    State* st = J.T.st;
-    const float keep = J.silt_keep;
-    double* book = J.T.books + 3;
-    Ctl* c = ctl_of(st);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && c->active) {
-        // The sync's start (:6339): the marks' box for the next step's wet
-        // set, and the live set and start span, rebuilt by k_clear_sync.
-        for (int k = 0; k < 4; ++k) c->mbox[k] = c->cbox[k];
-        if (step_goes(st)) {
-            st->live_foam = 0;
-            box_clear(st->live_box, S.res);
-            box_clear(st->tspan, S.res);
-        }
-    }
-    if (!step_goes(st) || box_empty(c->tspan2)) return;
-    const int res = S.res;
-    const float area = S.cell * S.cell;
-    int bi0, bi1, bj0, bj1;
-    grown(c->tspan2, res, bi0, bi1, bj0, bj1);
-    double b = 0.0;
-    LocalBox lb;
-    BOX_CELLS(res, bi0, bi1, bj0, bj1) {
-        const float h = S.water[g] + S.slurry[g];
-        const float column = finite_f(T[g]) ? fmaxf(T[g], 0.0f) : 0.0f;
-        if (column <= 0.0f) {
-            T[g] = 0.0f;
-            continue;
-        }
-        if (!finite_f(h) || h < 1.0e-5f) {
-            b += (double)(column * area);
-            T[g] = 0.0f;
-            continue;
-        }
-        const float stay = column * keep;
-        b += (double)((column - stay) * area);
-        T[g] = stay;
-        if (stay > 1.0e-8f) lb.add(i, j);
-    }
-    lb.commit(c->tspan3);
-    block_book(b, book);
 }
 
 // A tire push's constants for spawn_tire_tracers (:6599-6665), computed once
@@ -785,14 +689,15 @@ constexpr int SPAWN_SHARED_PUSHES = 32;
 // spawn_foam_and_silt (:6511-6520) on one wet cell (water h, film velocity
 // u, v, slurry hs): the tires in push order (spawn_tire_tracers :6599-6665),
 // then the shore (spawn_shore_tracers :6667-6684) and Froude breaking
-// (spawn_breaking_speed :6545-6558). `table`: the pushes' constants, or null
-// to compute them from `push` here.
-__device__ __forceinline__ void spawn_cell(const Sheet& S, int i, int j, uint8_t m, float h, float hs, float u,
-                                           float v, const PushK* table, const silt_tire_push* push, int np, float dt,
-                                           float& f, float& t, double& b) {
+// (spawn_breaking_speed :6545-6558). `table`: the pushes' constants, of which
+// those with a bit in `near` can reach the cell; or null to compute them all
+// from `push` here.
+__device__ __forceinline__ void spawn_cell(const Sheet& S, int i, int j, unsigned m, float h, float hs, float u,
+                                           float v, const PushK* table, unsigned near, const silt_tire_push* push,
+                                           int np, float dt, float& f, float& t, double& b) {
     const float cell = S.cell, area = cell * cell;
-    for (int k = 0; k < np; ++k) {
-        const PushK q = table ? table[k] : push_k(push[k], cell);
+    for (int at = 0; table ? near != 0u : at < np; ++at, near &= near - 1u) {
+        const PushK q = table ? table[__ffs(near) - 1] : push_k(push[at], cell);
         if (!q.live) continue;
         if (!finite_f(h) || h < 0.004f) continue;
         const float x = S.ox + ((float)i + 0.5f) * cell;
@@ -831,174 +736,209 @@ __device__ __forceinline__ void spawn_cell(const Sheet& S, int i, int j, uint8_t
         add_foam(f, prod, dt);
         if (silt_add > 0.0f) add_silt(t, fminf(silt_add * dt, 0.0012f), area, b);
     }
+    // A Froude number under 0.85 makes no foam: the square root of the squares
+    // and the two divisions behind it are left out where the squares are a
+    // thousandth below that (their rounding is under a millionth).
     const float hh = h + hs;
-    if (finite_f(hh) && !(hh < 0.004f)) {
-        if (finite_f(u) && finite_f(v) && !(hypot_rn(u, v) <= 0.05f)) add_foam(f, breaking_foam(hypot_rn(u, v), hh), dt);
+    if (finite_f(hh) && !(hh < 0.004f) && finite_f(u) && finite_f(v) &&
+        !(u * u + v * v < 0.999f * (0.85f * 0.85f) * 9.81f * hh)) {
+        const float speed = hypot_rn(u, v);
+        if (!(speed <= 0.05f)) add_foam(f, breaking_foam(speed, hh), dt);
     }
 }
 
-// The sources on every wet cell. They only add silt, so a cell above 1e-8
-// after the settling stays above it; the wet cells that end above it join
-// the span after the sources.
-__global__ void __launch_bounds__(256, 3) k_spawn(const Job* jobs) {
+// The pushes of `table` (np <= 32) that can reach a cell of the columns
+// i .. i + 127 of row j: a bit each, the same for the whole warp. The nearest
+// corner is found with the cells' own arithmetic, which is monotonic in i, so
+// a push left out fails every cell's own test too.
+__device__ __forceinline__ unsigned near_pushes(const Sheet& S, const PushK* table, int np, int i, int j) {
+    const int k = threadIdx.x & 31;
+    bool near = false;
+    if (k < np) {
+        const float x0 = S.ox + ((float)i + 0.5f) * S.cell, x1 = S.ox + ((float)(i + 127) + 0.5f) * S.cell;
+        const float dz = S.oz + ((float)j + 0.5f) * S.cell - table[k].z;
+        const float dx = table[k].x < x0 ? x0 - table[k].x : table[k].x > x1 ? table[k].x - x1 : 0.0f;
+        near = table[k].live && !(dx * dx + dz * dz > table[k].reach2);
+    }
+    return __ballot_sync(0xffffffffu, near);
+}
+
+// The rest of a cell's step: the advections take effect (foam on every wet or
+// foam-live cell, silt on the grown span), the silt of the span after the
+// transport settles (settle_turbid, :6473-6509), a wet cell takes its sources,
+// and the foam half of clear_dry_tracers (:6712-6739) and sync_foam_live
+// (:6339-6349) close it. A cell's foam and silt depend on no other cell here,
+// so they stay in registers from the advected value to the final one: as four
+// passes (commit, settle, spawn, clear and sync) they moved each foam value
+// six times and read marks and depths three times. Bound by DRAM and by the
+// latency of the two load rounds. The sources only add silt, so a settled cell
+// above 1e-8 stays above it; with the wet cells that end above it they are
+// the span after the sources. Outside the collection box no cell is wet, and
+// the live cells of the last sync lie inside it (it covers their box), so
+// every mark there is 0.
+__global__ void __launch_bounds__(256, 3) k_apply(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
-    const Job J = jobs[blockIdx.y];
-    const Sheet& S = J.S;
-    float* foam = J.T.foam[0];
-    float* T = J.T.turbid[0];
-    const uint8_t* mark = J.T.mark;
-    const float dt = J.dt;
-    double* book = J.T.books + 2;
-    Ctl* c = ctl_of(J.T.st);
-    if (!step_goes(J.T.st)) return;
+    JOB;
+    State* st = T.st;
+    Ctl* c = ctl_of(st);
+    if (!step_goes(st)) return;
+    float* foam = T.foam[0];
+    float* silt = T.turbid[0];
+    const float* ttmp = T.turbid[1];
+    uint8_t* mark = T.mark;
+    const float dt = J.dt, keep = J.silt_keep;
     __shared__ PushK table[SPAWN_SHARED_PUSHES];
     const int np = J.npush;
     const bool shared_table = np <= SPAWN_SHARED_PUSHES;
     if (shared_table && (int)threadIdx.x < np) table[threadIdx.x] = push_k(J.push[threadIdx.x], S.cell);
     __syncthreads();
     const int res = S.res;
-    double b = 0.0;
-    LocalBox lb;
+    const float area = S.cell * S.cell;
+    const bool foam_on = c->live_foam_prev != 0;
+    const float* foam_from = foam_on ? T.foam[1] : foam;
+    const Box none{0, -1, 0, -1};
     const Box cb = box_of(c->cbox);  // the wet cells lie inside
-    QUAD_ROWS(res, cb.i0, cb.i1, cb.j0, cb.j1) {
-        if (quiet_run(J.T.occ, res, j, ib - (int)(threadIdx.x & 31), Box{0, -1, 0, -1})) continue;
-        uint8_t mk[4];
+    const Box tb = box_empty(c->tspan1) ? none : grown_box(c->tspan1, res);  // advected
+    const Box zb = box_empty(c->tspan2) ? none : grown_box(c->tspan2, res);  // settling
+    const Box sb = box_union(tb, zb), u = box_union(cb, sb);
+    double stirred = 0.0, settled = 0.0;
+    unsigned int cnt = 0;
+    LocalBox live, span;
+    enum : unsigned { ADVECTED = 8, SETTLING = 16 };  // beside a cell's marks
+    // A run's marks are loaded while the run before is worked on: the planes
+    // that they ask for are then a round's one wait.
+    const Runs runs(u.i0, u.i1, u.j0, u.j1);
+    const unsigned warps = (of_ * blockDim.x) >> 5;
+    unsigned run = (at_ * blockDim.x + threadIdx.x) >> 5;
+    unsigned next[4];
+    int j_next = 0, ib_next = 0;
+    auto load_marks = [&](unsigned r) {
+        runs.at(r, ib_next, j_next);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            next[k] = in_box(cb, ib_next + 32 * k, j_next)
+                          ? mark[(unsigned)j_next * (unsigned)res + (unsigned)(ib_next + 32 * k)]
+                          : 0u;
+    };
+    if (run < runs.n) load_marks(run);
+    for (; run < runs.n; run += warps) {
+        const int j = j_next, ib = ib_next;
+        const unsigned g0 = (unsigned)j * (unsigned)res + (unsigned)ib;
+        unsigned is[4];
         float hw[4], hs[4], u4[4], v4[4], f4[4], t4[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            mk[k] = i <= cb.i1 ? mark[(unsigned)j * (unsigned)res + (unsigned)i] : (uint8_t)0;
+            is[k] = next[k];
+            if (in_box(tb, ib + 32 * k, j)) is[k] |= ADVECTED;
+            if (in_box(zb, ib + 32 * k, j)) is[k] |= SETTLING;
         }
+        if (run + warps < runs.n) load_marks(run + warps);
+        if (!__any_sync(0xffffffffu, (is[0] | is[1] | is[2] | is[3]) != 0u)) continue;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            if (!(mk[k] & WET)) continue;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)(ib + 32 * k);
-            hw[k] = S.water[g];
-            hs[k] = S.slurry[g];
-            u4[k] = S.uw[g];
-            v4[k] = S.vw[g];
-            f4[k] = foam[g];
-            t4[k] = T[g];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (!(mk[k] & WET)) continue;
-            const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            float f = f4[k], t = t4[k];
-            spawn_cell(S, i, j, mk[k], hw[k], hs[k], u4[k], v4[k], shared_table ? table : nullptr, J.push, np, dt, f,
-                       t, b);
-            foam[g] = f;
-            T[g] = t;
-            if (t > 1.0e-8f) lb.add(i, j);
-        }
-    }
-    lb.commit(c->tspan3);  // with the settled cells': the silt span after the sources
-    block_book(b, book);
-}
-
-// clear_dry_tracers (:6712-6739) then sync_foam_live (:6339-6349), per cell.
-// The clear only lowers silt, so the grown span after the sources holds every
-// cell above 1e-8 after it: those cells are the next step's start span.
-// Outside the collection box no cell is wet, and the live cells of the last
-// sync lie inside it (it covers their box), so every mark there is 0.
-__global__ void __launch_bounds__(256, 4) k_clear_sync(const Job* jobs) {
-    ::silt::dep_wait();
-    JOB;
-    float* foam = T.foam[0];
-    float* silt = T.turbid[0];
-    uint8_t* mark = T.mark;
-    State* st = T.st;
-    Ctl* c = ctl_of(st);
-    double* book = T.books + 3;
-    if (!step_goes(st)) return;
-    const int res = S.res;
-    const float area = S.cell * S.cell;
-    const Box cb = box_of(c->cbox);
-    const Box sb = box_empty(c->tspan3) ? Box{0, -1, 0, -1} : grown_box(c->tspan3, res);
-    const Box u = box_union(cb, sb);
-    double b = 0.0;
-    unsigned int cnt = 0;
-    LocalBox live, span;
-    QUAD_ROWS(res, u.i0, u.i1, u.j0, u.j1) {
-        if (quiet_run(T.occ, res, j, ib - (int)(threadIdx.x & 31), sb)) continue;
-        // Loads in two rounds: the marks, then what the wet cells and the
-        // span's cells read.
-        float hw[4], hs[4], f4[4], t4[4];
-        uint8_t mk[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            mk[k] = i <= u.i1 ? mark[(unsigned)j * (unsigned)res + (unsigned)i] : (uint8_t)0;
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            if (i > u.i1) continue;
-            const bool in_span = in_box(sb, i, j);
-            if (!(mk[k] & WET) && !in_span) continue;
-            hw[k] = S.water[g];
-            hs[k] = S.slurry[g];
-            if (mk[k] & WET) f4[k] = foam[g];
-            if (in_span) t4[k] = silt[g];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int i = ib + 32 * k;
-            const unsigned g = (unsigned)j * (unsigned)res + (unsigned)i;
-            if (i > u.i1) continue;
-            const uint8_t m = mk[k];
-            const bool in_span = in_box(sb, i, j);
-            if (!(m & WET) && !in_span) {
-                if (m != 0 && in_box(cb, i, j)) mark[g] = 0;  // a dry cell's marks (sync below)
-                continue;
+            const unsigned g = g0 + 32u * k;
+            if (is[k] & (WET | SETTLING)) {
+                hw[k] = S.water[g];
+                hs[k] = S.slurry[g];
             }
-            const float h = hw[k] + hs[k];
-            float f = (m & WET) ? f4[k] : 0.0f;
-            if (m & WET) {
-                if (!finite_f(h) || h < 0.004f || !finite_f(f)) {
-                    f = 0.0f;
-                    foam[g] = 0.0f;
-                }
+            if (is[k] & WET) {
+                u4[k] = S.uw[g];
+                v4[k] = S.vw[g];
             }
-            if (in_span) {
-                float t = t4[k];
-                if (!finite_f(h) || h < 1.0e-5f) {
-                    if (t > 0.0f) {
-                        b += (double)(t * area);
-                        t = 0.0f;
-                        silt[g] = 0.0f;
-                    }
-                } else if (!finite_f(t)) {
+            if ((is[k] & WET) || (foam_on && (is[k] & LIVE))) f4[k] = foam_from[g];
+            if (is[k] & (WET | ADVECTED | SETTLING)) t4[k] = (is[k] & ADVECTED ? ttmp : silt)[g];
+        }
+        const unsigned near = shared_table ? near_pushes(S, table, np, ib - (int)(threadIdx.x & 31), j) : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (is[k] == 0) continue;
+            const int i = ib + 32 * k;
+            const unsigned g = g0 + 32u * k;
+            const bool wet = is[k] & WET;
+            float t = t4[k];
+            if (is[k] & SETTLING) {
+                const float h = hw[k] + hs[k];
+                const float column = finite_f(t) ? fmaxf(t, 0.0f) : 0.0f;
+                if (column <= 0.0f) {
                     t = 0.0f;
-                    silt[g] = 0.0f;
+                } else if (!finite_f(h) || h < 1.0e-5f) {
+                    settled += (double)(column * area);
+                    t = 0.0f;
+                } else {
+                    t = column * keep;
+                    settled += (double)((column - t) * area);
                 }
-                if (t > 1.0e-8f) span.add(i, j);
             }
-            if (in_box(cb, i, j)) {
-                uint8_t mm = m & (WET | SHORE);
-                if ((mm & WET) && finite_f(f) && f > 1.0e-4f) {
-                    mm |= LIVE;
+            unsigned m = 0;
+            if (wet) {
+                float f = f4[k];
+                spawn_cell(S, i, j, is[k], hw[k], hs[k], u4[k], v4[k], shared_table ? table : nullptr, near, J.push, np,
+                           dt, f, t, stirred);
+                if (!finite_f(f)) f = 0.0f;  // a wet cell's depth is finite and at least 4 mm
+                foam[g] = f;
+                m = is[k] & (WET | SHORE);
+                if (f > 1.0e-4f) {
+                    m |= LIVE;
                     ++cnt;
                     live.add(i, j);
                 }
-                mark[g] = mm;
+            } else if (foam_on && (is[k] & LIVE)) {
+                foam[g] = f4[k];
             }
+            if (is[k] & (WET | ADVECTED | SETTLING)) {
+                silt[g] = t;
+                if ((is[k] & (WET | SETTLING)) && t > 1.0e-8f) span.add(i, j);
+            }
+            if (m != (is[k] & (WET | SHORE | LIVE))) mark[g] = (uint8_t)m;
         }
     }
     live.commit(st->live_box);
-    span.commit(st->tspan);
+    span.commit(c->tspan3);
     block_count(cnt, &st->live_foam);
-    block_book(b, book);
+    block_book(stirred, T.books + 2);
+    block_book(settled, T.books + 3);
+}
+
+// The silt half of clear_dry_tracers on the grown span. It only lowers silt,
+// so that span holds every cell above 1e-8 after it: those cells are the next
+// step's start span.
+__global__ void k_clear(const Job* jobs, const Slice* slices) {
+    ::silt::dep_wait();
+    JOB;
+    float* silt = T.turbid[0];
+    State* st = T.st;
+    Ctl* c = ctl_of(st);
+    if (!step_goes(st) || box_empty(c->tspan3)) return;
+    const int res = S.res;
+    const float area = S.cell * S.cell;
+    const Box sb = grown_box(c->tspan3, res);
+    double b = 0.0;
+    LocalBox span;
+    BOX_CELLS(res, sb.i0, sb.i1, sb.j0, sb.j1) {
+        const float h = S.water[g] + S.slurry[g];
+        const float was = silt[g];
+        float t = was;
+        if (!finite_f(h) || h < 1.0e-5f) {
+            if (t > 0.0f) {
+                b += (double)(t * area);
+                t = 0.0f;
+            }
+        } else if (!finite_f(t)) {
+            t = 0.0f;
+        }
+        if (__float_as_uint(t) != __float_as_uint(was)) silt[g] = t;
+        if (t > 1.0e-8f) span.add(i, j);
+    }
+    span.commit(st->tspan);
+    block_book(b, T.books + 3);
 }
 
 // ---------------------------------------------------------- step_suspended
 
-__global__ void k_susp_begin(const Job* jobs) {
+__global__ void k_susp_begin(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (threadIdx.x != 0 || at_ != 0) return;
     State* st = T.st;
     const int res = S.res;
     Ctl* c = ctl_of(st);
@@ -1019,7 +959,7 @@ __global__ void k_susp_begin(const Job* jobs) {
 // advect_suspended's first loop (:8826-8870): grains fall out at their fall
 // speed; a dry cell or a load above the water settles whole. Cells outside
 // the support box hold no load, and the loop leaves them as they are.
-__global__ void k_susp_settle(const Job* jobs) {
+__global__ void k_susp_settle(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     float* susp = T.susp[0];
@@ -1104,7 +1044,7 @@ __device__ __forceinline__ Donor donor_of(const Sheet& S, const float* susp, int
 // the donors, each donor's gives in its own order (advection x, z, then
 // mixing +x, -x, +z, -z), and records every accepted give in the donor's
 // slot; its total goes to `taken`.
-__global__ void k_susp_take(const Job* jobs) {
+__global__ void k_susp_take(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     const float* susp = T.susp[0];
@@ -1168,7 +1108,7 @@ __global__ void k_susp_take(const Job* jobs) {
 // Donors: each box cell gives its slots away in its own order, takes what
 // its neighbours gave it, then the load above the water or on a dry cell
 // settles (:8971-9000).
-__global__ void k_susp_give(const Job* jobs) {
+__global__ void k_susp_give(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
     float* susp = T.susp[0];
@@ -1245,7 +1185,7 @@ __global__ void k_susp_give(const Job* jobs) {
 // The idle report of every job with a report word: `last` 0 = the jobs
 // without a suspended pass (after step_tracers), 1 = the rest (after
 // step_suspended).
-__global__ void k_idle(const Job* jobs, int last) {
+__global__ void k_idle(const Job* jobs, const Slice*, int last) {
     ::silt::dep_wait();
     const Job& J = jobs[blockIdx.y];
     if (threadIdx.x != 0 || blockIdx.x != 0 || !J.idle_out || (J.susp_on != 0) != (last != 0)) return;
@@ -1316,19 +1256,45 @@ void entrain_box(const Sheet& S, const silt_tire_push* p, int n, int* b) {
     }
 }
 
-// Blocks per window of a launch over n windows: enough for the largest
-// window, about `total` blocks of 256 threads in all.
-int blocks_x(const Window* w, int n, int total) {
+// One launch sequence as the device sees it: its jobs, and over which blocks
+// the passes over cells go (`slices` null: `blocks` of the one job).
+struct Sequence {
+    const Job* jobs = nullptr;
+    const Slice* slices = nullptr;
+    int blocks = 1;
+};
+
+// The blocks of each window: about `total` of 256 threads in all, shared out by
+// the windows' cells (at least one each, at most one per 256 cells). An equal
+// share per window, as it was, let the largest of a mixed batch (64^2 to
+// 512^2) hold a whole pass back.
+template <class Each>
+int split_blocks(const Window* w, int n, int total, Each each) {
+    double cells = 0.0;
+    for (int k = 0; k < n; ++k) cells += (double)w[k].S.res * w[k].S.res;
+    int sum = 0;
+    for (int k = 0; k < n; ++k) {
+        const double own = (double)w[k].S.res * w[k].S.res;
+        const double most = std::max(1.0, ceil(own / 256.0));
+        const int b = (int)std::min(std::max(floor(total * (own / std::max(cells, 1.0)) + 0.5), 1.0), most);
+        each(k, b);
+        sum += b;
+    }
+    return sum;
+}
+
+// The blocks of each window where every one gets the same.
+int box_blocks(const Window* w, int n, int total) {
     size_t most = 1;
     for (int k = 0; k < n; ++k) most = std::max(most, (size_t)w[k].S.res * w[k].S.res);
     const size_t per = std::max<size_t>(1, (size_t)std::max(total, 1) / (size_t)std::max(n, 1));
     return (int)std::min((most + 255) / 256, per);
 }
 
-// Uploads the jobs (and their pushes) of one launch sequence; returns the
-// device array.
+// Uploads the jobs of one launch sequence, its slices and its pushes, in one
+// copy.
 cudaError_t upload(Runner& R, const Window* w, int n, float dt, float foam_decay, float silt_keep, cudaStream_t st,
-                   const Job** out) {
+                   Sequence* out) {
     const int slot = R.next;
     R.next = (R.next + 1) % Runner::SLOTS;
     cudaError_t e;
@@ -1339,37 +1305,40 @@ cudaError_t upload(Runner& R, const Window* w, int n, float dt, float foam_decay
     }
     size_t np = 0;
     for (int k = 0; k < n; ++k) np += (size_t)w[k].npush;
-    if ((size_t)n > R.cap_jobs[slot]) {
-        cudaFree(R.d_jobs[slot]);
-        if (R.h_jobs[slot]) cudaFreeHost(R.h_jobs[slot]);
-        R.d_jobs[slot] = nullptr;
-        R.h_jobs[slot] = nullptr;
-        R.cap_jobs[slot] = 0;
-        const size_t cap = (size_t)n * 2;
-        if ((e = cudaMalloc(&R.d_jobs[slot], cap * sizeof(Job))) != cudaSuccess) return e;
-        if ((e = cudaMallocHost(&R.h_jobs[slot], cap * sizeof(Job))) != cudaSuccess) return e;
-        R.cap_jobs[slot] = cap;
+    out->blocks = split_blocks(w, n, std::max(R.blocks_total, 1), [](int, int) {});
+    const size_t slices_at = ((size_t)n * sizeof(Job) + 15) & ~(size_t)15;
+    const size_t push_at = slices_at + (n > 1 ? (size_t)out->blocks * sizeof(Slice) : 0);
+    const size_t bytes = push_at + np * sizeof(silt_tire_push);
+    if (bytes > R.cap[slot]) {
+        cudaFree(R.d_buf[slot]);
+        if (R.h_buf[slot]) cudaFreeHost(R.h_buf[slot]);
+        R.d_buf[slot] = R.h_buf[slot] = nullptr;
+        R.cap[slot] = 0;
+        const size_t cap = bytes + bytes / 2;
+        if ((e = cudaMalloc(&R.d_buf[slot], cap)) != cudaSuccess) return e;
+        if ((e = cudaMallocHost(&R.h_buf[slot], cap)) != cudaSuccess) return e;
+        R.cap[slot] = cap;
     }
-    if (np > R.cap_push[slot]) {
-        cudaFree(R.d_push[slot]);
-        if (R.h_push[slot]) cudaFreeHost(R.h_push[slot]);
-        R.d_push[slot] = nullptr;
-        R.h_push[slot] = nullptr;
-        R.cap_push[slot] = 0;
-        const size_t cap = np * 2 + 16;
-        if ((e = cudaMalloc(&R.d_push[slot], cap * sizeof(silt_tire_push))) != cudaSuccess) return e;
-        if ((e = cudaMallocHost(&R.h_push[slot], cap * sizeof(silt_tire_push))) != cudaSuccess) return e;
-        R.cap_push[slot] = cap;
+    char* const h = (char*)R.h_buf[slot];
+    char* const d = (char*)R.d_buf[slot];
+    Job* const jobs = (Job*)h;
+    if (n > 1) {
+        Slice* to = (Slice*)(h + slices_at);
+        split_blocks(w, n, std::max(R.blocks_total, 1), [&to](int k, int b) {
+            for (int q = 0; q < b; ++q) *to++ = Slice{k, (unsigned)q, (unsigned)b, 0};
+        });
+        out->slices = (const Slice*)(d + slices_at);
     }
     size_t q = 0;
     for (int k = 0; k < n; ++k) {
-        Job& J = R.h_jobs[slot][k];
+        Job& J = jobs[k];
         memset(&J, 0, sizeof J);
         J.S = w[k].S;
         J.T = w[k].T;
         J.npush = w[k].npush;
-        J.push = w[k].npush ? R.d_push[slot] + q : nullptr;
-        if (w[k].npush) memcpy(R.h_push[slot] + q, w[k].push, (size_t)w[k].npush * sizeof(silt_tire_push));
+        J.push = w[k].npush ? (const silt_tire_push*)(d + push_at) + q : nullptr;
+        if (w[k].npush)
+            memcpy((silt_tire_push*)(h + push_at) + q, w[k].push, (size_t)w[k].npush * sizeof(silt_tire_push));
         q += (size_t)w[k].npush;
         bool wake = w[k].S.surface_driven != 0;
         for (int t = 0; t < w[k].npush; ++t) {
@@ -1388,30 +1357,31 @@ cudaError_t upload(Runner& R, const Window* w, int n, float dt, float foam_decay
         J.foam_decay = foam_decay;
         J.silt_keep = silt_keep;
     }
-    if (np && (e = cudaMemcpyAsync(R.d_push[slot], R.h_push[slot], np * sizeof(silt_tire_push),
-                                   cudaMemcpyHostToDevice, st)) != cudaSuccess)
-        return e;
-    if ((e = cudaMemcpyAsync(R.d_jobs[slot], R.h_jobs[slot], (size_t)n * sizeof(Job), cudaMemcpyHostToDevice, st)) !=
-        cudaSuccess)
-        return e;
+    if ((e = cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(R.ev[slot], st)) != cudaSuccess) return e;
-    *out = R.d_jobs[slot];
+    out->jobs = (const Job*)d;
     return cudaSuccess;
 }
 
-#define LAUNCH(kernel, bx, ...)                                                                \
-    do {                                                                                       \
-        ::silt::launch_dep(kernel, dim3((bx), (unsigned)n), dim3(256), 0, st, __VA_ARGS__);    \
-        ::silt::count_launch();                                                                \
-        const cudaError_t e_ = cudaGetLastError();                                             \
-        if (e_ != cudaSuccess) return e_;                                                      \
+// A pass over the windows' cells, and one with one block per window.
+#define LAUNCH_GRID(kernel, grid, slices, ...)                                                        \
+    do {                                                                                              \
+        ::silt::launch_dep(kernel, grid, dim3(256), 0, st, q.jobs, (const Slice*)(slices), ##__VA_ARGS__); \
+        ::silt::count_launch();                                                                       \
+        const cudaError_t e_ = cudaGetLastError();                                                    \
+        if (e_ != cudaSuccess) return e_;                                                             \
     } while (0)
+#define LAUNCH(kernel) LAUNCH_GRID(kernel, dim3((unsigned)q.blocks), q.slices)
+// A pass over small boxes (the span, the wake, the load's support), which do
+// not grow with the window: an equal share of the blocks for each.
+#define LAUNCH_BOX(kernel) LAUNCH_GRID(kernel, dim3((unsigned)box_blocks(w, n, R.blocks_total), (unsigned)n), nullptr)
+#define LAUNCH_ONE(kernel, ...) LAUNCH_GRID(kernel, dim3(1, (unsigned)n), nullptr, ##__VA_ARGS__)
 
 }  // namespace
 
 size_t plane_bytes(int res) {
     const size_t n = (size_t)res * res;
-    return 256 + 6 * n * sizeof(float) + 6 * n * sizeof(float) + n + (size_t)res * segments(res) + 256;
+    return 256 + 6 * n * sizeof(float) + 6 * n * sizeof(float) + n + 256;
 }
 
 cudaError_t attach(Planes& T, void* mem, int res, double* books, cudaStream_t st) {
@@ -1430,7 +1400,6 @@ cudaError_t attach(Planes& T, void* mem, int res, double* books, cudaStream_t st
     T.taken = T.susp[1];
     T.acc = f + 6 * n;
     T.mark = reinterpret_cast<uint8_t*>(f + 12 * n);
-    T.occ = T.mark + n;
     T.books = books;
     cudaError_t e = cudaMemsetAsync(mem, 0, plane_bytes(res), st);
     if (e != cudaSuccess) return e;
@@ -1439,24 +1408,21 @@ cudaError_t attach(Planes& T, void* mem, int res, double* books, cudaStream_t st
 
 void Runner::release() {
     for (int k = 0; k < SLOTS; ++k) {
-        cudaFree(d_jobs[k]);
-        cudaFree(d_push[k]);
-        if (h_jobs[k]) cudaFreeHost(h_jobs[k]);
-        if (h_push[k]) cudaFreeHost(h_push[k]);
+        cudaFree(d_buf[k]);
+        if (h_buf[k]) cudaFreeHost(h_buf[k]);
         if (ev[k]) cudaEventDestroy(ev[k]);
-        d_jobs[k] = h_jobs[k] = nullptr;
-        d_push[k] = h_push[k] = nullptr;
-        cap_jobs[k] = cap_push[k] = 0;
+        d_buf[k] = h_buf[k] = nullptr;
+        cap[k] = 0;
         ev[k] = nullptr;
     }
 }
 
 cudaError_t entrain(Runner& R, const Window* w, int n, float dt, cudaStream_t st) {
     if (n <= 0 || !(dt > 0.0f) || !std::isfinite(dt)) return cudaSuccess;
-    const Job* jobs = nullptr;
-    cudaError_t e = upload(R, w, n, dt, 0.0f, 0.0f, st, &jobs);
+    Sequence q;
+    cudaError_t e = upload(R, w, n, dt, 0.0f, 0.0f, st, &q);
     if (e != cudaSuccess) return e;
-    LAUNCH(k_entrain, blocks_x(w, n, R.blocks_total), jobs);
+    LAUNCH_BOX(k_entrain);
     return cudaSuccess;
 }
 
@@ -1465,40 +1431,36 @@ cudaError_t step_tracers(Runner& R, const Window* w, int n, float dt, cudaStream
     // The per-step factors, with the C library's expf as the reference's f32::exp.
     const float foam_decay = expf(-dt / 1.8f);  // FOAM_LIFE_S :112
     const float silt_keep = expf(-dt / 4.0f);   // SILT_SETTLE_S :119
-    const Job* jobs = nullptr;
-    cudaError_t e = upload(R, w, n, dt, foam_decay, silt_keep, st, &jobs);
+    Sequence q;
+    cudaError_t e = upload(R, w, n, dt, foam_decay, silt_keep, st, &q);
     if (e != cudaSuccess) return e;
-    const int bx = blocks_x(w, n, R.blocks_total);
     bool rescan = false;
     for (int k = 0; k < n; ++k) rescan = rescan || w[k].rescan;
-    if (rescan) LAUNCH(k_scan, bx, jobs);
-    LAUNCH(k_begin, 1, jobs);
-    LAUNCH(k_collect, bx, jobs);
-    LAUNCH(k_turbid_advect, bx, jobs);
-    LAUNCH(k_commit, bx, jobs);
-    LAUNCH(k_settle, bx, jobs);
-    LAUNCH(k_spawn, bx, jobs);
-    LAUNCH(k_clear_sync, bx, jobs);
+    if (rescan) LAUNCH(k_scan);
+    LAUNCH_ONE(k_begin);
+    LAUNCH(k_collect);
+    LAUNCH_BOX(k_turbid_advect);
+    LAUNCH(k_apply);
+    LAUNCH_BOX(k_clear);
     bool report = false;
     for (int k = 0; k < n; ++k) report = report || (w[k].idle_out && !w[k].susp_on);
-    if (report) LAUNCH(k_idle, 1, jobs, 0);
+    if (report) LAUNCH_ONE(k_idle, 0);
     return cudaSuccess;
 }
 
 cudaError_t step_suspended(Runner& R, const Window* w, int n, float dt, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const Job* jobs = nullptr;
-    cudaError_t e = upload(R, w, n, dt, 0.0f, 0.0f, st, &jobs);
+    Sequence q;
+    cudaError_t e = upload(R, w, n, dt, 0.0f, 0.0f, st, &q);
     if (e != cudaSuccess) return e;
-    LAUNCH(k_susp_begin, 1, jobs);
+    LAUNCH_ONE(k_susp_begin);
     if (!(dt > 0.0f) || !std::isfinite(dt)) return cudaSuccess;
-    const int bx = blocks_x(w, n, R.blocks_total);
-    LAUNCH(k_susp_settle, bx, jobs);
-    LAUNCH(k_susp_take, bx, jobs);
-    LAUNCH(k_susp_give, bx, jobs);
+    LAUNCH_BOX(k_susp_settle);
+    LAUNCH_BOX(k_susp_take);
+    LAUNCH_BOX(k_susp_give);
     bool report = false;
     for (int k = 0; k < n; ++k) report = report || w[k].idle_out;
-    if (report) LAUNCH(k_idle, 1, jobs, 1);
+    if (report) LAUNCH_ONE(k_idle, 1);
     return cudaSuccess;
 }
 

@@ -33,8 +33,6 @@ struct Planes {
     float* taken;       // suspended solids a cell takes from its neighbours this step
     float* acc;         // 6 planes: each donor's accepted gives (advection x, z; mixing +x, -x, +z, -z)
     uint8_t* mark;      // bit 0 wet, bit 1 shore, bit 2 foam-live
-    uint8_t* occ;       // per row and 128-cell segment (cells 128 s .. 128 s + 127): 1 when the wet-set pass
-                        // left a wet or foam-live mark in it (res x ceil(res / 128))
     State* st;
     double* books;      // [0] entrained, [1] settled suspended, [2] stirred, [3] settled silt (m^3, FP64)
 };
@@ -68,21 +66,26 @@ struct Job {
     float dt, foam_decay, silt_keep;
 };
 
+// One block of a launch over several windows: block `at` of the `of` that work
+// on job `job`.
+struct Slice {
+    int job;
+    unsigned at, of, pad;
+};
+
 // Host staging of the jobs of a launch sequence: windows and their pushes,
 // uploaded once per sequence into a ring of slots. A step uploads up to three
 // sequences, so a slot is reused about three steps later and its wait for
 // the earlier copy finds it long done: the host runs ahead of the device.
 struct Runner {
     static constexpr int SLOTS = 10;
-    Job* d_jobs[SLOTS] = {};
-    Job* h_jobs[SLOTS] = {};
-    silt_tire_push* d_push[SLOTS] = {};
-    silt_tire_push* h_push[SLOTS] = {};
-    size_t cap_jobs[SLOTS] = {}, cap_push[SLOTS] = {};
+    void* d_buf[SLOTS] = {};  // the jobs, the slices, the pushes
+    void* h_buf[SLOTS] = {};
+    size_t cap[SLOTS] = {};
     cudaEvent_t ev[SLOTS] = {};
     int next = 0;
     // Blocks of a pass over all the windows of a launch: 8 per SM (measured
-    // on config 2 against 16 and 32; any value gives the same planes).
+    // against 16 and 32; any value gives the same planes).
     int blocks_total = 1184;
     void release();
 };

@@ -201,6 +201,60 @@ def test_batch_tracers_equal_single_windows():
     batch.close()
 
 
+@pytest.mark.parametrize("count", [1, 32, 33])
+def test_tires_across_the_window_match_oracle(count):
+    """Tires from border to border of a window that is not a multiple of the
+    128 cells a warp takes: which of them can reach a run's cells is decided
+    per run up to 32 tires and per cell above. Bit for bit against the oracle
+    with the device's functions (its two builds themselves part by 2 ulp of one
+    suspended load here)."""
+    dt = 1.0 / 30.0
+    ref, dev = O.CoreRN(res=257), G.Sheet(res=257)
+    for c in (ref, dev):
+        c.pour_water(-25.7, 25.7, -6.0, 6.0, 0.05)
+    xs = np.linspace(-25.6, 25.6, count) if count > 1 else [-0.1]
+    for k in range(3):
+        for q, x in enumerate(xs):
+            t = dict(x=float(F(x)), z=float(F(((q * 7) % 11) - 5.0 + 0.1 * k)), forward_x=0.0, forward_z=1.0, radius=0.38,
+                     width=0.2, speed=3.0, slip=0.6)
+            ref.push_tire(**t)
+            dev.push_tire(**t)
+        ref.step(dt)
+        dev.step(dt)
+    check_planes(ref, dev)
+    check_books(ref, dev, 1e-12)
+    assert float(dev.get("foam").max()) > 0.0 and float(dev.get("turbid").max()) > 0.0
+
+
+def test_batch_tracers_of_unequal_windows_equal_single_windows():
+    """The blocks of a pass go to the windows by their cells: one block for the
+    smallest, most of them for the largest."""
+    import torch
+    scenes = [S.grid(res=r, seed=0x77 + r, puddles=3) for r in (40, 640, 64)]
+    stream = torch.cuda.Stream()
+    alone, grouped = ([G.Sheet(res=sc["res"], fine_res=64, layout=G.FINE_PER_TIRE, engine=G.ENGINE_GRID, stream=st)
+                       for sc in scenes] for st in (None, stream.cuda_stream))
+    for sheets in (alone, grouped):
+        for sh, sc in zip(sheets, scenes):
+            S.seed_core(sh, sc)
+    batch = G.Batch(grouped)
+    dt = 1.0 / 120.0
+    for k in range(1, 12):
+        idx, ts = [], []
+        for w in range(len(scenes)):
+            for t in S.tires_at(k * dt, speed=5.0, z0=-3.0):
+                alone[w].push_tire(**t)
+                idx.append(w)
+                ts.append(t)
+            alone[w].step(dt, want_spray=False)
+        batch.push_tires(idx, ts)
+        batch.step(dt)
+    for w in range(len(scenes)):
+        for n in ("water", "slurry") + TRACERS:
+            assert same_bits(alone[w].get(n), grouped[w].get(n)), (w, n)
+    batch.close()
+
+
 PUSH = dict(x=0.15, z=0.2, forward_x=0.0, forward_z=1.0, radius=0.38, width=0.28, speed=8.0, slip=1.2)
 
 
