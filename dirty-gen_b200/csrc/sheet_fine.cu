@@ -975,7 +975,7 @@ struct StepPlan {
 // Staging slots of the per-step tables: a slot is reused STAGING_SLOTS steps
 // later, so the wait for its earlier copy finds it done and the host plans
 // ahead of the device.
-constexpr int STAGING_SLOTS = 4;
+constexpr int STAGING_SLOTS = UPLOAD_RING;
 
 struct HostState {
     StepPlan plan;
@@ -983,6 +983,8 @@ struct HostState {
     char* h_tab[STAGING_SLOTS] = {};
     size_t cap[STAGING_SLOTS] = {};
     cudaEvent_t ev[STAGING_SLOTS] = {};
+    // The batch and its step that last used a slot through an upload lane (0: none).
+    unsigned long long used_batch[STAGING_SLOTS] = {}, used_step[STAGING_SLOTS] = {};
     int flip = 0;
 };
 
@@ -1023,8 +1025,10 @@ static int ensure_patches(Patches& P, int np, cudaStream_t st) {
     return SILT_OK;
 }
 
-// Plans one step's geometry on the host and ships it in one table copy.
-static int plan_step(Patches& P, silt_sheet* s, const std::vector<silt_tire_push>& ps, float dt) {
+// Plans one step's geometry on the host and ships it in one table copy, on
+// the lane where there is one.
+static int plan_step(Patches& P, silt_sheet* s, const std::vector<silt_tire_push>& ps, float dt,
+                     const UploadLane* lane = nullptr) {
     Impl& M = I(P);
     HostState& HS = H(P);
     StepPlan& L = HS.plan;
@@ -1324,8 +1328,15 @@ static int plan_step(Patches& P, silt_sheet* s, const std::vector<silt_tire_push
     // The pinned slot in use STAGING_SLOTS steps ago may still feed its copy.
     FCK(cudaEventSynchronize(HS.ev[slot]));
     memcpy(HS.h_tab[slot], tab.buf.data(), tab.buf.size());
-    FCK(cudaMemcpyAsync(HS.d_tab[slot], HS.h_tab[slot], tab.buf.size(), cudaMemcpyHostToDevice, W.st));
-    FCK(cudaEventRecord(HS.ev[slot], W.st));
+    const cudaStream_t up = lane ? lane->st : W.st;
+    if (lane) {
+        const bool old = HS.used_batch[slot] == lane->batch && HS.used_step[slot] + UPLOAD_RING <= lane->step;
+        FCK(cudaStreamWaitEvent(up, old ? lane->earlier : lane->now, 0));
+    }
+    HS.used_batch[slot] = lane ? lane->batch : 0;
+    HS.used_step[slot] = lane ? lane->step : 0;
+    FCK(cudaMemcpyAsync(HS.d_tab[slot], HS.h_tab[slot], tab.buf.size(), cudaMemcpyHostToDevice, up));
+    FCK(cudaEventRecord(HS.ev[slot], up));
     return SILT_OK;
 }
 
@@ -1889,7 +1900,7 @@ void batch_free(FineBatch* B) {
 }
 
 int batch_prepare(Patches& P, silt_sheet* s, const std::vector<silt_tire_push>& ps, float dt, StepOut& out,
-                  bool* has_work) {
+                  bool* has_work, const UploadLane* lane) {
     *has_work = false;
     Impl& M = I(P);
     int rc = restrict_all(P, s);
@@ -1902,7 +1913,7 @@ int batch_prepare(Patches& P, silt_sheet* s, const std::vector<silt_tire_push>& 
         return fade_only(P, s, dt);
     }
     M.spray_dirty = true;
-    if ((rc = plan_step(P, s, ps, dt))) return rc;
+    if ((rc = plan_step(P, s, ps, dt, lane))) return rc;
     StepPlan& L = H(P).plan;
     // The flags the single-window step reads between its launches.
     L.b_apply = M.near_maybe ? L.n_near : 0;

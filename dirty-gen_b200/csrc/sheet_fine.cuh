@@ -96,11 +96,24 @@ int peel_coarse(Patches& P, silt_sheet* s, const std::vector<silt_tire_push>& pu
 // when the window's patches go to the batched launches. batch_launch then
 // steps every such window's patches on `st` (after the uploads), and
 // batch_peel, after the coarse step, peels their coarse cells.
+//
+// The tables go up on a stream of their own (`st`), beside the kernels of the
+// steps before: in the batch's one order, 256 small copies held each step of
+// 256 windows up by 1.1 ms of 3.9. A table's slot is written again a ring's
+// turn later: when the batch itself used it that long ago, the copy waits for
+// the event `earlier`, recorded when the step of that use was queued whole;
+// after any other use for `now`, which follows all the work queued so far.
+struct UploadLane {
+    cudaStream_t st;
+    cudaEvent_t now, earlier;
+    unsigned long long batch, step;  // a batch's own number, and its steps counted from 1
+};
+constexpr int UPLOAD_RING = 4;  // steps from one use of a table's slot to the next
 struct FineBatch;
 FineBatch* batch_new();
 void batch_free(FineBatch* B);
 int batch_prepare(Patches& P, silt_sheet* s, const std::vector<silt_tire_push>& pushes, float dt, StepOut& out,
-                  bool* has_work);
+                  bool* has_work, const UploadLane* lane);
 int batch_launch(FineBatch* B, const std::vector<silt_sheet*>& sheets, const std::vector<Patches*>& patches, float dt,
                  cudaStream_t st);
 int batch_peel(FineBatch* B, const std::vector<silt_sheet*>& sheets, const std::vector<Patches*>& patches,

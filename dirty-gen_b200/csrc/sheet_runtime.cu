@@ -9,6 +9,7 @@
 // sheet subset: inflow, refine (restrict, lay the patches, near field), tire
 // shove on the patches, fine pair, fine spray, restrict, shove outside the
 // patches, coarse pair, coarse spray.
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -2045,8 +2046,8 @@ int silt_set_confinement(silt_sheet* s, int32_t form) {
 // between an event from the batch stream and one back to it.
 struct BatchWorkers {
     std::vector<std::thread> threads;
-    std::vector<cudaStream_t> streams;
-    std::vector<cudaEvent_t> done;
+    std::vector<cudaStream_t> streams, lanes;  // per worker: its kernels', its table uploads'
+    std::vector<cudaEvent_t> done, sent;
     std::vector<int> rc;
     std::vector<std::string> err;
     std::vector<unsigned long long> launches;
@@ -2096,7 +2097,9 @@ struct BatchWorkers {
         go.notify_all();
         for (auto& t : threads) t.join();
         for (cudaStream_t st : streams) cudaStreamDestroy(st);
+        for (cudaStream_t st : lanes) cudaStreamDestroy(st);
         for (cudaEvent_t e : done) cudaEventDestroy(e);
+        for (cudaEvent_t e : sent) cudaEventDestroy(e);
     }
 };
 
@@ -2116,7 +2119,9 @@ struct silt_batch {
     BatchTuner tuner;
     BatchWorkers* workers = nullptr;
     silt::fine::FineBatch* fine = nullptr;  // staging of the batched nested-patch launches
-    cudaEvent_t ev_start = nullptr;
+    // Recorded at the start of each step, in a ring (step k at k % UPLOAD_RING).
+    cudaEvent_t ev_start[silt::fine::UPLOAD_RING] = {};
+    unsigned long long id = 0, step = 0;  // this batch's number in the process, and its steps
     cudaStream_t st = nullptr;
     int device = 0;
     int max_tiles = 0;              // the largest window's tile count per layer
@@ -2167,7 +2172,8 @@ int batch_free(silt_batch* b) {
     }
     delete b->workers;
     silt::fine::batch_free(b->fine);
-    if (b->ev_start) cudaEventDestroy(b->ev_start);
+    for (cudaEvent_t e : b->ev_start)
+        if (e) cudaEventDestroy(e);
     cudaFree(b->list);
     cudaFree(b->entry_win);
     cudaFree(b->count);
@@ -2507,7 +2513,10 @@ int silt_batch_create(silt_sheet* const* sheets, int32_t n, silt_batch** out) {
         e = cudaMemcpy(b->d_ledger_src, src.data(), src.size() * sizeof(double*), cudaMemcpyHostToDevice);
     }
     b->fine = silt::fine::batch_new();
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_start, cudaEventDisableTiming);
+    static std::atomic<unsigned long long> batches{0};
+    b->id = ++batches;
+    for (cudaEvent_t& ev : b->ev_start)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (e == cudaSuccess) {
         unsigned hw = std::thread::hardware_concurrency();
         const int k = std::max(1, std::min({8, (int)(hw ? hw : 1), n}));
@@ -2515,12 +2524,14 @@ int silt_batch_create(silt_sheet* const* sheets, int32_t n, silt_batch** out) {
         W->device = b->device;
         b->workers = W;
         for (int q = 0; q < k && e == cudaSuccess; ++q) {
-            cudaStream_t st = nullptr;
-            cudaEvent_t ev = nullptr;
-            e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-            if (st) W->streams.push_back(st);
-            if (ev) W->done.push_back(ev);
+            for (int lane = 0; lane < 2 && e == cudaSuccess; ++lane) {
+                cudaStream_t st = nullptr;
+                cudaEvent_t ev = nullptr;
+                e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+                if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+                if (st) (lane ? W->lanes : W->streams).push_back(st);
+                if (ev) (lane ? W->sent : W->done).push_back(ev);
+            }
         }
         if (e == cudaSuccess) {
             W->rc.assign(k, 0);
@@ -2583,14 +2594,22 @@ int silt_batch_step(silt_batch* b, float dt) {
         if (!tw.empty()) CK(silt::tracers::entrain(b->tr_run, tw.data(), (int)tw.size(), dt, b->st));
     }
     phase(0);
-    CK(cudaEventRecord(b->ev_start, b->st));  // the workers' streams start after the batch's previous work
+    // The workers' streams start after the batch's previous work, their lanes
+    // for the tables after that of a ring's turn ago. A capture holds one
+    // order: there the tables go up on the workers' streams.
+    constexpr int RING = silt::fine::UPLOAD_RING;
+    const cudaEvent_t start = b->ev_start[++b->step % RING];
+    CK(cudaEventRecord(start, b->st));
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(b->st, &capture));
+    const bool lanes = capture == cudaStreamCaptureStatusNone;
     // Each window's tire pushes, inflow and nested-patch planning on the
-    // workers (the planning uploads the window's tables on the worker's
-    // stream); the patches themselves step in the batched launches below.
+    // workers; the patches themselves step in the batched launches below.
     Wk.run([&](int k) {
         Wk.rc[k] = 0;
         cudaStream_t wst = Wk.streams[k];
-        cudaError_t e = cudaStreamWaitEvent(wst, b->ev_start, 0);
+        cudaError_t e = cudaStreamWaitEvent(wst, start, 0);
+        const silt::fine::UploadLane lane = {Wk.lanes[k], start, b->ev_start[(b->step + 1) % RING], b->id, b->step};
         for (int w = k; w < n && e == cudaSuccess && Wk.rc[k] == 0; w += nk) {
             silt_sheet* s = b->sheets[w];
             cudaStream_t own = s->st;
@@ -2599,12 +2618,13 @@ int silt_batch_step(silt_batch* b, float dt) {
             ps[w].swap(s->pushes);
             bool has = false;
             Wk.rc[k] = step_inflow(s, dt);
-            if (!Wk.rc[k]) Wk.rc[k] = silt::fine::batch_prepare(s->fine, s, ps[w], dt, fo[w], &has);
+            if (!Wk.rc[k]) Wk.rc[k] = silt::fine::batch_prepare(s->fine, s, ps[w], dt, fo[w], &has, lanes ? &lane : nullptr);
             work[w] = has ? 1 : 0;
             s->st = own;
             if (Wk.rc[k]) Wk.err[k] = silt_last_error();
         }
         if (e == cudaSuccess) e = cudaEventRecord(Wk.done[k], wst);
+        if (e == cudaSuccess && lanes) e = cudaEventRecord(Wk.sent[k], lane.st);
         if (e != cudaSuccess && Wk.rc[k] == 0) {
             Wk.rc[k] = SILT_ECUDA;
             Wk.err[k] = std::string("batch worker: ") + cudaGetErrorString(e);
@@ -2615,7 +2635,10 @@ int silt_batch_step(silt_batch* b, float dt) {
             snprintf(g_err, sizeof g_err, "%s", Wk.err[k].c_str());
             return Wk.rc[k];
         }
-    for (int k = 0; k < nk; ++k) CK(cudaStreamWaitEvent(b->st, Wk.done[k], 0));
+    for (int k = 0; k < nk; ++k) {
+        CK(cudaStreamWaitEvent(b->st, Wk.done[k], 0));
+        if (lanes) CK(cudaStreamWaitEvent(b->st, Wk.sent[k], 0));
+    }
     phase(1);
     std::vector<silt_sheet*> fs;
     std::vector<silt::fine::Patches*> fp;

@@ -130,3 +130,38 @@ def test_batch_autotuner_times_real_steps_and_changes_no_bit():
     b.close()
     for _, bb, _ in runs.values():
         bb.close()
+
+
+@pytest.mark.parametrize("order", ["bbbbbbbbbbbb", "bsbssbsssbssssb", "bcbccbcccbb"])
+def test_uploads_beside_earlier_steps_change_no_bit(order):
+    """The nested patches' tables go up while earlier steps still run: steps of
+    one batch (b), of a second batch over the same windows (c) and of each
+    window by itself (s), queued without a wait in between, on windows large
+    enough that the host runs ahead, against windows stepped alone."""
+    import torch
+
+    stream = torch.cuda.Stream()
+    scenes = [S.grid(res=r, seed=0x99 + r, puddles=3) for r in (1024, 96)]
+    alone = [make(sc) for sc in scenes]
+    grouped = [make(sc, stream=stream.cuda_stream) for sc in scenes]
+    batches = {"b": G.Batch(grouped), "c": G.Batch(grouped)}
+    torch.cuda.synchronize()
+    for k, how in enumerate(order, 1):
+        if how == "s":
+            for sh in grouped:
+                push(sh, k, 4)
+                sh.step(DT, want_spray=False)
+        else:
+            tires = S.tires_at(k * DT, speed=5.0, z0=-3.0)[:4]
+            batches[how].push_tires([0] * len(tires) + [1] * len(tires), tires + tires)
+            batches[how].step(DT)
+    for k in range(1, len(order) + 1):
+        for sh in alone:
+            push(sh, k, 4)
+            sh.step(DT, want_spray=False)
+    for w in range(len(scenes)):
+        for name in ("water", "slurry", "uw", "vw", "us", "vs"):
+            a, b = alone[w].get(name), grouped[w].get(name)
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (w, name, float(np.abs(a - b).max()))
+    for b in batches.values():
+        b.close()
