@@ -1295,15 +1295,16 @@ int silt_step(silt_sheet* s, float dt, silt_spray_event* out, int32_t cap, int32
     phase(4);
     if (!skip_tracers) {
         // step_tracers (src/fluid_core.rs:6080), then the reach, then the
-        // suspended load (:6082-6089).
+        // suspended load (:6082-6089); in one sequence where no reach steps
+        // in between.
         silt::tracers::Window w = tracer_window(s, ps);
         w.susp_on = s->turbidity ? 1 : 0;
         w.idle_out = tracers_report_word(s);
-        CK(silt::tracers::step_tracers(s->tr_run, &w, 1, dt, s->st));
+        CK(silt::tracers::step_tracers(s->tr_run, &w, 1, dt, !s->reach_on, s->st));
         s->tr_rescan = false;
     }
     if ((rc = reach_step(s))) return rc;
-    if (s->turbidity && !skip_tracers) {
+    if (s->turbidity && !skip_tracers && s->reach_on) {
         silt::tracers::Window w = tracer_window(s, ps);
         w.susp_on = 1;
         w.idle_out = tracers_report_word(s);
@@ -2660,11 +2661,17 @@ int silt_batch_step(silt_batch* b, float dt) {
     phase(4);
     {
         // step_tracers of every window in one launch sequence, the reach, then
-        // the suspended load of the windows with turbidity on.
+        // the suspended load of the windows with turbidity on (in the same
+        // sequence where no window has a reach).
         std::vector<silt::tracers::Window> tw;
         tw.reserve(n);
-        for (int w = 0; w < n; ++w) tw.push_back(tracer_window(b->sheets[w], ps[w]));
-        CK(silt::tracers::step_tracers(b->tr_run, tw.data(), n, dt, b->st));
+        bool reach = false;
+        for (int w = 0; w < n; ++w) {
+            tw.push_back(tracer_window(b->sheets[w], ps[w]));
+            tw.back().susp_on = b->sheets[w]->turbidity ? 1 : 0;
+            reach = reach || b->sheets[w]->reach_on;
+        }
+        CK(silt::tracers::step_tracers(b->tr_run, tw.data(), n, dt, !reach, b->st));
         for (silt_sheet* s : b->sheets) {
             s->tr_rescan = false;
             s->tr_poke = true;  // stepped by the batch, which sends no idle reports
@@ -2672,8 +2679,11 @@ int silt_batch_step(silt_batch* b, float dt) {
         for (silt_sheet* s : b->sheets)
             if ((rc = reach_step(s))) return rc;
         std::vector<silt::tracers::Window> sw;
-        for (int w = 0; w < n; ++w)
-            if (b->sheets[w]->turbidity) sw.push_back(tracer_window(b->sheets[w], ps[w]));
+        for (int w = 0; w < n && reach; ++w) {
+            if (!b->sheets[w]->turbidity) continue;
+            sw.push_back(tracer_window(b->sheets[w], ps[w]));
+            sw.back().susp_on = 1;
+        }
         if (!sw.empty()) CK(silt::tracers::step_suspended(b->tr_run, sw.data(), (int)sw.size(), dt, b->st));
     }
     phase(5);

@@ -51,6 +51,7 @@ struct Ctl {
     int ssup[4];    // this step's suspended pass: a box holding every cell whose load is not 0
     int ssup_next[4];  // the same for the next step, grown by every writer of the load
     unsigned int live_foam_prev;
+    unsigned int arrived;  // blocks of a report's kernel that are done (0 between kernels)
 };
 
 __device__ __forceinline__ Ctl* ctl_of(State* s) { return reinterpret_cast<Ctl*>(s + 1); }
@@ -213,6 +214,45 @@ __device__ __forceinline__ void box_clear(int* box, int res) {
 
 __device__ __forceinline__ bool box_empty(const int* b) { return b[0] > b[1]; }
 
+// The idle report of a job with a report word, by the last of the job's `of`
+// blocks to end its last kernel (every block calls it): k_clear's for the jobs
+// without a suspended pass, k_susp_give's for the rest.
+__device__ __forceinline__ void report_idle(const Job& J, unsigned of) {
+    if (!J.idle_out) return;
+    __syncthreads();  // the block's span and support are out
+    if (threadIdx.x != 0) return;
+    State* st = J.T.st;
+    Ctl* c = ctl_of(st);
+    __threadfence();
+    if (atomicAdd(&c->arrived, 1u) != of - 1u) return;
+    c->arrived = 0u;
+    __threadfence();
+    const volatile int* span = st->tspan;
+    const volatile int* sup = c->ssup_next;
+    const bool idle = st->live_foam == 0u && span[0] > span[1] &&
+                      (J.susp_on ? sup[0] > sup[1] : !J.rescan);
+    *J.idle_out = idle ? 1u : 0u;
+}
+
+// The start of the suspended pass. The cells that may hold a load: every
+// writer since the last pass grew the next box; a river inlet carrying a load
+// writes its rows.
+__device__ __forceinline__ void susp_begin(const Job& J) {
+    State* st = J.T.st;
+    const int res = J.S.res;
+    Ctl* c = ctl_of(st);
+    box_clear(st->sbox, res);
+    st->capped = 0;
+    for (int k = 0; k < 4; ++k) c->ssup[k] = c->ssup_next[k];
+    if (J.sup_all) {
+        c->ssup[0] = 0;
+        c->ssup[1] = res - 1;
+        c->ssup[2] = 0;
+        c->ssup[3] = res - 1;
+    }
+    box_clear(c->ssup_next, res);
+}
+
 // turbid_span's result (:9766-9795): the box grown by one, clamped.
 __device__ __forceinline__ void grown(const int* b, int res, int& i0, int& i1, int& j0, int& j1) {
     i0 = max(b[0] - 1, 0);
@@ -370,14 +410,16 @@ __global__ void k_scan(const Job* jobs, const Slice* slices) {
 // The step's control words, then collect_tracer_wet's box (:6248-6293) and
 // tracer_visit_box (:6296-6337). `wake`: a tire with speed or slip, or a
 // surface drive (host-known); `pbox`: the tires' reach boxes (host-computed;
-// empty when none).
-__global__ void k_begin(const Job* jobs, const Slice* slices) {
+// empty when none). `both`: the suspended pass follows in the same sequence, and
+// starts here too.
+__global__ void k_begin(const Job* jobs, const Slice* slices, int both) {
     ::silt::dep_wait();
     JOB;
     if (threadIdx.x != 0 || at_ != 0) return;
     State* st = T.st;
     const int res = S.res, wake = J.wake;
     Ctl* c = ctl_of(st);
+    if (both && J.susp_on) susp_begin(J);
     box_clear(c->tspan2, res);
     box_clear(c->tspan3, res);
     box_clear(c->cbox, res);
@@ -908,7 +950,10 @@ __global__ void k_clear(const Job* jobs, const Slice* slices) {
     float* silt = T.turbid[0];
     State* st = T.st;
     Ctl* c = ctl_of(st);
-    if (!step_goes(st) || box_empty(c->tspan3)) return;
+    if (!step_goes(st) || box_empty(c->tspan3)) {
+        if (!J.susp_on) report_idle(J, of_);
+        return;
+    }
     const int res = S.res;
     const float area = S.cell * S.cell;
     const Box sb = grown_box(c->tspan3, res);
@@ -931,6 +976,7 @@ __global__ void k_clear(const Job* jobs, const Slice* slices) {
     }
     span.commit(st->tspan);
     block_book(b, T.books + 3);
+    if (!J.susp_on) report_idle(J, of_);
 }
 
 // ---------------------------------------------------------- step_suspended
@@ -938,22 +984,7 @@ __global__ void k_clear(const Job* jobs, const Slice* slices) {
 __global__ void k_susp_begin(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
-    if (threadIdx.x != 0 || at_ != 0) return;
-    State* st = T.st;
-    const int res = S.res;
-    Ctl* c = ctl_of(st);
-    box_clear(st->sbox, res);
-    st->capped = 0;
-    // The cells that may hold a load: every writer since the last pass grew
-    // the next box; a river inlet carrying a load writes its rows.
-    for (int k = 0; k < 4; ++k) c->ssup[k] = c->ssup_next[k];
-    if (J.sup_all) {
-        c->ssup[0] = 0;
-        c->ssup[1] = res - 1;
-        c->ssup[2] = 0;
-        c->ssup[3] = res - 1;
-    }
-    box_clear(c->ssup_next, res);
+    if (threadIdx.x == 0 && at_ == 0 && J.susp_on) susp_begin(J);
 }
 
 // advect_suspended's first loop (:8826-8870): grains fall out at their fall
@@ -962,6 +993,7 @@ __global__ void k_susp_begin(const Job* jobs, const Slice* slices) {
 __global__ void k_susp_settle(const Job* jobs, const Slice* slices) {
     ::silt::dep_wait();
     JOB;
+    if (!J.susp_on) return;
     float* susp = T.susp[0];
     State* st = T.st;
     Ctl* c = ctl_of(st);
@@ -1052,7 +1084,7 @@ __global__ void k_susp_take(const Job* jobs, const Slice* slices) {
     float* acc = T.acc;
     State* st = T.st;
     const float dt = J.dt;
-    if (box_empty(st->sbox)) return;
+    if (!J.susp_on || box_empty(st->sbox)) return;
     const int res = S.res;
     const size_t n = (size_t)res * res;
     int bi0, bi1, bj0, bj1;
@@ -1117,7 +1149,11 @@ __global__ void k_susp_give(const Job* jobs, const Slice* slices) {
     State* st = T.st;
     const float dt = J.dt;
     double* book = T.books + 1;
-    if (box_empty(st->sbox)) return;
+    if (!J.susp_on) return;
+    if (box_empty(st->sbox)) {
+        report_idle(J, of_);
+        return;
+    }
     const int res = S.res;
     const size_t n = (size_t)res * res;
     const float area = S.cell * S.cell;
@@ -1180,20 +1216,7 @@ __global__ void k_susp_give(const Job* jobs, const Slice* slices) {
     held.commit(ctl_of(st)->ssup_next);
     block_book(b, book);
     block_count(capped, &st->capped);
-}
-
-// The idle report of every job with a report word: `last` 0 = the jobs
-// without a suspended pass (after step_tracers), 1 = the rest (after
-// step_suspended).
-__global__ void k_idle(const Job* jobs, const Slice*, int last) {
-    ::silt::dep_wait();
-    const Job& J = jobs[blockIdx.y];
-    if (threadIdx.x != 0 || blockIdx.x != 0 || !J.idle_out || (J.susp_on != 0) != (last != 0)) return;
-    const State* st = J.T.st;
-    const Ctl* c = reinterpret_cast<const Ctl*>(st + 1);
-    const bool idle = st->live_foam == 0u && box_empty(st->tspan) && !J.rescan &&
-                      (!J.susp_on || box_empty(c->ssup_next));
-    *J.idle_out = idle ? 1u : 0u;
+    report_idle(J, of_);
 }
 
 __global__ void k_reset_live(uint8_t* mark, State* st, int res, size_t n) {
@@ -1283,12 +1306,13 @@ int split_blocks(const Window* w, int n, int total, Each each) {
     return sum;
 }
 
-// The blocks of each window where every one gets the same.
+// The blocks of each window where every one gets the same; 4 per SM are enough
+// for one window's boxes, and a block beyond them only costs its launch.
 int box_blocks(const Window* w, int n, int total) {
     size_t most = 1;
     for (int k = 0; k < n; ++k) most = std::max(most, (size_t)w[k].S.res * w[k].S.res);
     const size_t per = std::max<size_t>(1, (size_t)std::max(total, 1) / (size_t)std::max(n, 1));
-    return (int)std::min((most + 255) / 256, per);
+    return (int)std::min({(most + 255) / 256, per, (size_t)592});
 }
 
 // Uploads the jobs of one launch sequence, its slices and its pushes, in one
@@ -1426,7 +1450,14 @@ cudaError_t entrain(Runner& R, const Window* w, int n, float dt, cudaStream_t st
     return cudaSuccess;
 }
 
-cudaError_t step_tracers(Runner& R, const Window* w, int n, float dt, cudaStream_t st) {
+static cudaError_t suspended_passes(Runner& R, const Window* w, int n, const Sequence& q, cudaStream_t st) {
+    LAUNCH_BOX(k_susp_settle);
+    LAUNCH_BOX(k_susp_take);
+    LAUNCH_BOX(k_susp_give);
+    return cudaSuccess;
+}
+
+cudaError_t step_tracers(Runner& R, const Window* w, int n, float dt, bool suspended, cudaStream_t st) {
     if (n <= 0 || !(dt > 0.0f) || !std::isfinite(dt)) return cudaSuccess;
     // The per-step factors, with the C library's expf as the reference's f32::exp.
     const float foam_decay = expf(-dt / 1.8f);  // FOAM_LIFE_S :112
@@ -1434,18 +1465,18 @@ cudaError_t step_tracers(Runner& R, const Window* w, int n, float dt, cudaStream
     Sequence q;
     cudaError_t e = upload(R, w, n, dt, foam_decay, silt_keep, st, &q);
     if (e != cudaSuccess) return e;
-    bool rescan = false;
-    for (int k = 0; k < n; ++k) rescan = rescan || w[k].rescan;
+    bool rescan = false, any = false;
+    for (int k = 0; k < n; ++k) {
+        rescan = rescan || w[k].rescan;
+        any = any || w[k].susp_on;
+    }
     if (rescan) LAUNCH(k_scan);
-    LAUNCH_ONE(k_begin);
+    LAUNCH_ONE(k_begin, suspended ? 1 : 0);
     LAUNCH(k_collect);
     LAUNCH_BOX(k_turbid_advect);
     LAUNCH(k_apply);
     LAUNCH_BOX(k_clear);
-    bool report = false;
-    for (int k = 0; k < n; ++k) report = report || (w[k].idle_out && !w[k].susp_on);
-    if (report) LAUNCH_ONE(k_idle, 0);
-    return cudaSuccess;
+    return suspended && any ? suspended_passes(R, w, n, q, st) : cudaSuccess;
 }
 
 cudaError_t step_suspended(Runner& R, const Window* w, int n, float dt, cudaStream_t st) {
@@ -1455,13 +1486,7 @@ cudaError_t step_suspended(Runner& R, const Window* w, int n, float dt, cudaStre
     if (e != cudaSuccess) return e;
     LAUNCH_ONE(k_susp_begin);
     if (!(dt > 0.0f) || !std::isfinite(dt)) return cudaSuccess;
-    LAUNCH_BOX(k_susp_settle);
-    LAUNCH_BOX(k_susp_take);
-    LAUNCH_BOX(k_susp_give);
-    bool report = false;
-    for (int k = 0; k < n; ++k) report = report || w[k].idle_out;
-    if (report) LAUNCH_ONE(k_idle, 1);
-    return cudaSuccess;
+    return suspended_passes(R, w, n, q, st);
 }
 
 cudaError_t reset_indices(Planes& T, int res, cudaStream_t st) {

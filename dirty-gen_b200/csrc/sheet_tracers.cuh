@@ -98,7 +98,7 @@ struct Window {
     int npush;
     int rescan = 0;   // the planes were rewritten since the last tracer step (attach, window move)
     int sup_all = 0;  // a river inlet writes the suspended load outside the tracer kernels
-    int susp_on = 0;  // turbidity on: step_suspended follows step_tracers this step
+    int susp_on = 0;  // turbidity on: the suspended pass takes this window
     unsigned int* idle_out = nullptr;  // device word for the idle report (see step_tracers)
 };
 
@@ -108,8 +108,11 @@ cudaError_t attach(Planes& T, void* mem, int res, double* books, cudaStream_t st
 // entrain_wake (src/fluid_core.rs:8758-8815) on every window, before the step.
 cudaError_t entrain(Runner& R, const Window* w, int n, float dt, cudaStream_t st);
 // step_tracers (src/fluid_core.rs:6210-6237) after the coarse pair and its peel.
-// A window without turbidity then reports whether it is idle (below).
-cudaError_t step_tracers(Runner& R, const Window* w, int n, float dt, cudaStream_t st);
+// A window without turbidity then reports whether it is idle (below). With
+// `suspended`, the suspended pass of the windows with susp_on follows in the
+// same sequence (one upload, one start); where a river reach steps in between
+// the caller calls step_suspended by itself.
+cudaError_t step_tracers(Runner& R, const Window* w, int n, float dt, bool suspended, cudaStream_t st);
 // step_suspended (src/fluid_core.rs:8750-8756 with advect_suspended :8817-9002),
 // then every window reports whether it is idle: no live foam, no silt above
 // 1e-8 and no suspended load. An idle window whose next step has no wake (no
