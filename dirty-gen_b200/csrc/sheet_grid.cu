@@ -41,20 +41,24 @@ namespace silt {
 constexpr int FT = 32;       // force tile edge
 // Shared-memory layout of a force tile: the halo its widest stage reads and
 // the eight planes' width and size.
-template <int HALO>
+template <int HALO, int PLANES>
 struct TileGeom {
     static constexpr int H = HALO;
     static constexpr int W = FT + 2 * H;
     static constexpr int PLANE = W * W;
-    static constexpr size_t BYTES = sizeof(float) * 8 * PLANE;
+    static constexpr size_t BYTES = sizeof(float) * PLANES * PLANE;
 };
 constexpr int FORCE_THREADS = 512;
 // The snapshot form carries every stage of a cell through one tile:
-// p (2) + gravity (1) + vorticity (2) + projection (4).
-using Snap = TileGeom<9>;
+// p (2) + gravity (1) + vorticity (2) + projection (4). Seven planes (70 KB):
+// three CTAs share an SM. Their time is block barriers between ten short
+// stages, so a third tile on the SM fills the other two's waits: k_force on a
+// flooded 1000^2 grid 86 us with eight planes and two CTAs.
+using Snap = TileGeom<9, 7>;
+constexpr int SNAP_CTAS = 3;  // per SM
 // The sweep form's stages meet in global memory, so no stage reaches further
 // than the projection's 4 cells: 51 KB a tile instead of 80.
-using Sweep = TileGeom<4>;
+using Sweep = TileGeom<4, 8>;
 constexpr size_t SWEEP_SMEM = 2 * Sweep::BYTES;  // a CTA's two teams
 static_assert(2 * (SWEEP_SMEM + 2048) <= 228 * 1024, "two sweep CTAs share an SM");
 
@@ -226,17 +230,16 @@ __device__ __forceinline__ int tile_band(const LayerParams& P, int tx0, int ty0)
 // tile corner minus G::H).
 template <class G>
 struct ForcePlanes {
-    float* E;   // eta
-    float* TG;  // x-pass scratch
+    float* E;   // eta, then q
+    float* TG;  // x-pass scratch; the snapshot form's vorticity between the two blurs
     float* TS;
     float* PB;  // pressure p, then projection b
     float* U;   // u, v
     float* V;
     float* HS;  // depth
-    float* WQ;  // vorticity, then q
     __device__ explicit ForcePlanes(float* sm)
         : E(sm), TG(sm + G::PLANE), TS(sm + 2 * G::PLANE), PB(sm + 3 * G::PLANE), U(sm + 4 * G::PLANE), V(sm + 5 * G::PLANE),
-          HS(sm + 6 * G::PLANE), WQ(sm + 7 * G::PLANE) {}
+          HS(sm + 6 * G::PLANE) {}
 };
 
 #define NX(d) (EDGE ? (gy - oy) * G::W + (clampi(gx + (d), 0, res - 1) - ox) : s + (d))
@@ -328,7 +331,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
             const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
             float gq = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
             float sq = tap5(F.TS[s0], F.TS[s1], F.TS[s], F.TS[s3], F.TS[s4], kS0, kS1, kS2, in);
-            F.WQ[s] = 0.62f * gq + 0.38f * sq;
+            F.E[s] = 0.62f * gq + 0.38f * sq;
         });
         T.sync();
     }
@@ -337,8 +340,8 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         float uu = F.U[s], vv = F.V[s];
         if (F.HS[s] > eps) {
             if (P.project) {
-                float qx = fdiv(F.WQ[NX(1)] - F.WQ[NX(-1)], P.div_two);
-                float qz = fdiv(F.WQ[NZ(1)] - F.WQ[NZ(-1)], P.div_two);
+                float qx = fdiv(F.E[NX(1)] - F.E[NX(-1)], P.div_two);
+                float qz = fdiv(F.E[NZ(1)] - F.E[NZ(-1)], P.div_two);
                 uu += 0.012f * dt * qx;
                 vv += 0.012f * dt * qz;
             }
@@ -386,17 +389,17 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
         region<TM, G, EDGE, 5, 5>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             float dvdx = fdiv(F.V[NX(1)] - F.V[NX(-1)], P.div_two);
             float dudz = fdiv(F.U[NZ(1)] - F.U[NZ(-1)], P.div_two);
-            F.WQ[s] = dvdx - dudz;
+            F.TG[s] = dvdx - dudz;
         });
         T.sync();
         // Confinement kick from that snapshot, in place, radius 4
         // (src/fluid_core.rs:2348-2375, :2441-2470).
         region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
             if (F.HS[s] > eps) {
-                float w = F.WQ[s];
+                float w = F.TG[s];
                 if (finite_f(w) && !(fabsf(w) < 1.0e-4f)) {
-                    float wxp = fabsf(F.WQ[NX(1)]), wxm = fabsf(F.WQ[NX(-1)]);
-                    float wzp = fabsf(F.WQ[NZ(1)]), wzm = fabsf(F.WQ[NZ(-1)]);
+                    float wxp = fabsf(F.TG[NX(1)]), wxm = fabsf(F.TG[NX(-1)]);
+                    float wzp = fabsf(F.TG[NZ(1)]), wzm = fabsf(F.TG[NZ(-1)]);
                     float nx_ = fdiv(wxp - wxm, P.div_two);
                     float nz_ = fdiv(wzp - wzm, P.div_two);
                     float du = P.vort * dt * (-nz_ * w);
@@ -944,7 +947,7 @@ __global__ void __launch_bounds__(FORCE_THREADS, 2) k_force_sweep(ForceLaunch L)
 }
 
 // Persistent over the substep's tile list.
-__global__ void __launch_bounds__(FORCE_THREADS) k_force(ForceLaunch L) {
+__global__ void __launch_bounds__(FORCE_THREADS, SNAP_CTAS) k_force(ForceLaunch L) {
     ::silt::dep_wait();
     extern __shared__ float sm[];
     __shared__ LayerParams Ps[2];
@@ -1504,6 +1507,7 @@ __global__ void __launch_bounds__(256) k_batch_speed2(const WindowSubstep* ws, c
     }
 }
 
+// (At three CTAs per SM its registers spill: two.)
 __global__ void __launch_bounds__(FORCE_THREADS) k_batch_force(const WindowSubstep* ws, const int* list,
                                                                const int* entry_win, const int* count) {
     ::silt::dep_wait();
@@ -1722,7 +1726,7 @@ cudaError_t launch_force(const ForceLaunch& L, int res, int layers, cudaStream_t
     std::call_once(attr, [] { cudaFuncSetAttribute(k_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Snap::BYTES); });
     (void)res;
     (void)layers;
-    ::silt::launch_dep(k_force, dim3(148 * 2), dim3(FORCE_THREADS), Snap::BYTES, st, L);
+    ::silt::launch_dep(k_force, dim3(148 * SNAP_CTAS), dim3(FORCE_THREADS), Snap::BYTES, st, L);
     ::silt::count_launch();
     return cudaGetLastError();
 }

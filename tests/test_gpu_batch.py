@@ -165,3 +165,29 @@ def test_uploads_beside_earlier_steps_change_no_bit(order):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (w, name, float(np.abs(a - b).max()))
     for b in batches.values():
         b.close()
+
+
+@pytest.mark.parametrize("forms", [(1, 0, 0), (0, 1, 1), (1, 1, 1)])
+def test_batch_of_both_confinement_forms_equals_single_steps(forms):
+    """Windows confined from a snapshot (1) beside windows confined by the
+    sweep (0): in one batch each form takes its own launch over the one list."""
+    import torch
+
+    stream = torch.cuda.Stream()
+    scenes = [S.grid(res=r, seed=0x31 + r, puddles=3) for r in (96, 130, 200)]
+    alone = [make(sc, fast=True) for sc in scenes]
+    grouped = [make(sc, fast=True, stream=stream.cuda_stream) for sc in scenes]
+    for sheets in (alone, grouped):
+        for sh, snapshot in zip(sheets, forms):
+            if snapshot:
+                sh.set_confinement(G.CONFINE_SNAPSHOT)
+    batch = G.Batch(grouped)
+    for _ in range(6):
+        for sh in alone:
+            sh.step(DT, want_spray=False)
+        batch.step(DT)
+    for w in range(len(scenes)):
+        for name in ("water", "slurry", "uw", "vw", "us", "vs"):
+            a, b = alone[w].get(name), grouped[w].get(name)
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (w, name, float(np.abs(a - b).max()))
+    batch.close()
