@@ -23,6 +23,7 @@
 // no flux and no force. The full-grid pass therefore gives the reference's
 // depths and velocities on every cell that holds fluid.
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <mutex>
 #include <type_traits>
@@ -53,7 +54,7 @@ constexpr int FORCE_THREADS = 512;
 // p (2) + gravity (1) + vorticity (2) + projection (4). Seven planes (70 KB):
 // three CTAs share an SM. Their time is block barriers between ten short
 // stages, so a third tile on the SM fills the other two's waits: k_force on a
-// flooded 1000^2 grid 86 us with eight planes and two CTAs.
+// flooded 1000^2 grid 90 us with eight planes and two CTAs, 83 so.
 using Snap = TileGeom<9, 7>;
 constexpr int SNAP_CTAS = 3;  // per SM
 // The sweep form's stages meet in global memory, so no stage reaches further
@@ -176,6 +177,22 @@ __device__ __forceinline__ float cell_decay(const LayerParams& P, size_t g, floa
     const float rate = P.nu_mode == NU_TABLE ? P.damp_plane[g] : sheet_damp(cell_nu(P, g));
     return exp_rn(-rate * dt);
 }
+
+// The damping factor of the viscosity a thread met last, for a layer with a
+// viscosity plane (NU_PLANE; one such layer and one dt to a launch): a film of
+// one material has one viscosity, and the factor is a double-precision power
+// and exponential (k_force on a flooded 1000^2 grid of one viscosity 83 us
+// evaluating it per cell, 70 so).
+struct LastDamp {
+    float nu = NAN, factor = 0.0f;  // NAN: none yet
+    __device__ __forceinline__ float of(float x, float dt) {
+        if (x != nu) {
+            nu = x;
+            factor = exp_rn(-sheet_damp(x) * dt);
+        }
+        return factor;
+    }
+};
 
 // Every cell of the tile's region of radius (RX, RY): f(gx, gy, s, g) with s
 // the shared-memory index and g the global one. The rectangle is walked as one
@@ -300,7 +317,8 @@ __device__ __forceinline__ void pressure_field(const TM& T, const LayerParams& P
 // (radius 4), depth and eta (radius 4) (src/fluid_core.rs:1992-2037). Writes
 // every cell of the tile to u_out, v_out.
 template <class TM, class G, bool EDGE>
-__device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, const ForcePlanes<G>& F, int tx0, int ty0) {
+__device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, const ForcePlanes<G>& F, int tx0, int ty0,
+                                            LastDamp* last = nullptr) {
     const int res = P.res;
     const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float dt = P.dt, eps = P.eps;
@@ -345,7 +363,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
                 uu += 0.012f * dt * qx;
                 vv += 0.012f * dt * qz;
             }
-            float decay = cell_decay(P, g, dt);
+            float decay = last && P.nu_mode == NU_PLANE ? last->of(P.nu_plane[g], dt) : cell_decay(P, g, dt);
             uu = finite_speed(uu * decay, kSpeedCap);
             vv = finite_speed(vv * decay, kSpeedCap);
         }
@@ -360,7 +378,8 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
 // are plain offsets. Threads walk the regions as rows (one warp per row,
 // lanes along x).
 template <class TM, class G, bool EDGE>
-__device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0) {
+__device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, float* sm, int tx0, int ty0,
+                                           LastDamp* last) {
     const int res = P.res;
     const ForcePlanes<G> F(sm);
     const int ox = tx0 - G::H, oy = ty0 - G::H;
@@ -413,7 +432,7 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
         });
         T.sync();
     }
-    finish_tile<TM, G, EDGE>(T, P, F, tx0, ty0);
+    finish_tile<TM, G, EDGE>(T, P, F, tx0, ty0, last);
 }
 
 // Sweep form, part 1: the post-gravity velocity G of every cell of the tile
@@ -669,7 +688,8 @@ __device__ __forceinline__ bool tile_interior(int res, int tx0, int ty0) {
 // One list entry of the force pass (the sweep form's first part for a
 // sweeping layer). Returns true when it used shared memory.
 template <class G, class TM>
-__device__ __forceinline__ bool force_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int nxt, int e, float* sm) {
+__device__ __forceinline__ bool force_entry(const TM& T, const LayerParams& P, const TileFlags& tf, int nxt, int e, float* sm,
+                                            LastDamp* last = nullptr) {
     const int l = e >> 30, zero_fill = (e & ENTRY_ZERO) != 0, copy = (e & ENTRY_COPY) != 0, t = e & ENTRY_TILE;
     const int res = P.res;
     const int tx0 = (t % tf.tiles_x) * FT, ty0 = (t / tf.tiles_x) * FT;
@@ -704,9 +724,9 @@ __device__ __forceinline__ bool force_entry(const TM& T, const LayerParams& P, c
         else
             pre_tile<TM, G, true>(T, P, sm, tx0, ty0);
     } else if (interior) {
-        force_tile<TM, G, false>(T, P, sm, tx0, ty0);
+        force_tile<TM, G, false>(T, P, sm, tx0, ty0, last);
     } else {
-        force_tile<TM, G, true>(T, P, sm, tx0, ty0);
+        force_tile<TM, G, true>(T, P, sm, tx0, ty0, last);
     }
     if (T.tid == 0) pick(tf.zero_uv, l, nxt)[t] = 0;
     return true;
@@ -955,9 +975,10 @@ __global__ void __launch_bounds__(FORCE_THREADS, SNAP_CTAS) k_force(ForceLaunch 
     __syncthreads();
     const int n = *L.tf.count;
     const WholeCta T;
+    LastDamp last;
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const int e = L.tf.list[k];
-        if (force_entry<Snap>(T, Ps[e >> 30], L.tf, L.nxt, e, sm)) T.sync();  // shared memory is reused by the next tile
+        if (force_entry<Snap>(T, Ps[e >> 30], L.tf, L.nxt, e, sm, &last)) T.sync();  // shared memory is reused by the next tile
     }
 }
 

@@ -69,7 +69,7 @@ __device__ __forceinline__ float hypot_rn(float x, float y) {
 __device__ __forceinline__ float sheet_damp(float nu) {
     float rel = rclamp(fmaxf(nu, 0.05f) / 231.0f, 0.002f, 12.0f);
     if (rel >= 0.42f) return 1.70f * pow_rn(rel, 0.30f);
-    const float at_silt = 1.70f * pow_rn(0.42f, 0.30f);
+    constexpr float at_silt = 1.70f * 0x1.8aadfe0000000p-1f;  // 0.42^0.30 rounded once, as pow_rn gives it
     float t = rclamp(rel / 0.42f, 0.0f, 1.0f);
     return at_silt * pow_rn(t, 1.15f);
 }

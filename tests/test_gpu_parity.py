@@ -203,6 +203,25 @@ def test_free_step_sheet_above_512_matches_oracle(res, speed, depth):
     assert dh <= TOL_H, dh
 
 
+@pytest.mark.parametrize("pattern", ["cells", "rows", "halves"])
+def test_free_step_sheet_above_512_with_mixed_viscosity_matches_oracle(pattern):
+    """A thread keeps the damping factor of the viscosity it met last: planes
+    that change it at every cell, every row, and once."""
+    import torch
+    res = 513
+    step, dev, (h, u, v, bed, nu) = free_operator(res, 0.5, 0.05)
+    jj, ii = np.mgrid[0:res, 0:res]
+    key = {"cells": ii + jj, "rows": jj, "halves": (ii >= res // 2).astype(int)}[pattern]
+    nu = np.array([0.05, 0.9, 30.0, 240.0], np.float32)[key % 4].ravel()
+    dev[4].copy_(torch.tensor(nu))
+    gate, sc = np.ones(res * res, np.uint8), O.Scratch()
+    for _ in range(3):
+        O.step_sheet(h, u, v, bed, nu, gate, res, 0.1, 0.05, 0.02, scratch=sc)
+        assert step(0.05) == 0
+    dh = np.abs(dev[0].cpu().numpy() - h).max()
+    assert dh <= TOL_H, dh
+
+
 @pytest.mark.parametrize("res,speed,count", [(513, 0.5, 1), (600, 2.6, 4), (515, 5.0, 7)])
 def test_free_step_sheet_above_512_counts_its_substeps(res, speed, count):
     """The first substep's dt is the device's own count of the speed, the
