@@ -110,8 +110,13 @@ static_assert((TS * sizeof(float)) % 16 == 0, "a TMA box row is a multiple of 16
 static_assert((TPL * sizeof(float)) % 128 == 0, "each transport plane starts 128-byte aligned");
 static_assert(TS * TW * sizeof(float) <= TPL * sizeof(float), "a TMA box fits its plane");
 constexpr int TRANSPORT_THREADS = 256;
+// Per SM, by registers (six planes are 34 KB). The tile's six dependent stages
+// wait at block barriers, which a fifth CTA fills: with eight planes and four,
+// 34 us instead of 31 on a flooded 1000^2 grid, 283 instead of 272 on 256
+// windows.
+constexpr int TRANSPORT_CTAS = 5;
 
-size_t transport_smem_bytes() { return sizeof(float) * TPL * 8; }
+size_t transport_smem_bytes() { return sizeof(float) * TPL * 6; }
 
 // Five taps left to right. Away from the edge the reference starts from the
 // first product (accum5); near it from 0.0 (accum5_clamped,
@@ -1143,8 +1148,8 @@ __device__ __forceinline__ void transport_tile(const TransportParams& P, float* 
     float* FR = sm + 3 * PL;    // right-going flux
     float* HX = sm + 4 * PL;    // depth after the x pass
     float* VS = sm + 5 * PL;    // v
-    float* UP = sm + 6 * PL;    // up-going flux of row pair (r, r+1)
-    float* DN = sm + 7 * PL;    // down-going flux
+    float* UP = FL;             // up-going flux of row pair (r, r+1): the x fluxes are spent by then
+    float* DN = FR;             // down-going flux
     const int ox = tx0 - 4, oy = ty0 - 2;
 #define TIDX(gx, gy) (((gy) - oy) * TS + ((gx) - ox))
     const int ry0 = max(0, ty0 - 2), ry1 = min(res, ty1 + 1);
@@ -1346,7 +1351,7 @@ __device__ __forceinline__ void transport_entry(const TransportParams& P, const 
 }
 
 // Persistent over the substep's tile list.
-__global__ void __launch_bounds__(TRANSPORT_THREADS) k_transport(TransportLaunch L,
+__global__ void __launch_bounds__(TRANSPORT_THREADS, TRANSPORT_CTAS) k_transport(TransportLaunch L,
                                                                    const __grid_constant__ TransportMaps M) {
     ::silt::dep_wait();
     extern __shared__ __align__(128) float sm[];
@@ -1626,7 +1631,7 @@ __global__ void __launch_bounds__(FORCE_THREADS, 2) k_batch_force_sweep(const Wi
         batch_force_sweep<HalfCta>(ws, nwin, list, entry_win, n, S, slots, sm);
 }
 
-__global__ void __launch_bounds__(TRANSPORT_THREADS) k_batch_transport(const WindowSubstep* ws, const int* list,
+__global__ void __launch_bounds__(TRANSPORT_THREADS, TRANSPORT_CTAS) k_batch_transport(const WindowSubstep* ws, const int* list,
                                                                        const int* entry_win, const int* count) {
     ::silt::dep_wait();
     extern __shared__ float sm[];
@@ -1817,7 +1822,7 @@ cudaError_t launch_transport(const TransportLaunch& L, int res, int layers, cuda
         M.on[l] = P.res == res && P.h && P.u && P.v && transport_map(P.h, res, &M.map[l][0]) &&
                   transport_map(P.u, res, &M.map[l][1]) && transport_map(P.v, res, &M.map[l][2]);
     }
-    ::silt::launch_dep(k_transport, dim3(148 * 4), dim3(TRANSPORT_THREADS), transport_smem_bytes(), st, L, M);
+    ::silt::launch_dep(k_transport, dim3(148 * TRANSPORT_CTAS), dim3(TRANSPORT_THREADS), transport_smem_bytes(), st, L, M);
     ::silt::count_launch();
     return cudaGetLastError();
 }
