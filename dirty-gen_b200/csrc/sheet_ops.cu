@@ -193,18 +193,6 @@ __global__ void k_export(const float* bed, const float* water, const float* slur
     }
 }
 
-// FP64 sums of max(h, 0) for two planes (the ledger's column_sum, src/fluid_core.rs:4617).
-__global__ void k_sum2(const float* a, const float* b, size_t n, double* out) {
-    ::silt::dep_wait();
-    double sa = 0.0, sb = 0.0;
-    GRID_STRIDE(i, n) {
-        sa += (double)fmaxf(a[i], 0.0f);
-        sb += (double)fmaxf(b[i], 0.0f);
-    }
-    ::silt::block_add(sa, out);
-    ::silt::block_add(sb, out + 1);
-}
-
 // The last block of a launch to finish (the ticket counts finished blocks)
 // adds the blocks' partial pairs part[2k], part[2k + 1], k < nb, in a fixed
 // order into out[0], out[1] and re-arms the ticket, so the sum does not
@@ -237,8 +225,9 @@ __device__ __forceinline__ void ordered_finish(double sa, double sb, double* par
     }
 }
 
-// k_sum2 with a fixed grid and an ordered finish: the same planes give the
-// same bits on every call.
+// FP64 sums of max(h, 0) for two planes (the ledger's column_sum,
+// src/fluid_core.rs:4617), with a fixed grid and an ordered finish: the same
+// planes give the same bits on every call.
 __global__ void k_sum2_ordered(const float* a, const float* b, size_t n, double* out, double* part,
                                unsigned int* ticket) {
     ::silt::dep_wait();
@@ -440,16 +429,9 @@ cudaError_t op_export(const float* bed, const float* water, const float* slurry,
     return cudaGetLastError();
 }
 cudaError_t op_sum2(const float* a, const float* b, size_t n, double* out, cudaStream_t st, double* scratch) {
-    if (scratch) {
-        const int nb = std::min(blocks_for(n), SUM_BLOCKS);
-        unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch + 2 * SUM_BLOCKS);
-        ::silt::launch_dep(k_sum2_ordered, dim3(nb), dim3(256), 0, st, a, b, n, out, scratch, ticket);
-        ::silt::count_launch();
-        return cudaGetLastError();
-    }
-    cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(double), st);
-    if (e != cudaSuccess) return e;
-    ::silt::launch_dep(k_sum2, dim3(blocks_for(n)), dim3(256), 0, st, a, b, n, out);
+    const int nb = std::min(blocks_for(n), SUM_BLOCKS);
+    unsigned int* ticket = reinterpret_cast<unsigned int*>(scratch + 2 * SUM_BLOCKS);
+    ::silt::launch_dep(k_sum2_ordered, dim3(nb), dim3(256), 0, st, a, b, n, out, scratch, ticket);
     ::silt::count_launch();
     return cudaGetLastError();
 }

@@ -32,9 +32,9 @@ cudaError_t op_export(const float* bed, const float* water, const float* slurry,
 // a ticket (SUM_SCRATCH_BYTES, zeroed once).
 constexpr int SUM_BLOCKS = 1184;
 constexpr size_t SUM_SCRATCH_BYTES = (2 * SUM_BLOCKS + 2) * sizeof(double);
-// out[0..1] = FP64 sums of max(a, 0) and max(b, 0). With `scratch` the sum
-// is ordered (the same bits on every call); without it, blocks add atomically.
-cudaError_t op_sum2(const float* a, const float* b, size_t n, double* out, cudaStream_t st, double* scratch = nullptr);
+// out[0..1] = FP64 sums of max(a, 0) and max(b, 0), ordered: the same bits on
+// every call.
+cudaError_t op_sum2(const float* a, const float* b, size_t n, double* out, cudaStream_t st, double* scratch);
 // Every window's suspended and silt column sums into out[16 w + 14, 15], in
 // a fixed order; `scratch` (sum_tracers_scratch_bytes(n), zeroed once).
 size_t sum_tracers_scratch_bytes(int n);
