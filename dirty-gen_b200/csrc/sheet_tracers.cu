@@ -1287,6 +1287,16 @@ struct Sequence {
     int blocks = 1;
 };
 
+// The blocks of a pass over whole windows. One window's runs cost about the
+// same, so it gets the blocks that are resident at once (3 per SM by
+// registers), and each ends with one set of block sums: with 8 per SM, 2048^2
+// took 31 us in k_apply and 24 in k_collect instead of 22 and 21. Several
+// windows differ more, and more blocks even them out (256 windows: 171 and 102
+// us with 16 per SM, 233 and 147 with 6).
+int whole_window_blocks(const Runner& R, int n) {
+    return n == 1 ? std::min(std::max(R.blocks_total, 1), 148 * 3) : std::max(R.blocks_total, 1);
+}
+
 // The blocks of each window: about `total` of 256 threads in all, shared out by
 // the windows' cells (at least one each, at most one per 256 cells). An equal
 // share per window, as it was, let the largest of a mixed batch (64^2 to
@@ -1329,7 +1339,7 @@ cudaError_t upload(Runner& R, const Window* w, int n, float dt, float foam_decay
     }
     size_t np = 0;
     for (int k = 0; k < n; ++k) np += (size_t)w[k].npush;
-    out->blocks = split_blocks(w, n, std::max(R.blocks_total, 1), [](int, int) {});
+    out->blocks = split_blocks(w, n, whole_window_blocks(R, n), [](int, int) {});
     const size_t slices_at = ((size_t)n * sizeof(Job) + 15) & ~(size_t)15;
     const size_t push_at = slices_at + (n > 1 ? (size_t)out->blocks * sizeof(Slice) : 0);
     const size_t bytes = push_at + np * sizeof(silt_tire_push);
@@ -1348,7 +1358,7 @@ cudaError_t upload(Runner& R, const Window* w, int n, float dt, float foam_decay
     Job* const jobs = (Job*)h;
     if (n > 1) {
         Slice* to = (Slice*)(h + slices_at);
-        split_blocks(w, n, std::max(R.blocks_total, 1), [&to](int k, int b) {
+        split_blocks(w, n, whole_window_blocks(R, n), [&to](int k, int b) {
             for (int q = 0; q < b; ++q) *to++ = Slice{k, (unsigned)q, (unsigned)b, 0};
         });
         out->slices = (const Slice*)(d + slices_at);
