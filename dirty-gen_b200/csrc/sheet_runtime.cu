@@ -3043,8 +3043,9 @@ int silt_step_sheet(float* h, float* u, float* v, const float* bed, const float*
     count.cap = 8.0f;
     count.launched = 8;
     int rc = substep(dt, count);
+    const cudaError_t waited = cudaEventSynchronize(back->ev);  // also after a failure: the slot serves the next call
     if (rc) return rc;
-    CK(cudaEventSynchronize(back->ev));
+    CK(waited);
     const unsigned int bits = back->host[0];
     double sum;
     memcpy(&sum, back->host + 8, sizeof sum);
