@@ -36,30 +36,12 @@
 #include "block_sum.cuh"
 #include "sheet_math.cuh"
 #include "launch_count.cuh"
+#include "tile_geom.cuh"
 
 namespace silt {
 
-constexpr int FT = 32;       // force tile edge
-// Shared-memory layout of a force tile: the halo its widest stage reads and
-// the eight planes' width and size.
-template <int HALO, int PLANES>
-struct TileGeom {
-    static constexpr int H = HALO;
-    static constexpr int W = FT + 2 * H;
-    static constexpr int PLANE = W * W;
-    static constexpr size_t BYTES = sizeof(float) * PLANES * PLANE;
-};
 constexpr int FORCE_THREADS = 512;
-// The snapshot form carries every stage of a cell through one tile:
-// p (2) + gravity (1) + vorticity (2) + projection (4). Seven planes (70 KB):
-// three CTAs share an SM. Their time is block barriers between ten short
-// stages, so a third tile on the SM fills the other two's waits: k_force on a
-// flooded 1000^2 grid 90 us with eight planes and two CTAs, 83 so.
-using Snap = TileGeom<9, 7>;
 constexpr int SNAP_CTAS = 3;  // per SM
-// The sweep form's stages meet in global memory, so no stage reaches further
-// than the projection's 4 cells: 51 KB a tile instead of 80.
-using Sweep = TileGeom<4, 8>;
 constexpr size_t SWEEP_SMEM = 2 * Sweep::BYTES;  // a CTA's two teams
 static_assert(2 * (SWEEP_SMEM + 2048) <= 228 * 1024, "two sweep CTAs share an SM");
 
@@ -199,22 +181,6 @@ struct LastDamp {
     }
 };
 
-// Every cell of the tile's region of radius (RX, RY): f(gx, gy, s, g) with s
-// the shared-memory index and g the global one. The rectangle is walked as one
-// flat range (a compile-time width), which keeps every lane busy; on edge
-// tiles cells outside the grid are left out.
-template <class TM, class G, bool EDGE, int RX, int RY, class F>
-__device__ __forceinline__ void region(const TM& T, int tx0, int ty0, int res, F f) {
-    const int ox = tx0 - G::H, oy = ty0 - G::H;
-    constexpr int RW = FT + 2 * RX, RH = FT + 2 * RY;
-    for (int k = T.tid; k < RW * RH; k += TM::NT) {
-        const int r = k / RW;
-        const int gy = ty0 - RY + r, gx = tx0 - RX + (k - r * RW);
-        if (EDGE && ((unsigned)gx >= (unsigned)res || (unsigned)gy >= (unsigned)res)) continue;
-        f(gx, gy, (gy - oy) * G::W + (gx - ox), gy * res + gx);
-    }
-}
-
 // The velocity a substep starts from at (gx, gy), from the plane's (uu, vv):
 // the lazy dry cut of the previous substep, then the soft window border
 // (src/fluid_core.rs:9594-9622; a river reach's band keeps its current through
@@ -289,25 +255,25 @@ __device__ __forceinline__ void pressure_field(const TM& T, const LayerParams& P
     const int res = P.res;
     const int ox = tx0 - G::H, oy = ty0 - G::H;
     const float *depth = P.h, *bed = P.bed, *u = P.u, *v = P.v;
-    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         stage(&F.HS[s], depth + g);
         stage(&F.E[s], bed + g);
     });
-    region<TM, G, EDGE, RV, RV>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, RV, RV>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         stage(&F.U[s], u + g);
         stage(&F.V[s], v + g);
     });
     staged();
-    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int, int, int s, int) { F.E[s] += F.HS[s]; });
+    region<TM, G, EDGE, R + 2, R + 2>(T, tx0, ty0, res, [&](int, int, int s, typename G::Index) { F.E[s] += F.HS[s]; });
     T.sync();
-    region<TM, G, EDGE, R, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, R, R + 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
         float e0 = F.E[NX(-2)], e1 = F.E[NX(-1)], e2 = F.E[s], e3 = F.E[NX(1)], e4 = F.E[NX(2)];
         F.TG[s] = tap5(e0, e1, e2, e3, e4, kG0, kG1, kG2, in);
         F.TS[s] = tap5(e0, e1, e2, e3, e4, kS0, kS1, kS2, in);
     });
     T.sync();
-    region<TM, G, EDGE, R, R>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, R, R>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         const bool in = EDGE ? (gy >= 2 && gy <= res - 3) : true;
         const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
         float gb = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
@@ -329,7 +295,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
     const float dt = P.dt, eps = P.eps;
     if (P.project) {
         // b = div * overload - 0.015 * overload * lap(eta), radius 3 (:1992-2003).
-        region<TM, G, EDGE, 3, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 3, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             const int sxp = NX(1), sxm = NX(-1), szp = NZ(1), szm = NZ(-1);
             float ux = fdiv(F.U[sxp] - F.U[sxm], P.div_two);
             float vz = fdiv(F.V[szp] - F.V[szm], P.div_two);
@@ -341,7 +307,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         });
         T.sync();
         // x pass of both blurs of b: rows radius 3, columns radius 1.
-        region<TM, G, EDGE, 1, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 1, 3>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             const bool in = EDGE ? (gx >= 2 && gx <= res - 3) : true;
             float b0 = F.PB[NX(-2)], b1 = F.PB[NX(-1)], b2 = F.PB[s], b3 = F.PB[NX(1)], b4 = F.PB[NX(2)];
             F.TG[s] = tap5(b0, b1, b2, b3, b4, kG0, kG1, kG2, in);
@@ -349,7 +315,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         });
         T.sync();
         // q = 0.62 G(b) + 0.38 S(b), radius 1 (:2004-2011).
-        region<TM, G, EDGE, 1, 1>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 1, 1>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             const bool in = EDGE ? (gy >= 2 && gy <= res - 3) : true;
             const int s0 = NZ(-2), s1 = NZ(-1), s3 = NZ(1), s4 = NZ(2);
             float gq = tap5(F.TG[s0], F.TG[s1], F.TG[s], F.TG[s3], F.TG[s4], kG0, kG1, kG2, in);
@@ -359,7 +325,7 @@ __device__ __forceinline__ void finish_tile(const TM& T, const LayerParams& P, c
         T.sync();
     }
     // Projection kick, damping and the speed clamp on wet cells (:2015-2037).
-    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         float uu = F.U[s], vv = F.V[s];
         if (F.HS[s] > eps) {
             if (P.project) {
@@ -394,7 +360,7 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
     pressure_field<TM, G, EDGE, 7, 6>(T, P, F, tx0, ty0);
     // Velocity on radius 6 and gravity down the pressure gradient on wet
     // cells (src/fluid_core.rs:2234-2253).
-    region<TM, G, EDGE, 6, 6>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, 6, 6>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         float uu = F.U[s], vv = F.V[s];
         start_velocity(P, band, gx, gy, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
@@ -410,7 +376,7 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
     T.sync();
     // Vorticity of the post-gravity snapshot, radius 5 (src/fluid_core.rs:3498-3506).
     if (P.vort > 0.0f) {
-        region<TM, G, EDGE, 5, 5>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 5, 5>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             float dvdx = fdiv(F.V[NX(1)] - F.V[NX(-1)], P.div_two);
             float dudz = fdiv(F.U[NZ(1)] - F.U[NZ(-1)], P.div_two);
             F.TG[s] = dvdx - dudz;
@@ -418,7 +384,7 @@ __device__ __forceinline__ void force_tile(const TM& T, const LayerParams& P, fl
         T.sync();
         // Confinement kick from that snapshot, in place, radius 4
         // (src/fluid_core.rs:2348-2375, :2441-2470).
-        region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             if (F.HS[s] > eps) {
                 float w = F.TG[s];
                 if (finite_f(w) && !(fabsf(w) < 1.0e-4f)) {
@@ -451,7 +417,7 @@ __device__ __forceinline__ void pre_tile(const TM& T, const LayerParams& P, floa
     const int band = tile_band<G>(P, tx0, ty0);
     const float dt = P.dt, eps = P.eps;
     pressure_field<TM, G, EDGE, 1, 0>(T, P, F, tx0, ty0);
-    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+    region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
         float uu = F.U[s], vv = F.V[s];
         start_velocity(P, band, gx, gy, F.HS[s], uu, vv);
         if (F.HS[s] > eps) {
@@ -516,7 +482,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
     float *__restrict__ fu = P.fu, *__restrict__ fv = P.fv;
     auto own = [&](int gx, int gy) { return gx >= tx0 && gx < tx0 + FT && gy >= ty0 && gy < ty0 + FT; };
     if (reuse) {
-        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             if (!own(gx, gy) && HS[s] > eps) {
                 stage(&FU[s], fu + g);
                 stage(&FV[s], fv + g);
@@ -525,7 +491,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
         staged();
     } else {
         const float *depth = P.h, *u = P.u, *v = P.v, *gu = P.u_out, *gv = P.v_out;
-        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             stage(&HS[s], depth + g);
             stage(&PU[s], u + g);
             stage(&PV[s], v + g);
@@ -539,7 +505,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
         });
         staged();
         // The same thread's cells again.
-        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, int) {
+        region<TM, G, EDGE, 2, 2>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index) {
             const float hv = HS[s];
             float uu = PU[s], vv = PV[s];
             start_velocity(P, band, gx, gy, hv, uu, vv);
@@ -609,7 +575,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
                 if (HS[s] > eps) solve(gx, gy, s);
             }
         } else {
-            region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int) {
+            region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index) {
                 if (it > 0) {
                     if (!mark[s]) return;
                     mark[s] = 0;
@@ -622,7 +588,7 @@ __device__ bool sweep_tile(const TM& T, const LayerParams& P, float* sm, int tx0
         tile_changed = true;
     }
     if (tile_changed) {
-        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, int g) {
+        region<TM, G, EDGE, 0, 0>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index g) {
             if (HS[s] > eps) {
                 fu[g] = FU[s];
                 fv[g] = FV[s];
@@ -640,7 +606,7 @@ __device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, flo
     const int band = tile_band<G>(P, tx0, ty0);
     const float eps = P.eps;
     const float *depth = P.h, *bed = P.bed, *u = P.u, *v = P.v, *fu = P.fu, *fv = P.fv;
-    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int, int, int s, int g) {
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int, int, int s, typename G::Index g) {
         stage(&F.HS[s], depth + g);
         stage(&F.E[s], bed + g);
         stage(&F.U[s], u + g);
@@ -649,7 +615,7 @@ __device__ __forceinline__ void post_tile(const TM& T, const LayerParams& P, flo
         stage(&F.TS[s], fv + g);
     });
     staged();
-    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, int) {
+    region<TM, G, EDGE, 4, 4>(T, tx0, ty0, res, [&](int gx, int gy, int s, typename G::Index) {
         const float hv = F.HS[s];
         F.E[s] += hv;
         float uu = F.U[s], vv = F.V[s];
@@ -1164,7 +1130,8 @@ __device__ __forceinline__ void transport_tile(const TransportParams& P, float* 
     if (!by_tma) {
         const float *h = P.h, *u = P.u, *v = P.v;
         trows<EDGE, TT + 3, TT + 3>(cx0, cx1, ry0, ry1, [&](int gx, int gy) {
-            const int g = gy * res + gx, s = TIDX(gx, gy);
+            const size_t g = plane_index<size_t>(gx, gy, res);
+            const int s = TIDX(gx, gy);
             stage(&HSm[s], h + g);
             stage(&US[s], u + g);
             if (gx >= tx0 && gx < tx1) stage(&VS[s], v + g);
@@ -1552,7 +1519,7 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_batch_force(const WindowSubst
             nxt_s = D.F.nxt;
         }
         __syncthreads();
-        if (!Ps.sweep) force_entry<Snap>(T, Ps, Tf, nxt_s, e, sm);  // the others are k_batch_force_sweep's
+        if (!Ps.sweep) force_entry<SheetSnap>(T, Ps, Tf, nxt_s, e, sm);  // the others are k_batch_force_sweep's
         __syncthreads();  // the parameters and shared memory are reused by the next entry
     }
 }

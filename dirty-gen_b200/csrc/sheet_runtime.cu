@@ -37,6 +37,7 @@
 #include "sheet_park.cuh"
 #include "sheet_tracers.cuh"
 #include "sheet_window.cuh"
+#include "tile_geom.cuh"
 
 namespace {
 
@@ -627,7 +628,7 @@ void silt_cfg_default(silt_cfg* c) {
 
 int silt_sheet_create(const silt_cfg* cfg, silt_sheet** out) {
     if (!cfg || !out) return fail_arg("cfg/out");
-    if (cfg->res < 8 || cfg->res > 32768 || !(cfg->cell > 0.0f)) return fail_arg("res/cell");
+    if (cfg->res < 8 || cfg->res > silt::MAX_SHEET_RES || !(cfg->cell > 0.0f)) return fail_arg("res/cell");
     if (cfg->fine_res < 8 || cfg->fine_res > 1024 || !(cfg->fine_cell > 0.0f)) return fail_arg("fine_res/fine_cell");
     float ratio = cfg->cell / cfg->fine_cell;
     if (fabsf(ratio - roundf(ratio)) > 1.0e-3f || roundf(ratio) < 1.0f) return fail_arg("cell/fine_cell not whole");
