@@ -37,10 +37,13 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstdio>
+#include <map>
+#include <mutex>
 
 #include "../../include/silt_closure.h"
 #include "closure.cuh"
 #include "launch_count.cuh"
+#include "per_device.cuh"
 
 namespace silt {
 namespace closure {
@@ -603,26 +606,17 @@ __global__ void k_wait_probe(int* err, int polls) {
     if (!ok && threadIdx.x == 0 && err) atomicExch(err, 1);
 }
 
-template <class K>
-cudaError_t set_smem(K kernel, int bytes) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-}
-
 int sm_count() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
+    static PerDevice<int> n;
+    return n.of(query_sm_count);
 }
 
 template <int CIN, int COUT>
 cudaError_t conv_launch(const ConvArgs& a, cudaStream_t st) {
     using S = ConvShape<CIN, COUT>;
-    static cudaError_t attr = set_smem(k_conv3x3<CIN, COUT>, S::SMEM);
-    if (attr != cudaSuccess) return attr;
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_conv3x3<CIN, COUT>, S::SMEM); });
+    if (allowed != cudaSuccess) return allowed;
     const int tiles = a.n_img * ((a.H + TILE_H - 1) / TILE_H) * ((a.W + TILE_W - 1) / TILE_W);
     const int grid = std::min(tiles, S::CTAS * sm_count());
     ::silt::launch_dep(k_conv3x3<CIN, COUT>, dim3(grid), dim3(THREADS), S::SMEM, st, a);
@@ -633,8 +627,9 @@ cudaError_t conv_launch(const ConvArgs& a, cudaStream_t st) {
 template <int CIN, int COUT>
 cudaError_t wgrad_launch(const WgradArgs& a, cudaStream_t st) {
     using S = WgradShape<CIN, COUT>;
-    static cudaError_t attr = set_smem(k_conv3x3_wgrad<CIN, COUT>, S::SMEM);
-    if (attr != cudaSuccess) return attr;
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_conv3x3_wgrad<CIN, COUT>, S::SMEM); });
+    if (allowed != cudaSuccess) return allowed;
     const int tiles = a.n_img * ((a.H + TILE_H - 1) / TILE_H) * ((a.W + TILE_W - 1) / TILE_W);
     const int grid = std::min(tiles, 2 * sm_count());  // two CTAs an SM by shared memory
     ::silt::launch_dep(k_conv3x3_wgrad<CIN, COUT>, dim3(grid), dim3(WG_THREADS), S::SMEM, st, a);
@@ -642,8 +637,14 @@ cudaError_t wgrad_launch(const WgradArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// The current device's error word (nullptr when there is no memory for it).
 int* err_slot() {
-    static int* d = nullptr;
+    static std::mutex m;
+    static std::map<int, int*> words;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(m);
+    int*& d = words[dev];
     if (!d && cudaMalloc(&d, sizeof(int)) == cudaSuccess) cudaMemset(d, 0, sizeof(int));
     return d;
 }

@@ -36,6 +36,7 @@
 #include "block_sum.cuh"
 #include "sheet_math.cuh"
 #include "launch_count.cuh"
+#include "per_device.cuh"
 #include "tile_geom.cuh"
 
 namespace silt {
@@ -1640,15 +1641,17 @@ cudaError_t launch_batch_speed2(const WindowSubstep* d_ws, const int* list, cons
     return cudaGetLastError();
 }
 
-// Grid of a cooperative force launch: every CTA the device holds at once.
-template <class K>
-int coop_grid(K kernel) {
-    int dev = 0, nsm = 0, per = 0;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SWEEP_SMEM);
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, FORCE_THREADS, SWEEP_SMEM) != cudaSuccess) return 0;
-    return nsm * per;
+// CTAs of a cooperative force launch that the current device holds at once;
+// not positive when it cannot be told (the launch is refused then).
+template <class... KArgs>
+int coop_grid(void (*kernel)(KArgs...), int dev) {
+    int per = 0;
+    if (allow_smem(kernel, SWEEP_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, FORCE_THREADS, SWEEP_SMEM) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return query_sm_count(dev) * per;
 }
 
 template <class K, class... Args>
@@ -1672,23 +1675,17 @@ cudaError_t launch_coop(K kernel, int grid, cudaStream_t st, Args... args) {
 cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* list, const int* entry_win,
                                const int* count, SweepState* sweep, bool snapshot, cudaStream_t st, int ctas_per_sm) {
     if (sweep) {
-        static std::once_flag sattr;
-        static int grid = 0, nsm = 148;
-        std::call_once(sattr, [] {
-            grid = coop_grid(k_batch_force_sweep);
-            int dev = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm <= 0)
-                nsm = 148;
-            cudaGetLastError();
-        });
+        static PerDevice<int> grids, sms;
+        const int grid = grids.of([](int dev) { return coop_grid(k_batch_force_sweep, dev); });
+        const int nsm = sms.of(query_sm_count);
         // Fewer CTAs than the device holds stay co-resident: the launch is still cooperative.
         const int g = ctas_per_sm > 0 ? std::min(grid, ctas_per_sm * nsm) : grid;
         const cudaError_t e = launch_coop(k_batch_force_sweep, g, st, d_ws, nwin, list, entry_win, count, sweep);
         if (e != cudaSuccess || !snapshot) return e != cudaSuccess ? e : cudaGetLastError();
     }
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_batch_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Snap::BYTES); });
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_batch_force, Snap::BYTES); });
+    if (allowed != cudaSuccess) return allowed;
     ::silt::launch_dep(k_batch_force, dim3(148 * 2), dim3(FORCE_THREADS), Snap::BYTES, st, d_ws, list, entry_win, count);
     ::silt::count_launch();
     return cudaGetLastError();
@@ -1696,8 +1693,9 @@ cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* l
 
 cudaError_t launch_batch_transport(const WindowSubstep* d_ws, const int* list, const int* entry_win,
                                    const int* count, cudaStream_t st, int blocks) {
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_batch_transport, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)transport_smem_bytes()); });
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_batch_transport, transport_smem_bytes()); });
+    if (allowed != cudaSuccess) return allowed;
     const unsigned grid = blocks > 0 ? (unsigned)blocks : 148u * 4u;
     ::silt::launch_dep(k_batch_transport, dim3(grid), dim3(TRANSPORT_THREADS), transport_smem_bytes(), st, d_ws, list, entry_win, count);
     ::silt::count_launch();
@@ -1707,16 +1705,14 @@ cudaError_t launch_batch_transport(const WindowSubstep* d_ws, const int* list, c
 cudaError_t launch_force(const ForceLaunch& L, int res, int layers, cudaStream_t st) {
     if (L.lay[0].sweep || L.lay[1].sweep) {
         if (!L.tf.sweep) return cudaErrorInvalidValue;
-        static std::once_flag sattr;
-        static int grid = 0;
-        std::call_once(sattr, [] {
-            grid = coop_grid(k_force_sweep);
-        });
+        static PerDevice<int> grids;
+        const int grid = grids.of([](int dev) { return coop_grid(k_force_sweep, dev); });
         const cudaError_t e = launch_coop(k_force_sweep, grid, st, L);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Snap::BYTES); });
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_force, Snap::BYTES); });
+    if (allowed != cudaSuccess) return allowed;
     (void)res;
     (void)layers;
     ::silt::launch_dep(k_force, dim3(148 * SNAP_CTAS), dim3(FORCE_THREADS), Snap::BYTES, st, L);
@@ -1779,8 +1775,9 @@ bool transport_map(const float* plane, int res, CUtensorMap* out) {
 }  // namespace
 
 cudaError_t launch_transport(const TransportLaunch& L, int res, int layers, cudaStream_t st) {
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_transport, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)transport_smem_bytes()); });
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_transport, transport_smem_bytes()); });
+    if (allowed != cudaSuccess) return allowed;
     (void)layers;
     // Interior tiles of a grid a multiple of 4 cells wide arrive by TMA.
     TransportMaps M;

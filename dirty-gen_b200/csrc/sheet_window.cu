@@ -27,6 +27,7 @@
 #include "sheet_math.cuh"
 #include "sheet_window.cuh"
 #include "launch_count.cuh"
+#include "per_device.cuh"
 
 namespace silt {
 namespace window {
@@ -1874,10 +1875,12 @@ static int crew_for(int max_res) {
 // Dynamic shared memory of a launch: the wet bits of its largest window and the runs.
 static size_t wet_bytes(int max_res) { return ((size_t)max_res * wet_words(max_res) + MAX_RUNS) * 4; }
 
-// The largest crew the device can hold at once (a cluster of full-SM CTAs).
-static int crew_limit_query(cudaStream_t st) {
-    cudaFuncSetAttribute(k_window_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wet_bytes(MAX_RES));
-    cudaFuncSetAttribute(k_window_step_list, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wet_bytes(MAX_RES));
+// The largest crew the current device can hold at once (a cluster of full-SM
+// CTAs), after the kernels' attributes are set there; 0 when it takes none.
+static int crew_limit_query(int) {
+    if (allow_smem(k_window_step, wet_bytes(MAX_RES)) != cudaSuccess ||
+        allow_smem(k_window_step_list, wet_bytes(MAX_RES)) != cudaSuccess)
+        return 0;
     if (cudaFuncSetAttribute(k_window_step, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaFuncSetAttribute(k_window_step_list, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
@@ -1888,7 +1891,6 @@ static int crew_limit_query(cudaStream_t st) {
         cfg.gridDim = dim3((unsigned)c, 1, 1);
         cfg.blockDim = dim3(NT, 1, 1);
         cfg.dynamicSmemBytes = wet_bytes(MAX_RES);
-        cfg.stream = st;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = (unsigned)c;
@@ -1903,22 +1905,18 @@ static int crew_limit_query(cudaStream_t st) {
     return 1;
 }
 
-static int crew_limit(cudaStream_t st) {
-    static std::once_flag once;
-    static int limit = 1;
-    std::call_once(once, [st] { limit = crew_limit_query(st); });
-    return limit;
-}
-
 // The crew for `njobs` jobs: as large as the window and the device allow, and
 // small enough that all the jobs' CTAs fit on the GPU about twice over.
-static int crew_of(int njobs, int max_res, cudaStream_t st) {
-    return std::max(1, std::min({crew_for(max_res), crew_limit(st), 296 / std::max(njobs, 1)}));
+static int crew_of(int njobs, int max_res) {
+    static PerDevice<int> limits;
+    const int limit = limits.of(crew_limit_query);
+    return limit <= 0 ? 0 : std::max(1, std::min({crew_for(max_res), limit, 296 / std::max(njobs, 1)}));
 }
 
 cudaError_t launch_window_step_list(Job* const* d_job_list, int njobs, int max_res, cudaStream_t st) {
     if (njobs <= 0) return cudaSuccess;
-    const int crew = crew_of(njobs, max_res, st);
+    const int crew = crew_of(njobs, max_res);
+    if (crew <= 0) return cudaErrorInvalidConfiguration;  // no room for a CTA's shared memory on this device
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(njobs * crew), 1, 1);
     cfg.blockDim = dim3(NT, 1, 1);
@@ -1941,7 +1939,8 @@ cudaError_t launch_window_step_list(Job* const* d_job_list, int njobs, int max_r
 
 cudaError_t launch_window_step(const Job* d_jobs, int njobs, int max_res, cudaStream_t st) {
     if (njobs <= 0) return cudaSuccess;
-    const int crew = crew_of(njobs, max_res, st);
+    const int crew = crew_of(njobs, max_res);
+    if (crew <= 0) return cudaErrorInvalidConfiguration;  // no room for a CTA's shared memory on this device
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(njobs * crew), 1, 1);
     cfg.blockDim = dim3(NT, 1, 1);
