@@ -231,12 +231,13 @@ int tiles_dirty(silt_sheet* s) {
 // Materialise the lazy dry cut before anything reads or writes the planes.
 // `read_only`: the caller only reads them, so the tile flags still hold and
 // the next step keeps to its active tiles (a quiet tile has no depth, so after
-// the cut no velocity either); otherwise that step takes every tile.
+// the cut no velocity either). Otherwise that step takes every tile, whether
+// or not a cut was pending: the caller writes the planes or hands them out.
 int flush_cut(silt_sheet* s, bool read_only = false) {
+    if (!read_only) s->tiles_all = true;
     if (!s->cut_pending) return SILT_OK;
     for (int l = 0; l < 2; ++l) CK(silt::launch_apply_cut(s->H(l), s->U(l), s->V(l), s->n, 1.0e-6f, s->st));
     s->cut_pending = false;
-    if (!read_only) s->tiles_all = true;
     return SILT_OK;
 }
 

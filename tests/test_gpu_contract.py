@@ -153,3 +153,46 @@ def test_publish_between_steps_changes_no_bit(res):
     assert cells[0] <= cells[1]
     if res == 640:
         assert cells[0] < cells[1]
+
+
+@pytest.mark.parametrize("before", ["publish", "get", "coarse_cell", "none"])
+def test_water_written_through_a_handed_out_plane_flows(before):
+    """Depth written into a dry, quiet part of a grid sheet through
+    plane_device, whatever read the planes before: the next steps give the
+    bits of the same depth written by the sheet's own call."""
+    import torch
+
+    import silt_scenes as S
+
+    res = 640
+    scene = S.grid(res=res, puddles=2)
+    a, b = (G.Sheet(res=res, engine=G.ENGINE_GRID, fine_res=64, layout=G.FINE_PER_TIRE) for _ in range(2))
+    for sh in (a, b):
+        S.seed_core(sh, scene)
+        for _ in range(3):
+            sh.step(1.0 / 120.0, want_spray=False)
+    dry = a.get("water").reshape(res, res) == 0.0
+    rows, cols = slice(8, 40), slice(560, 600)  # spans tiles, none of them near water
+    assert dry[:128, 480:].all()
+    for sh in (a, b):
+        sh.step(1.0 / 120.0, want_spray=False)
+        sh.step(1.0 / 120.0, want_spray=False)
+        if before == "publish":
+            sh.publish()
+        elif before == "get":
+            sh.get("water")
+        elif before == "coarse_cell":
+            sh.coarse_cell(3, 3)
+    plane = a.plane_device("water")
+    a.sync()
+    plane[rows, cols] = 0.1
+    torch.cuda.synchronize()
+    w = b.get("water").reshape(res, res)
+    w[rows, cols] = 0.1
+    b.set("water", w.ravel())
+    for _ in range(3):
+        for sh in (a, b):
+            sh.step(1.0 / 120.0, want_spray=False)
+    for name in ("water", "slurry", "uw", "vw", "us", "vs"):
+        assert np.array_equal(a.get(name).view(np.uint32), b.get(name).view(np.uint32)), name
+    assert (a.get("water").reshape(res, res)[rows, cols] > 0.0).any()
