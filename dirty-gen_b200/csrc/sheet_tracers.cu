@@ -63,9 +63,12 @@ __device__ __forceinline__ bool step_goes(const State* st) {
     return c->active && (st->wet_any || st->live_silt);
 }
 
+// The grid engine's pending dry cut: a cell with less water than this carries
+// no water velocity. A wet cell of the tracers may be one: its film is water
+// and slurry together.
+constexpr float CUT_EPS = 1.0e-6f;
 __device__ __forceinline__ float vel(const float* u, const Sheet& S, size_t g) {
-    // The grid engine's pending dry cut: a cell under eps carries no velocity.
-    return (S.cut_pending && S.water[g] < 1.0e-6f) ? 0.0f : u[g];
+    return (S.cut_pending && S.water[g] < CUT_EPS) ? 0.0f : u[g];
 }
 
 __device__ __forceinline__ float smoothstep_f(float e0, float e1, float x) {  // :9688-9691
@@ -589,7 +592,7 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs, const Slice
         const int ib = ib_next, j = j_next;
         const unsigned g0 = (unsigned)j * (unsigned)res + (unsigned)ib;
         unsigned mk[4];
-        bool wet[4];
+        bool wet[4], moves[4];
         // A run with no wet cell and no foam-live mark: its cells' marks become
         // 0 and nothing else happens there.
         bool busy = false;
@@ -598,6 +601,7 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs, const Slice
             mk[k] = m_next[k];
             const float h = w_next[k] + s_next[k];
             wet[k] = finite_f(h) && !(h < 0.004f);
+            moves[k] = !S.cut_pending || !(w_next[k] < CUT_EPS);
             busy = busy || wet[k] || (mk[k] & LIVE);
         }
         if (run + warps < runs.n) load_head(run + warps);
@@ -622,8 +626,8 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs, const Slice
                 nb[k][3] = S.water[g + res];
             }
             if (foam_on) {
-                uw4[k] = S.uw[g];
-                vw4[k] = S.vw[g];
+                uw4[k] = moves[k] ? S.uw[g] : 0.0f;
+                vw4[k] = moves[k] ? S.vw[g] : 0.0f;
             }
         }
 #pragma unroll
@@ -642,7 +646,7 @@ __global__ void __launch_bounds__(256, 3) k_collect(const Job* jobs, const Slice
             if (m != mk[k]) mark[g] = (uint8_t)m;
             if (foam_on) {
                 if (m & WET) {
-                    const float uu = uw4[k], vv = vw4[k];  // wet cells are far above the dry cut
+                    const float uu = uw4[k], vv = vw4[k];
                     float sample = 0.0f;
                     if (finite_f(uu) && finite_f(vv)) {
                         const float x = (float)i - uu * dt / S.cell;
@@ -897,6 +901,7 @@ __global__ void __launch_bounds__(256, 3) k_apply(const Job* jobs, const Slice* 
             const int i = ib + 32 * k;
             const unsigned g = g0 + 32u * k;
             const bool wet = is[k] & WET;
+            if (wet && S.cut_pending && hw[k] < CUT_EPS) u4[k] = v4[k] = 0.0f;
             float t = t4[k];
             if (is[k] & SETTLING) {
                 const float h = hw[k] + hs[k];

@@ -363,3 +363,33 @@ def test_reach_walks_every_chunk_in_order(res, rows, half_width, inlet, outlet, 
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (name, float(np.abs(a - b).max()))
     led = dev.ledger()
     assert abs(led["reach_m3"] - ref.reach_bank_m3()) <= 1e-4 * abs(led["reach_m3"]) + 1e-6
+
+
+@pytest.mark.parametrize("engine", [G.ENGINE_WINDOW, G.ENGINE_GRID])
+def test_a_drained_film_carries_no_foam(engine):
+    """A moving water film over slurry that falls under the dry cut in one
+    step: its cells are still wet to the tracers (the slurry alone is 4 mm)
+    and move no more, so they neither break nor carry the foam that lies on
+    them. The grid engine leaves that cut for the next step's reads."""
+    dt, res = 1.0 / 30.0, 96
+    ref, dev = Pair(res=res), G.Sheet(res=res, engine=engine)
+    for c in (ref, dev):
+        c.set_near_field(False)
+        c.pour_slurry(-4.0, 4.0, -4.0, 4.0, 0.01, 0, 0.6)
+        c.pour_water(-4.0, 4.0, -4.0, 4.0, 0.03)
+    for _ in range(4):
+        for c in (ref, dev):
+            c.push_tire(**PUSH)
+            c.step(dt)
+    foam, slurry = ref.get("foam"), ref.get("slurry")
+    # Every third column a film of 1.1 um at 2.2 m/s: it gives a seventh away and falls under 1 um.
+    film = (slurry > 0.006) & (np.arange(res * res) % res % 3 == 1)
+    for c in (ref, dev):
+        c.set("water", np.where(film, F(1.1e-6), F(0.0)).astype(F))
+        c.set("uw", np.where(film, F(2.2), F(0.0)).astype(F))
+        c.set("vw", np.zeros(res * res, F))
+        c.push_tire(**PUSH)
+        c.step(dt)
+    drained = film & (ref.get("water") == 0.0) & (ref.get("slurry") >= F(0.004))
+    assert drained.sum() > 100 and (drained & (foam > 1.0e-4)).sum() > 4
+    ref.check(dev)
