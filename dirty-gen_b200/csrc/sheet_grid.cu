@@ -938,9 +938,9 @@ __global__ void __launch_bounds__(FORCE_THREADS, 2) k_force_sweep(ForceLaunch L)
         force_sweep<HalfCta>(L, Ps, n, sm);
 }
 
-// Persistent over the substep's tile list.
-__global__ void __launch_bounds__(FORCE_THREADS, SNAP_CTAS) k_force(ForceLaunch L) {
-    ::silt::dep_wait();
+// The snapshot form's force pass, persistent over the substep's tile list.
+template <class G>
+__device__ __forceinline__ void force_snapshot(const ForceLaunch& L) {
     extern __shared__ float sm[];
     __shared__ LayerParams Ps[2];
     if (threadIdx.x < 2) Ps[threadIdx.x] = force_params(L.lay[threadIdx.x], L.sc, threadIdx.x, blockIdx.x == 0);
@@ -950,8 +950,19 @@ __global__ void __launch_bounds__(FORCE_THREADS, SNAP_CTAS) k_force(ForceLaunch 
     LastDamp last;
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const int e = L.tf.list[k];
-        if (force_entry<Snap>(T, Ps[e >> 30], L.tf, L.nxt, e, sm, &last)) T.sync();  // shared memory is reused by the next tile
+        if (force_entry<G>(T, Ps[e >> 30], L.tf, L.nxt, e, sm, &last)) T.sync();  // shared memory is reused by the next tile
     }
+}
+
+__global__ void __launch_bounds__(FORCE_THREADS, SNAP_CTAS) k_force(ForceLaunch L) {
+    ::silt::dep_wait();
+    force_snapshot<Snap>(L);
+}
+
+// On a grid of more than MAX_NEAR_RES cells a side.
+__global__ void __launch_bounds__(FORCE_THREADS, SNAP_CTAS) k_force_far(ForceLaunch L) {
+    ::silt::dep_wait();
+    force_snapshot<FarSnap>(L);
 }
 
 // The list entry of tile t of layer l for this substep, or -1 for none.
@@ -1520,7 +1531,7 @@ __global__ void __launch_bounds__(FORCE_THREADS) k_batch_force(const WindowSubst
             nxt_s = D.F.nxt;
         }
         __syncthreads();
-        if (!Ps.sweep) force_entry<SheetSnap>(T, Ps, Tf, nxt_s, e, sm);  // the others are k_batch_force_sweep's
+        if (!Ps.sweep) force_entry<Snap>(T, Ps, Tf, nxt_s, e, sm);  // the others are k_batch_force_sweep's
         __syncthreads();  // the parameters and shared memory are reused by the next entry
     }
 }
@@ -1710,12 +1721,16 @@ cudaError_t launch_force(const ForceLaunch& L, int res, int layers, cudaStream_t
         const cudaError_t e = launch_coop(k_force_sweep, grid, st, L);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
-    static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_force, Snap::BYTES); });
-    if (allowed != cudaSuccess) return allowed;
-    (void)res;
     (void)layers;
-    ::silt::launch_dep(k_force, dim3(148 * SNAP_CTAS), dim3(FORCE_THREADS), Snap::BYTES, st, L);
+    static_assert(FarSnap::BYTES == Snap::BYTES, "one tile layout");
+    static PerDevice<cudaError_t> attr;
+    const cudaError_t allowed = attr.of([](int) {
+        const cudaError_t e = allow_smem(k_force, Snap::BYTES);
+        return e != cudaSuccess ? e : allow_smem(k_force_far, Snap::BYTES);
+    });
+    if (allowed != cudaSuccess) return allowed;
+    ::silt::launch_dep(res > MAX_NEAR_RES ? k_force_far : k_force, dim3(148 * SNAP_CTAS), dim3(FORCE_THREADS),
+                       Snap::BYTES, st, L);
     ::silt::count_launch();
     return cudaGetLastError();
 }

@@ -52,15 +52,19 @@ SILT_TILE_FN void region(const TM& T, int tx0, int ty0, int res, F f) {
 // three CTAs share an SM. Their time is block barriers between ten short
 // stages, so a third tile on the SM fills the other two's waits: k_force on a
 // flooded 1000^2 grid 90 us with eight planes and two CTAs, 83 so.
-// The free operator takes any grid whose planes the device holds, and from
-// 46341 cells a side on a place is past 2^31: 64-bit places.
-using Snap = TileGeom<9, 7, size_t>;
-// A sheet has at most MAX_SHEET_RES cells a side: 32-bit places, which cost no
-// register pair (the batch's snapshot kernel holds 64 registers a thread with
-// them, which two CTAs per SM need, and 73 with 64-bit ones).
+// 32-bit places reach MAX_NEAR_RES cells a side: every sheet (MAX_SHEET_RES at
+// most) and the free operator's grids up to there. The free operator takes any
+// grid whose planes the device holds (70 000 cells a side and more), and above
+// that size 64-bit places (FarSnap), which cost register pairs: on a flooded
+// 1000^2 grid k_force takes 67.7 us with 32-bit places and 69.0 with 64-bit
+// ones, and the batch's kernel 73 registers a thread for 64, one CTA per SM for
+// two.
+constexpr int MAX_NEAR_RES = 46340;
 constexpr int MAX_SHEET_RES = 32768;
-static_assert((long long)MAX_SHEET_RES * MAX_SHEET_RES <= 0x7fffffffLL, "a sheet's places fit an int");
-using SheetSnap = TileGeom<9, 7, int>;
+static_assert((long long)MAX_NEAR_RES * MAX_NEAR_RES <= 0x7fffffffLL && MAX_SHEET_RES <= MAX_NEAR_RES,
+              "a near grid's places fit an int");
+using Snap = TileGeom<9, 7, int>;
+using FarSnap = TileGeom<9, 7, size_t>;
 // The sweep form's stages meet in global memory, so no stage reaches further
 // than the projection's 4 cells: 51 KB a tile instead of 80. Only sheets take it.
 using Sweep = TileGeom<4, 8, int>;

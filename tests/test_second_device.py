@@ -21,6 +21,7 @@ RUNTIME = r"""
 
 // Two devices: the first of 148 SMs, the second of 60 that holds crews of up to 4.
 int device = 0, refused = 0;
+const void* kernel = nullptr;  // of the last launch
 int fail_attribute = -1;  // the device that refuses shared memory
 unsigned grid = 0, cluster = 0;
 static const int SMS[2] = {148, 60}, CREW[2] = {16, 4};
@@ -75,6 +76,7 @@ cudaError_t cudaGetDriverEntryPoint(const char*, void**, unsigned long long, cud
     return cudaErrorNotSupported;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* f, void**) {
+    kernel = f;
     grid = c->gridDim.x;
     cluster = 1;
     for (unsigned k = 0; k < c->numAttrs; ++k)
@@ -98,6 +100,7 @@ PROGRAM = r"""
 #include "sheet_window.cuh"
 
 extern int device, refused, fail_attribute;
+extern const void* kernel;
 extern unsigned grid, cluster;
 
 namespace silt {
@@ -128,6 +131,12 @@ int main(int argc, char** argv) {
         memset(&F, 0, sizeof F);
         F.tf.sweep = &sweep;
         ran(launch_force(F, 64, 2, nullptr));
+        // 32-bit places up to 46340 cells a side, a kernel of its own above.
+        const void* const near = kernel;
+        ran(launch_force(F, 46340, 2, nullptr));
+        failed += kernel != near;
+        ran(launch_force(F, 46341, 2, nullptr));
+        const int far = kernel != near;
         F.lay[0].sweep = 1;
         ran(launch_force(F, 64, 2, nullptr));
         const unsigned coop = grid;
@@ -141,7 +150,7 @@ int main(int argc, char** argv) {
         ran(closure::conv3x3(x, x, f, nullptr, x, nullptr, 64, 32, 32, 32, 32, 1, nullptr));
         const unsigned conv = grid;
         ran(closure::conv3x3_wgrad(x, x, f, f, 64, 32, 32, 32, 32, nullptr));
-        printf("%d %d %d %u %u %u %u\n", d, failed, refused, crew, coop, batch, conv);
+        printf("%d %d %d %u %u %u %u %d\n", d, failed, refused, crew, coop, batch, conv, far);
     }
 }
 """
@@ -166,7 +175,7 @@ def rows(program, *args):
 
 def test_every_launch_on_each_device(program):
     """No launch is refused, and crews and grids are each device's own."""
-    first, second = (0, 0, 0, 16, 148 * 2, 148 * 2, 512), (1, 0, 0, 4, 60 * 2, 60 * 2, 4 * 60)
+    first, second = (0, 0, 0, 16, 148 * 2, 148 * 2, 512, 1), (1, 0, 0, 4, 60 * 2, 60 * 2, 4 * 60, 1)
     assert rows(program) == [first, second, first, second]
 
 
@@ -175,4 +184,4 @@ def test_a_device_that_refuses_shared_memory_says_so(program):
     got = rows(program, "1")
     assert [r[0] for r in got] == [0, 1, 0, 1]
     assert all(r[1:3] == (0, 0) for r in got if r[0] == 0)
-    assert all(r[1:3] == (14, 0) for r in got if r[0] == 1)
+    assert all(r[1:3] == (16, 0) for r in got if r[0] == 1)

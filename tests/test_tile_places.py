@@ -42,11 +42,12 @@ void walk_all(int res) {
 
 int main(int, char** argv) {
     const int res = atoi(argv[1]);
-    walk_all<silt::Snap>(res);
-    if (res <= silt::MAX_SHEET_RES) {
-        walk_all<silt::SheetSnap>(res);
-        walk_all<silt::Sweep>(res);
-    }
+    // As launch_force picks: 32-bit places up to MAX_NEAR_RES.
+    if (res > silt::MAX_NEAR_RES)
+        walk_all<silt::FarSnap>(res);
+    else
+        walk_all<silt::Snap>(res);
+    if (res <= silt::MAX_SHEET_RES) walk_all<silt::Sweep>(res);
     printf("%lld %lld\n", seen, wrong);
 }
 """
