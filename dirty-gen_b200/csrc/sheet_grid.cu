@@ -94,9 +94,10 @@ static_assert((TPL * sizeof(float)) % 128 == 0, "each transport plane starts 128
 static_assert(TS * TW * sizeof(float) <= TPL * sizeof(float), "a TMA box fits its plane");
 constexpr int TRANSPORT_THREADS = 256;
 // Per SM, by registers (six planes are 34 KB). The tile's six dependent stages
-// wait at block barriers, which a fifth CTA fills: with eight planes and four,
-// 34 us instead of 31 on a flooded 1000^2 grid, 283 instead of 272 on 256
-// windows.
+// wait at block barriers, which a fifth CTA fills: k_transport, whose grid is
+// five per SM, 34 us with eight planes and four CTAs on a flooded 1000^2 grid
+// and 31 so. The batch's grid is its tuner's choice, four per SM by default: six
+// planes alone took it from 283 to 272 us on 256 windows.
 constexpr int TRANSPORT_CTAS = 5;
 
 size_t transport_smem_bytes() { return sizeof(float) * TPL * 6; }

@@ -81,9 +81,11 @@ struct TileFlags {
     unsigned long long* stepped;  // per layer: running total of tiles stepped (may be nullptr)
     int32_t tiles_x;
     SweepState* sweep;       // cleared by the tile-list kernel (may be nullptr)
-    // Per layer and tile (stamp[l * tiles_x^2 + t]): when the sweep last
-    // changed the tile, as epoch * 256 + pass + 1. A later pass solves a tile
-    // again only when its 3 x 3 neighbourhood changed since it was solved.
+    // Per layer and tile (stamp[l * tiles_x^2 + t]): when the sweep last changed
+    // a cell of the tile that another tile reads (columns 0, 30 and 31, rows 30
+    // and 31: sweep_tile's `exported`), as epoch * 256 + pass + 1. A later pass
+    // solves a tile again only when one of the five tiles whose cells it reads
+    // as earlier ones (left, right and the three above) was stamped since.
     unsigned int* stamp;
 };
 
@@ -166,7 +168,8 @@ cudaError_t launch_batch_speed2(const WindowSubstep* d_ws, const int* list, cons
 // cooperative launch (pre-sweep tiles, the sweep's fixed point, projection)
 // steps every such window; `snapshot`: some window takes the snapshot form,
 // in a launch of its own. `ctas_per_sm` caps the cooperative launch's CTAs per
-// SM (at most what the device holds at once; 0 = that maximum); `blocks` sizes the transport's persistent grid (0 = four per SM).
+// SM (at most what the device holds at once; 0 = that maximum); `blocks` sizes
+// the transport's persistent grid (0 = four per SM).
 // Every setting gives the same bits.
 cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* list, const int* entry_win,
                                const int* count, SweepState* sweep, bool snapshot, cudaStream_t st,

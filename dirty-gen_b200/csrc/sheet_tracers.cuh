@@ -84,8 +84,10 @@ struct Runner {
     size_t cap[SLOTS] = {};
     cudaEvent_t ev[SLOTS] = {};
     int next = 0;
-    // Blocks of a pass over all the windows of a launch: 8 per SM (measured
-    // against 16 and 32; any value gives the same planes).
+    // Blocks of a pass over all the windows of a launch; any value gives the
+    // same planes. A sheet's own runner keeps this bound, of which a pass takes
+    // what one window needs (whole_window_blocks, box_blocks); a batch sets its
+    // tuner's choice, 16 per SM by default.
     int blocks_total = 1184;
     void release();
 };

@@ -252,8 +252,9 @@ int silt_window_origin(float center_x, float center_z, int32_t res, float cell, 
 int silt_read_plane(silt_sheet* s, int32_t which, float* host);
 int silt_write_plane(silt_sheet* s, int32_t which, const float* host);
 /* Device pointer of plane `which` (same indices) in the handle's current
- * buffers, valid until the next step or write; the caller orders its reads
- * after the handle's stream. */
+ * buffers, valid until the next step or write; the caller orders its accesses
+ * after the handle's stream. The next step takes the planes as they then are
+ * (the grid engine steps every tile once). */
 int silt_plane_device(silt_sheet* s, int32_t which, void** out);
 /* Device-to-device copy of src's window state (depths, velocities, bed,
  * moisture, grain) into dst (same size and device); dst's nested patches and
