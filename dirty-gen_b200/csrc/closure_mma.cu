@@ -35,9 +35,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
-#include <map>
 #include <mutex>
 
 #include "../../include/silt_closure.h"
@@ -606,46 +606,58 @@ __global__ void k_wait_probe(int* err, int polls) {
     if (!ok && threadIdx.x == 0 && err) atomicExch(err, 1);
 }
 
-int sm_count() {
-    static PerDevice<int> n;
-    return n.of(query_sm_count);
-}
+// What a convolution's launch asks of a device: the leave for its shared
+// memory, and the SMs.
+struct LaunchRoom {
+    cudaError_t allowed = cudaSuccess;
+    int sms = 0;
+};
 
 template <int CIN, int COUT>
-cudaError_t conv_launch(const ConvArgs& a, cudaStream_t st) {
+cudaError_t conv_launch(const ConvArgs& a, int dev, cudaStream_t st) {
     using S = ConvShape<CIN, COUT>;
-    static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_conv3x3<CIN, COUT>, S::SMEM); });
-    if (allowed != cudaSuccess) return allowed;
+    static PerDevice<LaunchRoom> rooms;
+    const LaunchRoom room = rooms.of(dev, [](int d) {
+        return LaunchRoom{allow_smem(k_conv3x3<CIN, COUT>, S::SMEM), query_sm_count(d)};
+    });
+    if (room.allowed != cudaSuccess) return room.allowed;
     const int tiles = a.n_img * ((a.H + TILE_H - 1) / TILE_H) * ((a.W + TILE_W - 1) / TILE_W);
-    const int grid = std::min(tiles, S::CTAS * sm_count());
+    const int grid = std::min(tiles, S::CTAS * room.sms);
     ::silt::launch_dep(k_conv3x3<CIN, COUT>, dim3(grid), dim3(THREADS), S::SMEM, st, a);
     ::silt::count_launch();
     return cudaGetLastError();
 }
 
 template <int CIN, int COUT>
-cudaError_t wgrad_launch(const WgradArgs& a, cudaStream_t st) {
+cudaError_t wgrad_launch(const WgradArgs& a, int dev, cudaStream_t st) {
     using S = WgradShape<CIN, COUT>;
-    static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_conv3x3_wgrad<CIN, COUT>, S::SMEM); });
-    if (allowed != cudaSuccess) return allowed;
+    static PerDevice<LaunchRoom> rooms;
+    const LaunchRoom room = rooms.of(dev, [](int d) {
+        return LaunchRoom{allow_smem(k_conv3x3_wgrad<CIN, COUT>, S::SMEM), query_sm_count(d)};
+    });
+    if (room.allowed != cudaSuccess) return room.allowed;
     const int tiles = a.n_img * ((a.H + TILE_H - 1) / TILE_H) * ((a.W + TILE_W - 1) / TILE_W);
-    const int grid = std::min(tiles, 2 * sm_count());  // two CTAs an SM by shared memory
+    const int grid = std::min(tiles, 2 * room.sms);  // two CTAs an SM by shared memory
     ::silt::launch_dep(k_conv3x3_wgrad<CIN, COUT>, dim3(grid), dim3(WG_THREADS), S::SMEM, st, a);
     ::silt::count_launch();
     return cudaGetLastError();
 }
 
-// The current device's error word (nullptr when there is no memory for it).
-int* err_slot() {
+// The error word of device `dev`, which is current (nullptr when there is no
+// memory for it: asked again by the next call).
+int* err_slot(int dev) {
+    constexpr int KEPT = 64;
+    static std::atomic<int*> words[KEPT];
     static std::mutex m;
-    static std::map<int, int*> words;
-    int dev = 0;
-    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= KEPT) return nullptr;
+    int* d = words[dev].load(std::memory_order_acquire);
+    if (d) return d;
     std::lock_guard<std::mutex> lock(m);
-    int*& d = words[dev];
-    if (!d && cudaMalloc(&d, sizeof(int)) == cudaSuccess) cudaMemset(d, 0, sizeof(int));
+    d = words[dev].load(std::memory_order_relaxed);
+    if (!d && cudaMalloc(&d, sizeof(int)) == cudaSuccess) {
+        cudaMemset(d, 0, sizeof(int));
+        words[dev].store(d, std::memory_order_release);
+    }
     return d;
 }
 
@@ -653,27 +665,29 @@ int* err_slot() {
 
 cudaError_t conv3x3(const uint16_t* x, const uint16_t* w, const float* bias, const uint16_t* gate, uint16_t* y,
                     float* y32, int n_img, int h, int wd, int cin, int cout, int relu, cudaStream_t st) {
-    ConvArgs a{x, w, bias, gate, y, y32, n_img, h, wd, relu, ((uintptr_t)gate & 15u) == 0, err_slot()};
+    const int dev = current_device();
+    ConvArgs a{x, w, bias, gate, y, y32, n_img, h, wd, relu, ((uintptr_t)gate & 15u) == 0, err_slot(dev)};
     if (n_img <= 0 || h <= 0 || wd <= 0) return cudaSuccess;
-    if (cin == 16 && cout == 32) return conv_launch<16, 32>(a, st);
-    if (cin == 32 && cout == 32) return conv_launch<32, 32>(a, st);
-    if (cin == 32 && cout == 16) return conv_launch<32, 16>(a, st);
-    if (cin == 16 && cout == 16) return conv_launch<16, 16>(a, st);
+    if (cin == 16 && cout == 32) return conv_launch<16, 32>(a, dev, st);
+    if (cin == 32 && cout == 32) return conv_launch<32, 32>(a, dev, st);
+    if (cin == 32 && cout == 16) return conv_launch<32, 16>(a, dev, st);
+    if (cin == 16 && cout == 16) return conv_launch<16, 16>(a, dev, st);
     return cudaErrorInvalidValue;
 }
 
 cudaError_t conv3x3_wgrad(const uint16_t* x, const uint16_t* dy, float* dw, float* db, int n_img, int h, int wd,
                           int cin, int cout, cudaStream_t st) {
-    WgradArgs a{x, dy, dw, db, n_img, h, wd, ((uintptr_t)dw & 15u) == 0, err_slot()};
+    const int dev = current_device();
+    WgradArgs a{x, dy, dw, db, n_img, h, wd, ((uintptr_t)dw & 15u) == 0, err_slot(dev)};
     if (n_img <= 0 || h <= 0 || wd <= 0) return cudaSuccess;
-    if (cin == 16 && cout == 32) return wgrad_launch<16, 32>(a, st);
-    if (cin == 32 && cout == 32) return wgrad_launch<32, 32>(a, st);
-    if (cin == 32 && cout == 16) return wgrad_launch<32, 16>(a, st);
+    if (cin == 16 && cout == 32) return wgrad_launch<16, 32>(a, dev, st);
+    if (cin == 32 && cout == 32) return wgrad_launch<32, 32>(a, dev, st);
+    if (cin == 32 && cout == 16) return wgrad_launch<32, 16>(a, dev, st);
     return cudaErrorInvalidValue;
 }
 
 int device_error(cudaStream_t st, int* flag) {
-    int* d = err_slot();
+    int* d = err_slot(current_device());
     if (!d) return 0;
     if (cudaMemcpyAsync(flag, d, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return -1;
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;
@@ -762,7 +776,7 @@ int silt_closure_adam(float* param, float* m, float* v, const float* grad, int32
 
 int silt_closure_wait_status(int32_t* gave_up, void* stream) {
     if (!gave_up) return fail(SILT_EINVAL, "invalid argument: closure_wait_status");
-    int* d = err_slot();
+    int* d = err_slot(silt::current_device());
     if (!d) return fail(SILT_ECUDA, "closure_wait_status: no error slot");
     int flag = 0;
     const cudaStream_t st = (cudaStream_t)stream;
@@ -775,7 +789,7 @@ int silt_closure_wait_status(int32_t* gave_up, void* stream) {
 
 int silt_closure_wait_probe(int32_t polls, void* stream) {
     if (polls < 1 || polls > (1 << 20)) return fail(SILT_EINVAL, "invalid argument: closure_wait_probe polls");
-    int* d = err_slot();
+    int* d = err_slot(silt::current_device());
     if (!d) return fail(SILT_ECUDA, "closure_wait_probe: no error slot");
     ::silt::launch_dep(k_wait_probe, dim3(1), dim3(32), 0, (cudaStream_t)stream, d, (int)polls);
     ::silt::count_launch();

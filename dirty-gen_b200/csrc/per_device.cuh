@@ -9,6 +9,12 @@
 
 namespace silt {
 
+inline int current_device() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+
 template <class T>
 class PerDevice {
     static constexpr int KEPT = 64;  // device ordinals with a value of their own; beyond, it is made on each call
@@ -16,10 +22,8 @@ class PerDevice {
     T value_[KEPT] = {};
 
   public:
-    // The current device's value: make(device), called on the first use there.
-    T of(T (*make)(int)) {
-        int dev = 0;
-        cudaGetDevice(&dev);
+    // The value of device `dev`, which is current: make(dev), called on the first use there.
+    T of(int dev, T (*make)(int)) {
         if (dev < 0 || dev >= KEPT) return make(dev);
         std::call_once(once_[dev], [this, dev, make] { value_[dev] = make(dev); });
         return value_[dev];

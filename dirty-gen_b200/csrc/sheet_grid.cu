@@ -1688,15 +1688,16 @@ cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* l
                                const int* count, SweepState* sweep, bool snapshot, cudaStream_t st, int ctas_per_sm) {
     if (sweep) {
         static PerDevice<int> grids, sms;
-        const int grid = grids.of([](int dev) { return coop_grid(k_batch_force_sweep, dev); });
-        const int nsm = sms.of(query_sm_count);
+        const int dev = current_device();
+        const int grid = grids.of(dev, [](int d) { return coop_grid(k_batch_force_sweep, d); });
+        const int nsm = sms.of(dev, query_sm_count);
         // Fewer CTAs than the device holds stay co-resident: the launch is still cooperative.
         const int g = ctas_per_sm > 0 ? std::min(grid, ctas_per_sm * nsm) : grid;
         const cudaError_t e = launch_coop(k_batch_force_sweep, g, st, d_ws, nwin, list, entry_win, count, sweep);
         if (e != cudaSuccess || !snapshot) return e != cudaSuccess ? e : cudaGetLastError();
     }
     static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_batch_force, Snap::BYTES); });
+    const cudaError_t allowed = attr.of(current_device(), [](int) { return allow_smem(k_batch_force, Snap::BYTES); });
     if (allowed != cudaSuccess) return allowed;
     ::silt::launch_dep(k_batch_force, dim3(148 * 2), dim3(FORCE_THREADS), Snap::BYTES, st, d_ws, list, entry_win, count);
     ::silt::count_launch();
@@ -1706,7 +1707,7 @@ cudaError_t launch_batch_force(const WindowSubstep* d_ws, int nwin, const int* l
 cudaError_t launch_batch_transport(const WindowSubstep* d_ws, const int* list, const int* entry_win,
                                    const int* count, cudaStream_t st, int blocks) {
     static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_batch_transport, transport_smem_bytes()); });
+    const cudaError_t allowed = attr.of(current_device(), [](int) { return allow_smem(k_batch_transport, transport_smem_bytes()); });
     if (allowed != cudaSuccess) return allowed;
     const unsigned grid = blocks > 0 ? (unsigned)blocks : 148u * 4u;
     ::silt::launch_dep(k_batch_transport, dim3(grid), dim3(TRANSPORT_THREADS), transport_smem_bytes(), st, d_ws, list, entry_win, count);
@@ -1718,14 +1719,14 @@ cudaError_t launch_force(const ForceLaunch& L, int res, int layers, cudaStream_t
     if (L.lay[0].sweep || L.lay[1].sweep) {
         if (!L.tf.sweep) return cudaErrorInvalidValue;
         static PerDevice<int> grids;
-        const int grid = grids.of([](int dev) { return coop_grid(k_force_sweep, dev); });
+        const int grid = grids.of(current_device(), [](int d) { return coop_grid(k_force_sweep, d); });
         const cudaError_t e = launch_coop(k_force_sweep, grid, st, L);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
     (void)layers;
     static_assert(FarSnap::BYTES == Snap::BYTES, "one tile layout");
     static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) {
+    const cudaError_t allowed = attr.of(current_device(), [](int) {
         const cudaError_t e = allow_smem(k_force, Snap::BYTES);
         return e != cudaSuccess ? e : allow_smem(k_force_far, Snap::BYTES);
     });
@@ -1792,7 +1793,7 @@ bool transport_map(const float* plane, int res, CUtensorMap* out) {
 
 cudaError_t launch_transport(const TransportLaunch& L, int res, int layers, cudaStream_t st) {
     static PerDevice<cudaError_t> attr;
-    const cudaError_t allowed = attr.of([](int) { return allow_smem(k_transport, transport_smem_bytes()); });
+    const cudaError_t allowed = attr.of(current_device(), [](int) { return allow_smem(k_transport, transport_smem_bytes()); });
     if (allowed != cudaSuccess) return allowed;
     (void)layers;
     // Interior tiles of a grid a multiple of 4 cells wide arrive by TMA.

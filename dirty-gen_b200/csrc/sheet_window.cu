@@ -1909,7 +1909,7 @@ static int crew_limit_query(int) {
 // small enough that all the jobs' CTAs fit on the GPU about twice over.
 static int crew_of(int njobs, int max_res) {
     static PerDevice<int> limits;
-    const int limit = limits.of(crew_limit_query);
+    const int limit = limits.of(current_device(), crew_limit_query);
     return limit <= 0 ? 0 : std::max(1, std::min({crew_for(max_res), limit, 296 / std::max(njobs, 1)}));
 }
 
