@@ -998,10 +998,12 @@ __device__ __forceinline__ int tile_entry(const TileFlags& tf, int cur, int nxt,
 }
 
 __global__ void k_tile_list(TileFlags tf, int cur, int nxt, int all, int skip0, int skip1, SubstepCount sc,
-                            int* count_next, double* zero_ledger, unsigned int* zero_bits) {
+                            int* count_next, double* zero_ledger, unsigned int* zero_bits, const double* sum,
+                            double wet) {
     ::silt::dep_wait();
     const int nt = tf.tiles_x * tf.tiles_x;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (sum && !(*sum > wet)) return;
     if (k == 0) {
         if (count_next) *count_next = 0;
         if (zero_ledger) zero_ledger[0] = zero_ledger[1] = 0.0;
@@ -1017,14 +1019,14 @@ __global__ void k_tile_list(TileFlags tf, int cur, int nxt, int all, int skip0, 
 
 cudaError_t launch_tile_list(const TileFlags& tf, int cur, int nxt, int all, int skip0, int skip1,
                              const SubstepCount& sc, int* count_next, double* zero_ledger, unsigned int* zero_bits,
-                             cudaStream_t st) {
+                             cudaStream_t st, const double* sum, double wet) {
     if (!count_next) {
         cudaError_t e = cudaMemsetAsync(tf.count, 0, sizeof(int), st);
         if (e != cudaSuccess) return e;
     }
     const int n = 2 * tf.tiles_x * tf.tiles_x;
     ::silt::launch_dep(k_tile_list, dim3((n + 255) / 256), dim3(256), 0, st, tf, cur, nxt, all, skip0, skip1, sc, count_next, zero_ledger,
-                                                 zero_bits);
+                                                 zero_bits, sum, wet);
     ::silt::count_launch();
     return cudaGetLastError();
 }

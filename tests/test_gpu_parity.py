@@ -454,3 +454,40 @@ def test_work_boxes_of_awkward_wet_shapes_match_oracle(pattern, res):
     for name in ("water", "uw", "vw"):
         a, b = ref.get(name), dev.get(name)
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), (name, float(np.abs(a - b).max()))
+
+
+@pytest.mark.parametrize("res,level", [(513, 0.0), (700, 1.0e-12)])
+def test_a_dry_call_above_512_steps_no_tile(res, level):
+    """A call that finds nothing wet leaves the caller's planes and the
+    scratch planes, which only a substep writes, as they are; water on the
+    same arrays afterwards steps as on fresh ones."""
+    import torch
+
+    def arrays():
+        h = torch.full((res, res), level, device="cuda")
+        u = torch.full((res, res), 0.3, device="cuda")
+        v = torch.full((res, res), -0.2, device="cuda")
+        bed = torch.zeros((res, res), device="cuda")
+        nu = torch.full((res, res), 0.9, device="cuda")
+        scratch = torch.zeros(G.lib().silt_step_sheet_scratch_bytes(res) // 4 + 16, device="cuda")
+        return h, u, v, bed, nu, scratch
+
+    def step(a):
+        rc = G.lib().silt_step_sheet(*(x.data_ptr() for x in a[:5]), None, res, 0.2, 1.0 / 120.0, 0.08,
+                                     a[5].data_ptr(), None)
+        torch.cuda.synchronize()
+        return rc
+
+    a, b = arrays(), arrays()
+    planes = a[5][64:64 + 3 * res * res]  # u, v and h of a substep, behind 256 bytes
+    planes.fill_(7.0)
+    for _ in range(3):
+        assert step(a) == G.SILT_OK_NOOP
+    for x, y in zip(a[:5], b[:5]):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32))
+    assert bool((planes == 7.0).all())
+    for q in (a, b):
+        q[0][40:300, 100:333] = 0.05
+        assert step(q) == 0
+    for x, y in zip(a[:3], b[:3]):
+        assert torch.equal(x.view(torch.int32), y.view(torch.int32))
